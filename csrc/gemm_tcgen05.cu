@@ -26,8 +26,12 @@
 // slice (kept in tensor memory) the matching blocks of all peers, read through distributed shared
 // memory with 16-byte loads, in a fixed order (deterministic).  No global scratch.
 //
-// Warp roles (192 threads): warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer,
-// warps 2..5 = epilogue (warp w reads TMEM lanes 32*(w%4) .. +31).
+// Warp roles: warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer, the others = epilogue (warp w reads TMEM lanes
+// 32*(w%4) .. +31).  One CTA per SM (the accumulators and the stages fill it), so the epilogue runs behind the main loop
+// and its arithmetic and tensor-memory loads are bound by the warps that issue them: from 64 tokens on eight warps share it, two per
+// lane quarter with alternate columns (or, in the pair form, a tile each).  Four against eight warps:
+// 12288 x 2048 with SwiGLU at 13600 tokens 604 and 553 us, at 256 tokens 21.3 and 20.4; 2048 x 6144 with a residual at 3072
+// tokens 76.7 and 69.8 (there also because the producer loads the pair form's residual tiles behind the last k block)
 #include <cuda.h>
 #include <stdio.h>
 
@@ -108,7 +112,10 @@ struct GemmCfg {
   static constexpr int TMEM_COLS = COLS < 32 ? 32 : COLS;     // power of two >= 32 (BN is a power of two)
   static constexpr int SMEM_BYTES = NS * STAGE_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
   static constexpr int CHUNK = BN >= 32 ? 32 : 16;
+  static constexpr int EPI_WARPS = BN >= 64 ? 8 : 4;
+  static constexpr int THREADS = 64 + 32 * EPI_WARPS;
 };
+__device__ __forceinline__ int epi_threads() { return blockDim.x - 64; }
 
 template <int CHUNK>
 __device__ __forceinline__ void tmem_ld_chunk(uint32_t taddr, float* v) {
@@ -144,13 +151,13 @@ __device__ __forceinline__ void stage_one(__nv_bfloat16* slot, float a, float u,
   *slot = __float2bfloat16_rn(y);
 }
 
-// Activation pass over a staged tile (n_tok x 128 bf16 in shared memory), run by the 128 epilogue threads after
+// Activation pass over a staged tile (n_tok x 128 bf16 in shared memory), run by the epilogue threads after
 // they have all staged their rows: GELU (erf form) of the bf16-rounded outputs.  Kept out of the staging loops,
 // whose unrolled bodies every GEMM executes.
 __device__ __noinline__ void gelu_tile(__nv_bfloat16* stg, int n_tok) {
   const int e = threadIdx.x - 64;
   __nv_bfloat162* v = reinterpret_cast<__nv_bfloat162*>(stg);
-  for (int i = e; i < n_tok * 64; i += 128) {
+  for (int i = e; i < n_tok * 64; i += epi_threads()) {
     const float2 f = __bfloat1622float2(v[i]);
     v[i] = __floats2bfloat162_rn(gelu_erf(f.x), gelu_erf(f.y));
   }
@@ -164,7 +171,7 @@ __device__ __noinline__ void xielu_tile(__nv_bfloat16* stg, int n_tok, float up,
     return fmaf(0.5f, z, z > 0.f ? up * z * z : neg);
   };
 #pragma unroll 4
-  for (int i = threadIdx.x - 64; i < n_tok * 64; i += 128) {
+  for (int i = threadIdx.x - 64; i < n_tok * 64; i += epi_threads()) {
     const float2 f = __bfloat1622float2(v[i]);
     v[i] = __floats2bfloat162_rn(act(f.x), act(f.y));
   }
@@ -173,12 +180,13 @@ __device__ __noinline__ void xielu_tile(__nv_bfloat16* stg, int n_tok, float up,
 // Interleaved-SwiGLU epilogue of one accumulator tile (S == 1 path): lanes 2i / 2i + 1 of the tile hold gate_i / up_i.
 // Per token pair the even lane sends its gate of the odd token and receives the up value of the even token (one
 // shuffle), so each lane evaluates one SiLU per two tokens; results go to a [BN tokens][64 features] staging tile.
+// Columns from c_first on, every c_step-th chunk.
 template <int BN, int CHUNK>
-__device__ __noinline__ void swiglu_interleaved_tile(uint32_t trow, __nv_bfloat16* stg, int row) {
+__device__ __noinline__ void swiglu_interleaved_tile(uint32_t trow, __nv_bfloat16* stg, int row, int c_first, int c_step) {
   const bool odd = row & 1;
   const int fo = row >> 1;
 #pragma unroll 1
-  for (int c0 = 0; c0 < BN; c0 += CHUNK) {
+  for (int c0 = c_first; c0 < BN; c0 += c_step) {
     float a[CHUNK];
     tmem_ld_chunk<CHUNK>(trow + c0, a);
     tmem_ld_wait();
@@ -193,13 +201,13 @@ __device__ __noinline__ void swiglu_interleaved_tile(uint32_t trow, __nv_bfloat1
 }
 
 // Copy `n_tok` staged rows ([token][128 features] bf16 in shared memory, tokens ta..ta+n_tok) into the
-// owners' slot buffers with 16-byte peer stores (128 epilogue threads: 16 lanes per 256-byte row),
+// owners' slot buffers with 16-byte peer stores (16 lanes of the epilogue threads per 256-byte row),
 // then fence and advance each touched owner's arrival counter by the rows it received.
 __device__ __noinline__ void push_rows(const GemmParams& p, const __nv_bfloat16* stg, int ta, int n_tok, int f0) {
-  const int e = threadIdx.x - 64;                 // 0..127
+  const int e = threadIdx.x - 64;
   const int sub = e & 15, r0 = e >> 4;            // 16-byte piece of the row, first row of this thread
   const int H = p.push_ld;
-  for (int r = r0; r < n_tok; r += 8) {
+  for (int r = r0; r < n_tok; r += epi_threads() / 16) {
     const int t = ta + r;
     if (t >= p.M) break;
     const int owner = t / p.push_rpr;
@@ -207,7 +215,7 @@ __device__ __noinline__ void push_rows(const GemmParams& p, const __nv_bfloat16*
     __nv_bfloat16* dst = p.push_slot[owner] + ((size_t)p.push_rank * p.push_rpr + (t - owner * p.push_rpr)) * H + f0 + sub * 8;
     *reinterpret_cast<uint4*>(dst) = v;
   }
-  named_bar_sync(1, 128);
+  named_bar_sync(1, epi_threads());
   if (e == 0 && ta < p.M) {
     __threadfence_system();
     const int tb = min(p.M, ta + n_tok);
@@ -219,9 +227,9 @@ __device__ __noinline__ void push_rows(const GemmParams& p, const __nv_bfloat16*
 }
 
 // QKV epilogue on a staged tile: `stg` holds [n_tok tokens][128 features] bf16 = head `f0 / 128` of tokens
-// ta .. ta + n_tok.  First the 128 epilogue threads bring the per-token inputs into shared memory `aux` with
+// ta .. ta + n_tok.  First the epilogue threads bring the per-token inputs into shared memory `aux` with
 // coalesced loads (the tokens' RoPE rows, cache slots and depth selectors: one global round trip instead of
-// one per token); then the four warps take the tokens round robin; a lane owns four consecutive dims of the
+// one per token); then the warps take the tokens round robin; a lane owns four consecutive dims of the
 // head, so the head's sum of squares is one warp reduction and the rotate-half partner (dim +- 64) sits in
 // lane +- 16.  Same arithmetic and rounding as qk_norm_rope_kv_kernel.  `aux` needs n_tok * 264 bytes.
 #ifndef TAHB_QKV_U
@@ -230,7 +238,7 @@ __device__ __noinline__ void push_rows(const GemmParams& p, const __nv_bfloat16*
 #endif
 __device__ __noinline__ void qkv_epilogue(const GemmParams& p, const __nv_bfloat16* stg, uint8_t* aux, int ta,
                                              int n_tok, int f0) {
-  const int e = threadIdx.x - 64;                 // 0..127
+  const int e = threadIdx.x - 64, n_thr = epi_threads(), n_warps = n_thr >> 5;
   const int w4 = e >> 5, lane = e & 31;
   const int h = f0 >> 7;
   const bool is_q = h < p.nq;
@@ -241,19 +249,19 @@ __device__ __noinline__ void qkv_epilogue(const GemmParams& p, const __nv_bfloat
   int* s_sel = s_slot + n_tok;
   if (table && (is_q || is_k)) {
     const uint4* src = reinterpret_cast<const uint4*>(p.rope_cs);
-    for (int i = e; i < n_tok * 16; i += 128) {
+    for (int i = e; i < n_tok * 16; i += n_thr) {
       const int t = ta + (i >> 4);
       if (t < p.M) s_cs[i] = src[(size_t)t * 16 + (i & 15)];
     }
   }
   if (!is_q) {
-    for (int i = e; i < n_tok; i += 128) {
+    for (int i = e; i < n_tok; i += n_thr) {
       const int t = ta + i;
       s_slot[i] = (p.slot != nullptr && t < p.M) ? p.slot[t] : -1;
       s_sel[i] = (p.cache_sel != nullptr && t < p.M) ? p.cache_sel[t] : 0;
     }
   }
-  named_bar_sync(1, 128);
+  named_bar_sync(1, n_thr);
   const __nv_bfloat16* nw = is_q ? p.q_norm_w : p.k_norm_w;
   // Packed bf16x2 arithmetic: a bf16 x bf16 product is exact in fp32, so __hmul2 rounds once exactly like the
   // scalar statement bf16(float(a) * float(b)); this more than halves the instruction count of the loop, which
@@ -278,13 +286,13 @@ __device__ __noinline__ void qkv_epilogue(const GemmParams& p, const __nv_bfloat
   // Four tokens per warp and step, written phase by phase: the latency of a token's dependent chain (reduction,
   // shuffles) is hidden by the other three tokens' chains.
   constexpr int U = TAHB_QKV_U;
-  for (int r0 = w4; r0 < n_tok; r0 += 4 * U) {
+  for (int r0 = w4; r0 < n_tok; r0 += n_warps * U) {
     int rr[U];
     bool live[U];
     uint2 raw[U], outv[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      rr[u] = r0 + 4 * u;
+      rr[u] = r0 + n_warps * u;
       live[u] = rr[u] < n_tok && ta + rr[u] < p.M;
       raw[u] = live[u] ? *reinterpret_cast<const uint2*>(stg + rr[u] * 128 + lane * 4) : make_uint2(0u, 0u);
       outv[u] = raw[u];
@@ -376,7 +384,7 @@ __host__ __device__ constexpr int split_stage_offset(int S, int cols_per_rank) {
 }
 
 template <int BN, bool DUAL, bool PAIR = false>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(GemmCfg<BN, DUAL>::THREADS, 1)
 gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                const __grid_constant__ CUtensorMap tm_w2, const __grid_constant__ CUtensorMap tm_x2,
                const __grid_constant__ CUtensorMap tm_out, const __grid_constant__ CUtensorMap tm_res,
@@ -466,6 +474,17 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           tma_load_2d(st + C::W_BYTES, mx, x, t0, &full_bar[s]);
         }
       }
+      if constexpr (PAIR) {
+        // the residual tiles take the first two stages as the main loop frees them
+        if (p.tma_out && p.residual != nullptr && !*abort_flag) {
+          mbar_expect_tx(res_bar, BN * 256 * 2);
+#pragma unroll
+          for (int s = 0; s < 2; ++s) {
+            if (n_kb > s) mbar_wait(&empty_bar[s], ((n_kb - 1 - s) / C::NS) & 1, abort_flag, p.status, STATUS_TIMEOUT_STAGE_EMPTY);
+            if (!*abort_flag) tma_load_2d(smem + s * C::STAGE_BYTES, &tm_res, s ? p.up_off + f0 : f0, t0, res_bar);
+          }
+        }
+      }
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -504,6 +523,9 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     const int q = warp & 3;
     const int row = q * 32 + lane;
     const int f = f0 + row;
+    const int half = (warp - 2) >> 2;               // of the two warps of a lane quarter (eight epilogue warps)
+    constexpr int STEP = C::CHUNK * (C::EPI_WARPS / 4);
+    const int c_first = half * C::CHUNK;
     const uint32_t trow = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     mbar_wait(accum_bar, 0, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
     tc_fence_after();
@@ -513,44 +535,35 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       if constexpr (PAIR) {
         // Two plain output tiles (features f0.. and up_off + f0..) that shared the CTA's activation tile: per unit
         // of work a CTA pulls half the activation bytes, which is what bounds the GEMM at large token counts.
-        __nv_bfloat16* stg1 = stg + BN * 128;
+        __nv_bfloat16* stg1 = reinterpret_cast<__nv_bfloat16*>(smem + C::STAGE_BYTES);
         const bool il = p.act == 2;
-        if (res_tma) {
-          if (threadIdx.x == 64) {
-            mbar_expect_tx(res_bar, BN * 256 * 2);
-            tma_load_2d(stg, &tm_res, f0, t0, res_bar);
-            tma_load_2d(stg1, &tm_res, p.up_off + f0, t0, res_bar);
-          }
-          mbar_wait(res_bar, 0, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
-        }
+        static_assert(!PAIR || (C::STAGE_BYTES >= BN * 256 && C::NS >= 2), "a staged tile fits a stage");
+        if (res_tma) mbar_wait(res_bar, 0, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
         if (il) {
-          swiglu_interleaved_tile<BN, C::CHUNK>(trow, stg, row);
-          swiglu_interleaved_tile<BN, C::CHUNK>(trow + BN, stg1, row);
+          swiglu_interleaved_tile<BN, C::CHUNK>(trow + half * BN, half ? stg1 : stg, row, 0, C::CHUNK);
         } else {
+          __nv_bfloat16* mine = half ? stg1 : stg;
 #pragma unroll 1
           for (int c0 = 0; c0 < BN; c0 += C::CHUNK) {
-            float a[C::CHUNK], u[C::CHUNK];
-            tmem_ld_chunk<C::CHUNK>(trow + c0, a);
-            tmem_ld_chunk<C::CHUNK>(trow + BN + c0, u);
+            float a[C::CHUNK];
+            tmem_ld_chunk<C::CHUNK>(trow + half * BN + c0, a);
             tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < C::CHUNK; ++j) {
-              stage_one<false>(stg + (c0 + j) * 128 + row, a[j], 0.f, res_tma);
-              stage_one<false>(stg1 + (c0 + j) * 128 + row, u[j], 0.f, res_tma);
-            }
+            for (int j = 0; j < C::CHUNK; ++j) stage_one<false>(mine + (c0 + j) * 128 + row, a[j], 0.f, res_tma);
           }
         }
         if (p.push_world > 0) {
-          named_bar_sync(1, 128);
+          named_bar_sync(1, C::EPI_WARPS * 32);
           push_rows(p, stg, t0, BN, f0);
           push_rows(p, stg1, t0, BN, p.up_off + f0);
         } else {
           if (p.act == 3) {
-            named_bar_sync(1, 128);
-            xielu_tile(stg, 2 * BN, p.act_up, p.act_low);
+            named_bar_sync(1, C::EPI_WARPS * 32);
+            xielu_tile(stg, BN, p.act_up, p.act_low);
+            xielu_tile(stg1, BN, p.act_up, p.act_low);
           }
           fence_proxy_async_smem();
-          named_bar_sync(1, 128);
+          named_bar_sync(1, C::EPI_WARPS * 32);
           if (threadIdx.x == 64) {
             tma_store_2d(&tm_out, stg, il ? f0 / 2 : f0, t0);
             tma_store_2d(&tm_out, stg1, il ? (p.up_off + f0) / 2 : p.up_off + f0, t0);
@@ -568,10 +581,10 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       }
       const bool swiglu_il = !DUAL && p.act == 2;
       if (swiglu_il) {
-        if constexpr (!DUAL) swiglu_interleaved_tile<BN, C::CHUNK>(trow, stg, row);
+        if constexpr (!DUAL) swiglu_interleaved_tile<BN, C::CHUNK>(trow, stg, row, c_first, STEP);
       }
 #pragma unroll 1
-      for (int c0 = swiglu_il ? BN : 0; c0 < BN; c0 += C::CHUNK) {
+      for (int c0 = swiglu_il ? BN : c_first; c0 < BN; c0 += STEP) {
         float a[C::CHUNK];
         float u[DUAL ? C::CHUNK : 1];
         tmem_ld_chunk<C::CHUNK>(trow + c0, a);
@@ -590,21 +603,21 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         }
       }
       if (p.qkv_on) {
-        named_bar_sync(1, 128);
+        named_bar_sync(1, C::EPI_WARPS * 32);
         qkv_epilogue(p, stg, smem + BN * 256, t0, BN, f0);        // aux behind the staged tile
       } else if (p.push_world > 0) {
-        named_bar_sync(1, 128);
+        named_bar_sync(1, C::EPI_WARPS * 32);
         push_rows(p, stg, t0, BN, f0);
       } else if (p.tma_out) {
         if (p.act == 1) {
-          named_bar_sync(1, 128);
+          named_bar_sync(1, C::EPI_WARPS * 32);
           gelu_tile(stg, BN);
         } else if (p.act == 3) {
-          named_bar_sync(1, 128);
+          named_bar_sync(1, C::EPI_WARPS * 32);
           xielu_tile(stg, BN, p.act_up, p.act_low);
         }
         fence_proxy_async_smem();
-        named_bar_sync(1, 128);
+        named_bar_sync(1, C::EPI_WARPS * 32);
         if (threadIdx.x == 64) {
           tma_store_2d(&tm_out, stg, swiglu_il ? f0 / 2 : f0, t0);
           tma_store_commit();
@@ -633,6 +646,7 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       const int rs = C::NACC * per + 4;
       const uint32_t trow = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
       const uint32_t red_addr = smem_u32(smem);
+      const int c_first = C::EPI_WARPS == 8 ? ((warp - 2) >> 2) * 16 : 0, c_step = C::EPI_WARPS * 4;
 #pragma unroll 1
       for (int d = 0; d < S; ++d) {
         if (d == rank) continue;
@@ -642,7 +656,7 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
 #pragma unroll 1
         for (int acc = 0; acc < C::NACC; ++acc) {
 #pragma unroll 1
-          for (int c = 0; c < per; c += 16) {
+          for (int c = c_first; c < per; c += c_step) {
             float a[16];
             tmem_ld16(trow + acc * BN + d * per + c, a);
             tmem_ld_wait();
@@ -673,8 +687,9 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         }
         mbar_wait(res_bar, 0, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
       }
+      const int c_first = C::EPI_WARPS == 8 ? ((warp - 2) >> 2) * 16 : 0, c_step = C::EPI_WARPS * 4;
 #pragma unroll 1
-      for (int c = 0; c < per; c += 16) {
+      for (int c = c_first; c < per; c += c_step) {
         float a[16];
         float u[DUAL ? 16 : 1];
         tmem_ld16(trow + rank * per + c, a);
@@ -702,21 +717,21 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         }
       }
       if (p.qkv_on) {
-        named_bar_sync(1, 128);
+        named_bar_sync(1, C::EPI_WARPS * 32);
         qkv_epilogue(p, stg, reinterpret_cast<uint8_t*>(stg) + per * 256, t0 + rank * per, per, f0);
       } else if (p.push_world > 0) {
-        named_bar_sync(1, 128);
+        named_bar_sync(1, C::EPI_WARPS * 32);
         push_rows(p, stg, t0 + rank * per, per, f0);
       } else if (p.tma_out) {
         if (p.act == 1) {
-          named_bar_sync(1, 128);
+          named_bar_sync(1, C::EPI_WARPS * 32);
           gelu_tile(stg, per);
         } else if (p.act == 3) {
-          named_bar_sync(1, 128);
+          named_bar_sync(1, C::EPI_WARPS * 32);
           xielu_tile(stg, per, p.act_up, p.act_low);
         }
         fence_proxy_async_smem();
-        named_bar_sync(1, 128);
+        named_bar_sync(1, C::EPI_WARPS * 32);
         if (threadIdx.x == 64) {
           tma_store_2d(&tm_out, stg, f0, t0 + rank * per);
           tma_store_commit();
@@ -808,7 +823,7 @@ static int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMa
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((p.F + 127) / 128, (p.M + BN - 1) / BN, p.splits);
-  cfg.blockDim = dim3(192, 1, 1);
+  cfg.blockDim = dim3(C::THREADS, 1, 1);
   cfg.dynamicSmemBytes = C::SMEM_BYTES;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
