@@ -109,7 +109,7 @@ struct GemmCfg {
   static constexpr int NS = NS_RAW > 8 ? 8 : NS_RAW;
   static constexpr int NACC = DUAL ? 2 : 1;
   static constexpr int COLS = BN * NACC;
-  static constexpr int TMEM_COLS = COLS < 32 ? 32 : COLS;     // power of two >= 32 (BN is a power of two)
+  static constexpr int TMEM_COLS = COLS <= 32 ? 32 : COLS <= 64 ? 64 : COLS <= 128 ? 128 : COLS <= 256 ? 256 : 512;
   static constexpr int SMEM_BYTES = NS * STAGE_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
   static constexpr int CHUNK = BN >= 32 ? 32 : 16;
   static constexpr int EPI_WARPS = BN >= 64 ? 8 : 4;
@@ -845,7 +845,7 @@ using namespace tahb;
 
 // out[M, F] = X[M, K] W[F, K]^T (+ X2[M, R] W2[F, R]^T) (+ residual) ; dual != 0 => SwiGLU over W rows
 // [0, F) (gate) and [up_off, up_off + F) (up).  All matrices bf16 row-major; K and R multiples of 64.
-// bn = token-tile width (16/32/64/128/256, 0 = choose from M); splits = split-K cluster size (1,2,4,8).
+// bn = token-tile width (16/32/64/128/192/256, 0 = choose from M); splits = split-K cluster size (1,2,4,8).
 // Returns 0 on success, a negative code on a host-side error.  *status (device int) is set non-zero
 // by the kernel if a bounded wait ran out.
 // Host-side description of the fused QKV epilogue (see GemmParams::qkv_on); all pointers are device memory.
@@ -902,7 +902,7 @@ static int gemm_impl(const void* W, const void* X, void* out, const void* residu
     dual = 2;
     F = F / 2;
     up_off = F;
-    bn = 256;
+    if (bn != 128 && bn != 192) bn = 256;
     splits = 1;
   }
   if (pair && b_mn && M % 64) return -24;
@@ -991,7 +991,10 @@ static int gemm_impl(const void* W, const void* X, void* out, const void* residu
 #define TAHB_LAUNCH(BN_)                                                              \
   case BN_:                                                                           \
     return dual ? launch<BN_, true>(mw, mx, mw2, mx2, mo, mr, p, stream) : launch<BN_, false>(mw, mx, mw2, mx2, mo, mr, p, stream);
+  if (pair && bn == 128) return launch<128, true, true>(mw, mx, mw2, mx2, mo, mr, p, stream);
+  if (pair && bn == 192) return launch<192, true, true>(mw, mx, mw2, mx2, mo, mr, p, stream);
   if (pair) return launch<256, true, true>(mw, mx, mw2, mx2, mo, mr, p, stream);
+  if (bn == 192 && !dual) return launch<192, false>(mw, mx, mw2, mx2, mo, mr, p, stream);
   switch (bn) {
     TAHB_LAUNCH(16)
     TAHB_LAUNCH(32)

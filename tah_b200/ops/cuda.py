@@ -10,6 +10,7 @@ word; :func:`check_status` reads it (a host sync) and raises :class:`KernelTimeo
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from typing import List, Optional, Sequence
 
@@ -150,9 +151,32 @@ def plan_gemm(M: int, F: int, K: int, R: int = 0, dual: bool = False):
     return best[1], best[2]
 
 
-# token count from which the two-tile ("pair") GEMM is the default; TAH_B200_GEMM_PAIR=0 turns it off
+# the two-tile ("pair") GEMM is a candidate above 256 tokens; TAH_B200_GEMM_PAIR=0 turns it off
 PAIR_AUTO = os.environ.get("TAH_B200_GEMM_PAIR", "1") != "0"
-PAIR_MIN_TOKENS = 1024
+
+
+@functools.lru_cache(maxsize=4096)
+def plan_tiles(M: int, rows: int, K: int, can_pair: bool, can_split: bool):
+    """``(pair, bn, splits)`` for more than 256 tokens: tiles of 128 or (pair) 256 features by 128, 192 or 256 tokens, whichever fills the
+    SMs' waves best by a cost model.
+
+    Microseconds, 256 tokens always (paired from 1024 on) and the chosen form: 1500 tokens 67.4 and 41.1 (2048 x 6144), 30.0 and 18.0
+    (2048 x 2048); 3072 tokens 31.7 and 26.6 (2048 x 2048), 70.1 and 63.3 (2048 x 6144); 700 tokens 17.9 and 16.4 (4096 x 2048), 14.9 and
+    13.5 (2048 x 2048).  Over nine token counts from 300 to 13600 the choice was within 10 % of the best of all forms."""
+    best = None
+    for nf in (1, 2) if can_pair else (1,):
+        for bn in (128, 192, 256):
+            for s in (1, 2, 4) if can_split and nf == 1 else (1,):
+                kb = -(-K // 64) / s
+                if s > 1 and (kb < 4 or not _fits(bn, s, 1)):
+                    continue
+                waves = -(-(-(-rows // (128 * nf)) * -(-M // bn) * s) // SM_COUNT)
+                # microseconds per block of 64: tensor cores, and bytes into the SM at 87 KB/us
+                t_kb = max(0.39 * nf * bn / 256, (128 * nf + bn) * 0.125 / 87)
+                t = waves * (kb * t_kb + 0.5 + 0.005 * nf * bn / s + (1.5 + (s - 1) * bn / s * 0.5 / 19.0 if s > 1 else 0.0)) + 1.5
+                if best is None or t < best[0] - 1e-9:
+                    best = (t, nf == 2, bn, s)
+    return best[1:]
 
 
 def interleave_gate_up(w: torch.Tensor) -> torch.Tensor:
@@ -199,6 +223,25 @@ def wait_flags(flags: torch.Tensor, targets: torch.Tensor) -> None:
         "tahb_wait_flags")
 
 
+def _plan_tiles(M: int, rows: int, K: int, R: int, swiglu: bool, gelu: bool, swiglu_interleaved: bool, pair=None, bn: int = 0, splits=None):
+    """``(pair, bn, splits)`` of a tcgen05 product with a weight of ``rows`` rows."""
+    can_pair = not swiglu and not gelu and rows % 256 == 0
+    if pair is None and bn == 0 and splits is None and M > 256 and not swiglu:
+        return plan_tiles(M, rows, K + R, can_pair and PAIR_AUTO, not swiglu_interleaved)
+    pair = bool(pair) and can_pair
+    if pair:
+        bn, splits = bn or 256, 1
+    elif swiglu_interleaved:
+        splits = 1                       # the interleaved epilogue exists for unsplit tiles
+        if bn == 0:
+            bn = 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128 if M <= 128 else 256
+    elif splits is None and bn == 0:
+        bn, splits = plan_gemm(M, rows // 2 if swiglu else rows, K, R, swiglu)
+    elif splits is None:
+        splits = 1
+    return pair, bn, splits
+
+
 def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None,
          residual: Optional[torch.Tensor] = None, x2: Optional[torch.Tensor] = None,
          w2: Optional[torch.Tensor] = None, swiglu: bool = False, splits: Optional[int] = None,
@@ -209,10 +252,10 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
 
     ``gelu``: the epilogue applies the erf GELU to the bf16-rounded output (not together with ``residual``).
 
-    ``pair``: every CTA computes two 128-feature output tiles (features ``f`` and ``F/2 + f``) from one 256-token
-    activation tile, unsplit.  It halves the activation bytes a CTA pulls per unit of work, which is what bounds
-    the kernel at large token counts (1350-1400 vs 915-1100 TFLOP/s at 8192+ tokens); default: on from
-    ``PAIR_MIN_TOKENS`` tokens when the shape allows it (also with ``swiglu_interleaved``).
+    ``pair``: every CTA computes two 128-feature output tiles (features ``f`` and ``F/2 + f``) from one activation tile
+    of 256 tokens (or ``bn`` 128, 192), unsplit.  It halves the activation bytes a CTA pulls per unit of work, which is what
+    bounds the kernel at large token counts (1350-1400 vs 915-1100 TFLOP/s at 8192+ tokens); default: by
+    :func:`plan_tiles` above 256 tokens (also with ``swiglu_interleaved``).
 
     ``swiglu_interleaved``: the rows of ``w`` (and ``w2``) alternate ``gate_i, up_i`` (see :func:`interleave_gate_up`)
     and ``out[M, F/2] = silu(gate) * up``: one accumulator and one wide MMA per k step, the faster SwiGLU form.
@@ -246,20 +289,7 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
         _check_bf16_2d(out, "out")
     if residual is not None:
         _check_bf16_2d(residual, "residual")
-    if pair is None:
-        pair = (PAIR_AUTO and M >= PAIR_MIN_TOKENS and bn == 0 and splits is None and not swiglu and not gelu
-                and w.shape[0] % 256 == 0)
-    pair = bool(pair) and not swiglu and not gelu and w.shape[0] % 256 == 0
-    if pair:
-        bn, splits = 256, 1
-    elif swiglu_interleaved:
-        splits = 1                       # the interleaved epilogue exists for unsplit tiles
-        if bn == 0:
-            bn = 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128 if M <= 128 else 256
-    elif splits is None and bn == 0:
-        bn, splits = plan_gemm(M, F, K, R, swiglu)
-    elif splits is None:
-        splits = 1
+    pair, bn, splits = _plan_tiles(M, w.shape[0], K, R, swiglu, gelu, swiglu_interleaved, pair, bn, splits)
     args = (_p(w), _p(x), _p(out), _p(residual), _p(w2), _p(x2), c_int(M), c_int(F), c_int(K), c_int(R),
             c_ll(w.stride(0)), c_ll(x.stride(0)), c_ll(out.stride(0)),
             c_ll(residual.stride(0) if residual is not None else 0),
@@ -313,11 +343,12 @@ def gemm_t(x: torch.Tensor, w: torch.Tensor, *, x_t: bool = False, w_t: bool = F
         out = torch.empty(M, F, dtype=torch.bfloat16, device=x.device)
     if residual is not None:
         _check_bf16_2d(residual, "residual")
-    if pair is None:
-        pair = PAIR_AUTO and M >= PAIR_MIN_TOKENS and bn == 0 and splits is None
-    pair = bool(pair) and F % 256 == 0 and (not x_t or M % 64 == 0)
+    can_pair = F % 256 == 0 and (not x_t or M % 64 == 0)
+    if pair is None and bn == 0 and splits is None and M > 256:
+        pair, bn, splits = plan_tiles(M, F, Kx, can_pair and PAIR_AUTO, True)
+    pair = bool(pair) and can_pair
     if pair:
-        bn, splits = 256, 1
+        bn, splits = bn or 256, 1
     elif splits is None and bn == 0:
         bn, splits = plan_gemm(M, F, (Kx + 63) // 64 * 64, 0, False)
         if x_t:
@@ -608,8 +639,7 @@ def xielu_linear(x: torch.Tensor, w: torch.Tensor, up: float, low: float, out: O
         out = torch.empty(M, F, dtype=torch.bfloat16, device=x.device)
     for n, t in (("x", x), ("w", w), ("out", out)):
         _check_bf16_2d(t, n)
-    pair = PAIR_AUTO and M >= PAIR_MIN_TOKENS and F % 256 == 0
-    bn, splits = (256, 1) if pair else plan_gemm(M, F, Kd)
+    pair, bn, splits = _plan_tiles(M, F, Kd, 0, False, False, False)
     _rc(lib().tahb_gemm_xielu(_p(w), _p(x), _p(out), c_int(M), c_int(F), c_int(Kd), c_ll(w.stride(0)), c_ll(x.stride(0)), c_ll(out.stride(0)),
                               c_float(up), c_float(low), c_int(int(pair)), c_int(splits), c_int(bn), _p(status_word(x.device)), _stream()),
         "tahb_gemm_xielu")

@@ -92,7 +92,7 @@ def bench_gemm(a):
     t = _time(fn, a.iters, a.warmup)
     flops = 2.0 * M * wrows * (Kd + R)
     byts = (wrows * (Kd + R) + M * (Kd + R) + M * F) * 2
-    auto_pair = K.PAIR_AUTO and M >= K.PAIR_MIN_TOKENS and not a.bn and wrows % 256 == 0 and not a.swiglu
+    auto_pair = M > 256 and not a.bn and not a.swiglu and K.plan_tiles(M, wrows, Kd + R, K.PAIR_AUTO and wrows % 256 == 0, not il)[0]
     res = {"op": "gemm", "M": M, "F": F, "K": Kd, "R": R, "swiglu": a.swiglu, "swiglu_interleaved": il,
            "transposed": a.transposed, "pair": bool(a.pair) if a.pair is not None else auto_pair,
            "plan_bn_splits": [a.bn, a.splits] if a.bn else K.plan_gemm(M, F, Kd, R, a.swiglu)}

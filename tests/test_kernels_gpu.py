@@ -894,3 +894,29 @@ def test_soft_embedding_mix_forward_backward_kernels():
     _close(out, ref, atol=3e-2, rtol=3e-2)
     _close(logits.grad, lf.grad, atol=3e-2, rtol=5e-2)
     _close(E.grad, Ef.grad, atol=3e-2, rtol=5e-2)
+
+
+@pytest.mark.parametrize("M,F,K", [(257, 512, 256), (385, 256, 2048), (1000, 2048, 192), (192, 512, 64)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_gemm_tile_forms_give_the_same_bits(M, F, K, residual):
+    """Every tile the planner chooses from above 256 tokens: unsplit ones add in the same order, split ones stay within one rounding of
+    the sum and one of the result."""
+    Kc = _cuda()
+    x, w = _rand(M, K, seed=1), _rand(F, K, scale=K ** -0.5, seed=2)
+    res = _rand(M, F, seed=3) if residual else None
+    base = Kc.gemm(x, w, residual=res, pair=False, bn=256, splits=1)
+    z = x.double() @ w.double().t()
+    ref = z + (0.0 if res is None else res.double())
+    tol = 2.0 ** -8 * 1.01 * (z.abs() + ref.abs()) + 2e-5
+    assert bool(((base.double() - ref).abs() <= tol).all())
+    for pair, bn in ((False, 128), (False, 192), (True, 128), (True, 192), (True, 256)):
+        assert torch.equal(Kc.gemm(x, w, residual=res, pair=pair, bn=bn, splits=1), base), (pair, bn)
+        if not residual:
+            assert torch.equal(Kc.gemm(x, w, swiglu_interleaved=True, pair=pair, bn=bn),
+                               Kc.gemm(x, w, swiglu_interleaved=True, pair=False, bn=256))
+            assert torch.equal(Kc.gemm_t(x, w.t().contiguous(), w_t=True, pair=pair, bn=bn, splits=1), base)
+    for bn, splits in ((192, 2), (192, 4), (256, 2)):
+        out = Kc.gemm(x, w, residual=res, pair=False, bn=bn, splits=splits)
+        assert bool(((out.double() - ref).abs() <= tol).all())
+    assert bool(((Kc.gemm(x, w, residual=res).double() - ref).abs() <= tol).all())
+    Kc.check_status()
