@@ -58,7 +58,6 @@ __device__ __forceinline__ void locate_page(int i, const int* seg_pages, int& c,
 
 template <int HD, int G>
 __global__ void __launch_bounds__(160, (HD * G <= 256) ? 4 : 2) decode_attn_kernel(const DecodeAttnParams p) {
-  pdl_launch_dependents();
   pdl_wait();
   using C = AttCfg<HD>;
   constexpr int VEC = HD / 64;       // 16-byte chunks per lane per row: lane gl owns chunks gl, gl + 8, ...
@@ -228,6 +227,7 @@ __global__ void __launch_bounds__(160, (HD * G <= 256) ? 4 : 2) decode_attn_kern
     }
   }
 
+  pdl_launch_dependents();
   // merge the 16 groups through shared memory (the pipeline buffers are free now)
   __syncthreads();
   float* sm_m = reinterpret_cast<float*>(att_smem);          // [16][G]

@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 namespace tahb {
 
 constexpr unsigned long long WAIT_TIMEOUT_NS = 2000000000ull;  // 2 s
@@ -34,6 +36,10 @@ enum Status : int {
 // tail of kernel N.  Every such kernel executes pdl_wait on every path, so completion of a kernel
 // implies completion of all kernels before it.  Both instructions are no-ops in a kernel launched
 // without the attribute.
+//
+// Kernels of a few microseconds release their successor late, when their loads have arrived and only arithmetic
+// and stores are left: released at its start, a chain of such kernels piles several waiting grids up on the SMs,
+// and a tick of one row (336 launches) took 2.06 ms instead of 1.50 ms; 20 rows 3.51 and 3.04 ms.
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -20,7 +20,6 @@ __global__ void __launch_bounds__(128) rmsnorm_kernel(const __nv_bfloat16* __res
                                                       const __nv_bfloat16* __restrict__ w,
                                                       __nv_bfloat16* __restrict__ y, int H, long long ldx,
                                                       long long ldy, float eps) {
-  pdl_launch_dependents();
   pdl_wait();
   const int row = blockIdx.x;
   const int nvec = H / 8;
@@ -44,6 +43,7 @@ __global__ void __launch_bounds__(128) rmsnorm_kernel(const __nv_bfloat16* __res
   ss = warp_sum(ss);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
   __syncthreads();
+  pdl_launch_dependents();
   const float tot = red[0] + red[1] + red[2] + red[3];
   const float rstd = rsqrtf(tot / (float)H + eps);
   const uint4* wr = reinterpret_cast<const uint4*>(w);
@@ -89,7 +89,6 @@ __global__ void __launch_bounds__(256) rmsnorm_lora_kernel(const __nv_bfloat16* 
                                                            long long ldy, float eps, const int* __restrict__ gate,
                                                            const __nv_bfloat16* __restrict__ A,
                                                            __nv_bfloat16* __restrict__ T, int R, long long ldt) {
-  pdl_launch_dependents();
   pdl_wait();
   extern __shared__ uint4 srow[];            // H / 8 vectors: the normalised row (LoRA CTAs only)
   __shared__ float red[8];
@@ -160,6 +159,7 @@ __global__ void __launch_bounds__(256) rmsnorm_lora_kernel(const __nv_bfloat16* 
     float tot = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) tot += red[k];   // fixed order: every CTA of a row gets the same rstd
+    pdl_launch_dependents();
     const float rstd = rsqrtf(tot / (float)H + eps);
     uint4* yr = reinterpret_cast<uint4*>(y + (size_t)row * ldy);
 #pragma unroll
@@ -493,7 +493,6 @@ __global__ void __launch_bounds__(256) lora_a_rows_kernel(const __nv_bfloat16* _
                                                           int M, int K, int R, long long ldx, long long ldt,
                                                           const uint32_t* wait_flag, const uint32_t* wait_target,
                                                           int wait_world, int* status, unsigned long long wait_limit) {
-  pdl_launch_dependents();
   pdl_wait();
   __shared__ int s_rows[1024];
   __shared__ int s_warp[8];
@@ -515,6 +514,7 @@ __global__ void __launch_bounds__(256) lora_a_rows_kernel(const __nv_bfloat16* _
     if (lane >= o) incl += y;
   }
   if (lane == 31) s_warp[warp] = incl;
+  pdl_launch_dependents();
   __syncthreads();
   int base = 0;
   for (int w = 0; w < warp; ++w) base += s_warp[w];

@@ -1,0 +1,244 @@
+// Matrix product for a handful of tokens: out[t, f] = sum_k X[t, k] W[f, k] (+ sum_r X2[t, r] W2[f, r]) (+ residual),
+// with the epilogues of gemm_tcgen05.cu (plain, residual, GELU, interleaved SwiGLU, xIELU), for M <= 32, and for narrow weights at
+// token counts whose 32-token tiles (the grid's second dimension) still fit one wave.
+//
+// What bounds it: the weight is read once (2 F K bytes) and used M times, so this is a stream of HBM at 2 M FLOP per
+// weight; and it runs in a chain of small launches, so the time from the predecessor's end to the last store counts as
+// much as the bandwidth.  A 128-feature tensor-memory tile leaves most SMs without work at the layer sizes (F = 2048
+// gives 16 tiles, 64 CTAs with a cluster split), and pays for tensor-map fetch, tensor-memory allocation, a cluster
+// barrier pair and a staged TMA store in every launch.  Here a CTA owns 16 or 32 features, its warps split the
+// reduction, weights go from global memory straight into the registers that warp-level tensor instructions read,
+// and the warps' partial sums meet once in shared memory.
+//
+// Fragment layout: mma.m16n8k16 wants for lane (g = lane / 4, t = lane % 4) the reduction indices {2t, 2t+1, 2t+8, 2t+9} of
+// rows g and g + 8.  The order of the reduction is free as long as both operands agree, so a lane reads 16 consecutive
+// bytes (8 indices) of a row at 8 t and feeds two instructions with them: 64 contiguous bytes per row and step, no
+// shared memory, no shuffles.
+#include <cuda.h>
+
+#include "common.cuh"
+
+namespace tahb {
+
+struct FewParams {
+  const __nv_bfloat16 *W, *X, *W2, *X2, *residual;
+  __nv_bfloat16* out;
+  int M, F, K, R;
+  long long ldw, ldx, ldw2, ldx2, ldo, ldr;
+  int act;               // 0 none, 1 GELU, 2 SwiGLU of interleaved rows, 3 xIELU
+  int stacked;           // SwiGLU of a weight with all gate rows in front of the up rows: how many gate rows; 0: interleaved
+  float act_up, act_low;
+  int early;             // the weights are constants of the launch chain: read them ahead of the dependency wait
+};
+
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint4 ld_stream(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
+template <int NT, int MT>
+struct FewCfg {
+  static constexpr int ST = 4 / MT;                        // steps of 32 reduction indices per buffer, two buffers: 64 registers
+  static constexpr int PITCH = 16 * MT + 4;                // floats per token in the reduction area: no bank conflicts
+  static constexpr int red_bytes(int warps) { return warps * 8 * NT * PITCH * 4; }
+};
+
+template <int NT, int MT, int NW>
+__global__ void __launch_bounds__(NW * 32)
+gemm_few_kernel(const FewParams p) {
+  using C = FewCfg<NT, MT>;
+  constexpr int ST = C::ST, FT = 16 * MT;
+  extern __shared__ float red[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int f0 = blockIdx.x * FT;
+  const int tok0 = blockIdx.y * 8 * NT, M = min(p.M - tok0, 8 * NT);          // this CTA's tokens
+  const int steps = p.K >> 5, s0 = steps * warp / NW, s1 = steps * (warp + 1) / NW;
+
+  auto row_of = [&](int m, int h) {            // weight row of this lane's feature
+    const int v = min(f0 + 16 * m + 8 * h + g, p.F - 1);
+    return (size_t)(p.stacked ? (v >> 1) + (v & 1) * p.stacked : v);
+  };
+  const __nv_bfloat16* wr[MT][2];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) wr[m][h] = p.W + row_of(m, h) * p.ldw + t * 8;
+
+  uint4 w[2][ST][MT][2];
+  auto fetch = [&](uint4 (&b)[ST][MT][2], int s) {
+#pragma unroll
+    for (int i = 0; i < ST; ++i)
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          b[i][m][h] = s + i < s1 ? ld_stream(wr[m][h] + (size_t)(s + i) * 32) : make_uint4(0u, 0u, 0u, 0u);
+  };
+  if (!p.early) pdl_wait();
+  fetch(w[0], s0);
+  fetch(w[1], s0 + ST);
+  if (p.early) pdl_wait();
+
+  float acc[MT][NT][4];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[m][j][c] = 0.f;
+
+  const __nv_bfloat16* xr[NT];
+#pragma unroll
+  for (int j = 0; j < NT; ++j) xr[j] = p.X + (size_t)(tok0 + min(8 * j + g, M - 1)) * p.ldx + t * 8;
+
+  auto multiply = [&](const uint4 (&b)[MT][2], const uint4 (&x)[NT]) {
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        mma_16816(acc[m][j], b[m][0].x, b[m][1].x, b[m][0].y, b[m][1].y, x[j].x, x[j].y);
+        mma_16816(acc[m][j], b[m][0].z, b[m][1].z, b[m][0].w, b[m][1].w, x[j].z, x[j].w);
+      }
+  };
+  auto consume = [&](uint4 (&b)[ST][MT][2], int s) {
+    uint4 x[ST][NT];
+#pragma unroll
+    for (int i = 0; i < ST; ++i)
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+        x[i][j] = s + i < s1 ? *reinterpret_cast<const uint4*>(xr[j] + (size_t)(s + i) * 32) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int i = 0; i < ST; ++i) multiply(b[i], x[i]);
+  };
+  for (int s = s0; s < s1; s += 2 * ST) {
+    consume(w[0], s);
+    if (s + 2 * ST < s1) fetch(w[0], s + 2 * ST);
+    if (s + ST < s1) {
+      consume(w[1], s + ST);
+      if (s + 3 * ST < s1) fetch(w[1], s + 3 * ST);
+    }
+  }
+  // the K-extension: R / 32 more steps, one warp each in turn
+  for (int s = warp; s < (p.R >> 5); s += NW) {
+    uint4 b[MT][2], x[NT];
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        b[m][h] = ld_stream(p.W2 + row_of(m, h) * p.ldw2 + t * 8 + s * 32);
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+      x[j] = *reinterpret_cast<const uint4*>(p.X2 + (size_t)(tok0 + min(8 * j + g, M - 1)) * p.ldx2 + t * 8 + s * 32);
+    multiply(b, x);
+  }
+
+  pdl_launch_dependents();
+
+  // the warps' sums meet: [warp][token][feature]
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        red[(warp * 8 * NT + 8 * j + 2 * t + (c & 1)) * C::PITCH + 16 * m + g + 8 * (c >> 1)] = acc[m][j][c];
+  __syncthreads();
+  auto total = [&](int tok, int f) {
+    float v = 0.f;
+#pragma unroll
+    for (int k = 0; k < NW; ++k) v += red[(k * 8 * NT + tok) * C::PITCH + f];
+    return v;
+  };
+  if (p.act == 2) {
+    for (int o = threadIdx.x; o < M * (FT / 2); o += NW * 32) {
+      const int tok = o / (FT / 2), f = o % (FT / 2);
+      if (f0 + 2 * f >= p.F) continue;
+      const float gate = bf16_round(total(tok, 2 * f)), up = bf16_round(total(tok, 2 * f + 1));
+      p.out[(size_t)(tok0 + tok) * p.ldo + f0 / 2 + f] = __float2bfloat16_rn(bf16_round(silu(gate)) * up);
+    }
+    return;
+  }
+  for (int o = threadIdx.x; o < M * FT; o += NW * 32) {
+    const int tok = o / FT, f = f0 + o % FT;
+    if (f >= p.F) continue;
+    float v = total(tok, o % FT);
+    if (p.residual != nullptr) v = bf16_round(v) + __bfloat162float(p.residual[(size_t)(tok0 + tok) * p.ldr + f]);
+    if (p.act == 1) {
+      const float z = bf16_round(v);
+      v = 0.5f * z * (1.0f + erff(z * 0.70710678118654752f));
+    } else if (p.act == 3) {
+      const float z = bf16_round(v);
+      v = fmaf(0.5f, z, z > 0.f ? p.act_up * z * z : p.act_low * (ex2_approx(z * 1.4426950408889634f) - 1.0f - z));
+    }
+    p.out[(size_t)(tok0 + tok) * p.ldo + f] = __float2bfloat16_rn(v);
+  }
+}
+
+template <int NT, int MT, int NW>
+static int launch_few(const FewParams& p, cudaStream_t stream) {
+  constexpr int bytes = FewCfg<NT, MT>::red_bytes(NW);
+  auto kern = gemm_few_kernel<NT, MT, NW>;
+  if constexpr (bytes > 48 * 1024) {
+    static const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+    if (!ok) return -10;
+  }
+  return launch_chain(kern, dim3((p.F + 16 * MT - 1) / (16 * MT), (p.M + 8 * NT - 1) / (8 * NT)), dim3(NW * 32), bytes, stream, p) == cudaSuccess ? 0 : -12;
+}
+
+}  // namespace tahb
+
+using namespace tahb;
+
+// Same operands as tahb_gemm (act as its `dual`: 0 plain, 1 SwiGLU of stacked rows, 3 GELU, 4 interleaved SwiGLU; 5 xIELU with act_up /
+// act_low); F counts weight rows.  K and R multiples of 32, W / X / W2 / X2 on 16-byte boundaries with row pitches that are
+// multiples of 8 elements.
+//
+// The split, measured with weights out of HBM (us, M = 1 / 12 / 32; in brackets the tcgen05 form it takes the place of):
+//   F x K          2048 x 2048          4096 x 2048          2048 x 6144           12288 x 2048 SwiGLU     151936 x 2048
+//   1 tile, 16 w   2.8 / 3.2 / 4.1      5.6 / 6.2 / 8.2      5.9 / 6.4 / 8.6       16 / 18 / 24            144 / 167 / 230
+//   1 tile, 8 w    3.4 / 3.5 / 4.8      4.4 / 4.7 / 6.2      8.8 / 9.3 / 13.9      12.5 / 13.4 / 18.0      92 / 124 / 174
+//   2 tiles, 16 w  2.4 / 3.5 / 5.2      4.0 / 4.9 / 6.5      6.8 / 9.1 / 13.5      11.1 / 14.1 / 18.8      99 / 133 / 189
+//   2 tiles, 4 w   6.9 / 7.9 / 9.8      7.6 / 8.9 / 12.0     19 / 22 / 27          9.7 / 11.4 / 13.1       90 / 98 / 131
+//   (tcgen05)      13.1 / 13.3 / 9.4    13.7 / 13.8 / 9.9    33.5 / 33.5 / 19.7    14.2 / 14.2 / 15.0      120 / 122 / 125
+// Tiles of 16 features: about 16 warps per SM keep enough bytes in flight, more only add partial sums.  With four times as many
+// tiles as SMs, four warps a CTA and two tiles are the streaming form (activations read once per 32 features).  Up to 8 tokens a
+// reduction of 2048 lies in the two register buffers of 16 warps x 2 tiles: every weight byte is requested before the first wait.
+extern "C" int tahb_gemm_few(const void* W, const void* X, void* out, const void* residual, const void* W2, const void* X2, int M, int F,
+                             int K, int R, long long ldw, long long ldx, long long ldo, long long ldr, long long ldw2, long long ldx2,
+                             int act, float act_up, float act_low, int early, cudaStream_t stream) {
+  if (M <= 0 || F <= 0) return 0;
+  if (K <= 0 || K % 32 || R % 32 || ((act == 1 || act == 4) && (F % 2 || residual != nullptr))) return -20;
+  auto odd = [](const void* p, long long ld) { return (reinterpret_cast<uintptr_t>(p) & 15) || (ld & 7); };
+  if (odd(W, ldw) || odd(X, ldx) || (R > 0 && (odd(W2, ldw2) || odd(X2, ldx2)))) return -2;
+  FewParams p;
+  p.W = reinterpret_cast<const __nv_bfloat16*>(W);
+  p.X = reinterpret_cast<const __nv_bfloat16*>(X);
+  p.W2 = reinterpret_cast<const __nv_bfloat16*>(W2);
+  p.X2 = reinterpret_cast<const __nv_bfloat16*>(X2);
+  p.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
+  p.out = reinterpret_cast<__nv_bfloat16*>(out);
+  p.M = M; p.F = F; p.K = K; p.R = R;
+  p.ldw = ldw; p.ldx = ldx; p.ldw2 = ldw2; p.ldx2 = ldx2; p.ldo = ldo; p.ldr = ldr;
+  p.act = act == 3 ? 1 : (act == 1 || act == 4) ? 2 : act == 5 ? 3 : 0;
+  p.stacked = act == 1 ? F / 2 : 0;
+  p.act_up = act_up; p.act_low = act_low;
+  p.early = early;
+  const int tiles = (F + 15) / 16;
+#define TAHB_FEW(NT_)                                                                         \
+  {                                                                                           \
+    if (tiles >= 4 * 148) return launch_few<NT_, 2, 4>(p, stream);                             \
+    if (NT_ == 1 && K <= 2048) return launch_few<1, 2, 16>(p, stream);                         \
+    if (tiles <= 148 || K >= 4096) return launch_few<NT_, 1, 16>(p, stream);                   \
+    return launch_few<NT_, 1, 8>(p, stream);                                                  \
+  }
+  if (M <= 8) TAHB_FEW(1)
+  if (M <= 16) TAHB_FEW(2)
+  TAHB_FEW(4)
+#undef TAHB_FEW
+}

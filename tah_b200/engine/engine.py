@@ -485,7 +485,7 @@ class TaHEngine(DecodeEngine):
                 K.gemm(x, a_, out=t_buf)
         kw = dict(x2=t_buf, w2=b_) if lora else {}
         if tp is None:
-            K.gemm(x, w_, residual=h, out=h, **kw)
+            K.gemm(x, w_, residual=h, out=h, const_w=True, **kw)
             if next_lora is not None:
                 # the norm kernel also forms t = gate * xn A^T for the projection that consumes xn
                 return K.rms_norm_lora(h, ln_w, cfg.rms_norm_eps, gate, next_lora[0], out=xn_out, t_out=next_lora[1])[0]
@@ -549,7 +549,7 @@ class TaHEngine(DecodeEngine):
                            caches=pools[li], cache_sel=s.depth, slot=s.slot, page_size=self.page_size,
                            tp_wait=self._xn_wait, rope_cs=s.rope_cs, **kw)
             else:
-                K.gemm(xn, L.w_qkv, out=s.qkv, tp_wait=self._xn_wait, **kw)
+                K.gemm(xn, L.w_qkv, out=s.qkv, tp_wait=self._xn_wait, const_w=True, **kw)
                 K.qk_norm_rope_kv(s.qkv, L.q_norm, L.k_norm, s.pos, nq, nkv, hd, cfg.rms_norm_eps, cfg.rope_theta,
                                   q_out=s.q, caches=pools[li], cache_sel=s.depth, slot=s.slot, page_size=self.page_size)
             K.decode_attn(s.q, pools[li], kv.page_table, kv.len, s.depth, nq, nkv, hd, self.page_size, scale, out=s.o,
@@ -558,7 +558,7 @@ class TaHEngine(DecodeEngine):
                                     push=push, next_lora=(L.a_gu, s.t_gu) if fuse_norm_lora else None)
             if lora and not fuse_norm_lora:
                 K.lora_a_rows(xn, L.a_gu, s.gate, out=s.t_gu, tp_wait=self._xn_wait)
-            sw = dict(swiglu_interleaved=True) if w.gu_interleaved else dict(swiglu=True)
+            sw = dict(swiglu_interleaved=True, const_w=True) if w.gu_interleaved else dict(swiglu=True, const_w=True)
             if lora:
                 K.gemm(xn, L.w_gu, x2=s.t_gu, w2=L.b_gu, out=s.act, tp_wait=self._xn_wait, **sw)
             else:
@@ -573,7 +573,7 @@ class TaHEngine(DecodeEngine):
         if cfg.num_hidden_layers in tl:
             j = tl.index(cfg.num_hidden_layers)
             s.taps[:, j * H:(j + 1) * H].copy_(xn)
-        K.gemm(xn, w.lm_head, out=s.logits)
+        K.gemm(xn, w.lm_head, out=s.logits, const_w=True)
         lo, hi, _ = w.vocab_shard
         logits, cum = s.logits[:, :hi - lo], s.cum[:, :hi - lo]
         K.logits_post(logits, cum, s.depth, s.best, s.best_val)

@@ -397,7 +397,7 @@ class HybridEngine(DecodeEngine):
             y_ex, slot, weight = self._mixture(f, proj, b)
             if weight is not None:
                 raise NotImplementedError("weighted expert outputs beside a mixer")
-        K.linear(self._attention(li, L.mixer, proj, b, plan), L.mixer.w_o, out=b.y)
+        K.linear(self._attention(li, L.mixer, proj, b, plan), L.mixer.w_o, out=b.y, const_w=True)
         K.residual_add_norm(b.y, b.x, self.cfg.residual_mult, w_next, self.w.W, self.cfg.norm_groups, self.cfg.rms_norm_eps,
                             b.h, y_ex, slot)
 
@@ -413,11 +413,11 @@ class HybridEngine(DecodeEngine):
             L, follow = w.layers[r.layer], w.runs[ri + 1] if ri + 1 < len(w.runs) else None
             after = w.final_norm if follow is None else w.layers[follow.layer].norm1
             b.before = None if self.layer_hook is None or follow is None or follow.add is None else torch.empty_like(b.x)
-            proj = K.linear(b.h, L.mixer.w_in, out=b.proj[:, :L.mixer.w_in.shape[0]])
+            proj = K.linear(b.h, L.mixer.w_in, out=b.proj[:, :L.mixer.w_in.shape[0]], const_w=True)
             if L.parallel:
                 self._parallel_layer(ri, L, proj, after, b, plan)
             else:
-                K.linear(run[type(L.mixer)](ri, L.mixer, proj, b, plan), L.mixer.w_o, out=b.y)
+                K.linear(run[type(L.mixer)](ri, L.mixer, proj, b, plan), L.mixer.w_o, out=b.y, const_w=True)
                 if w.streams is not None:
                     K.streams_norm(b.y, b.x, L.hc1, after if L.norm2 is None else L.norm2, w.W, self.cfg.norm_groups, self.cfg.rms_norm_eps,
                                    b.h, y_bias=getattr(L.mixer, "o_bias", None))
@@ -448,10 +448,10 @@ class HybridEngine(DecodeEngine):
         if isinstance(L.ff, MixtureLayer):
             y, (ex["y_ex"], ex["slot"], ex["y_weight"]) = None, self._mixture(L.ff, None, b)
         elif isinstance(L.ff, XIELULayer):
-            K.linear(K.xielu_linear(b.h, L.w_up, L.ff.up, L.ff.low, out=b.act[:, :L.w_down.shape[1]]), L.w_down, out=y)
+            K.linear(K.xielu_linear(b.h, L.w_up, L.ff.up, L.ff.low, out=b.act[:, :L.w_down.shape[1]]), L.w_down, out=y, const_w=True)
         else:
-            act = K.swiglu_linear(b.h, L.w_gu, out=b.act[:, :L.w_down.shape[1]])
-            K.linear(act, L.w_down, out=y)
+            act = K.swiglu_linear(b.h, L.w_gu, out=b.act[:, :L.w_down.shape[1]], const_w=True)
+            K.linear(act, L.w_down, out=y, const_w=True)
         if w.streams is None:
             self._seam(y, L.out2, w_next, follow, b, plan)
         else:
@@ -678,7 +678,7 @@ class HybridEngine(DecodeEngine):
         w = self.w
         s.binding.tick_begin(None, None, None)
         self._embed(s.buf, s.plan)
-        K.linear(self._layers(s.buf, s.plan), w.head, out=s.logits)
+        K.linear(self._layers(s.buf, s.plan), w.head, out=s.logits, const_w=True)
         V = w.vocab
         K.logits_post(s.logits[:, :V], s.cum[:, :V], None, s.best, s.best_val)
         if sampling is not None and self.dtype != torch.bfloat16:

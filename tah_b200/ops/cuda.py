@@ -246,7 +246,7 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
          residual: Optional[torch.Tensor] = None, x2: Optional[torch.Tensor] = None,
          w2: Optional[torch.Tensor] = None, swiglu: bool = False, splits: Optional[int] = None,
          bn: int = 0, tp_push=None, tp_wait=None, gelu: bool = False, swiglu_interleaved: bool = False,
-         pair: Optional[bool] = None) -> torch.Tensor:
+         pair: Optional[bool] = None, const_w: bool = False) -> torch.Tensor:
     """``out[M,F] = x[M,K] @ w[F,K]^T (+ x2[M,R] @ w2[F,R]^T) (+ residual)``; with ``swiglu`` the
     weight is ``[2F, K]`` (gate rows then up rows) and ``out = silu(gate) * up``.
 
@@ -259,6 +259,9 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
 
     ``swiglu_interleaved``: the rows of ``w`` (and ``w2``) alternate ``gate_i, up_i`` (see :func:`interleave_gate_up`)
     and ``out[M, F/2] = silu(gate) * up``: one accumulator and one wide MMA per k step, the faster SwiGLU form.
+
+    ``const_w``: ``w`` and ``w2`` are weights that no kernel of this library writes; for few tokens they are then read while the
+    kernel before this one still runs.
 
     Tensor parallel (see :class:`tah_b200.parallel.tp.TensorParallel`): ``tp_push =
     (slot_ptrs, cnt_ptrs, rank, rows_per_rank)`` replaces the output by peer stores of the tile
@@ -289,6 +292,10 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
         _check_bf16_2d(out, "out")
     if residual is not None:
         _check_bf16_2d(residual, "residual")
+    if (not pair and bn == 0 and splits in (None, 1) and tp_push is None and tp_wait is None and
+            not ((swiglu or gelu) and (residual is not None or swiglu and gelu)) and _few_ok(x, w, x2, w2) and
+            (not (gelu or swiglu_interleaved) or _whole_pieces(out))):
+        return _gemm_few(x, w, out, residual, x2, w2, 1 if swiglu else 3 if gelu else 4 if swiglu_interleaved else 0, early=const_w)
     pair, bn, splits = _plan_tiles(M, w.shape[0], K, R, swiglu, gelu, swiglu_interleaved, pair, bn, splits)
     args = (_p(w), _p(x), _p(out), _p(residual), _p(w2), _p(x2), c_int(M), c_int(F), c_int(K), c_int(R),
             c_ll(w.stride(0)), c_ll(x.stride(0)), c_ll(out.stride(0)),
@@ -312,6 +319,36 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
             wait = (None, None, c_int(0))
         rc = lib().tahb_gemm_tp(*args, *push, *wait)
     _rc(rc, "tahb_gemm")
+    return out
+
+
+# Token count up to which the product is a stream of the weight (csrc/gemm_few.cu).  From 17 tokens on, a weight with more than 16384 rows
+# stays on the tensor-memory form: it has tiles for every SM and reads the activations once per 128 features (151936 x 2048 at 32
+# tokens: 125 us there, 131 us here; 12288 x 2048: 15.0 and 13.1 us).
+FEW_TOKENS, FEW_WIDE_TOKENS, FEW_WIDE_ROWS = 32, 16, 16384
+
+
+def _whole_pieces(t: torch.Tensor) -> bool:
+    return t.data_ptr() % 16 == 0 and t.stride(0) % 8 == 0
+
+
+def few_shape(M: int, rows: int, K: int, R: int = 0) -> bool:
+    """Whether a product of ``M`` tokens with a weight of ``rows`` rows takes the few-token form."""
+    few = M <= (FEW_WIDE_TOKENS if rows > FEW_WIDE_ROWS else FEW_TOKENS)
+    return few and M > 0 and K > 0 and K % 64 == 0 and R % 64 == 0
+
+
+def _few_ok(x, w, x2=None, w2=None) -> bool:
+    return (few_shape(x.shape[0], w.shape[0], x.shape[1], 0 if x2 is None else x2.shape[1]) and
+            all(t is None or _whole_pieces(t) for t in (x, w, x2, w2)))
+
+
+def _gemm_few(x, w, out, residual=None, x2=None, w2=None, act: int = 0, act_up: float = 0.0, act_low: float = 0.0, early: bool = False):
+    """``act``: 0 none, 1 SwiGLU of stacked rows, 3 GELU, 4 SwiGLU of interleaved rows, 5 xIELU."""
+    ld = lambda t: c_ll(0 if t is None else t.stride(0))
+    _rc(lib().tahb_gemm_few(_p(w), _p(x), _p(out), _p(residual), _p(w2), _p(x2), c_int(x.shape[0]), c_int(w.shape[0]), c_int(x.shape[1]),
+                            c_int(0 if x2 is None else x2.shape[1]), ld(w), ld(x), ld(out), ld(residual), ld(w2), ld(x2), c_int(act),
+                            c_float(act_up), c_float(act_low), c_int(1 if early else 0), _stream()), "tahb_gemm_few")
     return out
 
 
@@ -596,10 +633,10 @@ def _act_f32(*ts: torch.Tensor) -> int:
     return 1 if dt == torch.float32 else 0
 
 
-def linear(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+def linear(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, const_w: bool = False) -> torch.Tensor:
     """``out[M, F] = x[M, K] @ w[F, K]^T``: the tensor-core GEMM for bf16, the fp32 FMA kernel for fp32 operands."""
     if not _act_f32(x, w):
-        return gemm(x, w, out=out)
+        return gemm(x, w, out=out, const_w=const_w)
     if x.dim() != 2 or w.dim() != 2 or x.shape[1] != w.shape[1] or x.stride(1) != 1 or w.stride(1) != 1:
         raise ValueError(f"linear: x {tuple(x.shape)} w {tuple(w.shape)}")
     M, Kd = x.shape
@@ -610,11 +647,11 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None)
     return out
 
 
-def swiglu_linear(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+def swiglu_linear(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, const_w: bool = False) -> torch.Tensor:
     """``silu(gate) * up`` of ``x @ w^T``: bf16 weights have interleaved gate / up rows (:func:`interleave_gate_up`, the
     fused GEMM epilogue), fp32 weights the stacked ``[gate; up]`` rows (product, then an activation kernel)."""
     if not _act_f32(x, w):
-        return gemm(x, w, out=out, swiglu_interleaved=True)
+        return gemm(x, w, out=out, swiglu_interleaved=True, const_w=const_w)
     gu = linear(x, w)
     M, inter = gu.shape[0], gu.shape[1] // 2
     if out is None:
@@ -639,6 +676,8 @@ def xielu_linear(x: torch.Tensor, w: torch.Tensor, up: float, low: float, out: O
         out = torch.empty(M, F, dtype=torch.bfloat16, device=x.device)
     for n, t in (("x", x), ("w", w), ("out", out)):
         _check_bf16_2d(t, n)
+    if _few_ok(x, w) and _whole_pieces(out):
+        return _gemm_few(x, w, out, act=5, act_up=up, act_low=low)
     pair, bn, splits = _plan_tiles(M, F, Kd, 0, False, False, False)
     _rc(lib().tahb_gemm_xielu(_p(w), _p(x), _p(out), c_int(M), c_int(F), c_int(Kd), c_ll(w.stride(0)), c_ll(x.stride(0)), c_ll(out.stride(0)),
                               c_float(up), c_float(low), c_int(int(pair)), c_int(splits), c_int(bn), _p(status_word(x.device)), _stream()),
@@ -1284,13 +1323,16 @@ def varlen_attn_naive(q, ks, vs, bases, counts, nq, nkv, hd, scale, out=None):
 def attn_tiles(seq_counts: torch.Tensor, tile: int = 128):
     """Query tiles for :func:`prefill_attn`: every sequence's packed tokens (``seq_counts[b]`` of
     them, sequences laid out back to back) are cut into runs of at most ``tile`` tokens.  Returns
-    int32 ``(tile_q0, tile_qn)``."""
+    int32 ``(tile_q0, tile_qn)``, every sequence's first tiles first: the kernels start at the end, where the work is."""
     cnt = seq_counts.to(torch.int64)
     per = (cnt + tile - 1) // tile
     n_tiles = int(per.sum())
     dev = cnt.device
     seq_of = torch.repeat_interleave(torch.arange(cnt.numel(), device=dev), per, output_size=n_tiles)
     rank = torch.arange(n_tiles, device=dev) - (torch.cumsum(per, 0) - per)[seq_of]
+    if cnt.numel() > 1:
+        rank, order = torch.sort(rank, stable=True)
+        seq_of = seq_of[order]
     q0 = (torch.cumsum(cnt, 0) - cnt)[seq_of] + tile * rank
     qn = torch.clamp(cnt[seq_of] - tile * rank, max=tile)
     return q0.to(torch.int32).contiguous(), qn.to(torch.int32).contiguous()
@@ -1330,6 +1372,9 @@ def attn_kv_items(seq_kv_counts: torch.Tensor, seq_kv_base: torch.Tensor, seq_q_
     dev = cnt.device
     seq_of = torch.repeat_interleave(torch.arange(cnt.numel(), device=dev), per, output_size=n)
     rank = torch.arange(n, device=dev) - (torch.cumsum(per, 0) - per)[seq_of]
+    if cnt.numel() > 1:                      # the blocks that the most queries see first
+        rank, order = torch.sort(rank, stable=True)
+        seq_of = seq_of[order]
     kidx0 = block * rank
     row0 = seq_kv_base.to(torch.int64)[seq_of] + kidx0
     nkeys = torch.clamp(cnt[seq_of] - kidx0, max=block)

@@ -106,6 +106,50 @@ def test_gemm_swiglu_interleaved(M, I, K, R):
     assert torch.equal(out, dual)
 
 
+@pytest.mark.parametrize("M", [1, 8, 9, 17, 32, 33])
+@pytest.mark.parametrize("F,K,R", [(2048, 2048, 64), (40, 64, 0), (4096, 6144, 64), (9488, 128, 128), (16400, 192, 0)])
+@pytest.mark.parametrize("act", ["plain", "residual", "gelu", "swiglu", "xielu"])
+def test_gemm_few_tokens(M, F, K, R, act):
+    """The product for a handful of tokens at the edges of its token tiles, with rows, reduction steps and extension that do not divide
+    among its warps.  Bound: one bf16 rounding of the sum (half a unit of
+    8 significant bits: 2^-8 of it at most), one of the result, 32-bit sums far below; the epilogue functions have slopes below 1.2
+    (SwiGLU: times the other factor)."""
+    Kc = _cuda()
+    x, w = _rand(M, K, seed=1), _rand(F, K, scale=K ** -0.5, seed=2)
+    x2, w2 = (_rand(M, R, seed=3), _rand(F, R, scale=0.05, seed=4)) if R and act != "xielu" else (None, None)
+    z = x.double() @ w.double().t() + (x2.double() @ w2.double().t() if x2 is not None else 0.0)
+    eps = 2.0 ** -8
+    if act == "swiglu" and F == 40:
+        pytest.skip("an activation needs whole 16-byte pieces of output columns")
+    if act == "swiglu":
+        out = Kc.gemm(x, w, x2=x2, w2=w2, swiglu_interleaved=True)
+        g, u = z[:, 0::2], z[:, 1::2]
+        ref = torch.nn.functional.silu(g) * u
+        tol = 1.2 * eps * g.abs() * u.abs() + 2 * eps * ref.abs() + eps * ref.abs()
+    elif act == "gelu":
+        out, ref, tol = Kc.gemm(x, w, x2=x2, w2=w2, gelu=True), torch.nn.functional.gelu(z), 1.2 * eps * z.abs()
+    elif act == "xielu":
+        out = Kc.xielu_linear(x, w, 0.8, 1.1)
+        ref = torch.where(z > 0, 0.8 * z * z, 1.1 * (torch.expm1(z) - z)) + 0.5 * z
+        tol = eps * z.abs() * (1.6 * z.abs() + 0.5)
+    else:
+        res = _rand(M, F, seed=5) if act == "residual" else None
+        out, ref, tol = Kc.gemm(x, w, x2=x2, w2=w2, residual=res), z + (0.0 if res is None else res.double()), eps * z.abs()
+    Kc.check_status()
+    assert out.shape == ref.shape
+    assert bool(((out.double() - ref).abs() <= 1.01 * (tol + eps * ref.abs()) + 2e-5).all())
+
+
+def test_gemm_few_tokens_keeps_tokens_apart():
+    """An infinite or undefined token stays in its own output row, whatever part of the reduction it sits in."""
+    Kc = _cuda()
+    x, w = _rand(5, 2048, seed=1), _rand(64, 2048, scale=0.02, seed=2)
+    clean = Kc.gemm(x, w)
+    x[1, 2047], x[3, 0] = float("inf"), float("nan")
+    out = Kc.gemm(x, w)
+    assert torch.equal(out[[0, 2, 4]], clean[[0, 2, 4]]) and bool(out[3].isnan().all()) and bool(out[1].isinf().all())
+
+
 @pytest.mark.parametrize("M,F,K,R", [(256, 4096, 2048, 64), (1000, 512, 256, 0), (2048, 2048, 1024, 64), (77, 256, 128, 0)])
 @pytest.mark.parametrize("residual", [False, True])
 def test_gemm_pair_mode(M, F, K, R, residual):
