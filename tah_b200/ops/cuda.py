@@ -326,6 +326,9 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
 # stays on the tensor-memory form: it has tiles for every SM and reads the activations once per 128 features (151936 x 2048 at 32
 # tokens: 125 us there, 131 us here; 12288 x 2048: 15.0 and 13.1 us).
 FEW_TOKENS, FEW_WIDE_TOKENS, FEW_WIDE_ROWS = 32, 16, 16384
+# A narrow weight (an adapter's) has too few tensor-memory tiles to occupy the SMs at any token count: while tiles of 16 rows by 32 tokens
+# fit one wave, the few-token form is the faster one (64 x 2048 at 820 tokens 4.5 us, there 7.2; 192 x 2048 at 260 tokens 3.2 and 6.7; one
+# wave further 8.2 and 7.5, 7.7 and 7.3).
 
 
 def _whole_pieces(t: torch.Tensor) -> bool:
@@ -334,7 +337,7 @@ def _whole_pieces(t: torch.Tensor) -> bool:
 
 def few_shape(M: int, rows: int, K: int, R: int = 0) -> bool:
     """Whether a product of ``M`` tokens with a weight of ``rows`` rows takes the few-token form."""
-    few = M <= (FEW_WIDE_TOKENS if rows > FEW_WIDE_ROWS else FEW_TOKENS)
+    few = M <= (FEW_WIDE_TOKENS if rows > FEW_WIDE_ROWS else FEW_TOKENS) or -(-rows // 16) * -(-M // 32) <= SM_COUNT
     return few and M > 0 and K > 0 and K % 64 == 0 and R % 64 == 0
 
 
