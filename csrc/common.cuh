@@ -344,6 +344,25 @@ __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(_
 // main loop).  Relative error ~2^-21, far below the bf16 rounding that follows every use.
 __device__ __forceinline__ float silu(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
 
+// EPL consecutive bf16 of a lane, moved in one access when they lie on a boundary of their size (WIDE), else one by one.
+template <int EPL, bool WIDE>
+struct alignas(EPL * 2) QkvPiece {
+  __nv_bfloat16 v[EPL];
+  using Word = typename std::conditional<EPL == 4, uint2, uint32_t>::type;
+  __device__ __forceinline__ void load(const __nv_bfloat16* src) {
+    if constexpr (WIDE) *reinterpret_cast<Word*>(v) = *reinterpret_cast<const Word*>(src);
+    else
+#pragma unroll
+      for (int i = 0; i < EPL; ++i) v[i] = src[i];
+  }
+  __device__ __forceinline__ void store(__nv_bfloat16* dst) const {
+    if constexpr (WIDE) *reinterpret_cast<Word*>(dst) = *reinterpret_cast<const Word*>(v);
+    else
+#pragma unroll
+      for (int i = 0; i < EPL; ++i) dst[i] = v[i];
+  }
+};
+
 struct __align__(16) bf16x8 {
   __nv_bfloat162 v[4];
 };

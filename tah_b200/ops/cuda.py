@@ -1326,16 +1326,13 @@ def varlen_attn_naive(q, ks, vs, bases, counts, nq, nkv, hd, scale, out=None):
 def attn_tiles(seq_counts: torch.Tensor, tile: int = 128):
     """Query tiles for :func:`prefill_attn`: every sequence's packed tokens (``seq_counts[b]`` of
     them, sequences laid out back to back) are cut into runs of at most ``tile`` tokens.  Returns
-    int32 ``(tile_q0, tile_qn)``, every sequence's first tiles first: the kernels start at the end, where the work is."""
+    int32 ``(tile_q0, tile_qn)``."""
     cnt = seq_counts.to(torch.int64)
     per = (cnt + tile - 1) // tile
     n_tiles = int(per.sum())
     dev = cnt.device
     seq_of = torch.repeat_interleave(torch.arange(cnt.numel(), device=dev), per, output_size=n_tiles)
     rank = torch.arange(n_tiles, device=dev) - (torch.cumsum(per, 0) - per)[seq_of]
-    if cnt.numel() > 1:
-        rank, order = torch.sort(rank, stable=True)
-        seq_of = seq_of[order]
     q0 = (torch.cumsum(cnt, 0) - cnt)[seq_of] + tile * rank
     qn = torch.clamp(cnt[seq_of] - tile * rank, max=tile)
     return q0.to(torch.int32).contiguous(), qn.to(torch.int32).contiguous()
@@ -1375,9 +1372,6 @@ def attn_kv_items(seq_kv_counts: torch.Tensor, seq_kv_base: torch.Tensor, seq_q_
     dev = cnt.device
     seq_of = torch.repeat_interleave(torch.arange(cnt.numel(), device=dev), per, output_size=n)
     rank = torch.arange(n, device=dev) - (torch.cumsum(per, 0) - per)[seq_of]
-    if cnt.numel() > 1:                      # the blocks that the most queries see first
-        rank, order = torch.sort(rank, stable=True)
-        seq_of = seq_of[order]
     kidx0 = block * rank
     row0 = seq_kv_base.to(torch.int64)[seq_of] + kidx0
     nkeys = torch.clamp(cnt[seq_of] - kidx0, max=block)

@@ -940,6 +940,39 @@ def test_soft_embedding_mix_forward_backward_kernels():
     _close(E.grad, Ef.grad, atol=3e-2, rtol=5e-2)
 
 
+@pytest.mark.parametrize("hd,nq,nkv", [(128, 16, 8), (64, 4, 1), (128, 2, 2)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_qk_norm_rope_tokens_and_boundaries(hd, nq, nkv, shift):
+    """More heads than a pass of the warps takes and fewer, and rows that lie off the boundaries of wide accesses: the same bits either
+    way, forward and backward."""
+    Kc = _cuda()
+    M, F = 5, (nq + 2 * nkv) * hd
+    wide = _rand(M, F, seed=1)
+    flat = torch.empty(M * F + 8, dtype=torch.bfloat16, device="cuda")
+    qkv = flat[shift:shift + M * F].view(M, F)
+    qkv.copy_(wide)
+    qw, kw = _rand(hd, seed=2), _rand(hd, seed=3)
+    pos = torch.tensor([0, 1, 77, 4095, 39999], device="cuda", dtype=torch.int32)
+    gq, gk, gv = _rand(M, nq * hd, seed=4), _rand(M, nkv * hd, seed=5), _rand(M, nkv * hd, seed=6)
+    out = []
+    for x in (wide, qkv):
+        k, v = (torch.empty(M, nkv * hd, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        q = Kc.qk_norm_rope_kv(x, qw, kw, pos, nq, nkv, hd, 1e-6, 1e6, k_dense=k, v_dense=v)
+        gx, gwq, gwk = Kc.qk_norm_rope_bwd(x, qw, kw, gq, gk, gv, pos, nq, nkv, hd, 1e-6, 1e6)
+        out.append((q, k, v, gx))
+        xf, wq, wk = x.float().requires_grad_(True), qw.float().requires_grad_(True), kw.float().requires_grad_(True)
+        from tah_b200.models.qwen3 import apply_rope, rope_cos_sin
+        cos, sin = rope_cos_sin(pos[None].long(), hd, 1e6, torch.bfloat16)
+        parts = xf.split([nq * hd, nkv * hd, nkv * hd], -1)
+        norm = lambda t, w: w * t * torch.rsqrt(t.pow(2).mean(-1, keepdim=True) + 1e-6)
+        rot = lambda t, w, n: apply_rope(norm(t.view(1, M, n, hd), w), cos.float(), sin.float()).view(M, -1)
+        (rot(parts[0], wq, nq) * gq.float()).sum().add((rot(parts[1], wk, nkv) * gk.float()).sum()).add((parts[2] * gv.float()).sum()).backward()
+        _close(gx, xf.grad, atol=3e-2, rtol=2e-2)
+        _close(gwq, wq.grad, atol=2e-2 * nq ** 0.5, rtol=2e-2)
+        _close(gwk, wk.grad, atol=2e-2 * nkv ** 0.5, rtol=2e-2)
+    assert all(torch.equal(a, b) for a, b in zip(*out))
+
+
 @pytest.mark.parametrize("M,F,K", [(257, 512, 256), (385, 256, 2048), (1000, 2048, 192), (192, 512, 64)])
 @pytest.mark.parametrize("residual", [False, True])
 def test_gemm_tile_forms_give_the_same_bits(M, F, K, residual):
