@@ -7,11 +7,12 @@ namespace tahb {
 // ---------------------------------------------------------------------------------------------
 // RMSNorm backward.  y = w * (x * rstd),  rstd = rsqrt(mean(x^2) + eps).  With gn = gy * w:
 //     gx = rstd * (gn - xn * mean(gn * xn)),   gw = sum_rows gy * xn,   xn = x * rstd.
-// A CTA of 256 threads walks RMSB_ROWS consecutive rows; thread t owns columns 8t..8t+7 (+ 2048 k),
-// keeps its slice of gw in registers over those rows and adds it to the fp32 gw buffer once at the
-// end, so the atomics per launch are rows / RMSB_ROWS * H.
+// A CTA of 256 threads walks rows blockIdx, + gridDim, ...; thread t owns columns 8t..8t+7 (+ 2048 k), keeps its slice of gw in
+// registers over those rows and adds it to the fp32 gw buffer once at the end.  Bound: HBM (2048 columns, 3072 rows: 38 MB, 6 us); a
+// row is a chain of load, block reduction and store, so the next row is on its way while one is reduced, and two CTAs per SM share
+// the rows evenly.  32 rows in turn per CTA without that: 39 us at 3072 rows (96 CTAs), now 12.3 us.
 // ---------------------------------------------------------------------------------------------
-constexpr int RMSB_ROWS = 32;
+constexpr int RMSB_GRID = 296;
 
 template <int VPT>
 __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x,
@@ -35,9 +36,19 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const __nv_bfloat16* _
       for (int j = 0; j < 4; ++j) { const float2 f = __bfloat1622float2(h2[j]); wv[i][2 * j] = f.x; wv[i][2 * j + 1] = f.y; }
     }
   }
-  const int row_lo = blockIdx.x * RMSB_ROWS;
-  const int row_hi = min(M, row_lo + RMSB_ROWS);
-  for (int row = row_lo; row < row_hi; ++row) {
+  uint4 nx[VPT], ng[VPT];
+  auto fetch = [&](int row) {
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int idx = tid + i * 256;
+      if (idx < nvec) {
+        nx[i] = *reinterpret_cast<const uint4*>(x + (size_t)row * H + idx * 8);
+        ng[i] = *reinterpret_cast<const uint4*>(gy + (size_t)row * H + idx * 8);
+      }
+    }
+  };
+  if ((int)blockIdx.x < M) fetch(blockIdx.x);
+  for (int row = blockIdx.x; row < M; row += gridDim.x) {
     const size_t off = (size_t)row * H;
     float xv[VPT][8], gv[VPT][8];
     float ss = 0.f, dot = 0.f;
@@ -45,8 +56,7 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const __nv_bfloat16* _
     for (int i = 0; i < VPT; ++i) {
       const int idx = tid + i * 256;
       if (idx < nvec) {
-        const uint4 ux = *reinterpret_cast<const uint4*>(x + off + idx * 8);
-        const uint4 ug = *reinterpret_cast<const uint4*>(gy + off + idx * 8);
+        const uint4 ux = nx[i], ug = ng[i];
         const __nv_bfloat162* hx = reinterpret_cast<const __nv_bfloat162*>(&ux);
         const __nv_bfloat162* hg = reinterpret_cast<const __nv_bfloat162*>(&ug);
 #pragma unroll
@@ -62,6 +72,7 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const __nv_bfloat16* _
         }
       }
     }
+    if (row + (int)gridDim.x < M) fetch(row + gridDim.x);
     ss = warp_sum(ss);
     dot = warp_sum(dot);
     __syncthreads();
@@ -91,12 +102,18 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const __nv_bfloat16* _
     }
   }
   if (gw != nullptr) {
+    // a thread owns eight neighbouring columns: by way of shared memory a warp's additions fall into one 128-byte line instead of eight
+    __shared__ float slice[256 * 8];
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-      const int idx = tid + i * 256;
-      if (idx < nvec) {
+      __syncthreads();
 #pragma unroll
-        for (int j = 0; j < 8; ++j) atomicAdd(gw + idx * 8 + j, gwa[i][j]);
+      for (int j = 0; j < 8; ++j) slice[tid * 8 + j] = gwa[i][j];
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int c = j * 256 + tid;
+        if (i * 2048 + c < H) atomicAdd(gw + i * 2048 + c, slice[c]);
       }
     }
   }
@@ -136,10 +153,13 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __
 
 // ---------------------------------------------------------------------------------------------
 // Backward of the per-head QK RMSNorm + rotate-half RoPE (forward: qk_norm_rope_kv_kernel in
-// elementwise.cu).  One warp per (token, head), grid-stride; lane l owns elements l*EPL..+EPL-1.
+// elementwise.cu).  Lane l owns elements l*EPL..+EPL-1 of a head.
 //   n = w * (x * rstd),  y = n * cos + rot(n) * sin      (q and k heads; v heads pass through)
 //   gn = gy * cos +/- partner(gy) * sin ;  gx = rstd * (gn*w - xn * mean(gn*w*xn)) ;  gw += gn * xn
 // The weight gradients are summed per CTA in shared memory and added to the fp32 buffers once.
+// A CTA takes a token at a time, a warp four of its heads with all their loads in flight and the sines and cosines once for them (once
+// per CTA, by way of shared memory, 38 us: a barrier per token).  Bound: HBM (3072 tokens of 16 + 16 heads: 75 MB, 11 us); a warp per
+// head with one in flight and its own sincosf: 50 us, now 34.4 us.
 // ---------------------------------------------------------------------------------------------
 struct QkRopeBwdParams {
   const __nv_bfloat16* qkv;      // [M, (nq + 2 nkv) * HD] forward input
@@ -156,69 +176,77 @@ struct QkRopeBwdParams {
   float eps, log2_theta;
 };
 
-template <int HD>
-__global__ void __launch_bounds__(128) qk_norm_rope_bwd_kernel(const QkRopeBwdParams p) {
+constexpr int QKB_U = 4, QKB_WARPS = 8;
+template <int HD, bool WIDE>
+__global__ void __launch_bounds__(QKB_WARPS * 32) qk_norm_rope_bwd_kernel(const QkRopeBwdParams p) {
   constexpr int EPL = HD / 32;
+  using Piece = QkvPiece<EPL, WIDE>;
   __shared__ float s_gw[2][HD];
   for (int i = threadIdx.x; i < 2 * HD; i += blockDim.x) (&s_gw[0][0])[i] = 0.f;
   __syncthreads();
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int heads = p.nq + 2 * p.nkv;
-  const long long total = (long long)p.M * heads;
-  const long long stride = (long long)gridDim.x * (blockDim.x >> 5);
+  const bool upper = lane >= 16;
   float gw_q[EPL], gw_k[EPL];
+  float inv[EPL];
 #pragma unroll
-  for (int i = 0; i < EPL; ++i) { gw_q[i] = 0.f; gw_k[i] = 0.f; }
-  for (long long wg = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); wg < total; wg += stride) {
-    const int t = (int)(wg / heads);
-    const int h = (int)(wg % heads);
-    const bool is_q = h < p.nq;
-    const bool is_k = !is_q && h < p.nq + p.nkv;
-    __nv_bfloat16* dst = p.gqkv + ((size_t)t * heads + h) * HD + lane * EPL;
-    if (!is_q && !is_k) {
-      const __nv_bfloat16* g = p.gv + ((size_t)t * p.nkv + (h - p.nq - p.nkv)) * HD + lane * EPL;
+  for (int i = 0; i < EPL; ++i) inv[i] = exp2f(-(2.0f * (float)((lane & 15) * EPL + i) / (float)HD) * p.log2_theta);
+  Piece wq, wk;
+  wq.load(p.q_w + lane * EPL);
+  wk.load(p.k_w + lane * EPL);
 #pragma unroll
-      for (int i = 0; i < EPL; ++i) dst[i] = g[i];
-      continue;
-    }
-    const __nv_bfloat16* src = p.qkv + ((size_t)t * heads + h) * HD + lane * EPL;
-    const __nv_bfloat16* g = is_q ? p.gq + ((size_t)t * p.nq + h) * HD + lane * EPL
-                                  : p.gk + ((size_t)t * p.nkv + (h - p.nq)) * HD + lane * EPL;
-    const __nv_bfloat16* w = (is_q ? p.q_w : p.k_w) + lane * EPL;
-    float x[EPL], gy[EPL], wv[EPL], gpart[EPL];
-    float ss = 0.f;
+  for (int i = 0; i < EPL; ++i) gw_q[i] = gw_k[i] = 0.f;
+  for (int t = blockIdx.x; t < p.M; t += gridDim.x) {
+    float2 cs[EPL];
 #pragma unroll
     for (int i = 0; i < EPL; ++i) {
-      x[i] = __bfloat162float(src[i]);
-      gy[i] = __bfloat162float(g[i]);
-      wv[i] = __bfloat162float(w[i]);
-      ss += x[i] * x[i];
+      const float ang = (float)p.pos[t] * inv[i];
+      cs[i] = make_float2(bf16_round(cosf(ang)), bf16_round(sinf(ang)));
     }
-    ss = warp_sum(ss);
-    const float rstd = rsqrtf(ss / (float)HD + p.eps);
+    for (int h0 = warp; h0 < heads; h0 += QKB_U * QKB_WARPS) {
+      Piece xin[QKB_U], gin[QKB_U];
 #pragma unroll
-    for (int i = 0; i < EPL; ++i) gpart[i] = __shfl_xor_sync(0xffffffffu, gy[i], 16);
-    const float posf = (float)p.pos[t];
-    const bool upper = lane >= 16;
-    float gn[EPL], xn[EPL];
-    float dot = 0.f;
+      for (int u = 0; u < QKB_U; ++u) {
+        const int h = h0 + u * QKB_WARPS;
+        if (h >= heads) continue;
+        if (h < p.nq + p.nkv) xin[u].load(p.qkv + ((size_t)t * heads + h) * HD + lane * EPL);
+        gin[u].load((h < p.nq ? p.gq + ((size_t)t * p.nq + h) * HD
+                              : h < p.nq + p.nkv ? p.gk + ((size_t)t * p.nkv + h - p.nq) * HD
+                                                 : p.gv + ((size_t)t * p.nkv + h - p.nq - p.nkv) * HD) + lane * EPL);
+      }
 #pragma unroll
-    for (int i = 0; i < EPL; ++i) {
-      const int d = lane * EPL + i;
-      const int j = upper ? d - HD / 2 : d;
-      const float inv = exp2f(-(2.0f * (float)j / (float)HD) * p.log2_theta);
-      const float ang = posf * inv;
-      const float c = bf16_round(cosf(ang)), sn = bf16_round(sinf(ang));
-      gn[i] = gy[i] * c + (upper ? -gpart[i] : gpart[i]) * sn;
-      xn[i] = x[i] * rstd;
-      dot += gn[i] * wv[i] * xn[i];
-    }
-    dot = warp_sum(dot) / (float)HD;
+      for (int u = 0; u < QKB_U; ++u) {
+        const int h = h0 + u * QKB_WARPS;
+        if (h >= heads) continue;
+        Piece out = gin[u];
+        if (h < p.nq + p.nkv) {
+          const bool is_q = h < p.nq;
+          float x[EPL], gn[EPL], wv[EPL], ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < EPL; ++i) {
-      dst[i] = __float2bfloat16_rn(rstd * (gn[i] * wv[i] - xn[i] * dot));
-      if (is_q) gw_q[i] += gn[i] * xn[i];
-      else gw_k[i] += gn[i] * xn[i];
+          for (int i = 0; i < EPL; ++i) {
+            x[i] = __bfloat162float(xin[u].v[i]);
+            wv[i] = __bfloat162float(is_q ? wq.v[i] : wk.v[i]);
+            ss += x[i] * x[i];
+          }
+          const float rstd = rsqrtf(warp_sum(ss) / (float)HD + p.eps);
+          float dot = 0.f;
+#pragma unroll
+          for (int i = 0; i < EPL; ++i) {
+            const float gy = __bfloat162float(gin[u].v[i]), part = __shfl_xor_sync(0xffffffffu, gy, 16);
+            gn[i] = gy * cs[i].x + (upper ? -part : part) * cs[i].y;
+            x[i] *= rstd;
+            dot += gn[i] * wv[i] * x[i];
+          }
+          dot = warp_sum(dot) / (float)HD;
+#pragma unroll
+          for (int i = 0; i < EPL; ++i) {
+            out.v[i] = __float2bfloat16_rn(rstd * (gn[i] * wv[i] - x[i] * dot));
+            if (is_q) gw_q[i] += gn[i] * x[i];
+            else gw_k[i] += gn[i] * x[i];
+          }
+        }
+        out.store(p.gqkv + ((size_t)t * heads + h) * HD + lane * EPL);
+      }
     }
   }
 #pragma unroll
@@ -231,6 +259,55 @@ __global__ void __launch_bounds__(128) qk_norm_rope_bwd_kernel(const QkRopeBwdPa
     if (p.gq_w != nullptr) atomicAdd(p.gq_w + i, s_gw[0][i]);
     if (p.gk_w != nullptr) atomicAdd(p.gk_w + i, s_gw[1][i]);
   }
+}
+
+// d[row] = sum over hd of a[row][.] * b[row][.]: what the attention backward subtracts from every score gradient of a query head.  A lane
+// takes 16 bytes of each, hd / 8 lanes share a row.  HBM bound; the sum replaces two fp32 copies, their product and its reduction.
+__global__ void __launch_bounds__(256) rows_dot_kernel(const uint4* __restrict__ a, const uint4* __restrict__ b, float* __restrict__ d,
+                                                       long long rows, int lanes) {
+  const long long i = blockIdx.x * 256ll + threadIdx.x;
+  const long long row = i / lanes;
+  float s = 0.f;
+  if (row < rows) {
+    const uint4 u = a[i], v = b[i];
+    const __nv_bfloat162 *x = reinterpret_cast<const __nv_bfloat162*>(&u), *y = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __bfloat1622float2(x[j]), g = __bfloat1622float2(y[j]);
+      s += f.x * g.x + f.y * g.y;
+    }
+  }
+  for (int o = lanes >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (row < rows && i % lanes == 0) d[row] = s;
+}
+
+// Block-diagonal adapter factor of a fused projection, [F, n r]: rows begin[j] .. end[j] of columns j r .. (j + 1) r hold
+// B_j [., r] * scale, everything else is zero.
+struct BlockDiagParams {
+  const __nv_bfloat16* b[4];
+  int begin[4], end[4];
+  int n, r, F;
+  float scale;
+  __nv_bfloat16* out;
+};
+__global__ void __launch_bounds__(256) block_diag_kernel(const BlockDiagParams p) {
+  const int per = p.n * p.r / 8;                     // pieces of eight columns in a row
+  const long long i = blockIdx.x * 256ll + threadIdx.x;
+  if (i >= (long long)p.F * per) return;
+  const int row = (int)(i / per), col = (int)(i % per) * 8, j = col / p.r;
+  uint4 v = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (k != j || k >= p.n || row < p.begin[k] || row >= p.end[k]) continue;
+    v = *reinterpret_cast<const uint4*>(p.b[k] + (size_t)(row - p.begin[k]) * p.r + (col - k * p.r));
+    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float2 f = __bfloat1622float2(h[c]);
+      h[c] = __floats2bfloat162_rn(f.x * p.scale, f.y * p.scale);
+    }
+  }
+  *reinterpret_cast<uint4*>(p.out + (size_t)row * p.n * p.r + col) = v;
 }
 
 }  // namespace tahb
@@ -256,11 +333,15 @@ extern "C" int tahb_qk_norm_rope_bwd(const void* qkv, const void* q_w, const voi
   p.M = M; p.nq = nq; p.nkv = nkv;
   p.eps = eps;
   p.log2_theta = log2f(theta);
-  const long long warps = (long long)M * (nq + 2 * nkv);
-  long long blocks = (warps + 3) / 4;
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  if (hd == 128) qk_norm_rope_bwd_kernel<128><<<(int)blocks, 128, 0, stream>>>(p);
-  else if (hd == 64) qk_norm_rope_bwd_kernel<64><<<(int)blocks, 128, 0, stream>>>(p);
+  uintptr_t at = 0;
+  for (const void* q : {qkv, q_w, k_w, gq, gk, gv, (const void*)gqkv}) at |= reinterpret_cast<uintptr_t>(q);
+  const bool wide = at % (hd / 16) == 0;
+  const int blocks = M < 296 ? M : 296;            // two CTAs per SM, whose sums meet in the weight gradients' few lines
+#define TAHB_QKB(HD_)                                                                          \
+  (wide ? (void)(qk_norm_rope_bwd_kernel<HD_, true><<<blocks, QKB_WARPS * 32, 0, stream>>>(p)) \
+        : (void)(qk_norm_rope_bwd_kernel<HD_, false><<<blocks, QKB_WARPS * 32, 0, stream>>>(p)))
+  if (hd == 128) TAHB_QKB(128);
+  else if (hd == 64) TAHB_QKB(64);
   else return -2;
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
@@ -271,7 +352,7 @@ extern "C" int tahb_rmsnorm_bwd(const void* x, const void* w, const void* gy, vo
   if (M <= 0) return 0;
   if (H % 8) return -1;
   const int nvec = H / 8;
-  const int grid = (M + RMSB_ROWS - 1) / RMSB_ROWS;
+  const int grid = M < RMSB_GRID ? M : RMSB_GRID;
   auto X = reinterpret_cast<const __nv_bfloat16*>(x);
   auto W = reinterpret_cast<const __nv_bfloat16*>(w);
   auto GY = reinterpret_cast<const __nv_bfloat16*>(gy);
@@ -293,5 +374,32 @@ extern "C" int tahb_swiglu_bwd(const void* gu, const void* gy, void* dgu, long l
   swiglu_bwd_kernel<<<(int)blocks, 256, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(gu),
                                                      reinterpret_cast<const __nv_bfloat16*>(gy),
                                                      reinterpret_cast<__nv_bfloat16*>(dgu), M, I);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+// d [rows] fp32 = row sums of a * b, both [rows, hd] bf16 contiguous on 16-byte boundaries, hd 64 or 128.
+extern "C" int tahb_rows_dot(const void* a, const void* b, float* d, long long rows, int hd, cudaStream_t stream) {
+  if (rows <= 0) return 0;
+  if (hd != 64 && hd != 128) return -1;
+  const long long blocks = (rows * (hd / 8) + 255) / 256;
+  rows_dot_kernel<<<(unsigned)blocks, 256, 0, stream>>>(reinterpret_cast<const uint4*>(a), reinterpret_cast<const uint4*>(b), d, rows, hd / 8);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+// out [F, n r] from n <= 4 factors (see BlockDiagParams); r a multiple of 8, pointers on 16-byte boundaries.
+extern "C" int tahb_block_diag(void* const* b, const int* begin, const int* end, int n, int r, int F, float scale, void* out, cudaStream_t stream) {
+  if (F <= 0) return 0;
+  if (n < 1 || n > 4 || r <= 0 || r % 8) return -1;
+  BlockDiagParams p = {};
+  for (int j = 0; j < n; ++j) {
+    p.b[j] = reinterpret_cast<const __nv_bfloat16*>(b[j]);
+    p.begin[j] = begin[j];
+    p.end[j] = end[j];
+  }
+  p.n = n; p.r = r; p.F = F;
+  p.scale = scale;
+  p.out = reinterpret_cast<__nv_bfloat16*>(out);
+  const long long blocks = ((long long)F * (n * r / 8) + 255) / 256;
+  block_diag_kernel<<<(unsigned)blocks, 256, 0, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }

@@ -109,18 +109,31 @@ class _LoRALinear(torch.autograd.Function):
         return gx, gw, gt, gbd
 
 
+class _BlockDiag(torch.autograd.Function):
+    """The adapter's output factors, scaled, as one block-diagonal matrix."""
+
+    @staticmethod
+    def forward(ctx, F, spans, scaling, *blocks):
+        ctx.args = (spans, scaling, blocks[0].shape[1])
+        return K.block_diag([b.detach() for b in blocks], spans, F, scaling)
+
+    @staticmethod
+    def backward(ctx, g):
+        spans, scaling, r = ctx.args
+        return (None, None, None) + tuple(g[lo:hi, j * r:(j + 1) * r] * scaling if ctx.needs_input_grad[3 + j] else None
+                                          for j, (lo, hi) in enumerate(spans))
+
+
 def lora_linear(x, w, xa, lora_A, lora_B: List[torch.Tensor], adapted: Sequence[int], out_splits: Sequence[int],
                 r: int, scaling: float):
     R = len(adapted) * r
     if _gemm_ok(x, w) and R % 64 == 0 and lora_A.dtype == torch.bfloat16:
         t = linear(xa, lora_A)
-        bd = w.new_zeros(w.shape[0], R)
         off = [0]
         for sz in out_splits:
             off.append(off[-1] + sz)
-        for j, idx in enumerate(adapted):
-            bd[off[idx]:off[idx + 1], j * r:(j + 1) * r] = lora_B[j] * scaling
-        return _LoRALinear.apply(x, w, t, bd)
+        spans = tuple((off[idx], off[idx + 1]) for idx in adapted)
+        return _LoRALinear.apply(x, w, t, _BlockDiag.apply(w.shape[0], spans, scaling, *lora_B))
     y = linear(x, w)
     t = F.linear(xa, lora_A)
     pieces = list(y.split(list(out_splits), dim=-1))
@@ -372,7 +385,7 @@ class _SegmentAttention(torch.autograd.Function):
         ks = list(ctx.saved_tensors[3:3 + n_seg])
         vs = list(ctx.saved_tensors[3 + n_seg:])
         do2 = dout.reshape(B * Tq, nq * hd).contiguous()
-        dsum = (do2.float() * out.float()).view(B * Tq, nq, hd).sum(-1).contiguous()
+        dsum = K.rows_dot(do2, out, hd)
         scale = hd ** -0.5
         dq = K.attn_bwd_dq(q2, do2, ks, vs, meta.bases, meta.counts, meta.tile_q0, meta.tile_qn, nq, nkv, hd, scale,
                            lse, dsum, bounds=meta.bounds)

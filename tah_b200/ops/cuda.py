@@ -568,6 +568,31 @@ def swiglu_bwd(gate_up: torch.Tensor, gy: torch.Tensor) -> torch.Tensor:
     return out
 
 
+def rows_dot(a: torch.Tensor, b: torch.Tensor, hd: int) -> torch.Tensor:
+    """fp32 ``[N, heads]``: per head of ``hd``, the sum of ``a * b`` (contiguous bf16 ``[N, heads * hd]``)."""
+    if hd not in (64, 128) or any(t.dtype != torch.bfloat16 or not t.is_contiguous() or t.data_ptr() % 16 for t in (a, b)):
+        return (a.float() * b.float()).view(a.shape[0], -1, hd).sum(-1).contiguous()
+    d = torch.empty(a.shape[0], a.shape[1] // hd, dtype=torch.float32, device=a.device)
+    _rc(lib().tahb_rows_dot(_p(a), _p(b), _p(d), c_ll(d.numel()), c_int(hd), _stream()), "tahb_rows_dot")
+    return d
+
+
+def block_diag(blocks: Sequence[torch.Tensor], spans, F: int, scale: float) -> torch.Tensor:
+    """``[F, n r]``: block ``j [., r]`` times ``scale`` in rows ``spans[j]`` of columns ``j r ..``, zeros elsewhere."""
+    n, r = len(blocks), blocks[0].shape[1]
+    if (n > 4 or r % 8 or any(tuple(b.shape) != (hi - lo, r) or not 0 <= lo <= hi <= F for b, (lo, hi) in zip(blocks, spans)) or
+            any(b.dtype != torch.bfloat16 or not b.is_contiguous() or b.data_ptr() % 16 for b in blocks)):
+        out = torch.zeros(F, n * r, dtype=torch.bfloat16, device=blocks[0].device)
+        for j, (b, (lo, hi)) in enumerate(zip(blocks, spans)):
+            out[lo:hi, j * r:(j + 1) * r] = b * scale
+        return out
+    out = torch.empty(F, n * r, dtype=torch.bfloat16, device=blocks[0].device)
+    ints = lambda k: (c_int * n)(*[s[k] for s in spans])
+    _rc(lib().tahb_block_diag(_ptr_array(list(blocks)), ints(0), ints(1), c_int(n), c_int(r), c_int(F), c_float(scale), _p(out), _stream()),
+        "tahb_block_diag")
+    return out
+
+
 def qk_norm_rope_bwd(qkv, q_w, k_w, gq, gk, gv, pos, nq: int, nkv: int, hd: int, eps: float, theta: float):
     """Backward of :func:`qk_norm_rope_kv` (dense outputs): returns ``(gqkv, gq_w_fp32, gk_w_fp32)``."""
     M = qkv.shape[0]

@@ -973,6 +973,37 @@ def test_qk_norm_rope_tokens_and_boundaries(hd, nq, nkv, shift):
     assert all(torch.equal(a, b) for a, b in zip(*out))
 
 
+@pytest.mark.parametrize("M,H", [(1, 64), (295, 2048), (296, 2048), (700, 2056), (40, 8192)])
+def test_rms_norm_bwd_row_shares(M, H):
+    """Row counts around one row per CTA; the weight gradient is a 32-bit sum over the rows."""
+    Kc = _cuda()
+    x, w, gy = _rand(M, H, seed=1), _rand(H, seed=2), _rand(M, H, seed=3)
+    gx, gw = Kc.rms_norm_bwd(x, w, gy, 1e-6)
+    xf, wf = x.double().requires_grad_(True), w.double().requires_grad_(True)
+    (wf * xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + 1e-6) * gy.double()).sum().backward()
+    _close(gx, xf.grad, atol=1e-3, rtol=2.0 ** -8)
+    _close(gw, wf.grad, atol=1e-5 * M, rtol=1e-5)
+
+
+@pytest.mark.parametrize("spans,F,r", [(((0, 40), (40, 56), (56, 72)), 72, 8), (((0, 16), (32, 50)), 50, 24), (((0, 130),), 130, 64)])
+def test_block_diag_adapter_factor(spans, F, r):
+    Kc = _cuda()
+    blocks = [_rand(hi - lo, r, seed=j) for j, (lo, hi) in enumerate(spans)]
+    ref = torch.zeros(F, len(spans) * r, dtype=torch.bfloat16, device="cuda")
+    for j, (b, (lo, hi)) in enumerate(zip(blocks, spans)):
+        ref[lo:hi, j * r:(j + 1) * r] = b * 1.7
+    assert torch.equal(Kc.block_diag(blocks, spans, F, 1.7), ref)
+    odd = [torch.cat([b.flatten()[:1], b.flatten()])[1:].view_as(b) for b in blocks]       # off the 16-byte boundary
+    assert torch.equal(Kc.block_diag(odd, spans, F, 1.7), ref)
+
+
+@pytest.mark.parametrize("hd,heads,N", [(128, 16, 33), (64, 3, 1), (32, 2, 5)])
+def test_rows_dot(hd, heads, N):
+    Kc = _cuda()
+    a, b = _rand(N, heads * hd, seed=1), _rand(N, heads * hd, seed=2)
+    _close(Kc.rows_dot(a, b, hd), (a.double() * b.double()).view(N, heads, hd).sum(-1), atol=1e-5, rtol=1e-6)
+
+
 @pytest.mark.parametrize("M,F,K", [(257, 512, 256), (385, 256, 2048), (1000, 2048, 192), (192, 512, 64)])
 @pytest.mark.parametrize("residual", [False, True])
 def test_gemm_tile_forms_give_the_same_bits(M, F, K, residual):
