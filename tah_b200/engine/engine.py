@@ -228,7 +228,7 @@ class TaHEngine(DecodeEngine):
         # on four warps costs as much as the tile's main loop (prefill 272 ms fused, 254 ms with the separate kernel)
         fuse_qkv = hd == 128 and "qkv" in _fusions("")
         if tensor_core_attn:
-            tile_q0, tile_qn = K.attn_tiles(seq_counts)
+            tile_q0, tile_qn = K.attn_tiles(seq_counts, by_work=True)
         rope_cs = K.rope_table(pos, hd, cfg.rope_theta) if fuse_qkv else None     # once per pass, shared by the layers
         # tensor parallel: token counts that deal out in 16-row blocks take the push path (reduce-scatter in the
         # GEMM epilogue, consumers wait on landing flags), the others the pull kernel

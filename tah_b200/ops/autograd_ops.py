@@ -336,7 +336,7 @@ class SegmentMeta:
         B, Tq = q_pos.shape
         dev = q_pos.device
         self.B, self.Tq = B, Tq
-        self.tile_q0, self.tile_qn = K.attn_tiles(torch.full((B,), Tq, device=dev))
+        self.tile_q0, self.tile_qn = K.attn_tiles(torch.full((B,), Tq, device=dev), by_work=True)
         self.bases, self.counts, self.bounds, self.items, self.seg_T = [], [], [], [], []
         q_rows = torch.full((B,), Tq, device=dev)
         big = torch.iinfo(torch.int64).max

@@ -1028,3 +1028,32 @@ def test_gemm_tile_forms_give_the_same_bits(M, F, K, residual):
         assert bool(((out.double() - ref).abs() <= tol).all())
     assert bool(((Kc.gemm(x, w, residual=res).double() - ref).abs() <= tol).all())
     Kc.check_status()
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("nq,nkv", [(3, 1), (4, 4), (4, 1), (6, 3)])
+def test_attention_heads_of_a_kv_head(hd, nq, nkv):
+    """Forward and backward with odd and even numbers of query heads per KV head (even ones go two to a CTA), sequences around the sizes
+    of key blocks and query tiles; bounds as in the tests above."""
+    Kc = _cuda()
+    lens = [1, 63, 64, 65, 129, 300]
+    n = sum(lens)
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    b = [starts[i] for i, L in enumerate(lens) for _ in range(L)]
+    c = [j + 1 for L in lens for j in range(L)]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    q, k, v, dout = (_rand(n, h * hd, seed=j) for j, h in enumerate((nq, nkv, nkv, nq)))
+    cnt = torch.tensor(lens, device="cuda")
+    tq0, tqn = Kc.attn_tiles(cnt)
+    lse = torch.empty(n, nq, dtype=torch.float32, device="cuda")
+    out = Kc.prefill_attn(q, [k], [v], [i32(b)], [i32(c)], tq0, tqn, nq, nkv, hd, hd ** -0.5, lse=lse)
+    ref, rdq, rdk, rdv = _ref_attention_autograd(q, [k], [v], [b], [c], nq, nkv, hd, dout)
+    _close(out.view(n, nq, hd), ref, atol=2e-2, rtol=2e-2)
+    dsum = Kc.rows_dot(dout, out, hd)
+    dq = Kc.attn_bwd_dq(q, dout, [k], [v], [i32(b)], [i32(c)], tq0, tqn, nq, nkv, hd, hd ** -0.5, lse, dsum)
+    dk, dv = Kc.attn_bwd_dkv(q, dout, k, v, i32(c), Kc.attn_kv_items(cnt, torch.tensor(starts, device="cuda"), cnt), nq, nkv, hd, hd ** -0.5,
+                             lse, dsum)
+    Kc.check_status()
+    _close(dq.view(n, nq, hd), rdq, atol=3e-2, rtol=3e-2)
+    _close(dk.view(n, nkv, hd), rdk[0], atol=4e-2, rtol=4e-2)
+    _close(dv.view(n, nkv, hd), rdv[0], atol=4e-2, rtol=4e-2)
