@@ -5,16 +5,21 @@
 //
 // Two kernels, both recompute S and dP per block with tcgen05.mma from TMA-staged tiles:
 //
-//   attn_bwd_dq_kernel   one CTA per (128-query tile, query head), the forward's loop over 64-key
-//                        blocks of up to three KV segments.  S and dP in tensor memory, dS written to
-//                        shared memory (K-major) by 256 threads, dQ += dS K with K consumed MN-major.
-//                        Two CTAs per SM.
+//   attn_bwd_dq_kernel   one CTA per (128-query tile, two query heads of a KV head; one where their number
+//                        is odd), the forward's loop over 64-key blocks of up to three KV segments.  S and dP
+//                        in tensor memory, dS written to shared memory (K-major) by 256 threads per head,
+//                        dQ += dS K with K consumed MN-major.  One head's arithmetic runs under the other's
+//                        products, and the next block is loaded meanwhile: with a head per CTA, two CTAs per SM
+//                        and room for one K / V block each, its latency stood in every block.
+//                        16 heads on 8 KV heads, 3072 tokens in training: 231 us before, 213 with two heads, 179 with
+//                        the long tiles of all heads first.
 //   attn_bwd_dkv_kernel  one CTA per (128-key block of one sequence and segment, KV head): the keys sit
 //                        on the tensor-memory lanes.  Loop over the 64-query sub-tiles that can see the
 //                        block and over the query heads of the KV group: S^T = K Q^T, dP^T = V dO^T,
 //                        P^T and dS^T to shared memory, dV += P^T dO and dK += dS^T Q with the same
 //                        Q / dO tiles consumed MN-major.  dK and dV accumulate in tensor memory over the
-//                        whole loop (4 x 128 columns with the two score tiles).
+//                        whole loop (4 x 128 columns with the two score tiles).  The blocks that the most queries
+//                        see go first, of all heads: 209 us there, now 172.
 //
 // The duo-causal rule is the per-query bound key_index < count[segment][query]; no mask tensor.
 // All waits are bounded (common.cuh).
@@ -48,48 +53,52 @@ struct AttnBwdParams {
   int* status;
 };
 
-template <int HD>
+// NH: query heads of a CTA
+template <int HD, int NH>
 struct BwdQCfg {
   static constexpr int BK = 64;
   static constexpr int HALVES = HD / 64;
   static constexpr int QTILE = 128 * 64 * 2;
   static constexpr int KTILE = BK * 64 * 2;
-  static constexpr int Q_BYTES = HALVES * QTILE;               // Q and dO tiles
+  static constexpr int Q_BYTES = HALVES * QTILE;               // Q and dO tiles of a head
   static constexpr int K_BYTES = HALVES * KTILE;               // K and V blocks
-  static constexpr int DS_BYTES = 128 * BK * 2;
-  static constexpr int SMEM_BYTES = 2 * Q_BYTES + DS_BYTES + 2 * K_BYTES + 128;
-  static constexpr int TMEM_COLS = 256;                        // S at 0, dP at 64, dQ at 128
+  static constexpr int STAGE_BYTES = 2 * K_BYTES;
+  static constexpr int NSTAGE = NH;
+  static constexpr int DS_BYTES = 128 * BK * 2;                // of a head
+  static constexpr int SMEM_BYTES = NH * (2 * Q_BYTES + DS_BYTES) + NSTAGE * STAGE_BYTES + 128;
+  static constexpr int TMEM_COLS = NH * 256;                   // of every head: S at 0, dP at 64, dQ at 128
+  static constexpr int THREADS = 64 + NH * 256;
 };
 constexpr int BWD_THREADS = 320;
 
-template <int HD>
-__global__ void __launch_bounds__(BWD_THREADS, 2)
+template <int HD, int NH>
+__global__ void __launch_bounds__(BwdQCfg<HD, NH>::THREADS, NH == 2 ? 1 : 2)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                    const __grid_constant__ CUtensorMap tm_k0, const __grid_constant__ CUtensorMap tm_v0,
                    const __grid_constant__ CUtensorMap tm_k1, const __grid_constant__ CUtensorMap tm_v1,
                    const __grid_constant__ CUtensorMap tm_k2, const __grid_constant__ CUtensorMap tm_v2,
                    const AttnBwdParams p) {
-  using C = BwdQCfg<HD>;
+  using C = BwdQCfg<HD, NH>;
   constexpr int BK = C::BK;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* q_s = smem;
-  uint8_t* do_s = q_s + C::Q_BYTES;
-  uint8_t* ds_s = do_s + C::Q_BYTES;
-  uint8_t* k_s = ds_s + C::DS_BYTES;
-  uint8_t* v_s = k_s + C::K_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(v_s + C::K_BYTES);
+  uint8_t* do_s = q_s + NH * C::Q_BYTES;
+  uint8_t* ds_s = do_s + NH * C::Q_BYTES;
+  uint8_t* kv_s = ds_s + NH * C::DS_BYTES;                      // stages: [K | V]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(kv_s + C::NSTAGE * C::STAGE_BYTES);
   uint64_t* q_full = bars;
-  uint64_t* kv_full = bars + 1;
-  uint64_t* kv_empty = bars + 2;
-  uint64_t* s_full = bars + 3;
-  uint64_t* ds_ready = bars + 4;
-  uint64_t* dq_done = bars + 5;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6);
+  uint64_t* kv_full = bars + 1;                                 // [NSTAGE]
+  uint64_t* kv_empty = kv_full + C::NSTAGE;                     // [NSTAGE]
+  uint64_t* s_full = kv_empty + C::NSTAGE;                      // [NH]
+  uint64_t* ds_ready = s_full + NH;                             // [NH]
+  uint64_t* dq_done = ds_ready + NH;                            // [NH]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(dq_done + NH);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tile = blockIdx.x, head = blockIdx.y;
-  const int kvh = head / (p.nq / p.nkv);
+  // the last tiles of a sequence walk the most keys: all heads of them first, so that the short ones fill the last wave
+  const int n_hg = p.nq / NH, tile = gridDim.x / n_hg - 1 - blockIdx.x / n_hg, head0 = blockIdx.x % n_hg * NH;
+  const int kvh = head0 / (p.nq / p.nkv);
   const int q0 = p.tile_q0[tile], qn = p.tile_qn[tile];
   if ((smem_u32(smem) & 1023u) != 0) {
     if (threadIdx.x == 0) atomicCAS(p.status, 0, STATUS_BAD_INDEX);
@@ -108,11 +117,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   }
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
-    mbar_init(kv_full, 1);
-    mbar_init(kv_empty, 1);
-    mbar_init(s_full, 1);
-    mbar_init(ds_ready, 256);
-    mbar_init(dq_done, 1);
+    for (int s = 0; s < C::NSTAGE; ++s) { mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 1); }
+    for (int h = 0; h < NH; ++h) { mbar_init(&s_full[h], 1); mbar_init(&ds_ready[h], 256); mbar_init(&dq_done[h], 1); }
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -124,28 +130,29 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_s = tmem_base, tmem_dp = tmem_base + 64, tmem_dq = tmem_base + 128;
 
   if (warp == 0) {
     if (lane == 0) {
-      mbar_expect_tx(q_full, 2 * C::Q_BYTES);
+      mbar_expect_tx(q_full, 2 * NH * C::Q_BYTES);
 #pragma unroll
-      for (int h = 0; h < C::HALVES; ++h) {
-        tma_load_2d(q_s + h * C::QTILE, &tm_q, head * HD + h * 64, q0, q_full);
-        tma_load_2d(do_s + h * C::QTILE, &tm_do, head * HD + h * 64, q0, q_full);
+      for (int h = 0; h < NH * C::HALVES; ++h) {
+        tma_load_2d(q_s + h * C::QTILE, &tm_q, head0 * HD + h * 64, q0, q_full);
+        tma_load_2d(do_s + h * C::QTILE, &tm_do, head0 * HD + h * 64, q0, q_full);
       }
       int i = 0;
       for (int s = 0; s < p.n_seg; ++s) {
         const CUtensorMap* mk = s == 0 ? &tm_k0 : s == 1 ? &tm_k1 : &tm_k2;
         const CUtensorMap* mv = s == 0 ? &tm_v0 : s == 1 ? &tm_v1 : &tm_v2;
         for (int b = 0; b < seg_blocks[s]; ++b, ++i) {
-          mbar_wait(kv_empty, (i & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_STAGE_EMPTY);
-          mbar_expect_tx(kv_full, 2 * C::K_BYTES);
+          const int st = i % C::NSTAGE;
+          mbar_wait(&kv_empty[st], ((i / C::NSTAGE) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_STAGE_EMPTY);
+          mbar_expect_tx(&kv_full[st], C::STAGE_BYTES);
+          uint8_t* k_s = kv_s + st * C::STAGE_BYTES;
           const int y = seg_b0[s] + b * BK;
 #pragma unroll
           for (int h = 0; h < C::HALVES; ++h) {
-            tma_load_2d(k_s + h * C::KTILE, mk, kvh * HD + h * 64, y, kv_full);
-            tma_load_2d(v_s + h * C::KTILE, mv, kvh * HD + h * 64, y, kv_full);
+            tma_load_2d(k_s + h * C::KTILE, mk, kvh * HD + h * 64, y, &kv_full[st]);
+            tma_load_2d(k_s + C::K_BYTES + h * C::KTILE, mv, kvh * HD + h * 64, y, &kv_full[st]);
           }
         }
       }
@@ -157,34 +164,53 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       constexpr uint32_t idesc_q = umma_idesc_bf16_bmn(128, HD);
       mbar_wait(q_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
       const uint32_t q_addr = smem_u32(q_s), do_addr = smem_u32(do_s), ds_addr = smem_u32(ds_s);
-      const uint32_t k_addr = smem_u32(k_s), v_addr = smem_u32(v_s);
-      for (int i = 0; i < total_blocks; ++i) {
-        mbar_wait(kv_full, i & 1, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
-        tc_fence_after();
+      auto scores = [&](int i, int h) {             // S = Q K^T and dP = dO V^T over head_dim
+        const uint32_t k_addr = smem_u32(kv_s + (i % C::NSTAGE) * C::STAGE_BYTES), v_addr = k_addr + C::K_BYTES;
 #pragma unroll
-        for (int ks = 0; ks < HD / 16; ++ks) {      // S = Q K^T and dP = dO V^T over head_dim
-          const uint32_t qo = (ks / 4) * C::QTILE + (ks % 4) * 32;
+        for (int ks = 0; ks < HD / 16; ++ks) {
+          const uint32_t qo = h * C::Q_BYTES + (ks / 4) * C::QTILE + (ks % 4) * 32;
           const uint32_t ko = (ks / 4) * C::KTILE + (ks % 4) * 32;
-          umma_bf16(tmem_s, umma_desc_sw128(q_addr + qo), umma_desc_sw128(k_addr + ko), idesc_s, ks > 0 ? 1u : 0u);
-          umma_bf16(tmem_dp, umma_desc_sw128(do_addr + qo), umma_desc_sw128(v_addr + ko), idesc_s, ks > 0 ? 1u : 0u);
+          umma_bf16(tmem_base + h * 256, umma_desc_sw128(q_addr + qo), umma_desc_sw128(k_addr + ko), idesc_s, ks > 0 ? 1u : 0u);
+          umma_bf16(tmem_base + h * 256 + 64, umma_desc_sw128(do_addr + qo), umma_desc_sw128(v_addr + ko), idesc_s, ks > 0 ? 1u : 0u);
         }
-        umma_commit(s_full);
-        mbar_wait(ds_ready, i & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+        umma_commit(&s_full[h]);
+      };
+      auto block_here = [&](int i) {
+        mbar_wait(&kv_full[i % C::NSTAGE], (i / C::NSTAGE) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
         tc_fence_after();
+      };
+      if (total_blocks > 0) {
+        block_here(0);
+        for (int h = 0; h < NH; ++h) scores(0, h);
+      }
+      for (int i = 0; i < total_blocks; ++i) {
+        const uint32_t k_addr = smem_u32(kv_s + (i % C::NSTAGE) * C::STAGE_BYTES);
+        for (int h = 0; h < NH; ++h) {
+          // a head's threads have read its scores when they arrive here: the next block's follow its dQ product
+          mbar_wait(&ds_ready[h], i & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+          tc_fence_after();
 #pragma unroll
-        for (int ks = 0; ks < BK / 16; ++ks) {      // dQ += dS K, K consumed MN-major
-          const uint64_t db = umma_desc_mn_sw128(k_addr + ks * 2048, C::KTILE);
-          umma_bf16(tmem_dq, umma_desc_sw128(ds_addr + ks * 32), db, idesc_q, (i > 0 || ks > 0) ? 1u : 0u);
+          for (int ks = 0; ks < BK / 16; ++ks) {    // dQ += dS K, K consumed MN-major
+            const uint64_t db = umma_desc_mn_sw128(k_addr + ks * 2048, C::KTILE);
+            umma_bf16(tmem_base + h * 256 + 128, umma_desc_sw128(ds_addr + h * C::DS_BYTES + ks * 32), db, idesc_q,
+                      (i > 0 || ks > 0) ? 1u : 0u);
+          }
+          if (h == NH - 1) umma_commit(&kv_empty[i % C::NSTAGE]);
+          umma_commit(&dq_done[h]);
+          if (i + 1 < total_blocks) {
+            if (h == 0) block_here(i + 1);
+            scores(i + 1, h);
+          }
         }
-        umma_commit(kv_empty);
-        umma_commit(dq_done);
       }
     }
     __syncwarp();
   } else {
-    const int sw = warp - 2;
+    const int sw = (warp - 2) & 7, hi = (warp - 2) >> 3, head = head0 + hi;
     const int qd = warp & 3;
     const int half = sw >> 2;
+    const uint32_t tmem_s = tmem_base + hi * 256, tmem_dp = tmem_s + 64, tmem_dq = tmem_s + 128;
+    uint8_t* my_ds = ds_s + hi * C::DS_BYTES;
     const int row = qd * 32 + lane;
     const bool row_ok = row < qn;
     const uint32_t lane_off = static_cast<uint32_t>(qd * 32) << 16;
@@ -196,19 +222,18 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     for (int s = 0; s < p.n_seg; ++s) {
       const int cnt = row_ok ? p.seg_count[s][q0 + row] : 0;
       for (int b = 0; b < seg_blocks[s]; ++b, ++i) {
-        mbar_wait(s_full, i & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+        mbar_wait(&s_full[hi], i & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
         tc_fence_after();
         const int valid = cnt - b * BK - half * 32;
         float sv[32], dp[32];
         tmem_ld32(tmem_s + lane_off + half * 32, sv);
         tmem_ld32(tmem_dp + lane_off + half * 32, dp);
         tmem_ld_wait();
-        if (i > 0) mbar_wait(dq_done, (i - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
         const bool all_visible = __all_sync(0xffffffffu, valid >= 32);    // no masking inside this block
+        uint4 pk[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          uint4 pk;
-          __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&pk);
+          __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&pk[c]);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const int c0 = c * 8 + 2 * j;
@@ -220,15 +245,16 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             }
             p2[j] = __floats2bfloat162_rn(pa * fmaf(dp[c0], p.scale, -dsum_s), pb * fmaf(dp[c0 + 1], p.scale, -dsum_s));
           }
-          const int cc = half * 4 + c;
-          *reinterpret_cast<uint4*>(ds_s + row * 128 + ((cc ^ (row & 7)) << 4)) = pk;
         }
+        if (i > 0) mbar_wait(&dq_done[hi], (i - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4*>(my_ds + row * 128 + (((half * 4 + c) ^ (row & 7)) << 4)) = pk[c];
         fence_proxy_async_smem();
         tc_fence_before();
-        mbar_arrive(ds_ready);
+        mbar_arrive(&ds_ready[hi]);
       }
     }
-    if (total_blocks > 0) mbar_wait(dq_done, (total_blocks - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+    if (total_blocks > 0) mbar_wait(&dq_done[hi], (total_blocks - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
     tc_fence_after();
     __nv_bfloat16* dst = p.dq + ((size_t)(q0 + row) * p.nq + head) * HD + half * (HD / 2);
 #pragma unroll 1
@@ -305,7 +331,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int item = blockIdx.x, kvh = blockIdx.y;
+  const int item = blockIdx.x / p.nkv, kvh = blockIdx.x % p.nkv;      // the first key blocks are seen by the most queries
   const int G = p.nq / p.nkv;
   const int row0 = p.kv_row0[item], nkeys = p.kv_nkeys[item], kidx0 = p.kv_kidx0[item];
   const int qa = p.kv_qa[item], qb = p.kv_qb[item];
@@ -591,21 +617,24 @@ extern "C" int tahb_attn_bwd_dq(const void* q, const void* dout, void* dq, void*
   p.scale = scale;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = status;
-  dim3 grid(n_tiles, nq);
-#define TAHB_BQ(HD_)                                                                                            \
+  const bool two = (nq / nkv) % 2 == 0;
+#define TAHB_BQ(HD_, NH_)                                                                                       \
   {                                                                                                             \
+    using C = BwdQCfg<HD_, NH_>;                                                                                \
     static bool configured = false;                                                                             \
     if (!configured) {                                                                                          \
-      if (cudaFuncSetAttribute(attn_bwd_dq_kernel<HD_>, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
-                               BwdQCfg<HD_>::SMEM_BYTES) != cudaSuccess)                                        \
+      if (cudaFuncSetAttribute(attn_bwd_dq_kernel<HD_, NH_>, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
+                               C::SMEM_BYTES) != cudaSuccess)                                                   \
         return -10;                                                                                             \
       configured = true;                                                                                        \
     }                                                                                                           \
-    attn_bwd_dq_kernel<HD_><<<grid, BWD_THREADS, BwdQCfg<HD_>::SMEM_BYTES, stream>>>(mq, mdo, mk[0], mv[0], mk[1], \
-                                                                                     mv[1], mk[2], mv[2], p);   \
+    attn_bwd_dq_kernel<HD_, NH_><<<dim3(n_tiles * (nq / NH_)), C::THREADS, C::SMEM_BYTES, stream>>>(               \
+        mq, mdo, mk[0], mv[0], mk[1], mv[1], mk[2], mv[2], p);                                                  \
   }
-  if (hd == 128) TAHB_BQ(128)
-  else if (hd == 64) TAHB_BQ(64)
+  if (hd == 128 && two) TAHB_BQ(128, 2)
+  else if (hd == 128) TAHB_BQ(128, 1)
+  else if (hd == 64 && two) TAHB_BQ(64, 2)
+  else if (hd == 64) TAHB_BQ(64, 1)
   else return -2;
 #undef TAHB_BQ
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
@@ -639,7 +668,7 @@ extern "C" int tahb_attn_bwd_dkv(const void* q, const void* dout, const void* k,
   p.dk = reinterpret_cast<__nv_bfloat16*>(dk);
   p.dv = reinterpret_cast<__nv_bfloat16*>(dv);
   p.status = status;
-  dim3 grid(n_items, nkv);
+  dim3 grid(n_items * nkv);
 #define TAHB_BKV(HD_)                                                                                           \
   {                                                                                                             \
     static bool configured = false;                                                                             \

@@ -357,7 +357,7 @@ class SegmentMeta:
             self.bases.append(base[:, None].expand(B, Tq).reshape(-1).to(torch.int32).contiguous())
             self.counts.append(cnt.reshape(-1).to(torch.int32).contiguous())
             self.bounds.append(bound.reshape(-1).to(torch.int32).contiguous())
-            self.items.append(K.attn_kv_items(n_valid, base, q_rows))
+            self.items.append(K.attn_kv_items(n_valid, base, q_rows, by_work=True))
             self.seg_T.append(Ts)
 
 
