@@ -107,6 +107,53 @@ struct QkvPostParams {
   void* v_keep;               // [M, nkv * dv] or null
 };
 
+// Heads of 128 in bf16 without a rotation and without mixed values: a CTA per token, a warp takes four heads at a time with all loads in
+// flight, a lane four neighbouring dims.  Bound: HBM (7500 tokens of 16 + 16 heads: 61 MB in, 61 MB out, 18 us); the general kernel
+// below has one head per warp and loads of two bytes, 92 us there, this one 48 us.
+constexpr int QKVP_U = 4, QKVP_WARPS = 8;
+__global__ void __launch_bounds__(QKVP_WARPS * 32) qkv_post_128_kernel(const QkvPostParams p) {
+  pdl_launch_dependents();
+  pdl_wait();
+  constexpr int HD = 128;
+  const int heads = p.nq + 2 * p.nkv, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t = blockIdx.x, c = lane * 4;
+  const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(p.qkv) + (size_t)t * p.ld + c;
+  const int sl = p.nkv > 0 ? p.slot[t] : -1;
+  __nv_bfloat16* page = nullptr;
+  if (sl >= 0)
+    page = reinterpret_cast<__nv_bfloat16*>(p.cache) + ((size_t)(sl / p.page_size) * 2 * p.nkv * p.page_size + sl % p.page_size) * HD + c;
+  for (int h0 = warp; h0 < heads; h0 += QKVP_U * QKVP_WARPS) {
+    QkvPiece<4, true> in[QKVP_U];
+    float4 b[QKVP_U];
+#pragma unroll
+    for (int u = 0; u < QKVP_U; ++u) {
+      const int h = h0 + u * QKVP_WARPS;
+      if (h >= heads) continue;
+      in[u].load(src + (size_t)h * HD);
+      b[u] = p.bias != nullptr ? *reinterpret_cast<const float4*>(p.bias + h * HD + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < QKVP_U; ++u) {
+      const int h = h0 + u * QKVP_WARPS;
+      if (h >= heads) continue;
+      const bool is_q = h < p.nq, is_k = !is_q && h < p.nq + p.nkv;
+      float x[4] = {__bfloat162float(in[u].v[0]) + b[u].x, __bfloat162float(in[u].v[1]) + b[u].y,
+                    __bfloat162float(in[u].v[2]) + b[u].z, __bfloat162float(in[u].v[3]) + b[u].w};
+      const float* w = is_q ? p.q_w : is_k ? p.k_w : nullptr;
+      if (w != nullptr) {
+        const float r = 1.0f / sqrtf(warp_sum(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3]) / (float)p.dim + p.eps);
+        const float4 g = *reinterpret_cast<const float4*>(w + c);
+        x[0] *= r * g.x; x[1] *= r * g.y; x[2] *= r * g.z; x[3] *= r * g.w;
+      }
+      QkvPiece<4, true> out;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) out.v[i] = __float2bfloat16_rn(x[i]);
+      if (is_q) out.store(reinterpret_cast<__nv_bfloat16*>(p.q_out) + ((size_t)t * p.nq + h) * HD + c);
+      else if (page != nullptr) out.store(page + (size_t)(h - p.nq) * p.page_size * HD);
+    }
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(128) qkv_post_kernel(const QkvPostParams p) {
   pdl_launch_dependents();
@@ -612,12 +659,14 @@ __global__ void __launch_bounds__(128) window_decode_merge_kernel(const WindowAt
 
 // ---------------------------------------------------------------------------------------------
 // Portion kernel on the tensor cores (bf16, pages of 16): one CTA = a tile of up to 128 consecutive queries of one row
-// and one query head, walking the blocks of 64 keys that any of its queries sees (kept part, then window).  Same
-// structure as prefill_attn_kernel - S = Q K^T and O += P V by tcgen05 with S and O in tensor memory, two softmax
-// threads per query, lazily refreshed maximum, two-stage TMA ring - with K / V fetched page by page from the cache
+// and one or two query heads of a KV head, walking the blocks of 64 keys that any of its queries sees (kept part, then window).  Same
+// structure as prefill_attn_kernel - S = Q K^T and O += P V by tcgen05 with S (two buffers) and O in tensor memory, a softmax
+// thread per query, lazily refreshed maximum, TMA ring - with K / V fetched page by page from the cache
 // (four 16-row boxes per 64-key block form one swizzled tile; dims past dk / dv and pages past the last key read as
-// zeros) and with the distance bias added to the scores in registers.
-// Warp roles (320 threads): warp 0 TMA, warp 1 tensor memory + MMA, warps 2..9 softmax / epilogue.
+// zeros) and with the distance bias added to the scores in registers.  Two heads (an even number per KV head, dims up to 128) read a
+// block once and have four stages where two CTAs of one head have two each, whose latency then stands in every block.
+// 7500 tokens of 16 heads on 8 KV heads: 195 us with one head, 161 with two, 153 with the long tiles of all heads first.
+// Warp roles: warp 0 TMA, warp 1 tensor memory + MMA, four warps per head softmax / epilogue.
 // ---------------------------------------------------------------------------------------------
 struct WindowTiles {
   const int* q0;              // [n_tiles] first packed query
@@ -629,22 +678,23 @@ struct WindowTiles {
   int n_pool_pages;
 };
 
-// TIED: a stage holds keys only (and their factors, 64 floats behind all stages), which the second product reads too
-template <int HK, int HV, bool TIED = false>
+// TIED: a stage holds keys only (and their factors, 64 floats behind all stages), which the second product reads too.
+// NH: query heads of a CTA
+template <int HK, int HV, bool TIED, int NH>
 struct WpCfg {
   static constexpr int BK = 64;
   static constexpr int QTILE = 128 * 64 * 2, KTILE = BK * 64 * 2;
   static constexpr int Q_BYTES = HK * QTILE, K_BYTES = HK * KTILE, V_BYTES = HV * KTILE;
   static constexpr int P_BYTES = 128 * BK * 2;
   static constexpr int STAGE_BYTES = TIED ? K_BYTES : K_BYTES + V_BYTES;
-  static constexpr int NSTAGE = TIED ? 3 : 2;
+  static constexpr int NSTAGE = NH == 2 ? 4 : TIED ? 3 : 2;
   static constexpr int FACTOR_BYTES = TIED ? NSTAGE * BK * 4 : 0;
-  static constexpr int SMEM_BYTES = Q_BYTES + P_BYTES + NSTAGE * STAGE_BYTES + FACTOR_BYTES + 128;
-  static constexpr int XCOL = 64;                            // exchange columns between the two halves of a query
-  static constexpr int TMEM_COLS = HV <= 2 ? 256 : 512;      // S at 0, O at 128
-  static constexpr int MIN_CTAS = HK + HV <= 4 ? 2 : 1;
+  static constexpr int SMEM_BYTES = NH * (Q_BYTES + P_BYTES) + NSTAGE * STAGE_BYTES + FACTOR_BYTES + 192;
+  static constexpr int O_COL = NH * 128;                     // of every head: S, 2 x 64 columns; behind all of them O
+  static constexpr int TMEM_COLS = NH == 1 && HV <= 2 ? 256 : 512;
+  static constexpr int MIN_CTAS = NH == 1 && HK + HV <= 4 ? 2 : 1;
+  static constexpr int THREADS = 64 + NH * 128;
 };
-constexpr int WP_THREADS = 320;
 
 // cap * tanh(mul * v) of 32 scores of a thread.  The arguments of trained attention mostly lie well inside (-1, 1), where
 // x P(x^2) with a degree-5 minimax P (fitted for the absolute error, 3.3e-7 in fp32) needs no special-function unit, the
@@ -690,30 +740,31 @@ __device__ __forceinline__ void soft_cap32(float* v, float mul, float cap) {
 }
 
 // TIED: tm_v describes the matrix of pooled blocks (or is unused), whose blocks come first
-template <int HK, int HV, bool CAP, bool TIED>
-__global__ void __launch_bounds__(WP_THREADS, WpCfg<HK, HV, TIED>::MIN_CTAS)
+template <int HK, int HV, bool CAP, bool TIED, int NH>
+__global__ void __launch_bounds__(WpCfg<HK, HV, TIED, NH>::THREADS, WpCfg<HK, HV, TIED, NH>::MIN_CTAS)
 window_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                       const __grid_constant__ CUtensorMap tm_v, const WindowAttnParams p, const WindowTiles tl) {
-  using C = WpCfg<HK, HV, TIED>;
+  using C = WpCfg<HK, HV, TIED, NH>;
   constexpr int BK = C::BK;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* q_s = smem;
-  uint8_t* p_s = q_s + C::Q_BYTES;
-  uint8_t* kv_s = p_s + C::P_BYTES;
+  uint8_t* p_s = q_s + NH * C::Q_BYTES;
+  uint8_t* kv_s = p_s + NH * C::P_BYTES;
   float* factor_s = reinterpret_cast<float*>(kv_s + C::NSTAGE * C::STAGE_BYTES);      // [NSTAGE][BK], tied
   uint64_t* bars = reinterpret_cast<uint64_t*>(kv_s + C::NSTAGE * C::STAGE_BYTES + C::FACTOR_BYTES);
   uint64_t* q_full = bars;
   uint64_t* kv_full = bars + 1;
   uint64_t* kv_empty = kv_full + C::NSTAGE;
   uint64_t* s_full = kv_empty + C::NSTAGE;
-  uint64_t* p_ready = s_full + 1;
-  uint64_t* pv_done = p_ready + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 1);
+  uint64_t* p_ready = s_full + 2 * NH;          // s_full: [NH][2], p_ready and pv_done: [NH]
+  uint64_t* pv_done = p_ready + NH;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + NH);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tile = blockIdx.x, head = blockIdx.y;
-  const int kvh = head / (p.nq / p.nkv);
+  // the last tiles of a portion walk the most keys: all heads of them first, so that the short ones fill the last wave
+  const int n_hg = p.nq / NH, tile = gridDim.x / n_hg - 1 - blockIdx.x / n_hg, head0 = blockIdx.x % n_hg * NH;
+  const int kvh = head0 / (p.nq / p.nkv);
   if ((smem_u32(smem) & 1023u) != 0) {          // the swizzled tiles need a 1024-byte aligned base
     if (threadIdx.x == 0) atomicCAS(p.status, 0, STATUS_BAD_INDEX);
     return;
@@ -721,9 +772,12 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int s = 0; s < C::NSTAGE; ++s) { mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 1); }
-    mbar_init(s_full, 1);
-    mbar_init(p_ready, 256);
-    mbar_init(pv_done, 1);
+    for (int h = 0; h < NH; ++h) {
+      mbar_init(&s_full[2 * h], 1);
+      mbar_init(&s_full[2 * h + 1], 1);
+      mbar_init(&p_ready[h], 128);
+      mbar_init(&pv_done[h], 1);
+    }
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -735,7 +789,7 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + 128;
+  const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + C::O_COL;
 
   const int q0 = tl.q0[tile], qn = tl.qn[tile];
   const int i0 = p.pos[q0], i_last = i0 + qn - 1;             // the tile's positions are consecutive
@@ -749,9 +803,9 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
-      mbar_expect_tx(q_full, C::Q_BYTES);
+      mbar_expect_tx(q_full, NH * C::Q_BYTES);
 #pragma unroll
-      for (int h = 0; h < HK; ++h) tma_load_2d(q_s + h * C::QTILE, &tm_q, head * p.dk + h * 64, q0, q_full);
+      for (int h = 0; h < NH * HK; ++h) tma_load_2d(q_s + h * C::QTILE, &tm_q, (head0 + h / HK) * p.dk + h % HK * 64, q0, q_full);
       const int* pt = p.page_table + (size_t)p.row[q0] * p.max_pages;
       const int last_page = i_last / WD_PAGE, pool0 = pooled ? tl.pool_base[tile] : 0;
       for (int n = 0; n < total_blocks; ++n) {
@@ -796,33 +850,46 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       constexpr uint32_t idesc_o = umma_idesc_bf16_bmn(128, HV * 64);
       mbar_wait(q_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
       const uint32_t q_addr = smem_u32(q_s), p_addr = smem_u32(p_s);
-      for (int n = 0; n < total_blocks; ++n) {
+      auto scores = [&](int n) {
         const int st = n % C::NSTAGE;
         mbar_wait(&kv_full[st], (n / C::NSTAGE) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
         tc_fence_after();
         const uint32_t k_addr = smem_u32(kv_s + st * C::STAGE_BYTES);
-        const uint32_t v_addr = TIED ? k_addr : k_addr + C::K_BYTES;
 #pragma unroll
-        for (int ks = 0; ks < HK * 4; ++ks) {
-          const uint32_t qo = (ks / 4) * C::QTILE + (ks % 4) * 32;
-          const uint32_t ko = (ks / 4) * C::KTILE + (ks % 4) * 32;
-          umma_bf16(tmem_s, umma_desc_sw128(q_addr + qo), umma_desc_sw128(k_addr + ko), idesc_s, ks > 0 ? 1u : 0u);
+        for (int h = 0; h < NH; ++h) {
+#pragma unroll
+          for (int ks = 0; ks < HK * 4; ++ks) {
+            const uint32_t qo = h * C::Q_BYTES + (ks / 4) * C::QTILE + (ks % 4) * 32;
+            const uint32_t ko = (ks / 4) * C::KTILE + (ks % 4) * 32;
+            umma_bf16(tmem_s + h * 128 + (n & 1) * BK, umma_desc_sw128(q_addr + qo), umma_desc_sw128(k_addr + ko), idesc_s, ks > 0 ? 1u : 0u);
+          }
+          umma_commit(&s_full[2 * h + (n & 1)]);
         }
-        umma_commit(s_full);
-        mbar_wait(p_ready, n & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
-        tc_fence_after();
+      };
+      if (total_blocks > 0) scores(0);
+      for (int n = 0; n < total_blocks; ++n) {
+        if (n + 1 < total_blocks) scores(n + 1);        // its buffer's last reader arrived at p_ready for block n - 1
+        const int st = n % C::NSTAGE;
+        const uint32_t v_addr = smem_u32(kv_s + st * C::STAGE_BYTES) + (TIED ? 0 : C::K_BYTES);
 #pragma unroll
-        for (int ks = 0; ks < BK / 16; ++ks)
-          umma_bf16(tmem_o, umma_desc_sw128(p_addr + ks * 32), umma_desc_mn_sw128(v_addr + ks * 2048, C::KTILE), idesc_o,
-                    (n > 0 || ks > 0) ? 1u : 0u);
-        umma_commit(&kv_empty[st]);
-        umma_commit(pv_done);
+        for (int h = 0; h < NH; ++h) {
+          mbar_wait(&p_ready[h], n & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+          tc_fence_after();
+#pragma unroll
+          for (int ks = 0; ks < BK / 16; ++ks)
+            umma_bf16(tmem_o + h * 128, umma_desc_sw128(p_addr + h * C::P_BYTES + ks * 32), umma_desc_mn_sw128(v_addr + ks * 2048, C::KTILE),
+                      idesc_o, (n > 0 || ks > 0) ? 1u : 0u);
+          if (h == NH - 1) umma_commit(&kv_empty[st]);
+          umma_commit(&pv_done[h]);
+        }
       }
     }
     __syncwarp();
   } else {
-    // ---------------- softmax / epilogue: two threads per query, 32 key columns each ----------------
-    const int qd = warp & 3, half = (warp - 2) >> 2;
+    // ---------------- softmax / epilogue: a thread per query, two patches of 32 key columns ----------------
+    const int qd = warp & 3, hi = (warp - 2) >> 2, head = head0 + hi;
+    const uint32_t my_s = tmem_s + hi * 128, my_o = tmem_o + hi * 128;
+    uint8_t* my_p = p_s + hi * C::P_BYTES;
     const int row = qd * 32 + lane;
     const bool row_ok = row < qn;
     const uint32_t lane_off = static_cast<uint32_t>(qd * 32) << 16;
@@ -838,122 +905,112 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const int blocks = pooled ? visible_blocks(i, p.window, p.pool) : 0;
     float m_ref = -INFINITY, l = 0.f;
     for (int n = 0; n < total_blocks; ++n) {
-      const int j0 = (n < kb ? n : w0 + n - kb) * BK + half * 32;        // first key column of this thread
-      mbar_wait(s_full, n & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+      mbar_wait(&s_full[2 * hi + (n & 1)], (n >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
       tc_fence_after();
-      float sv[32];
-      tmem_ld32(tmem_s + lane_off + half * 32, sv);
+      float sc64[BK];
+      tmem_ld32(my_s + lane_off + (n & 1) * BK, sc64);
+      tmem_ld32(my_s + lane_off + (n & 1) * BK + 32, sc64 + 32);
       tmem_ld_wait();
-      const int dmin = iw0 - (j0 + 31), dmax = iw1 - j0;                 // distances inside the warp's 32 x 32 patch
       const bool means = pooled && n < kb;
-      if constexpr (CAP) soft_cap32(sv, cap_mul, cap);
-      if constexpr (TIED) {
-        if (p.factor != nullptr && !means) {
-          const int st = n % C::NSTAGE;
-          mbar_wait(&kv_full[st], (n / C::NSTAGE) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
-          const float4* f4 = reinterpret_cast<const float4*>(factor_s + st * BK + half * 32);
+      float mx = -INFINITY;
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const float4 f = f4[c];
-            sv[4 * c] *= f.x; sv[4 * c + 1] *= f.y; sv[4 * c + 2] *= f.z; sv[4 * c + 3] *= f.w;
+      for (int half = 0; half < 2; ++half) {
+        float* sv = sc64 + half * 32;
+        const int j0 = (n < kb ? n : w0 + n - kb) * BK + half * 32;        // first key column of the patch
+        const int dmin = iw0 - (j0 + 31), dmax = iw1 - j0;                 // distances inside the warp's 32 x 32 patch
+        if constexpr (CAP) soft_cap32(sv, cap_mul, cap);
+        if constexpr (TIED) {
+          if (p.factor != nullptr && !means) {
+            const int st = n % C::NSTAGE;
+            mbar_wait(&kv_full[st], (n / C::NSTAGE) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
+            const float4* f4 = reinterpret_cast<const float4*>(factor_s + st * BK + half * 32);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+              const float4 f = f4[c];
+              sv[4 * c] *= f.x; sv[4 * c + 1] *= f.y; sv[4 * c + 2] *= f.z; sv[4 * c + 3] *= f.w;
+            }
           }
         }
-      }
-      if (p.slope != nullptr) {
-        const float d0 = -slope * (float)(i - j0);
+        if (p.slope != nullptr) {
+          const float d0 = -slope * (float)(i - j0);
 #pragma unroll
-        for (int c = 0; c < 32; ++c) sv[c] = fmaf(sv[c], sc, fmaf(slope, (float)c, d0));
-      } else if (CAP && bias == nullptr) {
-      } else if (bias == nullptr || dmin >= p.far) {
+          for (int c = 0; c < 32; ++c) sv[c] = fmaf(sv[c], sc, fmaf(slope, (float)c, d0));
+        } else if (CAP && bias == nullptr) {
+        } else if (bias == nullptr || dmin >= p.far) {
 #pragma unroll
-        for (int c = 0; c < 32; ++c) sv[c] = fmaf(sv[c], sc, far_bias);
-      } else if (dmin >= 0 && dmax <= p.far) {
-        const float* b = bias + (i - j0);
+          for (int c = 0; c < 32; ++c) sv[c] = fmaf(sv[c], sc, far_bias);
+        } else if (dmin >= 0 && dmax <= p.far) {
+          const float* b = bias + (i - j0);
 #pragma unroll
-        for (int c = 0; c < 32; ++c) sv[c] = fmaf(sv[c], sc, __ldg(b - c));
-      } else {
+          for (int c = 0; c < 32; ++c) sv[c] = fmaf(sv[c], sc, __ldg(b - c));
+        } else {
 #pragma unroll
-        for (int c = 0; c < 32; ++c) sv[c] = fmaf(sv[c], sc, __ldg(bias + min(max(i - j0 - c, 0), p.far)));
-      }
-      if (means) {
-#pragma unroll
-        for (int c = 0; c < 32; ++c)
-          if (j0 + c >= blocks) sv[c] = -INFINITY;
-      } else if (!(dmin >= 0 && (j0 >= lo_w1 || j0 + 31 < p.keep_first))) {
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          const int j = j0 + c;
-          if (j > i || (j < lo && j >= p.keep_first)) sv[c] = -INFINITY;
+          for (int c = 0; c < 32; ++c) sv[c] = fmaf(sv[c], sc, __ldg(bias + min(max(i - j0 - c, 0), p.far)));
         }
-      }
-      float mx = sv[0];
+        if (means) {
 #pragma unroll
-      for (int c = 1; c < 32; ++c) mx = fmaxf(mx, sv[c]);
-      const uint32_t xcol = tmem_base + lane_off + C::XCOL + (n & 1) * 2;
-      tmem_st1(xcol + half, mx);
-      tmem_st_wait();
-      tc_fence_before();
-      named_bar_sync(1, 256);
-      tc_fence_after();
-      mx = fmaxf(mx, tmem_ld1(xcol + (half ^ 1)));
+          for (int c = 0; c < 32; ++c)
+            if (j0 + c >= blocks) sv[c] = -INFINITY;
+        } else if (!(dmin >= 0 && (j0 >= lo_w1 || j0 + 31 < p.keep_first))) {
+#pragma unroll
+          for (int c = 0; c < 32; ++c) {
+            const int j = j0 + c;
+            if (j > i || (j < lo && j >= p.keep_first)) sv[c] = -INFINITY;
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 32; ++c) mx = fmaxf(mx, sv[c]);
+      }
       const bool grow = mx > m_ref + 8.0f;
       const float m_new = grow ? mx : m_ref;
       const float f = (grow && m_ref != -INFINITY) ? exp2f(m_ref - m_new) : 1.0f;
-      if (n > 0) mbar_wait(pv_done, (n - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
-      tc_fence_after();
-      if (n > 0 && __any_sync(0xffffffffu, f != 1.0f)) {
-#pragma unroll 1
-        for (int c = 0; c < HV * 32; c += 32) {
-          float o[32];
-          tmem_ld32(tmem_o + lane_off + half * (HV * 32) + c, o);
-          tmem_ld_wait();
-#pragma unroll
-          for (int e = 0; e < 32; ++e) o[e] *= f;
-          tmem_st32(tmem_o + lane_off + half * (HV * 32) + c, o);
-        }
-        tmem_st_wait();
-      }
       l *= f;
       m_ref = m_new;
       const float neg_m = (m_ref == -INFINITY) ? 0.f : -m_ref;
       float ps0 = 0.f, ps1 = 0.f;
+      uint4 pk[BK / 8];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint4 pk;
-        __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&pk);
+      for (int c = 0; c < BK / 8; ++c) {
+        __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&pk[c]);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float a = ex2_approx(sv[c * 8 + 2 * e] + neg_m);
-          const float b = ex2_approx(sv[c * 8 + 2 * e + 1] + neg_m);
+          const float a = ex2_approx(sc64[c * 8 + 2 * e] + neg_m);
+          const float b = ex2_approx(sc64[c * 8 + 2 * e + 1] + neg_m);
           p2[e] = __floats2bfloat162_rn(a, b);
           ps0 += a;
           ps1 += b;
         }
-        *reinterpret_cast<uint4*>(p_s + row * 128 + (((half * 4 + c) ^ (row & 7)) << 4)) = pk;
       }
       l += ps0 + ps1;
+      // the product of the block before reads P and writes O
+      if (n > 0) mbar_wait(&pv_done[hi], (n - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+      tc_fence_after();
+      if (n > 0 && __any_sync(0xffffffffu, f != 1.0f)) {
+#pragma unroll 1
+        for (int c = 0; c < HV * 64; c += 32) {
+          float o[32];
+          tmem_ld32(my_o + lane_off + c, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 32; ++e) o[e] *= f;
+          tmem_st32(my_o + lane_off + c, o);
+        }
+        tmem_st_wait();
+      }
+#pragma unroll
+      for (int c = 0; c < BK / 8; ++c) *reinterpret_cast<uint4*>(my_p + row * 128 + ((c ^ (row & 7)) << 4)) = pk[c];
       fence_proxy_async_smem();
       tc_fence_before();
-      mbar_arrive(p_ready);
+      mbar_arrive(&p_ready[hi]);
     }
-    if (total_blocks > 0) mbar_wait(pv_done, (total_blocks - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+    if (total_blocks > 0) mbar_wait(&pv_done[hi], (total_blocks - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
     tc_fence_after();
-    {
-      const uint32_t xcol = tmem_base + lane_off + C::XCOL;
-      named_bar_sync(1, 256);
-      tmem_st1(xcol + half, l);
-      tmem_st_wait();
-      tc_fence_before();
-      named_bar_sync(1, 256);
-      tc_fence_after();
-      l += tmem_ld1(xcol + (half ^ 1));
-    }
     const float inv = row_ok ? finish_scale(p, q0 + row, head, m_ref, l) : 0.f;
     __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)(q0 + row) * p.ld_out + (size_t)head * p.dv;
 #pragma unroll 1
-    for (int c = half * (HV * 32); c < (half + 1) * (HV * 32); c += 32) {
+    for (int c = 0; c < HV * 64; c += 32) {
       float o[32];
-      tmem_ld32(tmem_o + lane_off + c, o);
+      tmem_ld32(my_o + lane_off + c, o);
       tmem_ld_wait();
       if (row_ok) {
 #pragma unroll
@@ -1013,18 +1070,27 @@ static int launch_window_decode(const WindowAttnParams& p, cudaStream_t stream) 
   return exact ? launch_window_decode_as<VEC, GB, true, false>(p, stream) : launch_window_decode_as<VEC, GB, false, false>(p, stream);
 }
 
-template <int HK, int HV, bool CAP, bool TIED = false>
-static int launch_window_prefill_as(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
-                                 const WindowAttnParams& p, const WindowTiles& tl, int n_tiles, cudaStream_t stream) {
+template <int HK, int HV, bool CAP, bool TIED, int NH>
+static int launch_window_prefill_heads(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+                                       const WindowAttnParams& p, const WindowTiles& tl, int n_tiles, cudaStream_t stream) {
+  using C = WpCfg<HK, HV, TIED, NH>;
+  auto kern = window_prefill_kernel<HK, HV, CAP, TIED, NH>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(window_prefill_kernel<HK, HV, CAP, TIED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             WpCfg<HK, HV, TIED>::SMEM_BYTES) != cudaSuccess)
-      return -10;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES) != cudaSuccess) return -10;
     configured = true;
   }
-  window_prefill_kernel<HK, HV, CAP, TIED><<<dim3(n_tiles, p.nq), WP_THREADS, WpCfg<HK, HV, TIED>::SMEM_BYTES, stream>>>(mq, mk, mv, p, tl);
+  kern<<<dim3(n_tiles * (p.nq / NH)), C::THREADS, C::SMEM_BYTES, stream>>>(mq, mk, mv, p, tl);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+template <int HK, int HV, bool CAP, bool TIED = false>
+static int launch_window_prefill_as(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+                                    const WindowAttnParams& p, const WindowTiles& tl, int n_tiles, cudaStream_t stream) {
+  if constexpr (HK <= 2 && HV <= 2) {
+    if ((p.nq / p.nkv) % 2 == 0) return launch_window_prefill_heads<HK, HV, CAP, TIED, 2>(mq, mk, mv, p, tl, n_tiles, stream);
+  }
+  return launch_window_prefill_heads<HK, HV, CAP, TIED, 1>(mq, mk, mv, p, tl, n_tiles, stream);
 }
 
 template <int HK, int HV>
@@ -1086,6 +1152,11 @@ extern "C" int tahb_qkv_post(const QkvPostParams* q, int f32, cudaStream_t strea
   if (p.dk > 256 || p.dv > 256 || p.dk % 8 || p.dv % 8 || p.dim > p.dk) return -2;
   if (p.rope != nullptr && (p.rot % 2 || p.rot < 2 || p.rot > p.dim)) return -2;
   if (p.v_first != nullptr && p.lambda == nullptr) return -2;
+  const uintptr_t wide = reinterpret_cast<uintptr_t>(p.qkv) | reinterpret_cast<uintptr_t>(p.q_out) | reinterpret_cast<uintptr_t>(p.cache) |
+                         (uintptr_t)(p.ld * 2);
+  const uintptr_t full = reinterpret_cast<uintptr_t>(p.bias) | reinterpret_cast<uintptr_t>(p.q_w) | reinterpret_cast<uintptr_t>(p.k_w);
+  if (!f32 && p.dk == 128 && p.dv == 128 && p.rope == nullptr && p.v_first == nullptr && p.v_keep == nullptr && wide % 8 == 0 && full % 16 == 0)
+    return launch_chain(qkv_post_128_kernel, dim3(p.M), dim3(QKVP_WARPS * 32), 0, stream, p) == cudaSuccess ? 0 : -3;
   const long long warps = (long long)p.M * (p.nq + 2 * p.nkv);
   const dim3 grid((unsigned)((warps + 3) / 4));
   cudaError_t e = f32 ? launch_chain(qkv_post_kernel<float>, grid, dim3(128), 0, stream, p)

@@ -575,3 +575,29 @@ def test_playground_command_line_and_evaluation_backend(tmp_path):
     for rows_n in (1, 2):
         got = infer.serve_all([Ids.decode(p) for p in prompts], rows_n)
         assert [Ids.encode(t) for t, _ in got] == rows
+
+
+@pytest.mark.parametrize("nq,nkv", [(16, 8), (40, 8), (6, 0), (0, 3)])
+@pytest.mark.parametrize("norm", [True, False])
+def test_qkv_post_heads_of_128(nq, nkv, norm):
+    """The form for heads of 128 against the general one (which a row pitch off the wide accesses' boundary selects): the same values up to
+    one rounding to bf16, since the norm's 32-bit sum has another order."""
+    from tah_b200.ops import cuda as K
+    M, hd, page = 7, 128, 16
+    g = torch.Generator(device="cuda").manual_seed(nq)
+    F = (nq + 2 * nkv) * hd
+    base = torch.randn(M, F, generator=g, device="cuda").bfloat16()
+    bias = torch.randn(F, generator=g, device="cuda")
+    qw, kw = (torch.randn(hd, generator=g, device="cuda") if norm else None for _ in range(2))
+    slot = torch.tensor([0, 5, 16, 31, -1, 40, 47], dtype=torch.int32, device="cuda")
+    got = []
+    for pitch in (F, F + 2):
+        x = torch.zeros(M, pitch, dtype=torch.bfloat16, device="cuda")
+        x[:, :F] = base
+        q = torch.zeros(M, max(1, nq) * hd, dtype=torch.bfloat16, device="cuda")
+        cache = torch.zeros(3, 2 * max(1, nkv) * page * hd, dtype=torch.bfloat16, device="cuda")
+        K.qkv_post(x[:, :F], bias, qw, kw, q if nq else None, cache, slot, nq, nkv, hd, hd, hd, page, 1e-6)
+        got.append((q, cache))
+    for a, b in zip(*got):
+        torch.testing.assert_close(a.float(), b.float(), rtol=2.0 ** -7, atol=1e-30)
+    assert (nkv == 0) == bool((got[0][1] == 0).all())
