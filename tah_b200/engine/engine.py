@@ -229,6 +229,21 @@ class TaHEngine(DecodeEngine):
         fuse_qkv = hd == 128 and "qkv" in _fusions("")
         if tensor_core_attn:
             tile_q0, tile_qn = K.attn_tiles(seq_counts, by_work=True)
+        if tp is None and tensor_core_attn and not fuse_qkv and w.pass_weights is not None and (lora or depth == 0 or w.r == 0):
+            # the plain form on one GPU: every launch of the pass from one native call
+            kv = bf(nL, 2, n, nkv * hd)
+            own = [(kv[li, 0], kv[li, 1]) for li in range(nL)]
+            taps = None if taps_out is None else {li: bf(n, cfg.hidden_size) for li in tap_layers if li < nL}
+            K.packed_pass(w.pass_weights, w.final_norm, h, xn_buf, [self.kv.layer_pool(depth, li) for li in range(nL)], [k for k, _ in own],
+                          [v for _, v in own], seg_k, seg_v, seg_base, seg_count, pos, slots, tile_q0, tile_qn, nq=nq, nkv=nkv, hd=hd,
+                          inter=w.inter, ranks=(w.r_qkv, w.r_o, w.r_gu, w.r_down) if lora else (0, 0, 0, 0),
+                          gu_interleaved=w.gu_interleaved, page_size=self.page_size, eps=cfg.rms_norm_eps, theta=cfg.rope_theta, scale=scale,
+                          taps=taps)
+            if taps_out is not None:
+                taps_out.update(taps)
+                if nL in tap_layers:
+                    taps_out[nL] = xn_buf
+            return xn_buf, own
         rope_cs = K.rope_table(pos, hd, cfg.rope_theta) if fuse_qkv else None     # once per pass, shared by the layers
         # tensor parallel: token counts that deal out in 16-row blocks take the push path (reduce-scatter in the
         # GEMM epilogue, consumers wait on landing flags), the others the pull kernel

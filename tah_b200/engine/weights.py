@@ -135,6 +135,7 @@ class EngineWeights:
                     lw.b_gu = K.interleave_gate_up(lw.b_gu)
             lw.a_down, lw.b_down = _lora_pair(mlp.down_proj, cols=d_cols)
             self.layers.append(lw)
+        self.pass_weights = K.pass_weights(self.layers)      # None: the layers' launches come one by one
         l0 = self.layers[0]
         width = lambda a: 0 if a is None else a.shape[0]
         self.r_qkv, self.r_o, self.r_gu, self.r_down = width(l0.a_qkv), width(l0.a_o), width(l0.a_gu), width(l0.a_down)

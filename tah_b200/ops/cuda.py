@@ -1390,6 +1390,93 @@ def prefill_attn(q, ks, vs, bases, counts, tile_q0, tile_qn, nq, nkv, hd, scale,
     return out
 
 
+class _ProductPlan(ctypes.Structure):
+    _fields_ = [(f, c_int) for f in ("few", "dual", "splits", "bn")]
+
+
+class _PassWeights(ctypes.Structure):
+    _fields_ = [(f, c_void_p) for f in ("ln1", "ln2", "q_norm", "k_norm", "w_qkv", "w_o", "w_gu", "w_down", "a_qkv", "b_qkv", "a_o", "b_o",
+                                        "a_gu", "b_gu", "a_down", "b_down")]
+
+
+_VP = ctypes.POINTER(c_void_p)
+
+
+class _Pass(ctypes.Structure):
+    _fields_ = [("layers", ctypes.POINTER(_PassWeights))] + \
+        [(f, c_void_p) for f in ("final_norm", "h", "xn", "qkv", "q", "o", "act", "t_qkv", "t_o", "t_gu", "t_down")] + \
+        [(f, _VP) for f in ("taps", "k_own", "v_own", "pool")] + \
+        [("k_seg", _VP * 3), ("v_seg", _VP * 3), ("n_kv", c_ll * 3), ("base", c_void_p * 3), ("count", c_void_p * 3)] + \
+        [(f, c_void_p) for f in ("pos", "slots", "tile_q0", "tile_qn", "status")] + \
+        [(f, c_int) for f in ("n_layers", "n", "hidden", "inter", "nq", "nkv", "hd", "page_size", "n_seg", "n_tiles", "gu_dual", "r_qkv",
+                              "r_o", "r_gu", "r_down")] + \
+        [(f, c_float) for f in ("eps", "theta", "scale")] + \
+        [(f, _ProductPlan) for f in ("p_qkv", "p_o", "p_gu", "p_down", "p_a_qkv", "p_a_o", "p_a_gu", "p_a_down")]
+
+
+def pass_weights(layers):
+    """The layers' weights as :func:`packed_pass` takes them, or None when one does not lie on a 16-byte boundary in contiguous rows.
+    Like a captured tick it stands for these tensors, and keeps them alive."""
+    arr = (_PassWeights * len(layers))()
+    arr.tensors = []
+    for a, l in zip(arr, layers):
+        for f, _ in _PassWeights._fields_:
+            t = getattr(l, f)
+            if t is not None and (t.data_ptr() % 16 or not t.is_contiguous() or t.shape[-1] % 8):
+                return None
+            setattr(a, f, 0 if t is None else t.data_ptr())
+            arr.tensors.append(t)
+    return arr
+
+
+def packed_pass(weights, final_norm, h, xn, pools, k_own, v_own, seg_k, seg_v, bases, counts, pos, slots, tile_q0, tile_qn, *, nq: int, nkv: int,
+                hd: int, inter: int, ranks: Sequence[int], gu_interleaved: bool, page_size: int, eps: float, theta: float, scale: float,
+                taps=None):
+    """All layers of a pass over the packed tokens ``h [n, H]`` (updated in place) in one call (``csrc/packed_pass.cu``); the final norm's
+    output goes to ``xn``.  ``k_own`` / ``v_own``: per layer, this pass's keys and values; ``seg_k`` / ``seg_v``: those of the shallower
+    passes; ``ranks``: adapter widths of qkv, o, gate / up and down, zeros without it; ``taps``: layer -> buffer for its input."""
+    global launch_count
+    if len(bases) > 3:
+        raise RuntimeError("tahb_packed_pass failed on the host side (more than three passes deep)")
+    n, H = h.shape
+    L, D = len(k_own), nq * hd
+    bf = lambda cols: torch.empty(n, cols, dtype=torch.bfloat16, device=h.device) if cols else None
+    bufs = dict(qkv=bf((nq + 2 * nkv) * hd), q=bf(D), o=bf(D), act=bf(inter), t_qkv=bf(ranks[0]), t_o=bf(ranks[1]), t_gu=bf(ranks[2]),
+                t_down=bf(ranks[3]))
+    a = _Pass()
+    a.layers = weights
+    a.final_norm, a.h, a.xn = final_norm.data_ptr(), h.data_ptr(), xn.data_ptr()
+    for f, t in bufs.items():
+        setattr(a, f, 0 if t is None else t.data_ptr())
+    a.taps = (c_void_p * (L + 1))(*[0 if taps is None or i not in taps else taps[i].data_ptr() for i in range(L + 1)])
+    a.k_own, a.v_own, a.pool = _ptr_array(k_own), _ptr_array(v_own), _ptr_array(pools)
+    for s, (ks, vs) in enumerate(zip(seg_k, seg_v)):
+        a.k_seg[s], a.v_seg[s], a.n_kv[s] = _ptr_array(ks), _ptr_array(vs), ks[0].shape[0]
+    a.n_kv[len(seg_k)] = n
+    for s, (b, c) in enumerate(zip(bases, counts)):
+        a.base[s], a.count[s] = b.data_ptr(), c.data_ptr()
+    a.pos, a.slots, a.tile_q0, a.tile_qn = pos.data_ptr(), slots.data_ptr(), tile_q0.data_ptr(), tile_qn.data_ptr()
+    a.status = status_word(h.device).data_ptr()
+    a.n_layers, a.n, a.hidden, a.inter, a.nq, a.nkv, a.hd, a.page_size = L, n, H, inter, nq, nkv, hd, page_size
+    a.n_seg, a.n_tiles, a.gu_dual = len(bases), tile_q0.numel(), 0 if gu_interleaved else 1
+    a.r_qkv, a.r_o, a.r_gu, a.r_down = ranks
+    a.eps, a.theta, a.scale = eps, theta, scale
+
+    def plan(rows, K, R=0, glu=False):
+        stacked, il = glu and not gu_interleaved, glu and gu_interleaved
+        if few_shape(n, rows, K, R):
+            return _ProductPlan(1, 4 if il else 1 if stacked else 0, 1, 0)
+        pair, bn, splits = _plan_tiles(n, rows, K, R, stacked, False, il)
+        return _ProductPlan(0, 1 if stacked else (6 if pair else 4) if il else 2 if pair else 0, splits, bn)
+
+    a.p_qkv, a.p_o = plan((nq + 2 * nkv) * hd, H, ranks[0]), plan(H, D, ranks[1])
+    a.p_gu, a.p_down = plan(2 * inter, H, ranks[2], glu=True), plan(H, inter, ranks[3])
+    a.p_a_qkv, a.p_a_o, a.p_a_gu, a.p_a_down = plan(ranks[0], H), plan(ranks[1], D), plan(ranks[2], H), plan(ranks[3], inter)
+    launches = c_int(0)
+    _rc(lib().tahb_packed_pass(ctypes.byref(a), ctypes.byref(launches), _stream()), "tahb_packed_pass")
+    launch_count += launches.value - 1
+
+
 def attn_kv_items(seq_kv_counts: torch.Tensor, seq_kv_base: torch.Tensor, seq_q_counts: torch.Tensor, block: int = 128,
                   by_work: bool = False):
     """Work items of :func:`attn_bwd_dkv` for one KV segment: every sequence's ``seq_kv_counts[b]`` keys
