@@ -37,7 +37,7 @@ from tah_b200.utils.observe import nvtx_range
 def _fusions(default: str):
     """Kernel fusions selected by ``TAH_B200_FUSE``: "1" = all, "0" = none, or a comma list of "qkv" (QK-norm, RoPE
     and the K/V write in the QKV GEMM's epilogue) and "lora" (LoRA-A of the gated rows inside the RMSNorm launch);
-    unset = ``default`` (nothing: the chains of separate launches measured faster in decode and in prefill)."""
+    unset = ``default`` ("lora" in ticks of up to eight rows, else nothing)."""
     v = os.environ.get("TAH_B200_FUSE", default)
     if v == "1":
         return {"qkv", "lora"}
@@ -526,9 +526,10 @@ class TaHEngine(DecodeEngine):
         tl = self._tap_layers()
         H = cfg.hidden_size
         nL = len(w.layers)
-        # Optional fusions of the decode chain.  Off by default: at 256 rows the chain of separate launches measured
-        # 1.7 % faster per tick than the fused kernels (whose extra work runs on four epilogue warps per CTA).
-        fuse = _fusions("")
+        # Optional fusions of the decode chain.  RMSNorm and LoRA-A in one launch pays while launches are what a tick is made of (1 row:
+        # 1.49 -> 1.35 ms, 6 rows 1.75 -> 1.67 ms); from 20 rows on the gated rows' products hold up the norm (2.98 -> 3.12 ms), and at
+        # 256 rows the chain of separate launches is faster, also than the QKV epilogue on the GEMM's epilogue warps.
+        fuse = _fusions("lora" if B <= 8 else "")
         fuse_norm_lora = "lora" in fuse and lora and tp is None  # RMSNorm + LoRA-A of the gated rows in one launch
         fuse_qkv = "qkv" in fuse and hd == 128                   # QK-norm + RoPE + KV write in the QKV GEMM epilogue
         rope = dict(rope_cs=s.rope_cs, hd=hd, theta=cfg.rope_theta) if fuse_qkv else {}
