@@ -59,7 +59,7 @@ def available() -> bool:
 
 
 def _stream() -> c_void_p:
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    return c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def _p(t: Optional[torch.Tensor]) -> c_void_p:
@@ -70,6 +70,8 @@ _status = {}
 
 
 def status_word(device=None) -> torch.Tensor:
+    if isinstance(device, torch.device) and device.type == "cuda" and device.index in _status:
+        return _status[device.index]
     dev = torch.device(device if device is not None else torch.cuda.current_device())
     if dev.type != "cuda":
         dev = torch.device("cuda", torch.cuda.current_device())
@@ -121,6 +123,7 @@ def _fits(bn: int, s: int, nacc: int) -> bool:
     return red + per * 256 <= ns * stage
 
 
+@functools.lru_cache(maxsize=4096)
 def plan_gemm(M: int, F: int, K: int, R: int = 0, dual: bool = False):
     """Pick the token-tile width and the split-K cluster size with a small cost model.
 
