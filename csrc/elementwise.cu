@@ -751,7 +751,7 @@ extern "C" int tahb_rmsnorm_lora(const void* x, const void* w, void* y, int M, i
                                  cudaStream_t stream) {
   if (M <= 0) return 0;
   if (H % 8 || H > 8192 || R <= 0 || M > 1024) return -1;
-  const int lora_ctas = gate != nullptr ? NORM_LORA_SLOTS * NORM_LORA_SLICES : 0;
+  const int lora_ctas = gate != nullptr ? (M < NORM_LORA_SLOTS ? M : NORM_LORA_SLOTS) * NORM_LORA_SLICES : 0;
   cudaError_t e = launch_chain(rmsnorm_lora_kernel, dim3(M + lora_ctas), dim3(256), (size_t)H * 2, stream,
                                reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(w),
                                reinterpret_cast<__nv_bfloat16*>(y), M, H, ldx, ldy, eps, gate,
