@@ -7,11 +7,22 @@
 //   [page][2 (K,V)][n_kv_heads][page_size][HD]  bf16
 // with a page table pt[c][row][i] and a length len[c][row].
 //
-// Work split: grid (n_kv_heads, rows, n_split).  A CTA has 4 warps = 16 groups of 8 lanes; a
-// group owns one KV token at a time and each lane HD/8 of its dims, so a token's K (or V) row is
-// one contiguous 2*HD-byte read by 8 lanes.  All G = nq/nkv query heads that share the KV head are
-// handled together, so K/V are read once.  Online softmax in base 2; groups are merged through
-// shared memory; with n_split > 1 partial (m, l, acc) go to a workspace and a second kernel merges.
+// Work split: an item is (KV head, row, split), one CTA; its pages go to its four (or two) warps in turn.  All G = nq / nkv query
+// heads that share the KV head are handled together, so K / V are read once, straight from global memory into the registers that
+// warp-level tensor instructions read (a page and a half of a warp's in flight; no shared memory ring):
+//
+//     scores [16 entries][8 columns] = K Q^T      a lane reads 16 consecutive bytes of a K row and of Q at the same dims: the order
+//                                                 of a reduction is free as long as both operands agree (see gemm_few.cu)
+//     O^T [16 dims][8 columns] += V^T P           a lane reads eight dims of four entries and pairs them
+//
+// Column = (part, head): P in fp32 is the sum of three bf16 parts, exactly, and the parts take columns that one or two heads leave
+// empty, so nothing of a probability is lost.  Online softmax in base 2; the warps merge through shared memory; with n_split > 1
+// partial (m, l, acc) go to a workspace and a second kernel merges.
+//
+// What bounds it: HBM, and for short rows the chain of dependent loads of an item (length, page number, page).  The kernel before had
+// four copy-fed warps per item on fp32 multiply-adds, 190 instructions for four entries of a warp, and was bound by their issue:
+// us, 16 heads on 8 KV heads, before and now: 1 row at 60 entries 4.6 and 3.5, 6 rows at 220 10.0 and 8.5, 20 rows at 1300 34.7 and 29.4,
+// 256 rows at 80 31.9 and 25.6, at 600 116 and 109 (5.9 TB/s).
 #include "common.cuh"
 #include "tah_b200_noalloc.h"
 
@@ -32,18 +43,16 @@ struct DecodeAttnParams {
   float scale_log2;             // softmax scale * log2(e)
 };
 
-// Geometry of the pipelined kernel: pages of 16 tokens; a pipeline stage holds STAGE_PAGES pages
-// (K and V blocks of one KV head: 2 * 16 * HD bf16 each page), NSTAGE stages in flight per CTA.
 constexpr int ATT_PAGE = 16;
-constexpr int ATT_STAGE_PAGES = 2;
-constexpr int ATT_NSTAGE = 3;
 
-template <int HD>
+template <int HD, int G>
 struct AttCfg {
-  static constexpr int BLK_ELEMS = ATT_PAGE * HD;                          // one K (or V) block of a page
-  static constexpr int STAGE_ELEMS = ATT_STAGE_PAGES * 2 * BLK_ELEMS;
-  static constexpr int STAGE_BYTES = STAGE_ELEMS * 2;
-  static constexpr int SMEM_BYTES = ATT_NSTAGE * STAGE_BYTES + 256;
+  static constexpr int STEPS = HD / 32;             // 16-byte pieces of a K row per lane
+  static constexpr int HALVES = HD / 64;
+  static constexpr int COLS = 3 * G;                // (part, head): see decode_attn_kernel
+  static constexpr int TILES = (COLS + 7) / 8;
+  static constexpr int PITCH = HD + 4;              // floats per column in the merge area
+  static constexpr int WARPS = TILES == 2 ? 8 : HD == 64 ? 16 : 12;      // resident per SM, without spills
 };
 
 // Maps the i-th visible page of a row (pages of cache 0 first, then cache 1, ...) to its cache and
@@ -56,20 +65,41 @@ __device__ __forceinline__ void locate_page(int i, const int* seg_pages, int& c,
     if (c == cc && local >= seg_pages[cc]) { local -= seg_pages[cc]; c = cc + 1; }
 }
 
-template <int HD, int G>
-__global__ void __launch_bounds__(160, (HD * G <= 256) ? 4 : 2) decode_attn_kernel(const DecodeAttnParams p) {
-  pdl_wait();
-  using C = AttCfg<HD>;
-  constexpr int VEC = HD / 64;       // 16-byte chunks per lane per row: lane gl owns chunks gl, gl + 8, ...
-  constexpr int DPL = VEC * 8;       // dims per lane
-  extern __shared__ __align__(128) uint8_t att_smem[];
-  __nv_bfloat16* stages = reinterpret_cast<__nv_bfloat16*>(att_smem);
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(att_smem + ATT_NSTAGE * C::STAGE_BYTES);
-  uint64_t* empty_bar = full_bar + ATT_NSTAGE;
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(empty_bar + ATT_NSTAGE);
+// c += A B.  The tensor core truncates where it adds to its accumulator: a product of its own per step and a rounded addition
+// keep the sums as close to the exact ones as fp32 multiply-adds are.
+__device__ __forceinline__ void att_mma_add(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  float d0, d1, d2, d3;
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+               : "=f"(d0), "=f"(d1), "=f"(d2), "=f"(d3)
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+  c[0] += d0; c[1] += d1; c[2] += d2; c[3] += d3;
+}
+__device__ __forceinline__ uint4 att_ld(const __nv_bfloat16* p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+// 8x8 tile of 16-bit values: lane (g, t) gives row g, columns 2t and 2t + 1, and gets column g, rows 2t and 2t + 1
+__device__ __forceinline__ uint32_t att_transpose(uint32_t v) {
+  uint32_t r;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
+}
+// part 0, 1, 2 of x: x = part 0 + part 1 + part 2 exactly, eight bits each
+__device__ __forceinline__ float bf16_part(float x, int part) {
+  const float hi = bf16_round(x), r1 = x - hi, mid = bf16_round(r1);
+  return part == 0 ? hi : part == 1 ? mid : part == 2 ? r1 - mid : 0.f;
+}
 
+template <int HD, int G, int NW>
+__global__ void __launch_bounds__(NW * 32, AttCfg<HD, G>::WARPS / NW) decode_attn_kernel(const DecodeAttnParams p) {
+  pdl_wait();
+  using C = AttCfg<HD, G>;
+  constexpr int S = C::STEPS, NH = C::HALVES, NT = C::TILES;
+  __shared__ float part[NW][C::COLS][C::PITCH];
+  __shared__ float part_ml[NW][G][2];
   const int kvh = blockIdx.x, row = blockIdx.y, split = blockIdx.z;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
 
   int seg_len[MAX_CACHES], seg_pages[MAX_CACHES];
   int total_pages = 0;
@@ -83,183 +113,172 @@ __global__ void __launch_bounds__(160, (HD * G <= 256) ? 4 : 2) decode_attn_kern
   const int ppc = (total_pages + p.n_split - 1) / p.n_split;
   const int pb = split * ppc;
   const int pe = min(total_pages, pb + ppc);
-  const int n_iter = pe > pb ? (pe - pb + ATT_STAGE_PAGES - 1) / ATT_STAGE_PAGES : 0;
+  const int n = pe - pb > warp ? (pe - pb - warp + NW - 1) / NW : 0;      // pages pb + warp, + 4, ... are this warp's
 
-  if (tid == 0) {
-    for (int s = 0; s < ATT_NSTAGE; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 4);          // one arrival per consumer warp
-    }
-    *abort_flag = 0;
-    mbar_fence_init();
-  }
-  __syncthreads();
-
-  float m[G], l[G], acc[G][DPL];
+  // 32 of the warp's pages at a time, one per lane: K block of this head, entries that are visible in it
+  const __nv_bfloat16* blk = nullptr;
+  int entries = 0;
+  auto look_up = [&](int i) {
+    const int pg = pb + warp + NW * (i + lane);
+    if (pg >= pe) return;
+    int c, local;
+    locate_page(pg, seg_pages, c, local);
+    int len = seg_len[0];
 #pragma unroll
-  for (int g = 0; g < G; ++g) {
-    m[g] = -INFINITY;
-    l[g] = 0.f;
+    for (int cc = 1; cc < MAX_CACHES; ++cc) if (c == cc) len = seg_len[cc];
+    const int page = p.page_table[c][(size_t)row * p.max_pages[c] + local];
+    blk = p.cache[c] + ((size_t)page * 2 * p.nkv + kvh) * (ATT_PAGE * HD);
+    entries = len - local * ATT_PAGE;
+  };
+  auto block_of = [&](int i) {
+    return reinterpret_cast<const __nv_bfloat16*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(blk), i & 31));
+  };
+  uint4 kx[S], ky[S], v[NH][4];
+  auto load_k = [&](const __nv_bfloat16* b) {           // entries g and g + 8
 #pragma unroll
-    for (int i = 0; i < DPL; ++i) acc[g][i] = 0.f;
-  }
-  const int grp = (warp & 3) * 4 + (lane >> 3);   // token slot inside a page (consumer warps only)
-  const int gl = lane & 7;
-
-  if (warp == 4) {
-    // ---------------- producer: bulk copies of whole K / V page blocks ----------------
-    if (lane == 0) {
-      for (int it = 0; it < n_iter; ++it) {
-        const int s = it % ATT_NSTAGE;
-        const uint32_t ph = (it / ATT_NSTAGE) & 1;
-        mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, STATUS_TIMEOUT_STAGE_EMPTY);
-        const int first = pb + it * ATT_STAGE_PAGES;
-        const int n_here = min(ATT_STAGE_PAGES, pe - first);
-        mbar_expect_tx(&full_bar[s], n_here * 2 * C::BLK_ELEMS * 2);
-        for (int u = 0; u < n_here; ++u) {
-          int c, local;
-          locate_page(first + u, seg_pages, c, local);
-          const int page = p.page_table[c][(size_t)row * p.max_pages[c] + local];
-          const __nv_bfloat16* kp = p.cache[c] + (((size_t)page * 2 + 0) * p.nkv + kvh) * C::BLK_ELEMS;
-          const __nv_bfloat16* vp = kp + (size_t)p.nkv * C::BLK_ELEMS;
-          __nv_bfloat16* dst = stages + (size_t)s * C::STAGE_ELEMS + (size_t)u * 2 * C::BLK_ELEMS;
-          bulk_load(dst, kp, C::BLK_ELEMS * 2, &full_bar[s]);
-          bulk_load(dst + C::BLK_ELEMS, vp, C::BLK_ELEMS * 2, &full_bar[s]);
-        }
-      }
+    for (int s = 0; s < S; ++s) {
+      kx[s] = att_ld(b + g * HD + s * 32 + t * 8);
+      ky[s] = att_ld(b + (g + 8) * HD + s * 32 + t * 8);
     }
-    __syncwarp();
+  };
+  auto load_v = [&](const __nv_bfloat16* b) {           // entries 2t, 2t + 1, 2t + 8, 2t + 9
+    b += (size_t)p.nkv * (ATT_PAGE * HD);
+#pragma unroll
+    for (int h = 0; h < NH; ++h)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[h][e] = att_ld(b + (2 * t + (e & 1) + 8 * (e >> 1)) * HD + h * 64 + g * 8);
+  };
+  look_up(0);
+  if (n > 0) {
+    const __nv_bfloat16* b = block_of(0);
+    load_k(b);
+    load_v(b);
+  }
+
+  // column g of the score tile: head g % G
+  uint4 q[S];
+  const __nv_bfloat16* qs = p.q + ((size_t)row * p.nq + kvh * G + g % G) * HD + t * 8;
+  if ((reinterpret_cast<uintptr_t>(p.q) & 15) == 0) {
+#pragma unroll
+    for (int s = 0; s < S; ++s) q[s] = *reinterpret_cast<const uint4*>(qs + s * 32);
   } else {
-    // ---------------- consumers: 16 groups of 8 lanes, one token of each page per group ----------------
-    float qv[G][DPL];
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      const __nv_bfloat16* qp = p.q + ((size_t)row * p.nq + kvh * G + g) * HD;
+    for (int s = 0; s < S; ++s) {
+      __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(&q[s]);
 #pragma unroll
-      for (int v = 0; v < VEC; ++v)
-#pragma unroll
-        for (int i = 0; i < 8; ++i) qv[g][v * 8 + i] = __bfloat162float(qp[(v * 8 + gl) * 8 + i]) * p.scale_log2;
+      for (int j = 0; j < 8; ++j) e[j] = qs[s * 32 + j];
     }
-    for (int it = 0; it < n_iter; ++it) {
-      const int s = it % ATT_NSTAGE;
-      const uint32_t ph = (it / ATT_NSTAGE) & 1;
-      mbar_wait(&full_bar[s], ph, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
-      const __nv_bfloat16* st = stages + (size_t)s * C::STAGE_ELEMS;
-      float sc[ATT_STAGE_PAGES][G];
-      bool ok[ATT_STAGE_PAGES];
+  }
+
+  // this lane's columns 2t and 2t + 1: maximum, its entries' share of the weight, and O
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, acc[NT][NH][4][4];
 #pragma unroll
-      for (int u = 0; u < ATT_STAGE_PAGES; ++u) {
-        const int gi = pb + it * ATT_STAGE_PAGES + u;
-        ok[u] = false;
-        if (gi < pe) {
-          int c, local;
-          locate_page(gi, seg_pages, c, local);
-          int len_c = seg_len[0];
+  for (int a = 0; a < NT * NH * 16; ++a) (&acc[0][0][0][0])[a] = 0.f;
+
+  for (int i = 0; i < n; ++i) {
+    float sc[4] = {0.f, 0.f, 0.f, 0.f};                 // entries g (0, 1) and g + 8 (2, 3), columns 2t and 2t + 1
 #pragma unroll
-          for (int cc = 1; cc < MAX_CACHES; ++cc) if (c == cc) len_c = seg_len[cc];
-          ok[u] = local * ATT_PAGE + grp < len_c;
-        }
-        const __nv_bfloat16* kp = st + (size_t)u * 2 * C::BLK_ELEMS + grp * HD;
-        float se[G], so[G];            // two partial sums per head: shorter dependent FMA chains
-#pragma unroll
-        for (int g = 0; g < G; ++g) { se[g] = 0.f; so[g] = 0.f; }
-#pragma unroll
-        for (int v = 0; v < VEC; ++v) {
-          const uint4 kr = *reinterpret_cast<const uint4*>(kp + (v * 8 + gl) * 8);
-          const __nv_bfloat162* kh = reinterpret_cast<const __nv_bfloat162*>(&kr);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float2 kf = __bfloat1622float2(kh[j]);
-#pragma unroll
-            for (int g = 0; g < G; ++g) {
-              se[g] = fmaf(qv[g][v * 8 + 2 * j], kf.x, se[g]);
-              so[g] = fmaf(qv[g][v * 8 + 2 * j + 1], kf.y, so[g]);
-            }
-          }
-        }
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-          float t = se[g] + so[g];
-          t += __shfl_xor_sync(0xffffffffu, t, 1);
-          t += __shfl_xor_sync(0xffffffffu, t, 2);
-          t += __shfl_xor_sync(0xffffffffu, t, 4);
-          sc[u][g] = ok[u] ? t : -INFINITY;
-        }
-      }
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
-        float mx = m[g];
-#pragma unroll
-        for (int u = 0; u < ATT_STAGE_PAGES; ++u) mx = fmaxf(mx, sc[u][g]);
-        const float corr = (m[g] == -INFINITY) ? 0.f : exp2f(m[g] - mx);
-        m[g] = mx;
-        l[g] *= corr;
-#pragma unroll
-        for (int i = 0; i < DPL; ++i) acc[g][i] *= corr;
-      }
-#pragma unroll
-      for (int u = 0; u < ATT_STAGE_PAGES; ++u) {
-        const __nv_bfloat16* vp = st + (size_t)u * 2 * C::BLK_ELEMS + C::BLK_ELEMS + grp * HD;
-        float pw[G];
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-          pw[g] = ok[u] ? exp2f(sc[u][g] - m[g]) : 0.f;
-          l[g] += pw[g];
-        }
-        if (!ok[u]) continue;   // never touch stage memory that holds no page: it may contain NaN bits
-#pragma unroll
-        for (int v = 0; v < VEC; ++v) {
-          const uint4 vr = *reinterpret_cast<const uint4*>(vp + (v * 8 + gl) * 8);
-          const __nv_bfloat162* vh = reinterpret_cast<const __nv_bfloat162*>(&vr);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float2 vf = __bfloat1622float2(vh[j]);
-#pragma unroll
-            for (int g = 0; g < G; ++g) {
-              acc[g][v * 8 + 2 * j] += pw[g] * vf.x;
-              acc[g][v * 8 + 2 * j + 1] += pw[g] * vf.y;
-            }
-          }
-        }
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty_bar[s]);
+    for (int s = 0; s < S; ++s) {
+      att_mma_add(sc, kx[s].x, ky[s].x, kx[s].y, ky[s].y, q[s].x, q[s].y);
+      att_mma_add(sc, kx[s].z, ky[s].z, kx[s].w, ky[s].w, q[s].z, q[s].w);
     }
+    const int have = __shfl_sync(0xffffffffu, entries, i & 31);
+    const bool more = i + 1 < n;
+    if (more && ((i + 1) & 31) == 0) look_up(i + 1);
+    const __nv_bfloat16* next = block_of(i + 1);
+    if (more) load_k(next);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) sc[c] = g + 8 * (c >> 1) < have ? sc[c] * p.scale_log2 : -INFINITY;
+    const float mx[2] = {fmaxf(sc[0], sc[2]), fmaxf(sc[1], sc[3])};
+    if (__any_sync(0xffffffffu, mx[0] > m[0] || mx[1] > m[1])) {
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        float top = fmaxf(m[c], mx[c]);
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        const float f = m[c] == -INFINITY ? 0.f : exp2f(m[c] - top);
+        m[c] = top;
+        l[c] *= f;
+#pragma unroll
+        for (int a = 0; a < NT * NH * 8; ++a) (&acc[0][0][0][0])[2 * a + c] *= f;
+      }
+    }
+    float w[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      w[c] = sc[c] == -INFINITY ? 0.f : exp2f(sc[c] - m[c & 1]);
+      l[c & 1] += w[c];
+    }
+    uint32_t b[NT][2];
+#pragma unroll
+    for (int a = 0; a < NT; ++a)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const __nv_bfloat162 pair = __floats2bfloat162_rn(bf16_part(w[2 * r], (8 * a + 2 * t) / G), bf16_part(w[2 * r + 1], (8 * a + 2 * t + 1) / G));
+        b[a][r] = att_transpose(*reinterpret_cast<const uint32_t*>(&pair));
+      }
+    if (have < ATT_PAGE) {                              // what lies behind the last entry may be NaN bits
+#pragma unroll
+      for (int h = 0; h < NH; ++h)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (2 * t + (e & 1) + 8 * (e >> 1) >= have) v[h][e] = make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int h = 0; h < NH; ++h) {
+      const uint32_t* e0 = reinterpret_cast<const uint32_t*>(&v[h][0]);
+      const uint32_t* e1 = reinterpret_cast<const uint32_t*>(&v[h][1]);
+      const uint32_t* e2 = reinterpret_cast<const uint32_t*>(&v[h][2]);
+      const uint32_t* e3 = reinterpret_cast<const uint32_t*>(&v[h][3]);
+#pragma unroll
+      for (int d = 0; d < 4; ++d) {                     // rows g and g + 8 of the tile: dims 8 g + 2 d and 8 g + 2 d + 1
+        const uint32_t a0 = __byte_perm(e0[d], e1[d], 0x5410), a1 = __byte_perm(e0[d], e1[d], 0x7632);
+        const uint32_t a2 = __byte_perm(e2[d], e3[d], 0x5410), a3 = __byte_perm(e2[d], e3[d], 0x7632);
+#pragma unroll
+        for (int a = 0; a < NT; ++a) att_mma_add(acc[a][h][d], a0, a1, a2, a3, b[a][0], b[a][1]);
+      }
+    }
+    if (more) load_v(next);
   }
 
   pdl_launch_dependents();
-  // merge the 16 groups through shared memory (the pipeline buffers are free now)
-  __syncthreads();
-  float* sm_m = reinterpret_cast<float*>(att_smem);          // [16][G]
-  float* sm_l = sm_m + 16 * G;                               // [16][G]
-  float* sm_acc = sm_l + 16 * G;                             // [16][G][HD]
-  if (warp < 4) {
-    if (gl == 0) {
+  // the warps meet in shared memory
 #pragma unroll
-      for (int g = 0; g < G; ++g) { sm_m[grp * G + g] = m[g]; sm_l[grp * G + g] = l[g]; }
+  for (int c = 0; c < 2; ++c) {
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) l[c] += __shfl_xor_sync(0xffffffffu, l[c], o);
+    if (g == 0 && 2 * t + c < G) {
+      part_ml[warp][2 * t + c][0] = m[c];
+      part_ml[warp][2 * t + c][1] = l[c];
     }
 #pragma unroll
-    for (int g = 0; g < G; ++g)
+    for (int a = 0; a < NT; ++a) {
+      const int col = 8 * a + 2 * t + c;
+      if (col >= C::COLS) continue;
 #pragma unroll
-      for (int v = 0; v < VEC; ++v)
-#pragma unroll
-        for (int i = 0; i < 8; ++i) sm_acc[(grp * G + g) * HD + (v * 8 + gl) * 8 + i] = acc[g][v * 8 + i];
+      for (int h = 0; h < NH; ++h) {
+        float4* dst = reinterpret_cast<float4*>(&part[warp][col][h * 64 + g * 8]);
+        dst[0] = make_float4(acc[a][h][0][c], acc[a][h][0][2 + c], acc[a][h][1][c], acc[a][h][1][2 + c]);
+        dst[1] = make_float4(acc[a][h][2][c], acc[a][h][2][2 + c], acc[a][h][3][c], acc[a][h][3][2 + c]);
+      }
+    }
   }
   __syncthreads();
-  for (int idx = tid; idx < G * HD; idx += 160) {
-    const int g = idx / HD, d = idx % HD;
+  for (int idx = tid; idx < G * HD; idx += NW * 32) {
+    const int hg = idx / HD, d = idx % HD;
     float mx = -INFINITY;
 #pragma unroll
-    for (int k = 0; k < 16; ++k) mx = fmaxf(mx, sm_m[k * G + g]);
+    for (int w = 0; w < NW; ++w) mx = fmaxf(mx, part_ml[w][hg][0]);
     float num = 0.f, den = 0.f;
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const float mk = sm_m[k * G + g];
-      const float w = (mk == -INFINITY) ? 0.f : exp2f(mk - mx);
-      num += w * sm_acc[(k * G + g) * HD + d];
-      den += w * sm_l[k * G + g];
+    for (int w = 0; w < NW; ++w) {
+      const float mw = part_ml[w][hg][0];
+      const float f = (mw == -INFINITY) ? 0.f : exp2f(mw - mx);
+      const float hi = part[w][hg][d], v = hi + (part[w][G + hg][d] + part[w][2 * G + hg][d]);
+      num += f * (fabsf(v) < INFINITY ? v : hi);        // an infinite entry: its products with the parts of one weight may cancel
+      den += f * part_ml[w][hg][1];
     }
-    const int head = kvh * G + g;
+    const int head = kvh * G + hg;
     if (p.n_split == 1) {
       p.out[((size_t)row * p.nq + head) * HD + d] = __float2bfloat16_rn(den > 0.f ? num / den : 0.f);
     } else {
@@ -347,15 +366,15 @@ __global__ void __launch_bounds__(128) varlen_attn_naive_kernel(const VarlenAttn
 
 template <int HD, int G>
 static int launch_decode(const DecodeAttnParams& p, cudaStream_t stream) {
-  dim3 grid(p.nkv, p.rows, p.n_split);
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(decode_attn_kernel<HD, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             AttCfg<HD>::SMEM_BYTES) != cudaSuccess)
-      return -10;
-    configured = true;
-  }
-  cudaError_t e = launch_chain(decode_attn_kernel<HD, G>, grid, dim3(160), AttCfg<HD>::SMEM_BYTES, stream, p);
+  const dim3 grid(p.nkv, p.rows, p.n_split);
+  // Four warps per item.  Two where more items than four times the resident ones have at most ten pages per cache: the dependent
+  // loads at the start of an item then cost half the warps (256 rows x 8 heads at 80 entries 25.6 us, with four 29.9; at 600 entries
+  // 116 and 109).
+  int pages = 0;
+  for (int c = 0; c < p.n_caches; ++c) pages = p.max_pages[c] > pages ? p.max_pages[c] : pages;
+  const bool small = (long long)p.nkv * p.rows * p.n_split > 148ll * AttCfg<HD, G>::WARPS && pages <= 10;
+  cudaError_t e = small ? launch_chain(decode_attn_kernel<HD, G, 2>, grid, dim3(64), 0, stream, p)
+                        : launch_chain(decode_attn_kernel<HD, G, 4>, grid, dim3(128), 0, stream, p);
   if (e == cudaSuccess && p.n_split > 1)
     e = launch_chain(decode_attn_merge_kernel<HD>, dim3(p.rows * p.nq), dim3(HD), 0, stream, p.ws, p.out, p.n_split);
   return e == cudaSuccess ? 0 : -3;

@@ -453,7 +453,10 @@ class TaHEngine(DecodeEngine):
         s = self._alloc_scheduler_state(B, max_new)
         # split the KV walk of a row when (rows x local KV heads) CTAs would leave SM slots empty
         # (small batches, wide tensor-parallel groups); the partial results meet in a merge kernel
-        s.attn_split = max(1, min(4, (148 * 4) // max(1, B * w.nkv)))
+        # one item per (row, KV head), 444 resident at once.  Few of them are split until they make up to two waves: with uneven rows and
+        # a quarter of the slots idle, 160 items in two took 30.9 us, in three 32.4 and in four 29.4 (in one 45)
+        items = max(1, B * w.nkv)
+        s.attn_split = min(4, 888 // items) if items <= 296 else 1
         s.attn_ws = None
         if s.attn_split > 1:
             n_ws = int(K.lib().tahb_decode_attn_ws_floats(B, w.nq, cfg.head_dim, s.attn_split))

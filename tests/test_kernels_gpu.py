@@ -407,6 +407,35 @@ def test_decode_attention_two_caches(hd, nq, nkv, n_split):
         _close(out[r].view(nq, hd), ref, atol=2e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("hd,nq,nkv", [(128, 16, 8), (64, 8, 8), (128, 12, 3)])
+@pytest.mark.parametrize("n_split", [1, 2])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_decode_attention_more_items_than_ctas(hd, nq, nkv, n_split, shift):
+    """Every CTA walks several rows: empty ones, one entry, whole pages, more pages than a stage ring and than 32 page numbers."""
+    Kc = _cuda()
+    page, rows = 16, 5 * 148 * 4 // (nkv * n_split) // 2
+    some0, some1 = [0, 1, 16, 33, 96, 7, 560, 32], [0, 5, 16, 0, 40]
+    lens0, lens1 = [some0[r * 7 % 8] for r in range(rows)], [some1[r % 5] for r in range(rows)]
+    c0, pt0, l0 = _paged_setup(rows, lens0, nkv, hd, page, 1)
+    c1, pt1, l1 = _paged_setup(rows, lens1, nkv, hd, page, 2)
+    depth = torch.tensor([r % 3 % 2 for r in range(rows)], dtype=torch.int32, device="cuda")
+    q = _rand(rows * nq * hd + shift, seed=3)[shift:].view(rows, nq * hd)
+    scale = hd ** -0.5
+    out = Kc.decode_attn(q, [c0, c1], [pt0, pt1], [l0, l1], depth, nq, nkv, hd, page, scale, n_split=n_split)
+    Kc.check_status()
+    for r in range(rows):
+        n1 = lens1[r] if int(depth[r]) else 0
+        parts = [_gather_paged(c, pt[r], n, page) for c, pt, n in ((c0, pt0, lens0[r]), (c1, pt1, n1)) if n]
+        if not parts:
+            assert not out[r].any()
+            continue
+        k, v = (torch.cat(x).float().repeat_interleave(nq // nkv, dim=1) for x in zip(*parts))
+        s = torch.einsum("hd,nhd->hn", q[r].view(nq, hd).float(), k) * scale
+        ref = torch.einsum("hn,nhd->hd", torch.softmax(s, -1), v)
+        # fp32 inside, one rounding to bf16 (2^-8 of the value) at the end; fp32 sums of up to 600 terms of order one stay below 1e-4
+        _close(out[r].view(nq, hd), ref, atol=1e-4, rtol=2 ** -8)
+
+
 def test_varlen_attention_duo_segments():
     Kc = _cuda()
     nq, nkv, hd = 4, 2, 64
