@@ -224,6 +224,33 @@ def test_engine_with_head_dim_128_fused_kernels_match_unfused(monkeypatch):
     assert same >= 0.9 * B * n_new, same
 
 
+@pytest.mark.parametrize("head_dim,T", [(64, 5), (64, 20), (128, 150)])
+def test_native_pass_gives_the_bits_of_the_loop(head_dim, T):
+    """The passes of a prompt (three deep, some tokens each) from one native call and launch by launch: the same kernels on the same plans."""
+    from tah_b200.engine import TaHEngine
+    B = 3
+    model = tiny_tah(max_iter=3, dtype=torch.bfloat16, head_dim=head_dim, num_attention_heads=4, num_key_value_heads=2).cuda().eval()
+    ids = torch.randint(0, 1024, (B, T), generator=torch.Generator().manual_seed(3)).cuda()
+    outs = []
+    for native in (True, False):
+        eng = TaHEngine(model, max_rows=B, max_seq_len=T + 4, use_cuda_graph=False, deep_fraction=1.0)
+        eng.hard_override = eng.make_bernoulli_override(B, (0.6, 0.6), seed=5)
+        assert eng.w.pass_weights is not None
+        if not native:
+            eng.w.pass_weights = None
+        seen, one_pass = [], eng._packed_pass
+
+        def spy(*a, **k):
+            hn, kv = one_pass(*a, **k)
+            seen.append([hn.clone()] + [t.clone() for pair in kv for t in pair])
+            return hn, kv
+        eng._packed_pass = spy
+        eng.generate(ids, None, max_new_tokens=2, do_sample=False)
+        outs.append(seen)
+    assert len(outs[0]) == len(outs[1]) == 3
+    assert all(torch.equal(a, b) for x, y in zip(*outs) for a, b in zip(x, y))
+
+
 def test_learned_mlp_decider_kernel_chain_matches_module_and_drives_the_engine():
     """``MLPIterDecider`` (tapped hidden states + sorted top-k logits -> residual MLP) as the engine's kernel chain
     against the PyTorch module, and a generation driven by it (no override)."""
