@@ -114,13 +114,14 @@ class _BlockDiag(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, F, spans, scaling, *blocks):
-        ctx.args = (spans, scaling, blocks[0].shape[1])
+        ctx.args = (spans, scaling, blocks[0].shape[1], [b.dtype for b in blocks])
         return K.block_diag([b.detach() for b in blocks], spans, F, scaling)
 
     @staticmethod
     def backward(ctx, g):
-        spans, scaling, r = ctx.args
-        return (None, None, None) + tuple(g[lo:hi, j * r:(j + 1) * r] * scaling if ctx.needs_input_grad[3 + j] else None
+        spans, scaling, r, types = ctx.args
+        # scaled in the factor's own type: a gradient of 32-bit factors is not rounded once more
+        return (None, None, None) + tuple(g[lo:hi, j * r:(j + 1) * r].to(types[j]) * scaling if ctx.needs_input_grad[3 + j] else None
                                           for j, (lo, hi) in enumerate(spans))
 
 

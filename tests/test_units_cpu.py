@@ -401,3 +401,24 @@ def test_kv_cache_guard_pages(monkeypatch):
     assert not kv.check_guards()
     monkeypatch.delenv("TAH_B200_CANARY")
     assert PagedKVCache(CacheGeometry(2, 2, 64, 16), 3, 40, 2, device="cpu").check_guards()
+
+
+def test_adapter_factor_keeps_gradients_of_32_bit_factors():
+    """The block-diagonal factor and its gradients are those of assigning each scaled block to its place, to the bit."""
+    from tah_b200.ops.autograd_ops import _BlockDiag
+    spans, F, r, scaling = ((0, 12), (12, 20)), 24, 8, 1.7
+    g = torch.Generator().manual_seed(0)
+    first = [torch.randn(hi - lo, r, generator=g) for lo, hi in spans]
+    gy = torch.randn(F, len(spans) * r, generator=g).to(torch.bfloat16)
+    got = []
+    for assign in (False, True):
+        blocks = [b.clone().requires_grad_() for b in first]
+        if assign:
+            out = torch.zeros(F, len(spans) * r, dtype=torch.bfloat16)
+            for j, (lo, hi) in enumerate(spans):
+                out[lo:hi, j * r:(j + 1) * r] = blocks[j] * scaling
+        else:
+            out = _BlockDiag.apply(F, spans, scaling, *blocks)
+        out.backward(gy)
+        got.append([out.detach()] + [b.grad for b in blocks])
+    assert all(torch.equal(a, b) for a, b in zip(*got))
