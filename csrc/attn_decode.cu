@@ -96,7 +96,8 @@ __global__ void __launch_bounds__(NW * 32, AttCfg<HD, G>::WARPS / NW) decode_att
   pdl_wait();
   using C = AttCfg<HD, G>;
   constexpr int S = C::STEPS, NH = C::HALVES, NT = C::TILES;
-  __shared__ float part[NW][C::COLS][C::PITCH];
+  static_assert(C::PITCH % 4 == 0, "a column's 16-byte pieces");
+  __shared__ __align__(16) float part[NW][C::COLS][C::PITCH];      // written as float4
   __shared__ float part_ml[NW][G][2];
   const int kvh = blockIdx.x, row = blockIdx.y, split = blockIdx.z;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
