@@ -226,11 +226,13 @@ def wait_flags(flags: torch.Tensor, targets: torch.Tensor) -> None:
         "tahb_wait_flags")
 
 
-def _plan_tiles(M: int, rows: int, K: int, R: int, swiglu: bool, gelu: bool, swiglu_interleaved: bool, pair=None, bn: int = 0, splits=None):
-    """``(pair, bn, splits)`` of a tcgen05 product with a weight of ``rows`` rows."""
+def _plan_tiles(M: int, rows: int, K: int, R: int, swiglu: bool, gelu: bool, swiglu_interleaved: bool, pair=None, bn: int = 0, splits=None,
+                staged: bool = True):
+    """``(pair, bn, splits)`` of a tcgen05 product with a weight of ``rows`` rows.  ``staged``: output and residual can be moved as whole
+    tiles (:func:`_whole_pieces`), the only way the pair form has."""
     can_pair = not swiglu and not gelu and rows % 256 == 0
     if pair is None and bn == 0 and splits is None and M > 256 and not swiglu:
-        return plan_tiles(M, rows, K + R, can_pair and PAIR_AUTO, not swiglu_interleaved)
+        return plan_tiles(M, rows, K + R, can_pair and PAIR_AUTO and staged, not swiglu_interleaved)
     pair = bool(pair) and can_pair
     if pair:
         bn, splits = bn or 256, 1
@@ -299,7 +301,8 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
             not ((swiglu or gelu) and (residual is not None or swiglu and gelu)) and _few_ok(x, w, x2, w2) and
             (not (gelu or swiglu_interleaved) or _whole_pieces(out))):
         return _gemm_few(x, w, out, residual, x2, w2, 1 if swiglu else 3 if gelu else 4 if swiglu_interleaved else 0, early=const_w)
-    pair, bn, splits = _plan_tiles(M, w.shape[0], K, R, swiglu, gelu, swiglu_interleaved, pair, bn, splits)
+    staged = tp_push is not None or (_whole_pieces(out) and (residual is None or _whole_pieces(residual)))
+    pair, bn, splits = _plan_tiles(M, w.shape[0], K, R, swiglu, gelu, swiglu_interleaved, pair, bn, splits, staged)
     args = (_p(w), _p(x), _p(out), _p(residual), _p(w2), _p(x2), c_int(M), c_int(F), c_int(K), c_int(R),
             c_ll(w.stride(0)), c_ll(x.stride(0)), c_ll(out.stride(0)),
             c_ll(residual.stride(0) if residual is not None else 0),
@@ -388,7 +391,8 @@ def gemm_t(x: torch.Tensor, w: torch.Tensor, *, x_t: bool = False, w_t: bool = F
         _check_bf16_2d(residual, "residual")
     can_pair = F % 256 == 0 and (not x_t or M % 64 == 0)
     if pair is None and bn == 0 and splits is None and M > 256:
-        pair, bn, splits = plan_tiles(M, F, Kx, can_pair and PAIR_AUTO, True)
+        staged = _whole_pieces(out) and (residual is None or _whole_pieces(residual))
+        pair, bn, splits = plan_tiles(M, F, Kx, can_pair and PAIR_AUTO and staged, True)
     pair = bool(pair) and can_pair
     if pair:
         bn, splits = bn or 256, 1

@@ -1086,3 +1086,24 @@ def test_attention_heads_of_a_kv_head(hd, nq, nkv):
     _close(dq.view(n, nq, hd), rdq, atol=3e-2, rtol=3e-2)
     _close(dk.view(n, nkv, hd), rdk[0], atol=4e-2, rtol=4e-2)
     _close(dv.view(n, nkv, hd), rdv[0], atol=4e-2, rtol=4e-2)
+
+
+@pytest.mark.parametrize("M,F", [(300, 12288), (800, 6144), (1100, 512)])
+@pytest.mark.parametrize("what", ["base", "pitch", "residual"])
+def test_gemm_output_off_the_boundaries_of_whole_tiles(M, F, what):
+    """Token counts for which the planner takes two tiles per CTA, which only move whole tiles: an output or a residual that lies off the
+    16-byte boundaries takes a form that stores element by element.  Bound: one bf16 rounding of the sum, one of the result."""
+    Kc = _cuda()
+    Kd = 256
+    x, w = _rand(M, Kd, seed=1), _rand(F, Kd, scale=Kd ** -0.5, seed=2)
+    assert M > 1024 or Kc.plan_tiles(M, F, Kd, True, True)[0]
+    out = torch.empty(M * F + 8, dtype=torch.bfloat16, device="cuda")[1:M * F + 1].view(M, F) if what == "base" else \
+        torch.empty(M, F + 2, dtype=torch.bfloat16, device="cuda")[:, :F] if what == "pitch" else None
+    res = _rand(M * F + 1, seed=3)[1:].view(M, F) if what == "residual" else None
+    z = x.double() @ w.double().t()
+    ref = z if res is None else z + res.double()
+    for product, weight, kw in ((Kc.gemm, w, {}), (Kc.gemm_t, w.t().contiguous(), dict(w_t=True))):
+        got = product(x, weight, out=out, residual=res, **kw)
+        assert bool(((got.double() - ref).abs() <= 2.0 ** -8 * 1.01 * (z.abs() + ref.abs()) + 2e-5).all())
+        got.fill_(float("nan"))
+    Kc.check_status()
