@@ -158,25 +158,36 @@ def plan_gemm(M: int, F: int, K: int, R: int = 0, dual: bool = False):
 PAIR_AUTO = os.environ.get("TAH_B200_GEMM_PAIR", "1") != "0"
 
 
-@functools.lru_cache(maxsize=4096)
-def plan_tiles(M: int, rows: int, K: int, can_pair: bool, can_split: bool):
-    """``(pair, bn, splits)`` for more than 256 tokens: tiles of 128 or (pair) 256 features by 128, 192 or 256 tokens, whichever fills the
-    SMs' waves best by a cost model.
+# CTAs of a launch with clusters of four that run at once: a cluster lies in one group of SMs, and what is left of a group holds none (of 148
+# SMs 132 did run in one wave, 144 in two)
+CLUSTER4_CTAS = 132
 
-    Microseconds, 256 tokens always (paired from 1024 on) and the chosen form: 1500 tokens 67.4 and 41.1 (2048 x 6144), 30.0 and 18.0
-    (2048 x 2048); 3072 tokens 31.7 and 26.6 (2048 x 2048), 70.1 and 63.3 (2048 x 6144); 700 tokens 17.9 and 16.4 (4096 x 2048), 14.9 and
-    13.5 (2048 x 2048).  Over nine token counts from 300 to 13600 the choice was within 10 % of the best of all forms."""
+
+@functools.lru_cache(maxsize=4096)
+def plan_tiles(M: int, rows: int, K: int, can_pair: bool, can_split: bool, x_t: bool = False):
+    """``(pair, bn, splits)`` for more than 256 tokens: tiles of 128 features by 64 to 256 tokens or (pair) 256 features by 128 to 256,
+    whichever fills the SMs' waves best by a cost model.  ``x_t``: activations are read transposed (weight gradients).
+
+    The constants are fitted to every form at weights of 64 to 12288 rows, reductions of 300 to 12288 and 257 to 13600 tokens (weight and
+    data gradients to 4000): a wave takes a third of a microsecond per block of 64 of the reduction whatever the width of a one-tile form,
+    so wide tiles pay only where they save a wave.  The choice lies within 5 % of the best form everywhere, 0.1 % on average.  Microseconds, by
+    the plan for up to 256 tokens (256-token pairs from 1024 on) / by this one: 1536 x 2048 at 450 tokens 11.2 / 11.0, 2048 x 2048 at 1000
+    13.8 / 13.5, 4096 x 2048 at 400 14.3 / 13.8, 2048 x 6144 at 520 25.7 / 23.3, at 5200 136 / 117, its weight gradient over 940 tokens
+    46.4 / 35.5."""
     best = None
     for nf in (1, 2) if can_pair else (1,):
-        for bn in (128, 192, 256):
+        for bn in (64, 128, 192, 256) if nf == 1 else (128, 192, 256):
             for s in (1, 2, 4) if can_split and nf == 1 else (1,):
                 kb = -(-K // 64) / s
                 if s > 1 and (kb < 4 or not _fits(bn, s, 1)):
                     continue
-                waves = -(-(-(-rows // (128 * nf)) * -(-M // bn) * s) // SM_COUNT)
-                # microseconds per block of 64: tensor cores, and bytes into the SM at 87 KB/us
-                t_kb = max(0.39 * nf * bn / 256, (128 * nf + bn) * 0.125 / 87)
-                t = waves * (kb * t_kb + 0.5 + 0.005 * nf * bn / s + (1.5 + (s - 1) * bn / s * 0.5 / 19.0 if s > 1 else 0.0)) + 1.5
+                waves = -(-(-(-rows // (128 * nf)) * -(-M // bn) * s) // (CLUSTER4_CTAS if s == 4 else SM_COUNT))
+                # microseconds: the main loop, the epilogue, the exchange of split sums
+                if x_t:
+                    t_kb, out = (0.29 + 0.164 * bn / 256, 2.6 + 0.0195 * bn) if nf == 1 else (0.31 + 0.297 * bn / 256, 3.0 + 0.038 * bn)
+                else:
+                    t_kb, out = (0.31 + 0.03 * bn / 256, 2.0 + 0.0143 * bn) if nf == 1 else (0.345 + 0.235 * bn / 256, 2.0 + 0.022 * bn)
+                t = waves * (kb * t_kb + out + {1: 0.0, 2: 1.1 + 0.003 * bn, 4: 0.65 + 0.0133 * bn}[s])
                 if best is None or t < best[0] - 1e-9:
                     best = (t, nf == 2, bn, s)
     return best[1:]
@@ -392,7 +403,7 @@ def gemm_t(x: torch.Tensor, w: torch.Tensor, *, x_t: bool = False, w_t: bool = F
     can_pair = F % 256 == 0 and (not x_t or M % 64 == 0)
     if pair is None and bn == 0 and splits is None and M > 256:
         staged = _whole_pieces(out) and (residual is None or _whole_pieces(residual))
-        pair, bn, splits = plan_tiles(M, F, Kx, can_pair and PAIR_AUTO and staged, True)
+        pair, bn, splits = plan_tiles(M, F, Kx, can_pair and PAIR_AUTO and staged, True, x_t)
     pair = bool(pair) and can_pair
     if pair:
         bn, splits = bn or 256, 1

@@ -1107,3 +1107,25 @@ def test_gemm_output_off_the_boundaries_of_whole_tiles(M, F, what):
         assert bool(((got.double() - ref).abs() <= 2.0 ** -8 * 1.01 * (z.abs() + ref.abs()) + 2e-5).all())
         got.fill_(float("nan"))
     Kc.check_status()
+
+
+@pytest.mark.parametrize("M,F,T", [(320, 512, 300), (704, 256, 1000)])
+def test_gemm_tile_forms_of_weight_gradients(M, F, T):
+    """Both operands read transposed, added to what the output holds, in every form of the planner: unsplit ones give the same bits, split ones
+    stay within one rounding of the sum and one of the result.  Neither size is a multiple of the wider tiles."""
+    Kc = _cuda()
+    gy, x, grad = _rand(T, M, seed=1), _rand(T, F, scale=T ** -0.5, seed=2), _rand(M, F, seed=3)
+
+    def run(**kw):
+        out = grad.clone()
+        return Kc.gemm_t(gy, x, x_t=True, w_t=True, residual=out, out=out, **kw)
+    base = run(pair=False, bn=256, splits=1)
+    z = gy.double().t() @ x.double()
+    tol = 2.0 ** -8 * 1.01 * (z.abs() + (z + grad.double()).abs()) + 2e-5
+    assert bool(((base.double() - z - grad.double()).abs() <= tol).all())
+    for pair, bn in ((False, 64), (False, 128), (False, 192), (True, 128), (True, 192), (True, 256)):
+        assert torch.equal(run(pair=pair, bn=bn, splits=1), base), (pair, bn)
+    for bn, splits in ((64, 2), (64, 4), (128, 4), (192, 2), (192, 4), (256, 2)):
+        assert bool(((run(pair=False, bn=bn, splits=splits).double() - z - grad.double()).abs() <= tol).all()), (bn, splits)
+    assert bool(((run().double() - z - grad.double()).abs() <= tol).all())
+    Kc.check_status()

@@ -42,6 +42,8 @@ def test_config_merge_precedence(tmp_path):
 
 
 # ---- compaction -------------------------------------------------------------------------------------
+
+
 def test_gather_scatter_round_trip():
     g = torch.Generator().manual_seed(0)
     for _ in range(20):
@@ -68,6 +70,8 @@ def test_active_set_empty():
 
 
 # ---- duo-causal predicate --------------------------------------------------------------------------
+
+
 def test_duo_mask_matches_brute_force():
     g = torch.Generator().manual_seed(1)
     B, Tq, Tk = 2, 5, 9
@@ -100,6 +104,8 @@ def test_depth0_queries_never_see_deeper_kv():
 
 
 # ---- soft embedding / deciders ----------------------------------------------------------------------
+
+
 def test_topk_softmax_input_update():
     E = torch.randn(50, 8)
     logits = torch.randn(3, 50)
@@ -150,6 +156,8 @@ def test_mlp_decider_features_keys_and_persistence(tmp_path):
 
 
 # ---- losses -----------------------------------------------------------------------------------------
+
+
 def test_fixed_cross_entropy_normalisation():
     x, t = torch.randn(6, 9), torch.tensor([1, 2, -100, 4, -100, 0])
     ref_sum = torch.nn.functional.cross_entropy(x, t, ignore_index=-100, reduction="sum")
@@ -199,6 +207,8 @@ def test_next_token_loss_matches_shifted_ce():
 
 
 # ---- sampler ----------------------------------------------------------------------------------------
+
+
 def test_sampler_filters_in_order():
     logits = torch.log(torch.tensor([[0.5, 0.25, 0.15, 0.06, 0.04]]))
     g = torch.Generator().manual_seed(0)
@@ -214,6 +224,8 @@ def test_sampler_filters_in_order():
 
 
 # ---- forward bookkeeping ----------------------------------------------------------------------------
+
+
 def test_force_one_continuation_and_uniform_passes():
     model = tiny_tah(decider="MLPIterDecider",
                      decider_kwargs=dict(topk=10, hidden_states_size=256, hidden_states_layer_nums=[1, 4],
@@ -422,3 +434,16 @@ def test_adapter_factor_keeps_gradients_of_32_bit_factors():
         out.backward(gy)
         got.append([out.detach()] + [b.grad for b in blocks])
     assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+def test_tile_plan_counts_the_clusters_that_fit():
+    """Clusters of four do not fill every SM: no plan counts on a wave of more than 132 of their CTAs; a narrow weight gets narrow tiles."""
+    from tah_b200.ops import cuda
+    for rows in (64, 192, 512, 1024, 1536, 2048, 2560, 4096):
+        for K in (1024, 2048, 6144):
+            for M in range(257, 3000, 31):
+                pair, bn, splits = cuda.plan_tiles(M, rows, K, rows % 256 == 0, True)
+                ctas = -(-rows // 128) * -(-M // bn) * splits
+                assert splits < 4 or not 132 < ctas <= 148, (M, rows, K)
+    assert cuda.plan_tiles(1536, 64, 2048, False, True) == (False, 64, 4)
+    assert cuda.plan_tiles(450, 1536, 2048, True, True) == (False, 128, 2)
