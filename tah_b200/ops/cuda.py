@@ -309,7 +309,7 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
     if residual is not None:
         _check_bf16_2d(residual, "residual")
     if (not pair and bn == 0 and splits in (None, 1) and tp_push is None and tp_wait is None and
-            not ((swiglu or gelu) and (residual is not None or swiglu and gelu)) and _few_ok(x, w, x2, w2) and
+            not ((swiglu or gelu) and (residual is not None or swiglu and gelu)) and _few_ok(x, w, x2, w2, const_w and (swiglu or swiglu_interleaved)) and
             (not (gelu or swiglu_interleaved) or _whole_pieces(out))):
         return _gemm_few(x, w, out, residual, x2, w2, 1 if swiglu else 3 if gelu else 4 if swiglu_interleaved else 0, early=const_w)
     staged = tp_push is not None or (_whole_pieces(out) and (residual is None or _whole_pieces(residual)))
@@ -339,27 +339,32 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
     return out
 
 
-# Token count up to which the product is a stream of the weight (csrc/gemm_few.cu).  From 17 tokens on, a weight with more than 16384 rows
-# stays on the tensor-memory form: it has tiles for every SM and reads the activations once per 128 features (151936 x 2048 at 32
-# tokens: 125 us there, 131 us here; 12288 x 2048: 15.0 and 13.1 us).
-FEW_TOKENS, FEW_WIDE_TOKENS, FEW_WIDE_ROWS = 32, 16, 16384
+# Up to 16 tokens the product is a stream of the weight (csrc/gemm_few.cu).  From 17 to 32 tokens its CTAs hold four token tiles and fewer of
+# them fit an SM, and the tensor-memory form has the better time for weights that need a second wave of them: two CTAs of 8 warps per SM up to
+# 4736 rows (us, few / tensor memory at 24 tokens: 2048 x 6144 9.1 / 19.8, 4096 x 2048 6.6 / 9.9, 4096 x 4096 12.7 / 14.6; 6144 x 2048 11.6 / 9.6,
+# 8192 x 2048 12.4 / 10.1).  The SwiGLU weight of a decode tick, read ahead of the dependency wait, is level while one wave of three CTAs of 4
+# warps per SM holds it (12288 x 2048 15.0 / 15.0, not read ahead 15.8; 16384 x 2048 26 / 14.6).
+FEW_TOKENS, FEW_WIDE_TOKENS, FEW_WIDE_WAVE, FEW_GLU_WAVE = 32, 16, 2 * SM_COUNT, 3 * SM_COUNT
 # A narrow weight (an adapter's) has too few tensor-memory tiles to occupy the SMs at any token count: while tiles of 16 rows by 32 tokens
-# fit one wave, the few-token form is the faster one (64 x 2048 at 820 tokens 4.5 us, there 7.2; 192 x 2048 at 260 tokens 3.2 and 6.7; one
-# wave further 8.2 and 7.5, 7.7 and 7.3).
+# fit one wave, the few-token form is the faster one (64 x 2048 at 1184 tokens 3.5 us, there 6.9; 64 x 6144 7.2 and 12.2; 192 x 2048 at 300
+# tokens 3.4 and 6.8; 192 x 6144 7.0 and 12.2; a wave further 6.0 and 6.9, 12.7 and 12.3).
 
 
 def _whole_pieces(t: torch.Tensor) -> bool:
     return t.data_ptr() % 16 == 0 and t.stride(0) % 8 == 0
 
 
-def few_shape(M: int, rows: int, K: int, R: int = 0) -> bool:
-    """Whether a product of ``M`` tokens with a weight of ``rows`` rows takes the few-token form."""
-    few = M <= (FEW_WIDE_TOKENS if rows > FEW_WIDE_ROWS else FEW_TOKENS) or -(-rows // 16) * -(-M // 32) <= SM_COUNT
+def few_shape(M: int, rows: int, K: int, R: int = 0, const_glu: bool = False) -> bool:
+    """Whether a product of ``M`` tokens with a weight of ``rows`` rows takes the few-token form.  ``const_glu``: SwiGLU of a weight that is
+    read ahead of the dependency wait."""
+    few = (M <= FEW_WIDE_TOKENS or
+           M <= FEW_TOKENS and (-(-rows // 16) <= FEW_WIDE_WAVE or const_glu and K <= 2048 and -(-rows // 32) <= FEW_GLU_WAVE) or
+           -(-rows // 16) * -(-M // 32) <= SM_COUNT)
     return few and M > 0 and K > 0 and K % 64 == 0 and R % 64 == 0
 
 
-def _few_ok(x, w, x2=None, w2=None) -> bool:
-    return (few_shape(x.shape[0], w.shape[0], x.shape[1], 0 if x2 is None else x2.shape[1]) and
+def _few_ok(x, w, x2=None, w2=None, const_glu: bool = False) -> bool:
+    return (few_shape(x.shape[0], w.shape[0], x.shape[1], 0 if x2 is None else x2.shape[1], const_glu) and
             all(t is None or _whole_pieces(t) for t in (x, w, x2, w2)))
 
 
@@ -1482,7 +1487,7 @@ def packed_pass(weights, final_norm, h, xn, pools, k_own, v_own, seg_k, seg_v, b
 
     def plan(rows, K, R=0, glu=False):
         stacked, il = glu and not gu_interleaved, glu and gu_interleaved
-        if few_shape(n, rows, K, R):
+        if few_shape(n, rows, K, R, glu):
             return _ProductPlan(1, 4 if il else 1 if stacked else 0, 1, 0)
         pair, bn, splits = _plan_tiles(n, rows, K, R, stacked, False, il)
         return _ProductPlan(0, 1 if stacked else (6 if pair else 4) if il else 2 if pair else 0, splits, bn)

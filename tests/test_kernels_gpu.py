@@ -1129,3 +1129,20 @@ def test_gemm_tile_forms_of_weight_gradients(M, F, T):
         assert bool(((run(pair=False, bn=bn, splits=splits).double() - z - grad.double()).abs() <= tol).all()), (bn, splits)
     assert bool(((run().double() - z - grad.double()).abs() <= tol).all())
     Kc.check_status()
+
+
+@pytest.mark.parametrize("M,rows", [(17, 9504), (32, 12288), (32, 14208), (32, 14240)])
+def test_gemm_few_tokens_wide_swiglu(M, rows):
+    """SwiGLU of a weight that is read ahead, 17 to 32 tokens: the few-token form up to one wave of its CTAs, the tensor-memory form behind it;
+    bound as in test_gemm_few_tokens."""
+    Kc = _cuda()
+    x, w = _rand(M, 192, seed=1), _rand(rows, 192, scale=192 ** -0.5, seed=2)
+    assert Kc.few_shape(M, rows, 192, 0, True) == (rows <= 14208) and not Kc.few_shape(M, rows, 192)
+    z = x.double() @ w.double().t()
+    g, u = z[:, 0::2], z[:, 1::2]
+    ref, eps = torch.nn.functional.silu(g) * u, 2.0 ** -8
+    tol = 1.2 * eps * g.abs() * u.abs() + 4 * eps * ref.abs()
+    for const in (True, False):
+        out = Kc.gemm(x, w, swiglu_interleaved=True, const_w=const)
+        assert bool(((out.double() - ref).abs() <= 1.01 * tol + 2e-5).all())
+    Kc.check_status()
