@@ -7,7 +7,7 @@
 //   [page][2 (K,V)][n_kv_heads][page_size][HD]  bf16
 // with a page table pt[c][row][i] and a length len[c][row].
 //
-// Work split: an item is (KV head, row, split), one CTA; its pages go to its four (or two) warps in turn.  All G = nq / nkv query
+// Work split: an item is (KV head, row, split), one CTA; its pages go to its two to four warps in turn.  All G = nq / nkv query
 // heads that share the KV head are handled together, so K / V are read once, straight from global memory into the registers that
 // warp-level tensor instructions read (a page and a half of a warp's in flight; no shared memory ring):
 //
@@ -45,6 +45,9 @@ struct DecodeAttnParams {
 
 constexpr int ATT_PAGE = 16;
 
+// Warps of the decode kernel that fit an SM without spills.
+constexpr int att_resident_warps(int hd, int G) { return 3 * G > 8 ? (hd == 64 ? 12 : 8) : hd == 64 ? 16 : 12; }
+
 template <int HD, int G>
 struct AttCfg {
   static constexpr int STEPS = HD / 32;             // 16-byte pieces of a K row per lane
@@ -52,7 +55,7 @@ struct AttCfg {
   static constexpr int COLS = 3 * G;                // (part, head): see decode_attn_kernel
   static constexpr int TILES = (COLS + 7) / 8;
   static constexpr int PITCH = HD + 4;              // floats per column in the merge area
-  static constexpr int WARPS = TILES == 2 ? 8 : HD == 64 ? 16 : 12;      // resident per SM, without spills
+  static constexpr int WARPS = att_resident_warps(HD, G);
 };
 
 // Maps the i-th visible page of a row (pages of cache 0 first, then cache 1, ...) to its cache and
@@ -114,7 +117,7 @@ __global__ void __launch_bounds__(NW * 32, AttCfg<HD, G>::WARPS / NW) decode_att
   const int ppc = (total_pages + p.n_split - 1) / p.n_split;
   const int pb = split * ppc;
   const int pe = min(total_pages, pb + ppc);
-  const int n = pe - pb > warp ? (pe - pb - warp + NW - 1) / NW : 0;      // pages pb + warp, + 4, ... are this warp's
+  const int n = pe - pb > warp ? (pe - pb - warp + NW - 1) / NW : 0;      // pages pb + warp, + NW, ... are this warp's
 
   // 32 of the warp's pages at a time, one per lane: K block of this head, entries that are visible in it
   const __nv_bfloat16* blk = nullptr;
@@ -365,17 +368,46 @@ __global__ void __launch_bounds__(128) varlen_attn_naive_kernel(const VarlenAttn
     p.out[((size_t)t * p.nq + h) * HD + lane * EPL + i] = __float2bfloat16_rn(l > 0.f ? acc[i] / l : 0.f);
 }
 
+// Estimated cost of `items` (row, KV head) items of up to `pages` pages, every one cut into `split` parts of `warps` warps: microseconds when
+// all are that long plus microseconds when their lengths are spread.  A CTA takes the start of an item (length, page number, page: dependent
+// loads) and its warps' pages in turn, a page at its latency or, with enough warps on the chip, at its share of HBM; a split adds the merge
+// kernel.  Equal items run in waves; uneven ones fill the SMs as they end, and behind them the longest one stands alone.  Fitted to 1 to 256
+// rows of 60 to 2099 entries, equal and spread from a quarter to all of them, in all six geometries: the choice among 2 to 4 warps and 1 to 4
+// parts is 0.9 % behind the best for each on average.
+static double decode_estimate(int hd, int G, long long items, int pages, int split, int warps) {
+  constexpr double START = 4.5, HBM_KB = 6500.0, MEAN = 0.5, ALONE = 0.65;
+  const long long n = items * split, resident = 148ll * (att_resident_warps(hd, G) / warps);
+  const int whole = (pages + split - 1) / split;
+  const double steps = 0.5 * ((whole + warps - 1) / warps + (double)pages / split / warps);
+  const double latency = hd == 128 ? (3 * G > 8 ? 1.7 : 2.1) : (3 * G > 8 ? 1.45 : 1.9), page = ATT_PAGE * hd * 4 / 1000.0 / HBM_KB;
+  auto wave = [&](long long ctas) { return ctas > 0 ? START + steps * fmax(latency, ctas * warps * page) : 0.0; };
+  const double equal = n / resident * wave(resident) + wave(n % resident), moved = n * warps * steps * MEAN * page, turns = (double)n / resident;
+  const double spread = n <= resident ? START + fmax(steps * latency, moved)
+                                      : fmax(turns * (START + MEAN * steps * latency), turns * START + moved) + ALONE * (START + steps * latency);
+  return equal + spread + (split > 1 ? 2.0 * (6.2 + 0.0007 * n) : 0.0);
+}
+
+static int decode_warps(int hd, int G, long long items, int pages, int split) {
+  int best = 4;
+  for (int w = 3; w >= 2; --w)          // three of eight resident warps fit no more items than four: they are never taken there
+    if (decode_estimate(hd, G, items, pages, split, w) < decode_estimate(hd, G, items, pages, split, best)) best = w;
+  return best;
+}
+
+// Two to four warps per item, by the estimate: with four, 444 items of heads of 128 run at once, with three 592, with two 888.  Four / the
+// number taken, us, 8 KV heads of two heads of 128: 64 rows at 60 entries 10.2 / 8.0 (three), at 300 23.4 / 17.5, at 1024 61.6 / 46.1 (spread
+// from a quarter of that 41.8 / 39.5); 96 rows at 140 17.2 / 14.1 (two); 256 rows at 60 25.2 / 21.4 (two); 128 rows at 1024 96.6 / 87.7 (three;
+// spread 63.4 / 69.1, the other way round).
 template <int HD, int G>
 static int launch_decode(const DecodeAttnParams& p, cudaStream_t stream) {
   const dim3 grid(p.nkv, p.rows, p.n_split);
-  // Four warps per item.  Two where more items than four times the resident ones have at most ten pages per cache: the dependent
-  // loads at the start of an item then cost half the warps (256 rows x 8 heads at 80 entries 25.6 us, with four 29.9; at 600 entries
-  // 116 and 109).
   int pages = 0;
   for (int c = 0; c < p.n_caches; ++c) pages = p.max_pages[c] > pages ? p.max_pages[c] : pages;
-  const bool small = (long long)p.nkv * p.rows * p.n_split > 148ll * AttCfg<HD, G>::WARPS && pages <= 10;
-  cudaError_t e = small ? launch_chain(decode_attn_kernel<HD, G, 2>, grid, dim3(64), 0, stream, p)
-                        : launch_chain(decode_attn_kernel<HD, G, 4>, grid, dim3(128), 0, stream, p);
+  const int warps = decode_warps(HD, G, (long long)p.nkv * p.rows, pages, p.n_split);
+  constexpr int THREE = AttCfg<HD, G>::WARPS == 8 ? 4 : 3;
+  cudaError_t e = warps == 2   ? launch_chain(decode_attn_kernel<HD, G, 2>, grid, dim3(64), 0, stream, p)
+                  : warps == 3 ? launch_chain(decode_attn_kernel<HD, G, THREE>, grid, dim3(32 * THREE), 0, stream, p)
+                               : launch_chain(decode_attn_kernel<HD, G, 4>, grid, dim3(128), 0, stream, p);
   if (e == cudaSuccess && p.n_split > 1)
     e = launch_chain(decode_attn_merge_kernel<HD>, dim3(p.rows * p.nq), dim3(HD), 0, stream, p.ws, p.out, p.n_split);
   return e == cudaSuccess ? 0 : -3;
@@ -388,6 +420,23 @@ using namespace tahb;
 // Workspace floats needed by tahb_decode_attn when n_split > 1.
 extern "C" long long tahb_decode_attn_ws_floats(int rows, int nq, int hd, int n_split) {
   return n_split > 1 ? (long long)rows * nq * n_split * (hd + 2) : 0;
+}
+
+// The number of warps per item that a launch takes.
+extern "C" int tahb_decode_attn_warps(int rows, int nq, int nkv, int hd, int pages, int n_split) {
+  return decode_warps(hd, nq / nkv, (long long)rows * nkv, pages, n_split);
+}
+
+// How many parts (1 to 4) every (row, KV head) item is best cut into when rows hold up to `pages` pages; no launch, no GPU needed.
+extern "C" int tahb_decode_attn_split(int rows, int nq, int nkv, int hd, int pages) {
+  if (rows <= 0 || nkv <= 0 || nq < nkv) return 1;
+  const int G = nq / nkv;
+  const long long items = (long long)rows * nkv;
+  auto cost = [&](int s) { return decode_estimate(hd, G, items, pages, s, decode_warps(hd, G, items, pages, s)); };
+  int best = 1;
+  for (int s = 2; s <= 4; ++s)
+    if (cost(s) < cost(best)) best = s;
+  return best;
 }
 
 extern "C" int tahb_decode_attn(const void* q, void* out, void* const* caches, const int* const* page_tables,

@@ -453,17 +453,7 @@ class TaHEngine(DecodeEngine):
         s = self._alloc_scheduler_state(B, max_new)
         # split the KV walk of a row when (rows x local KV heads) CTAs would leave SM slots empty
         # (small batches, wide tensor-parallel groups); the partial results meet in a merge kernel
-        # one item per (row, KV head), 444 resident at once.  Few of them are split until they make up to two waves: with uneven rows and
-        # a quarter of the slots idle, 160 items in two took 30.9 us, in three 32.4 and in four 29.4 (in one 45)
-        items = max(1, B * w.nkv)
-        if items <= 296:
-            s.attn_split = min(4, 888 // items)
-        elif 444 < items <= 592 and self.kv.max_pages[0] > 64:
-            # just more than fit: the second wave of long rows would be nearly empty (64 rows at 2099 entries 121 us in one, 105 in two, 99
-            # in three and in four; at 1024 entries 63 and 56; 72 rows at 2099 125 in one, 105 in three)
-            s.attn_split = max(range(1, 5), key=lambda n: items * n / 444 / -(-items * n // 444))
-        else:
-            s.attn_split = 1
+        s.attn_split = K.decode_attn_split(B, w.nq, w.nkv, cfg.head_dim, max(self.kv.max_pages))
         s.attn_ws = None
         if s.attn_split > 1:
             n_ws = int(K.lib().tahb_decode_attn_ws_floats(B, w.nq, cfg.head_dim, s.attn_split))

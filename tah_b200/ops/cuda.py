@@ -1343,6 +1343,11 @@ def gla_recurrent(qkvg, low, w2, b2, norm_w, out, state, pos, row, **kw):
 # -------------------------------------------------------------------------------------------
 # attention
 # -------------------------------------------------------------------------------------------
+def decode_attn_split(rows: int, nq: int, nkv: int, hd: int, pages: int) -> int:
+    """How many parts :func:`decode_attn` best cuts every row into when rows hold up to ``pages`` pages of the cache."""
+    return int(lib().tahb_decode_attn_split(c_int(rows), c_int(nq), c_int(nkv), c_int(hd), c_int(pages)))
+
+
 def decode_attn(q, caches: Sequence[torch.Tensor], page_tables: Sequence[torch.Tensor], lens: Sequence[torch.Tensor],
                 depth, nq: int, nkv: int, hd: int, page_size: int, scale: float, out=None, n_split: int = 1,
                 ws: Optional[torch.Tensor] = None):

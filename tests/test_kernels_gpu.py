@@ -436,6 +436,44 @@ def test_decode_attention_more_items_than_ctas(hd, nq, nkv, n_split, shift):
         _close(out[r].view(nq, hd), ref, atol=1e-4, rtol=2 ** -8)
 
 
+@pytest.mark.parametrize("hd,nq,nkv", [(128, 8, 8), (128, 16, 8), (128, 16, 4), (64, 8, 8), (64, 16, 8), (64, 32, 8)])
+@pytest.mark.parametrize("warps", [2, 3, 4])
+def test_decode_attention_warps_per_item(hd, nq, nkv, warps):
+    """Two, three and four warps per item, as many rows as take that number: rows around page boundaries, empty ones, two caches; undefined
+    bits behind the last entry of a page stay out of the result."""
+    Kc = _cuda()
+    page, most = 16, 11
+    takes = lambda rows: Kc.lib().tahb_decode_attn_warps(rows, nq, nkv, hd, most, 1)
+    rows = next((r for r in range(20, 400) if takes(r) == warps), None)
+    if rows is None:
+        assert (hd, nq, nkv, warps) == (128, 16, 4, 3)      # eight warps per SM: as many items of four as of three
+        return
+    some0, some1 = [0, 1, 15, 16, 17, 140, 33, 160], [0, 5, 16, 17, 40]
+    lens0, lens1 = [some0[r * 5 % 8] for r in range(rows)], [some1[r % 5] for r in range(rows)]
+    c0, pt0, l0 = _paged_setup(rows, lens0, nkv, hd, page, 1)
+    c1, pt1, l1 = _paged_setup(rows, lens1, nkv, hd, page, 2)
+    for c, pt, lens in ((c0, pt0, lens0), (c1, pt1, lens1)):
+        for r, n in enumerate(lens):
+            if n % page:
+                c[int(pt[r, n // page]), :, :, n % page:] = float("nan")
+    assert pt0.shape[1] == most
+    depth = torch.tensor([r % 3 % 2 for r in range(rows)], dtype=torch.int32, device="cuda")
+    q = _rand(rows, nq * hd, seed=3)
+    scale = hd ** -0.5
+    out = Kc.decode_attn(q, [c0, c1], [pt0, pt1], [l0, l1], depth, nq, nkv, hd, page, scale)
+    Kc.check_status()
+    for r in range(rows):
+        n1 = lens1[r] if int(depth[r]) else 0
+        parts = [_gather_paged(c, pt[r], n, page) for c, pt, n in ((c0, pt0, lens0[r]), (c1, pt1, n1)) if n]
+        if not parts:
+            assert not out[r].any()
+            continue
+        k, v = (torch.cat(x).float().repeat_interleave(nq // nkv, dim=1) for x in zip(*parts))
+        ref = torch.einsum("hn,nhd->hd", torch.softmax(torch.einsum("hd,nhd->hn", q[r].view(nq, hd).float(), k) * scale, -1), v)
+        # fp32 inside, one rounding to bf16 (2^-8 of the value) at the end; fp32 sums of 200 terms of order one stay below 1e-4
+        _close(out[r].view(nq, hd), ref, atol=1e-4, rtol=2 ** -8)
+
+
 def test_varlen_attention_duo_segments():
     Kc = _cuda()
     nq, nkv, hd = 4, 2, 64

@@ -42,8 +42,6 @@ def test_config_merge_precedence(tmp_path):
 
 
 # ---- compaction -------------------------------------------------------------------------------------
-
-
 def test_gather_scatter_round_trip():
     g = torch.Generator().manual_seed(0)
     for _ in range(20):
@@ -70,8 +68,6 @@ def test_active_set_empty():
 
 
 # ---- duo-causal predicate --------------------------------------------------------------------------
-
-
 def test_duo_mask_matches_brute_force():
     g = torch.Generator().manual_seed(1)
     B, Tq, Tk = 2, 5, 9
@@ -104,8 +100,6 @@ def test_depth0_queries_never_see_deeper_kv():
 
 
 # ---- soft embedding / deciders ----------------------------------------------------------------------
-
-
 def test_topk_softmax_input_update():
     E = torch.randn(50, 8)
     logits = torch.randn(3, 50)
@@ -156,8 +150,6 @@ def test_mlp_decider_features_keys_and_persistence(tmp_path):
 
 
 # ---- losses -----------------------------------------------------------------------------------------
-
-
 def test_fixed_cross_entropy_normalisation():
     x, t = torch.randn(6, 9), torch.tensor([1, 2, -100, 4, -100, 0])
     ref_sum = torch.nn.functional.cross_entropy(x, t, ignore_index=-100, reduction="sum")
@@ -207,8 +199,6 @@ def test_next_token_loss_matches_shifted_ce():
 
 
 # ---- sampler ----------------------------------------------------------------------------------------
-
-
 def test_sampler_filters_in_order():
     logits = torch.log(torch.tensor([[0.5, 0.25, 0.15, 0.06, 0.04]]))
     g = torch.Generator().manual_seed(0)
@@ -224,8 +214,6 @@ def test_sampler_filters_in_order():
 
 
 # ---- forward bookkeeping ----------------------------------------------------------------------------
-
-
 def test_force_one_continuation_and_uniform_passes():
     model = tiny_tah(decider="MLPIterDecider",
                      decider_kwargs=dict(topk=10, hidden_states_size=256, hidden_states_layer_nums=[1, 4],
@@ -434,6 +422,21 @@ def test_adapter_factor_keeps_gradients_of_32_bit_factors():
         out.backward(gy)
         got.append([out.detach()] + [b.grad for b in blocks])
     assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+def test_decode_attention_split_follows_the_warps_that_fit():
+    """The split of the rows among CTAs is derived from how many the kernel keeps resident, which its geometry decides."""
+    from tah_b200.ops import cuda
+    if not os.path.exists(cuda._LIB_PATH):
+        pytest.skip("the library is not built")
+    split = lambda rows, nq, nkv, hd, pages: cuda.decode_attn_split(rows, nq, nkv, hd, pages)
+    for nq, hd in ((8, 128), (16, 128), (32, 128), (8, 64), (16, 64), (32, 64)):
+        at = [split(rows, nq, 8, hd, 70) for rows in range(1, 300)]
+        assert at[0] == 4 and all(1 <= s <= 4 for s in at)          # one row of 70 pages is spread as far as it goes
+        assert {split(rows, nq, 8, hd, 4) for rows in (1, 16, 64, 256)} == {1}      # four pages: a merge costs more than it gives
+    # 64 rows of 8 KV heads and few pages: one wave holds them with three warps where 12 are resident, with two of eight, with four of 16
+    warps = lambda nq, hd: cuda.lib().tahb_decode_attn_warps(64, nq, 8, hd, 6, 1)
+    assert [warps(16, 128), warps(32, 128), warps(16, 64), warps(32, 64)] == [3, 2, 4, 3]
 
 
 def test_tile_plan_counts_the_clusters_that_fit():
