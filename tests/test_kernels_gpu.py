@@ -1147,6 +1147,21 @@ def test_gemm_output_off_the_boundaries_of_whole_tiles(M, F, what):
     Kc.check_status()
 
 
+@pytest.mark.parametrize("M,H", [(1, 2048), (2, 2056), (7, 64), (8, 8192), (31, 2048), (33, 4096), (64, 2048), (64, 3000)])
+def test_rms_norm_bwd_of_few_rows_repeats_itself(M, H):
+    """Up to 64 rows are summed in a fixed order: the same bits every time; the weight gradient is a 32-bit sum over the rows."""
+    Kc = _cuda()
+    x, w, gy = _rand(M, H, seed=1), _rand(H, seed=2), _rand(M, H, seed=3)
+    first = Kc.rms_norm_bwd(x, w, gy, 1e-6)
+    for _ in range(20):
+        assert all(torch.equal(a, b) for a, b in zip(first, Kc.rms_norm_bwd(x, w, gy, 1e-6)))
+    xf, wf = x.double().requires_grad_(True), w.double().requires_grad_(True)
+    (wf * xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + 1e-6) * gy.double()).sum().backward()
+    _close(first[0], xf.grad, atol=1e-3, rtol=2.0 ** -8)
+    _close(first[1], wf.grad, atol=1e-5 * M, rtol=1e-5)
+    assert Kc.rms_norm_bwd(x, w, gy, 1e-6, want_gw=False)[1] is None
+
+
 @pytest.mark.parametrize("M,F,T", [(320, 512, 300), (704, 256, 1000)])
 def test_gemm_tile_forms_of_weight_gradients(M, F, T):
     """Both operands read transposed, added to what the output holds, in every form of the planner: unsplit ones give the same bits, split ones
