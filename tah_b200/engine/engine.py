@@ -34,6 +34,9 @@ from tah_b200.ops import cuda as K
 from tah_b200.utils.observe import nvtx_range
 
 
+KV_BLOCK_BYTES = 1 << 29
+
+
 def _fusions(default: str):
     """Kernel fusions selected by ``TAH_B200_FUSE``: "1" = all, "0" = none, or a comma list of "qkv" (QK-norm, RoPE
     and the K/V write in the QKV GEMM's epilogue) and "lora" (LoRA-A of the gated rows inside the RMSNorm launch);
@@ -231,8 +234,11 @@ class TaHEngine(DecodeEngine):
             tile_q0, tile_qn = K.attn_tiles(seq_counts, by_work=True)
         if tp is None and tensor_core_attn and not fuse_qkv and w.pass_weights is not None and (lora or depth == 0 or w.r == 0):
             # the plain form on one GPU: every launch of the pass from one native call
-            kv = bf(nL, 2, n, nkv * hd)
-            own = [(kv[li, 0], kv[li, 1]) for li in range(nL)]
+            # Keys and values of as many layers at once as KV_BLOCK_BYTES hold: few blocks make first calls on new lengths quick (twelve prompts
+            # of 45 to 5000 tokens in turn ask the driver for 292 blocks, with one per layer 436; 3100 tokens 34 and 121 ms), but a pass
+            # over tens of thousands of tokens must not need gigabytes in one piece.
+            step = max(1, min(nL, KV_BLOCK_BYTES // max(1, 4 * n * nkv * hd)))
+            own = [(kv[0], kv[1]) for li in range(0, nL, step) for kv in bf(min(step, nL - li), 2, n, nkv * hd)]
             taps = None if taps_out is None else {li: bf(n, cfg.hidden_size) for li in tap_layers if li < nL}
             K.packed_pass(w.pass_weights, w.final_norm, h, xn_buf, [self.kv.layer_pool(depth, li) for li in range(nL)], [k for k, _ in own],
                           [v for _, v in own], seg_k, seg_v, seg_base, seg_count, pos, slots, tile_q0, tile_qn, nq=nq, nkv=nkv, hd=hd,

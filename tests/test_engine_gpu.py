@@ -251,6 +251,29 @@ def test_native_pass_gives_the_bits_of_the_loop(head_dim, T):
     assert all(torch.equal(a, b) for x, y in zip(*outs) for a, b in zip(x, y))
 
 
+@pytest.mark.parametrize("layers", [1, 2, 100])
+def test_native_pass_keeps_keys_and_values_in_bounded_blocks(monkeypatch, layers):
+    """A block of memory holds the keys and values of as many layers as fit its bound, one at least; the pass gives the same bits."""
+    from tah_b200.engine import TaHEngine
+    from tah_b200.engine import engine as module
+    model = tiny_tah(max_iter=2, dtype=torch.bfloat16, head_dim=128, num_attention_heads=4, num_key_value_heads=2).cuda().eval()
+    ids = torch.randint(0, 1024, (2, 150), generator=torch.Generator().manual_seed(3)).cuda()
+    got = []
+    for bound in (module.KV_BLOCK_BYTES, layers * 4 * 300 * 256 + 1000):
+        monkeypatch.setattr(module, "KV_BLOCK_BYTES", bound)
+        eng = TaHEngine(model, max_rows=2, max_seq_len=200, use_cuda_graph=False)
+        seen, one_pass = [], eng._packed_pass
+
+        def spy(*a, **k):
+            seen.append(one_pass(*a, **k))
+            return seen[-1]
+        eng._packed_pass = spy
+        got.append((eng.prefill(ids, None, 1)[0], [t for pair in seen[0][1] for t in pair]))
+    assert all(torch.equal(a, b) for a, b in zip(got[0][1], got[1][1])) and torch.equal(got[0][0], got[1][0])
+    assert len(got[1][1]) == 2 * len(eng.w.layers)
+    assert max(t.untyped_storage().nbytes() for t in got[1][1]) == min(layers, len(eng.w.layers)) * 4 * 300 * 256
+
+
 def test_learned_mlp_decider_kernel_chain_matches_module_and_drives_the_engine():
     """``MLPIterDecider`` (tapped hidden states + sorted top-k logits -> residual MLP) as the engine's kernel chain
     against the PyTorch module, and a generation driven by it (no override)."""
