@@ -232,7 +232,8 @@ class TaHEngine(DecodeEngine):
         fuse_qkv = hd == 128 and "qkv" in _fusions("")
         if tensor_core_attn:
             tile_q0, tile_qn = K.attn_tiles(seq_counts, by_work=True)
-        if tp is None and tensor_core_attn and not fuse_qkv and w.pass_weights is not None and (lora or depth == 0 or w.r == 0):
+        native = w.native_pass() if tp is None and tensor_core_attn and not fuse_qkv and (lora or depth == 0 or w.r == 0) else None
+        if native is not None:
             # the plain form on one GPU: every launch of the pass from one native call
             # Keys and values of as many layers at once as KV_BLOCK_BYTES hold: few blocks make first calls on new lengths quick (twelve prompts
             # of 45 to 5000 tokens in turn ask the driver for 292 blocks, with one per layer 436; 3100 tokens 34 and 121 ms), but a pass
@@ -240,7 +241,7 @@ class TaHEngine(DecodeEngine):
             step = max(1, min(nL, KV_BLOCK_BYTES // max(1, 4 * n * nkv * hd)))
             own = [(kv[0], kv[1]) for li in range(0, nL, step) for kv in bf(min(step, nL - li), 2, n, nkv * hd)]
             taps = None if taps_out is None else {li: bf(n, cfg.hidden_size) for li in tap_layers if li < nL}
-            K.packed_pass(w.pass_weights, w.final_norm, h, xn_buf, [self.kv.layer_pool(depth, li) for li in range(nL)], [k for k, _ in own],
+            K.packed_pass(native, w.final_norm, h, xn_buf, [self.kv.layer_pool(depth, li) for li in range(nL)], [k for k, _ in own],
                           [v for _, v in own], seg_k, seg_v, seg_base, seg_count, pos, slots, tile_q0, tile_qn, nq=nq, nkv=nkv, hd=hd,
                           inter=w.inter, ranks=(w.r_qkv, w.r_o, w.r_gu, w.r_down) if lora else (0, 0, 0, 0),
                           gu_interleaved=w.gu_interleaved, page_size=self.page_size, eps=cfg.rms_norm_eps, theta=cfg.rope_theta, scale=scale,

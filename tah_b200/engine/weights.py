@@ -12,6 +12,7 @@ from __future__ import annotations
 from dataclasses import dataclass
 from typing import List, Optional
 
+import itertools
 import os
 
 import torch
@@ -21,6 +22,9 @@ from tah_b200.ops import cuda as K
 
 def _pad64(n: int) -> int:
     return (n + 63) // 64 * 64
+
+
+_EDITIONS = itertools.count()
 
 
 @dataclass
@@ -41,6 +45,10 @@ class LayerWeights:
     b_gu: Optional[torch.Tensor] = None
     a_down: Optional[torch.Tensor] = None
     b_down: Optional[torch.Tensor] = None
+
+    def __setattr__(self, name, value):
+        object.__setattr__(self, name, value)
+        object.__setattr__(self, "edition", next(_EDITIONS))      # no two states of any layer have the same
 
 
 def _lora_pair(lin, rows: Optional[torch.Tensor] = None, cols: Optional[torch.Tensor] = None):
@@ -136,8 +144,16 @@ class EngineWeights:
             lw.a_down, lw.b_down = _lora_pair(mlp.down_proj, cols=d_cols)
             self.layers.append(lw)
         self.pass_weights = K.pass_weights(self.layers)      # None: the layers' launches come one by one
+        self._pass_editions = [l.edition for l in self.layers]
         l0 = self.layers[0]
         width = lambda a: 0 if a is None else a.shape[0]
         self.r_qkv, self.r_o, self.r_gu, self.r_down = width(l0.a_qkv), width(l0.a_o), width(l0.a_gu), width(l0.a_down)
         if self.r > 0 and min(self.r_qkv, self.r_o, self.r_gu, self.r_down) == 0:
             raise NotImplementedError("the engine expects LoRA on all seven projections (target_modules='all-linear')")
+
+    def native_pass(self):
+        """The layers as :func:`K.packed_pass` takes them, with the tensors that they hold now, or None."""
+        now = [l.edition for l in self.layers]
+        if self.pass_weights is not None and now != self._pass_editions:
+            self.pass_weights, self._pass_editions = K.pass_weights(self.layers), now
+        return self.pass_weights

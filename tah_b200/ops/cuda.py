@@ -1443,14 +1443,15 @@ class _Pass(ctypes.Structure):
 
 
 def pass_weights(layers):
-    """The layers' weights as :func:`packed_pass` takes them, or None when one does not lie on a 16-byte boundary in contiguous rows.
+    """The layers' weights as :func:`packed_pass` takes them, or None when one is not bf16 or does not lie on a 16-byte boundary in
+    contiguous rows.
     Like a captured tick it stands for these tensors, and keeps them alive."""
     arr = (_PassWeights * len(layers))()
     arr.tensors = []
     for a, l in zip(arr, layers):
         for f, _ in _PassWeights._fields_:
             t = getattr(l, f)
-            if t is not None and (t.data_ptr() % 16 or not t.is_contiguous() or t.shape[-1] % 8):
+            if t is not None and (t.data_ptr() % 16 or not t.is_contiguous() or t.shape[-1] % 8 or t.dtype != torch.bfloat16):
                 return None
             setattr(a, f, 0 if t is None else t.data_ptr())
             arr.tensors.append(t)

@@ -424,6 +424,27 @@ def test_adapter_factor_keeps_gradients_of_32_bit_factors():
     assert all(torch.equal(a, b) for a, b in zip(*got))
 
 
+def test_native_pass_reads_the_tensors_that_the_layers_hold_now():
+    from tah_b200.engine.weights import EngineWeights
+    from tah_b200.ops import cuda
+    w = EngineWeights(tiny_tah(max_iter=2, dtype=torch.bfloat16).simple_base_model)
+    held = lambda: [[getattr(a, f) for f, _ in a._fields_] for a in w.native_pass()]
+    want = lambda: [[0 if getattr(l, f) is None else getattr(l, f).data_ptr() for f, _ in w.native_pass()._type_._fields_] for l in w.layers]
+    before = held()
+    assert before == want() and w.native_pass() is w.native_pass()
+    w.layers[1].w_o = w.layers[1].w_o.clone()
+    assert held() == want() != before
+    w.layers[0] = type(w.layers[0])(**{f: getattr(w.layers[1], f) for f, _ in w.native_pass()._type_._fields_})
+    assert held() == want()
+    ln1 = w.layers[1].ln1
+    for other in (torch.zeros(ln1.numel() + 1, dtype=torch.bfloat16)[1:], ln1.float()):       # off the boundary, another type: launch by launch
+        w.layers[1].ln1 = ln1
+        w.pass_weights = w.pass_weights or cuda.pass_weights(w.layers)
+        assert w.native_pass() is not None
+        w.layers[1].ln1 = other
+        assert w.native_pass() is None
+
+
 def test_decode_attention_split_follows_the_warps_that_fit():
     """The split of the rows among CTAs is derived from how many the kernel keeps resident, which its geometry decides."""
     from tah_b200.ops import cuda
