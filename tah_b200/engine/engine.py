@@ -155,9 +155,7 @@ class TaHEngine(DecodeEngine):
         if taps.shape[1] == n_taps * H:
             feats = torch.empty(M, (n_taps + 1) * H, dtype=torch.bfloat16, device=taps.device)
             feats[:, :n_taps * H].copy_(taps)
-        tv = getattr(self, "_mlp_tv", None)
-        if tv is None or tv.shape[0] < M:
-            tv = self._mlp_tv = torch.zeros(max(M, self.max_rows), 128, dtype=torch.bfloat16, device=taps.device)
+        tv = self._kept_rows("_mlp_tv", M, lambda n: torch.zeros(n, 128, dtype=torch.bfloat16, device=taps.device))
         tv[:M, :k].copy_(topk_vals[:, :k])
         ones = w["ones"][:M]
         K.gemm(tv[:M], w["lp"], x2=ones, w2=w["lp_b"], out=feats[:, n_taps * H:])
@@ -169,6 +167,16 @@ class TaHEngine(DecodeEngine):
             x = K.gemm(u, b["w2"], x2=ones, w2=b["b2"], residual=x, out=x)
         return K.layer_norm_dot(x, w["oln_w"], w["oln_b"], w["ow"], w["ob"], w["oeps"])
 
+    def _kept_rows(self, name: str, M: int, make):
+        """A buffer of at least ``M`` rows.  Captured ticks hold the address of the one that they were captured with, so a smaller one is kept
+        when a longer prompt asks for more (twice as many at least: together the kept ones are no larger than the last)."""
+        kept = self.__dict__.setdefault(name, [])
+        fit = next((t for t in kept if M <= t.shape[0]), None)
+        if fit is None:
+            fit = make(max(M, self.max_rows, 2 * kept[-1].shape[0] if kept else 0))
+            kept.append(fit)
+        return fit
+
     def _score_simple_mlp(self, dec: SimpleMLPIterDecider, taps: torch.Tensor) -> torch.Tensor:
         """The two-layer decider as kernels: tcgen05 GEMM for the first layer (its bias enters the fp32
         accumulation as a K-extension: a column of ones times the bias), then SiLU + dot + bias per row."""
@@ -178,14 +186,18 @@ class TaHEngine(DecodeEngine):
             return dec.score(taps).float()
         M = taps.shape[0]
         cache = getattr(self, "_dec_cache", None)
-        if cache is None or cache[0] is not w1 or cache[1].shape[0] < M:
-            ones = torch.zeros(max(M, self.max_rows), 64, dtype=torch.bfloat16, device=taps.device)
-            ones[:, 0] = 1
+        if cache is None or cache[0] is not w1:
             bias_ext = torch.zeros(w1.shape[0], 64, dtype=torch.bfloat16, device=taps.device)
             if dec.fc1.bias is not None:
                 bias_ext[:, 0] = dec.fc1.bias.detach()
-            cache = self._dec_cache = (w1, ones, bias_ext)
-        _, ones, bias_ext = cache
+            cache = self._dec_cache = (w1, bias_ext)
+        bias_ext = cache[1]
+
+        def column(n):
+            t = torch.zeros(n, 64, dtype=torch.bfloat16, device=taps.device)
+            t[:, 0] = 1
+            return t
+        ones = self._kept_rows("_dec_ones", M, column)
         x = taps if taps.is_contiguous() else taps.contiguous()
         h1 = K.gemm(x, w1.detach(), x2=ones[:M], w2=bias_ext)
         return K.decider_head(h1, dec.fc2.weight.detach()[0].contiguous(), dec.fc2.bias.detach() if dec.fc2.bias is not None else None)

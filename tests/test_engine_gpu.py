@@ -251,29 +251,6 @@ def test_native_pass_gives_the_bits_of_the_loop(head_dim, T):
     assert all(torch.equal(a, b) for x, y in zip(*outs) for a, b in zip(x, y))
 
 
-@pytest.mark.parametrize("layers", [1, 2, 100])
-def test_native_pass_keeps_keys_and_values_in_bounded_blocks(monkeypatch, layers):
-    """A block of memory holds the keys and values of as many layers as fit its bound, one at least; the pass gives the same bits."""
-    from tah_b200.engine import TaHEngine
-    from tah_b200.engine import engine as module
-    model = tiny_tah(max_iter=2, dtype=torch.bfloat16, head_dim=128, num_attention_heads=4, num_key_value_heads=2).cuda().eval()
-    ids = torch.randint(0, 1024, (2, 150), generator=torch.Generator().manual_seed(3)).cuda()
-    got = []
-    for bound in (module.KV_BLOCK_BYTES, layers * 4 * 300 * 256 + 1000):
-        monkeypatch.setattr(module, "KV_BLOCK_BYTES", bound)
-        eng = TaHEngine(model, max_rows=2, max_seq_len=200, use_cuda_graph=False)
-        seen, one_pass = [], eng._packed_pass
-
-        def spy(*a, **k):
-            seen.append(one_pass(*a, **k))
-            return seen[-1]
-        eng._packed_pass = spy
-        got.append((eng.prefill(ids, None, 1)[0], [t for pair in seen[0][1] for t in pair]))
-    assert all(torch.equal(a, b) for a, b in zip(got[0][1], got[1][1])) and torch.equal(got[0][0], got[1][0])
-    assert len(got[1][1]) == 2 * len(eng.w.layers)
-    assert max(t.untyped_storage().nbytes() for t in got[1][1]) == min(layers, len(eng.w.layers)) * 4 * 300 * 256
-
-
 def test_learned_mlp_decider_kernel_chain_matches_module_and_drives_the_engine():
     """``MLPIterDecider`` (tapped hidden states + sorted top-k logits -> residual MLP) as the engine's kernel chain
     against the PyTorch module, and a generation driven by it (no override)."""
@@ -400,3 +377,60 @@ def test_kv_guard_pages_stay_untouched(monkeypatch):
     prompts = [torch.randint(0, 1024, (n,), generator=g) for n in (9, 30, 14, 5, 21)]
     eng.serve(prompts, max_new_tokens=12, rows=2, check_every=4)
     assert eng.kv.check_guards()
+
+
+@pytest.mark.parametrize("layers", [1, 2, 100])
+def test_native_pass_keeps_keys_and_values_in_bounded_blocks(monkeypatch, layers):
+    """A block of memory holds the keys and values of as many layers as fit its bound, one at least; the pass gives the same bits."""
+    from tah_b200.engine import TaHEngine
+    from tah_b200.engine import engine as module
+    model = tiny_tah(max_iter=2, dtype=torch.bfloat16, head_dim=128, num_attention_heads=4, num_key_value_heads=2).cuda().eval()
+    ids = torch.randint(0, 1024, (2, 150), generator=torch.Generator().manual_seed(3)).cuda()
+    got = []
+    for bound in (module.KV_BLOCK_BYTES, layers * 4 * 300 * 256 + 1000):
+        monkeypatch.setattr(module, "KV_BLOCK_BYTES", bound)
+        eng = TaHEngine(model, max_rows=2, max_seq_len=200, use_cuda_graph=False)
+        seen, one_pass = [], eng._packed_pass
+
+        def spy(*a, **k):
+            seen.append(one_pass(*a, **k))
+            return seen[-1]
+        eng._packed_pass = spy
+        got.append((eng.prefill(ids, None, 1)[0], [t for pair in seen[0][1] for t in pair]))
+    assert all(torch.equal(a, b) for a, b in zip(got[0][1], got[1][1])) and torch.equal(got[0][0], got[1][0])
+    assert len(got[1][1]) == 2 * len(eng.w.layers)
+    assert max(t.untyped_storage().nbytes() for t in got[1][1]) == min(layers, len(eng.w.layers)) * 4 * 300 * 256
+
+
+@pytest.mark.parametrize("decider", ["SimpleMLPIterDecider", "MLPIterDecider"])
+def test_decider_buffers_of_a_tick_stay_where_they_are(monkeypatch, decider):
+    """Captured ticks hold the addresses of the decider's buffers: a prompt with more tokens than the engine has rows leaves them alone."""
+    from tah_b200.engine import TaHEngine
+    from tah_b200.engine import engine as module
+    kw = dict(hidden_states_size=256, inner_size=64, threshold=0.5) if decider.startswith("Simple") else \
+        dict(hidden_states_size=256, topk=100, hidden_states_layer_nums=[1, 3, 4], hidden_dims=[128, 128, 128])
+    with torch.random.fork_rng():
+        model = tiny_tah(max_iter=2, dtype=torch.bfloat16, decider=decider, decider_kwargs=kw)
+    model = model.cuda().to(torch.bfloat16).eval()
+    eng = TaHEngine(model, max_rows=4, max_seq_len=64, use_cuda_graph=False, deep_fraction=1.0)
+    dec, seen, gemm = eng._decider()[1], [], module.K.gemm
+    def spy(x, w, **k):
+        own = [x] if not decider.startswith("Simple") and not seen else []          # the first product's sorted logits lie in such a buffer
+        seen.append([t.data_ptr() for t in (w, k["x2"], k["w2"], *own)])
+        return gemm(x, w, **k)
+    monkeypatch.setattr(module.K, "gemm", spy)
+
+    def score(rows):
+        width = len(eng._tap_layers()) * 256
+        taps = torch.ones(rows, width, dtype=torch.bfloat16, device="cuda")
+        del seen[:]
+        if decider.startswith("Simple"):
+            eng._score_simple_mlp(dec, taps)
+        else:
+            eng._score_mlp(dec, taps, torch.ones(rows, 128, device="cuda"))
+        return [list(a) for a in seen]
+    first = score(2)
+    assert first
+    score(50)
+    keep = [torch.empty(n, dtype=torch.uint8, device="cuda") for n in (512, 4096, 8192, 65536) for _ in range(50)]      # takes what was freed
+    assert score(2) == first and keep
