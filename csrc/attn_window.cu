@@ -663,9 +663,10 @@ __global__ void __launch_bounds__(128) window_decode_merge_kernel(const WindowAt
 // structure as prefill_attn_kernel - S = Q K^T and O += P V by tcgen05 with S (two buffers) and O in tensor memory, a softmax
 // thread per query, lazily refreshed maximum, TMA ring - with K / V fetched page by page from the cache
 // (four 16-row boxes per 64-key block form one swizzled tile; dims past dk / dv and pages past the last key read as
-// zeros) and with the distance bias added to the scores in registers.  Two heads (an even number per KV head, dims up to 128) read a
-// block once and have four stages where two CTAs of one head have two each, whose latency then stands in every block.
-// 7500 tokens of 16 heads on 8 KV heads: 195 us with one head, 161 with two, 153 with the long tiles of all heads first.
+// zeros) and with the distance bias added to the scores in registers.  Two heads per CTA read a block once and have four stages where two CTAs
+// of one head have two each; that pays where long portions make more than one wave (the caller's rule), and holds up short ones.
+// us, 16 heads of 128 on 8 KV heads, two threads per query / one head / two heads: 100 tokens 9.9 / 9.1 / 11.7, 700 26.7 / 23.7 / 27.6, two portions
+// of 2048 95.4 / 82.4 / 71.2, four 164 / 136 / 126; with a score cap 172 / 137 / 145.
 // Warp roles: warp 0 TMA, warp 1 tensor memory + MMA, four warps per head softmax / epilogue.
 // ---------------------------------------------------------------------------------------------
 struct WindowTiles {
@@ -676,6 +677,7 @@ struct WindowTiles {
                               // token, and a page is 16 consecutive rows
   const int* pool_base;       // [n_tiles] first page (16 rows) of the tile's row in the matrix of pooled blocks
   int n_pool_pages;
+  int heads;                  // query heads per CTA: 1, or 2 where the launcher has that form (see window_prefill_kernel)
 };
 
 // TIED: a stage holds keys only (and their factors, 64 floats behind all stages), which the second product reads too.
@@ -903,6 +905,7 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const float far_bias = bias == nullptr ? 0.f : bias[p.far];
     const float slope = p.slope == nullptr ? 0.f : p.slope[head];
     const int blocks = pooled ? visible_blocks(i, p.window, p.pool) : 0;
+    const float gate = p.gate != nullptr && row_ok ? gate_of(p, q0 + row, head) : 0.f;
     float m_ref = -INFINITY, l = 0.f;
     for (int n = 0; n < total_blocks; ++n) {
       mbar_wait(&s_full[2 * hi + (n & 1)], (n >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
@@ -1003,14 +1006,26 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       tc_fence_before();
       mbar_arrive(&p_ready[hi]);
     }
+    // the element gates of 32 dims are on their way while the last product runs, then while the 32 before them are written
+    uint4 z_in[4];
+    auto fetch_gates = [&](int c) {
+      const __nv_bfloat16* z = reinterpret_cast<const __nv_bfloat16*>(p.wide_gate) + (size_t)(q0 + row) * p.ld_gate + (size_t)head * p.dv + c;
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+        if (row_ok && c + v * 8 < p.dv) z_in[v] = *reinterpret_cast<const uint4*>(z + v * 8);
+    };
+    if (p.wide_gate != nullptr) fetch_gates(0);
     if (total_blocks > 0) mbar_wait(&pv_done[hi], (total_blocks - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
     tc_fence_after();
-    const float inv = row_ok ? finish_scale(p, q0 + row, head, m_ref, l) : 0.f;
+    float inv = row_ok ? finish_mass(p, head, m_ref, l) : 0.f;
+    if (p.gate != nullptr) inv *= sigmoid_f(gate);
     __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)(q0 + row) * p.ld_out + (size_t)head * p.dv;
 #pragma unroll 1
     for (int c = 0; c < HV * 64; c += 32) {
       float o[32];
       tmem_ld32(my_o + lane_off + c, o);
+      const uint4 z_now[4] = {z_in[0], z_in[1], z_in[2], z_in[3]};
+      if (p.wide_gate != nullptr && c + 32 < HV * 64) fetch_gates(c + 32);
       tmem_ld_wait();
       if (row_ok) {
 #pragma unroll
@@ -1020,7 +1035,7 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&pk);
             if (p.wide_gate != nullptr) {
               float z[8];
-              load8(reinterpret_cast<const __nv_bfloat16*>(p.wide_gate) + (size_t)(q0 + row) * p.ld_gate + (size_t)head * p.dv + c + v * 8, z);
+              load8(reinterpret_cast<const __nv_bfloat16*>(&z_now[v]), z);
 #pragma unroll
               for (int e = 0; e < 8; ++e) o[v * 8 + e] = __fdividef(o[v * 8 + e], 1.0f + __expf(-z[e]));
             }
@@ -1087,8 +1102,8 @@ static int launch_window_prefill_heads(const CUtensorMap& mq, const CUtensorMap&
 template <int HK, int HV, bool CAP, bool TIED = false>
 static int launch_window_prefill_as(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                                     const WindowAttnParams& p, const WindowTiles& tl, int n_tiles, cudaStream_t stream) {
-  if constexpr (HK <= 2 && HV <= 2) {
-    if ((p.nq / p.nkv) % 2 == 0) return launch_window_prefill_heads<HK, HV, CAP, TIED, 2>(mq, mk, mv, p, tl, n_tiles, stream);
+  if constexpr (HK == 2 && HV == 2 && !CAP) {
+    if (tl.heads == 2) return launch_window_prefill_heads<HK, HV, CAP, TIED, 2>(mq, mk, mv, p, tl, n_tiles, stream);
   }
   return launch_window_prefill_heads<HK, HV, CAP, TIED, 1>(mq, mk, mv, p, tl, n_tiles, stream);
 }
@@ -1195,14 +1210,16 @@ extern "C" int tahb_window_attn_decode(const WindowAttnParams* p, cudaStream_t s
 // Query tiles of portions; n_pages = pages of the layer's pool; kv_ld: see WindowTiles.  bias and sink in log2 units.
 // Tied layers with pooled blocks: p->pooled is a matrix [16 * n_pool_pages, nkv * dk] whose page pool_base[tile] is the first of the
 // tile's row.
+// heads: query heads per CTA, 1 or (an even number per KV head, dims of 65 to 128, no score cap) 2.
 extern "C" int tahb_window_attn_tiles(const WindowAttnParams* p, const int* q0, const int* qn, int n_tiles, int n_pages,
-                                      long long kv_ld, const int* pool_base, int n_pool_pages, cudaStream_t stream) {
+                                      long long kv_ld, const int* pool_base, int n_pool_pages, int heads, cudaStream_t stream) {
   if (p->n <= 0 || n_tiles <= 0) return 0;
   if (check_window_attn(p) || p->ld_out % 8 || (p->wide_gate != nullptr && (p->ld_gate % 8 || (reinterpret_cast<uintptr_t>(p->wide_gate) & 15))))
     return -2;
   if (kv_ld != 0 && kv_ld < (long long)p->nkv * (p->dk + p->dv)) return -2;
   if (p->tied && (kv_ld != 0 || n_pages < 1 || (p->pooled != nullptr && pool_base == nullptr))) return -2;
   if (p->page_size != WD_PAGE) return -5;
+  if (heads != 1 && (heads != 2 || (p->nq / p->nkv) % 2 || p->dk <= 64 || p->dk > 128 || p->dv <= 64 || p->dv > 128 || p->softcap > 0.f)) return -2;
   const size_t page_elems = (size_t)p->nkv * WD_PAGE * (p->dk + (p->tied ? 0 : p->dv));
   CUtensorMap mq, mk, mv;
   int rc;
@@ -1221,7 +1238,7 @@ extern "C" int tahb_window_attn_tiles(const WindowAttnParams* p, const int* q0, 
     if (!p->tied && (rc = make_page_map(&mv, kv + (size_t)p->nkv * WD_PAGE * p->dk, p->dv, p->nkv, n_pages, p->dv, (size_t)WD_PAGE * p->dv,
                             page_elems))) return rc;
   }
-  WindowTiles tl{q0, qn, n_pages, kv_ld, pool_base, n_pool_pages};
+  WindowTiles tl{q0, qn, n_pages, kv_ld, pool_base, n_pool_pages, heads};
   const int hk = p->dk <= 64 ? 1 : p->dk <= 128 ? 2 : 4, hv = p->dv <= 64 ? 1 : p->dv <= 128 ? 2 : 4;
   if (p->softcap == 0.f && p->dk > 128 && p->dk <= 192 && p->dv <= 128)
     return p->dv <= 64 ? launch_window_prefill_as<3, 1, false>(mq, mk, mv, *p, tl, n_tiles, stream)

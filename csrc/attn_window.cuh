@@ -96,18 +96,23 @@ template <> struct Row8<__nv_bfloat16> { using type = uint4; };
 constexpr int WD_PAGE = 16;
 constexpr float LOG2E = 1.4426950408889634f;
 
-// o = sum / (mass + exp2(sink - m)), times the head's gate; m, mass, sink in log2 units
-__device__ __forceinline__ float finish_scale(const WindowAttnParams& p, int t, int h, float m, float mass) {
+// o = sum / (mass + exp2(sink - m)); m, mass, sink in log2 units
+__device__ __forceinline__ float finish_mass(const WindowAttnParams& p, int h, float m, float mass) {
   float f = 1.0f;
   if (p.sink != nullptr) {
     const float top = fmaxf(m, p.sink[h]);
     f = exp2f(m - top);
     mass = mass * f + exp2f(p.sink[h] - top);
   }
-  f = mass > 0.f ? f / mass * p.out_scale : 0.f;
-  if (p.gate != nullptr)
-    f *= sigmoid_f(__bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.gate)[(size_t)t * p.ld_gate + h]));
-  return f;
+  return mass > 0.f ? f / mass * p.out_scale : 0.f;
+}
+__device__ __forceinline__ float gate_of(const WindowAttnParams& p, int t, int h) {      // pre-activation
+  return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.gate)[(size_t)t * p.ld_gate + h]);
+}
+// the same, times the head's gate
+__device__ __forceinline__ float finish_scale(const WindowAttnParams& p, int t, int h, float m, float mass) {
+  const float f = finish_mass(p, h, m, mass);
+  return p.gate != nullptr ? f * sigmoid_f(gate_of(p, t, h)) : f;
 }
 
 // factor of output element d of head h from its own gate

@@ -279,7 +279,7 @@ class HybridEngine(DecodeEngine):
                 kw["pooled"] = None if rows == 0 else K.pool_gather(kw["pooled"], src, m.nkv, m.dk, kw["pool_rows"],
                                                                     b.pooled[:rows * m.nkv * m.dk].view(rows, m.nkv * m.dk))
                 kw["pool_base"] = base
-            K.window_attn_tiles(q, o, pool, pt, plan.pos, plan.row, plan.tile_q0, plan.tile_qn, self.kv.n_pages[0], **kw)
+            K.window_attn_tiles(q, o, pool, pt, plan.pos, plan.row, plan.tile_q0, plan.tile_qn, self.kv.n_pages[0], longest=plan.longest, **kw)
         return o
 
     def _branches(self, li: int, m: BranchesLayer, proj: torch.Tensor, b: _Buffers, plan: _Plan) -> torch.Tensor:

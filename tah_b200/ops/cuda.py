@@ -922,20 +922,33 @@ def window_attn_decode(q, out, pool, page_table, pos, row, **kw):
     return out
 
 
-def window_attn_tiles(q, out, pool, page_table, pos, row, tile_q0, tile_qn, n_pages: int, kv_ld: int = 0, pool_base=None, **kw):
+def two_heads_per_cta(n_tiles: int, nq: int, nkv: int, longest: int) -> bool:
+    """Whether tiles of two query heads of a KV head pay in attention over sequences of up to ``longest`` tokens: they read a key block once and
+    have more of them in flight, but halve the CTAs, and what one head's product hides of the other's arithmetic needs several blocks.  So
+    long sequences (five tiles) in more than one wave of one-head CTAs, of which two fit an SM."""
+    return (nq // nkv) % 2 == 0 and longest > 4 * 128 and n_tiles * nq > 2 * SM_COUNT
+
+
+def window_attn_tiles(q, out, pool, page_table, pos, row, tile_q0, tile_qn, n_pages: int, kv_ld: int = 0, pool_base=None, longest: int = 0,
+                      heads: Optional[int] = None, **kw):
     """Windowed attention of prompt portions on the tensor cores (bf16, pages of 16): tiles of up to 128 consecutive
     tokens of one row.  ``bias``, ``sink`` and ``slope`` in log2 units.  ``kv_ld``: ``pool`` is not a paged cache but a matrix of that
     pitch whose rows ``[keys of all heads | values of all heads]`` are a token each, 16 of them a page.  ``wide_gate``: gate
     pre-activations of every output element (``gate``: of every head).  ``pooled`` is then the matrix of :func:`pool_gather`, and
-    ``pool_base`` the first of its pages of 16 rows that belongs to a tile's row."""
+    ``pool_base`` the first of its pages of 16 rows that belongs to a tile's row.  ``longest``: tokens of the longest portion, if known;
+    ``heads``: query heads per CTA (default: by :func:`two_heads_per_cta`; a score cap, pooled blocks and dims up to 64 were never faster
+    in pairs)."""
     a = window_attn_args(q, out, pool, page_table, pos, row, **kw)
     pooled = kw.get("pooled")
     _rc(lib().tahb_window_attn_tiles(ctypes.byref(a), _p(tile_q0), _p(tile_qn), c_int(tile_q0.numel()), c_int(n_pages),
-                                     c_ll(kv_ld), _p(pool_base), c_int(0 if pooled is None else pooled.shape[0] // 16), _stream()),
+                                     c_ll(kv_ld), _p(pool_base), c_int(0 if pooled is None else pooled.shape[0] // 16), c_int(heads), _stream()),
         "tahb_window_attn_tiles")
     return out
 
 
+    if heads is None:
+        heads = 2 if (two_heads_per_cta(tile_q0.numel(), kw["nq"], kw["nkv"], longest) and not kw.get("softcap") and pooled is None and
+                      64 < kw["dk"] <= 128 and 64 < kw["dv"] <= 128) else 1
 class _TiedKeys(ctypes.Structure):
     _fields_ = [(n, c_void_p) for n in ("k", "cache", "pooled", "slot", "pos", "row", "page_table")] + \
                [(n, c_int) for n in ("M", "nkv", "dk", "page_size", "max_pages", "pool", "pool_rows")] + [("ld", c_ll)]

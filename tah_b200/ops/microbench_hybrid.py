@@ -49,7 +49,7 @@ def bench_window_prefill(a):
     q0 = [b * T + t for b in range(B) for t in range(0, T, 128)]
     qn = [min(128, T - t) for b in range(B) for t in range(0, T, 128)]
     q0, qn, kw = _i32(q0), _i32(qn), _window_kw(a)
-    fn = lambda i: K.window_attn_tiles(q, out, pool, pt, pos, row, q0, qn, pool.shape[0], gate=gate, **kw)
+    fn = lambda i: K.window_attn_tiles(q, out, pool, pt, pos, row, q0, qn, pool.shape[0], gate=gate, longest=T, **kw)
     pairs = B * sum(_visible(i, a) for i in range(T))
     res = {"op": "window_prefill", "seqs": B, "T": T, "window": a.window, "keep": a.keep}
     return res, fn, 4.0 * pairs * a.nq * a.hd, n * (2 * a.nq + 2 * a.nkv) * a.hd * 2
@@ -99,7 +99,7 @@ def bench_tied_prefill(a):
     else:
         kw["wide_gate"] = _bf(n, a.nq * a.hd)
     q0, qn = _i32(q0), _i32(qn)
-    fn = lambda i: K.window_attn_tiles(q, out, pool, pt, pos, row, q0, qn, pool.shape[0], **kw)
+    fn = lambda i: K.window_attn_tiles(q, out, pool, pt, pos, row, q0, qn, pool.shape[0], longest=T, **kw)
     pairs = B * sum(_visible(i, a) + _blocks(i, a) for i in range(T))
     res = {"op": "tied_prefill", "seqs": B, "T": T, "window": a.window, "block": a.block}
     return res, fn, 4.0 * pairs * a.nq * a.hd, n * (2 * a.nq + a.nkv + (0 if a.block else a.nq)) * a.hd * 2

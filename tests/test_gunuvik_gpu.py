@@ -154,6 +154,38 @@ def test_windowed_attention_kernels(kernel, case, peaked):
     check_ok()
 
 
+@pytest.mark.parametrize("tied", [False, True])
+@pytest.mark.parametrize("window", [70, 2 ** 31 - 1])
+def test_windowed_attention_two_heads_per_cta(tied, window):
+    """Portions with two query heads per CTA: the same products in the same order as with one, so the same bits (biases, sink and gate of a
+    head; keys that are the values, with factors, slopes and element gates)."""
+    from tah_b200.ops import cuda as K
+    T, nq, G, d = 700, 8, 2, 104
+    g = torch.Generator(device="cuda").manual_seed(2)
+    rnd = lambda *shape: torch.randn(*shape, generator=g, device="cuda").to(BF16)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    pages = T // 16 + 1
+    pool, pt = rnd(pages, (1 if tied else 2) * G * 16 * d), i32([list(range(pages))])
+    kw = dict(nq=nq, nkv=G, dk=d, dv=d, page_size=16, scale=d ** -0.5, window=window, keep_first=0 if tied else 3)
+    if tied:
+        kw.update(tied=True, factor=torch.rand(pages, 16, generator=g, device="cuda"), slope=torch.rand(nq, generator=g, device="cuda") * 0.05,
+                  wide_gate=rnd(T, nq * d))
+    else:
+        kw.update(bias=torch.randn(nq, 33, generator=g, device="cuda"), sink=torch.randn(nq, generator=g, device="cuda"), gate=rnd(T, nq))
+    q = rnd(T, nq * d)
+    for a, b in ((0, T), (37, T), (500, 629)):
+        n, t0, out = b - a, list(range(0, b - a, 128)), []
+        part = dict(kw, **{x: kw[x][a:b] for x in ("gate", "wide_gate") if x in kw})
+        for heads in (1, 2):
+            out.append(torch.zeros(n, nq * d, dtype=BF16, device="cuda"))
+            K.window_attn_tiles(q[a:b], out[-1], pool, pt, i32(list(range(a, b))), i32([0] * n), i32(t0), i32([min(128, n - x) for x in t0]), pages,
+                                heads=heads, **part)
+        check_ok()
+        assert out[0].isfinite().all() and out[0].any() and torch.equal(*out)
+    with pytest.raises(RuntimeError):
+        K.window_attn_tiles(q[:9], out[0][:9], pool, pt, i32(list(range(9))), i32([0] * 9), i32([0]), i32([9]), pages, heads=2, **dict(part, nkv=nq))
+
+
 def test_attention_options_absent():
     """No bias, no sink, no gate: ordinary causal softmax attention."""
     from tah_b200.engine.hybrid import NO_WINDOW
