@@ -5,14 +5,14 @@
 //
 // Two kernels, both recompute S and dP per block with tcgen05.mma from TMA-staged tiles:
 //
-//   attn_bwd_dq_kernel   one CTA per (128-query tile, two query heads of a KV head; one where their number
-//                        is odd), the forward's loop over 64-key blocks of up to three KV segments.  S and dP
-//                        in tensor memory, dS written to shared memory (K-major) by 256 threads per head,
-//                        dQ += dS K with K consumed MN-major.  One head's arithmetic runs under the other's
-//                        products, and the next block is loaded meanwhile: with a head per CTA, two CTAs per SM
-//                        and room for one K / V block each, its latency stood in every block.
-//                        16 heads on 8 KV heads, 3072 tokens in training: 231 us before, 213 with two heads, 179 with
-//                        the long tiles of all heads first.
+//   attn_bwd_dq_kernel   one CTA per (128-query tile, query head, or two heads of a KV head), the forward's loop over
+//                        64-key blocks of up to three KV segments.  S and dP in tensor memory, dS written to shared
+//                        memory (K-major) by 256 threads per head, dQ += dS K with K consumed MN-major.  With a head
+//                        per CTA, two CTAs per SM and room for one K / V block each, a block's latency stands in
+//                        every block; with two heads one's arithmetic runs under the other's products and the next
+//                        block is loaded meanwhile, which pays for long sequences in more than a wave (the rule and
+//                        its figures: tah_b200/ops/cuda.py).  The long tiles of all heads go first: 16 heads on 8 KV
+//                        heads, one sequence of 3000 tokens 153 us head by head, 109 now; four of 2048 223 and 173.
 //   attn_bwd_dkv_kernel  one CTA per (128-key block of one sequence and segment, KV head): the keys sit
 //                        on the tensor-memory lanes.  Loop over the 64-query sub-tiles that can see the
 //                        block and over the query heads of the KV group: S^T = K Q^T, dP^T = V dO^T,
@@ -229,11 +229,13 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         tmem_ld32(tmem_s + lane_off + half * 32, sv);
         tmem_ld32(tmem_dp + lane_off + half * 32, dp);
         tmem_ld_wait();
+        // the scores of this block were issued behind the dQ product of the one before, which has read dS
+        if (i > 0) mbar_wait(&dq_done[hi], (i - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
         const bool all_visible = __all_sync(0xffffffffu, valid >= 32);    // no masking inside this block
-        uint4 pk[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&pk[c]);
+          uint4 pk;
+          __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const int c0 = c * 8 + 2 * j;
@@ -245,10 +247,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             }
             p2[j] = __floats2bfloat162_rn(pa * fmaf(dp[c0], p.scale, -dsum_s), pb * fmaf(dp[c0 + 1], p.scale, -dsum_s));
           }
+          *reinterpret_cast<uint4*>(my_ds + row * 128 + (((half * 4 + c) ^ (row & 7)) << 4)) = pk;
         }
-        if (i > 0) mbar_wait(&dq_done[hi], (i - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4*>(my_ds + row * 128 + (((half * 4 + c) ^ (row & 7)) << 4)) = pk[c];
         fence_proxy_async_smem();
         tc_fence_before();
         mbar_arrive(&ds_ready[hi]);
@@ -583,15 +583,16 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
 using namespace tahb;
 
 // dQ of the packed attention.  Arguments as tahb_prefill_attn plus dout [n_q, nq*hd], lse and dsum
-// ([n_q, nq] fp32) and the output dq [n_q, nq*hd].
+// ([n_q, nq] fp32) and the output dq [n_q, nq*hd]; heads: query heads per CTA, 1 or (an even number per KV head) 2.
 extern "C" int tahb_attn_bwd_dq(const void* q, const void* dout, void* dq, void* const* ks, void* const* vs,
                                 const long long* n_kv, const int* const* bases, const int* const* counts,
                                 const int* const* bounds, int n_seg,
                                 const int* tile_q0, const int* tile_qn, int n_tiles, long long n_q, int nq, int nkv,
-                                int hd, float scale, const float* lse, const float* dsum, int* status,
+                                int hd, float scale, const float* lse, const float* dsum, int heads, int* status,
                                 cudaStream_t stream) {
   if (n_tiles <= 0 || n_q <= 0) return 0;
   if (n_seg < 1 || n_seg > PF_MAX_SEG || (nq % nkv)) return -1;
+  if (heads != 1 && (heads != 2 || (nq / nkv) % 2)) return -1;
   CUtensorMap mq, mdo, mk[PF_MAX_SEG], mv[PF_MAX_SEG];
   int rc;
   if ((rc = pf_make_map(&mq, q, n_q, (long long)nq * hd, 128u))) return rc;
@@ -617,7 +618,7 @@ extern "C" int tahb_attn_bwd_dq(const void* q, const void* dout, void* dq, void*
   p.scale = scale;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = status;
-  const bool two = (nq / nkv) % 2 == 0;
+  const bool two = heads == 2;
 #define TAHB_BQ(HD_, NH_)                                                                                       \
   {                                                                                                             \
     using C = BwdQCfg<HD_, NH_>;                                                                                \

@@ -448,7 +448,7 @@ class HybridEngine(DecodeEngine):
         if isinstance(L.ff, MixtureLayer):
             y, (ex["y_ex"], ex["slot"], ex["y_weight"]) = None, self._mixture(L.ff, None, b)
         elif isinstance(L.ff, XIELULayer):
-            K.linear(K.xielu_linear(b.h, L.w_up, L.ff.up, L.ff.low, out=b.act[:, :L.w_down.shape[1]]), L.w_down, out=y, const_w=True)
+            K.linear(K.xielu_linear(b.h, L.w_up, L.ff.up, L.ff.low, out=b.act[:, :L.w_down.shape[1]], const_w=True), L.w_down, out=y, const_w=True)
         else:
             act = K.swiglu_linear(b.h, L.w_gu, out=b.act[:, :L.w_down.shape[1]], const_w=True)
             K.linear(act, L.w_down, out=y, const_w=True)

@@ -389,7 +389,7 @@ class _SegmentAttention(torch.autograd.Function):
         dsum = K.rows_dot(do2, out, hd)
         scale = hd ** -0.5
         dq = K.attn_bwd_dq(q2, do2, ks, vs, meta.bases, meta.counts, meta.tile_q0, meta.tile_qn, nq, nkv, hd, scale,
-                           lse, dsum, bounds=meta.bounds)
+                           lse, dsum, bounds=meta.bounds, longest=Tq)
         grads = []
         for s in range(n_seg):
             dk, dv = K.attn_bwd_dkv(q2, do2, ks[s], vs[s], meta.counts[s], meta.items[s], nq, nkv, hd, scale, lse, dsum,

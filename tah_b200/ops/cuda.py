@@ -238,12 +238,15 @@ def wait_flags(flags: torch.Tensor, targets: torch.Tensor) -> None:
 
 
 def _plan_tiles(M: int, rows: int, K: int, R: int, swiglu: bool, gelu: bool, swiglu_interleaved: bool, pair=None, bn: int = 0, splits=None,
-                staged: bool = True):
-    """``(pair, bn, splits)`` of a tcgen05 product with a weight of ``rows`` rows.  ``staged``: output and residual can be moved as whole
-    tiles (:func:`_whole_pieces`), the only way the pair form has."""
+                stores=()):
+    """``(pair, bn, splits)`` of a tcgen05 product with a weight of ``rows`` rows.  ``stores``: the output and the residual where there is
+    one; the pair form can only move them as whole tiles (:func:`_whole_pieces`)."""
     can_pair = not swiglu and not gelu and rows % 256 == 0
     if pair is None and bn == 0 and splits is None and M > 256 and not swiglu:
-        return plan_tiles(M, rows, K + R, can_pair and PAIR_AUTO and staged, not swiglu_interleaved)
+        plan = plan_tiles(M, rows, K + R, can_pair and PAIR_AUTO, not swiglu_interleaved)
+        if plan[0] and not all(t is None or _whole_pieces(t) for t in stores):
+            plan = plan_tiles(M, rows, K + R, False, not swiglu_interleaved)
+        return plan
     pair = bool(pair) and can_pair
     if pair:
         bn, splits = bn or 256, 1
@@ -309,11 +312,11 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
     if residual is not None:
         _check_bf16_2d(residual, "residual")
     if (not pair and bn == 0 and splits in (None, 1) and tp_push is None and tp_wait is None and
-            not ((swiglu or gelu) and (residual is not None or swiglu and gelu)) and _few_ok(x, w, x2, w2, const_w and (swiglu or swiglu_interleaved)) and
+            not ((swiglu or gelu) and (residual is not None or swiglu and gelu)) and _few_ok(x, w, x2, w2, const_w) and
             (not (gelu or swiglu_interleaved) or _whole_pieces(out))):
         return _gemm_few(x, w, out, residual, x2, w2, 1 if swiglu else 3 if gelu else 4 if swiglu_interleaved else 0, early=const_w)
-    staged = tp_push is not None or (_whole_pieces(out) and (residual is None or _whole_pieces(residual)))
-    pair, bn, splits = _plan_tiles(M, w.shape[0], K, R, swiglu, gelu, swiglu_interleaved, pair, bn, splits, staged)
+    pair, bn, splits = _plan_tiles(M, w.shape[0], K, R, swiglu, gelu, swiglu_interleaved, pair, bn, splits,
+                                   () if tp_push is not None else (out, residual))
     args = (_p(w), _p(x), _p(out), _p(residual), _p(w2), _p(x2), c_int(M), c_int(F), c_int(K), c_int(R),
             c_ll(w.stride(0)), c_ll(x.stride(0)), c_ll(out.stride(0)),
             c_ll(residual.stride(0) if residual is not None else 0),
@@ -342,9 +345,10 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
 # Up to 16 tokens the product is a stream of the weight (csrc/gemm_few.cu).  From 17 to 32 tokens its CTAs hold four token tiles and fewer of
 # them fit an SM, and the tensor-memory form has the better time for weights that need a second wave of them: two CTAs of 8 warps per SM up to
 # 4736 rows (us, few / tensor memory at 24 tokens: 2048 x 6144 9.1 / 19.8, 4096 x 2048 6.6 / 9.9, 4096 x 4096 12.7 / 14.6; 6144 x 2048 11.6 / 9.6,
-# 8192 x 2048 12.4 / 10.1).  The SwiGLU weight of a decode tick, read ahead of the dependency wait, is level while one wave of three CTAs of 4
-# warps per SM holds it (12288 x 2048 15.0 / 15.0, not read ahead 15.8; 16384 x 2048 26 / 14.6).
-FEW_TOKENS, FEW_WIDE_TOKENS, FEW_WIDE_WAVE, FEW_GLU_WAVE = 32, 16, 2 * SM_COUNT, 3 * SM_COUNT
+# 8192 x 2048 12.4 / 10.1).  Those are products in a row; in a decode tick, between kernels that leave the tensor-memory form's start-up in the
+# open, a weight that is read ahead of the dependency wait takes the few-token form while one wave of three CTAs of 4 warps per SM holds it:
+# 20 rows at 2300 entries 2.57 / 2.65 ms (xIELU feed-forwards of 6144), 2.84 / 2.87 (SwiGLU of 12288 rows); a wave further 26 / 14.6 us (16384).
+FEW_TOKENS, FEW_WIDE_TOKENS, FEW_WIDE_WAVE, FEW_CONST_WAVE = 32, 16, 2 * SM_COUNT, 3 * SM_COUNT
 # A narrow weight (an adapter's) has too few tensor-memory tiles to occupy the SMs at any token count: while tiles of 16 rows by 32 tokens
 # fit one wave, the few-token form is the faster one (64 x 2048 at 1184 tokens 3.5 us, there 6.9; 64 x 6144 7.2 and 12.2; 192 x 2048 at 300
 # tokens 3.4 and 6.8; 192 x 6144 7.0 and 12.2; a wave further 6.0 and 6.9, 12.7 and 12.3).
@@ -354,17 +358,18 @@ def _whole_pieces(t: torch.Tensor) -> bool:
     return t.data_ptr() % 16 == 0 and t.stride(0) % 8 == 0
 
 
-def few_shape(M: int, rows: int, K: int, R: int = 0, const_glu: bool = False) -> bool:
-    """Whether a product of ``M`` tokens with a weight of ``rows`` rows takes the few-token form.  ``const_glu``: SwiGLU of a weight that is
-    read ahead of the dependency wait."""
+@functools.lru_cache(maxsize=4096)
+def few_shape(M: int, rows: int, K: int, R: int = 0, const: bool = False) -> bool:
+    """Whether a product of ``M`` tokens with a weight of ``rows`` rows takes the few-token form.  ``const``: the weight is read ahead of the
+    dependency wait."""
     few = (M <= FEW_WIDE_TOKENS or
-           M <= FEW_TOKENS and (-(-rows // 16) <= FEW_WIDE_WAVE or const_glu and K <= 2048 and -(-rows // 32) <= FEW_GLU_WAVE) or
+           M <= FEW_TOKENS and (-(-rows // 16) <= FEW_WIDE_WAVE or const and -(-rows // 32) <= FEW_CONST_WAVE) or
            -(-rows // 16) * -(-M // 32) <= SM_COUNT)
     return few and M > 0 and K > 0 and K % 64 == 0 and R % 64 == 0
 
 
-def _few_ok(x, w, x2=None, w2=None, const_glu: bool = False) -> bool:
-    return (few_shape(x.shape[0], w.shape[0], x.shape[1], 0 if x2 is None else x2.shape[1], const_glu) and
+def _few_ok(x, w, x2=None, w2=None, const: bool = False) -> bool:
+    return (few_shape(x.shape[0], w.shape[0], x.shape[1], 0 if x2 is None else x2.shape[1], const) and
             all(t is None or _whole_pieces(t) for t in (x, w, x2, w2)))
 
 
@@ -712,7 +717,8 @@ def swiglu_linear(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] 
     return out
 
 
-def xielu_linear(x: torch.Tensor, w: torch.Tensor, up: float, low: float, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+def xielu_linear(x: torch.Tensor, w: torch.Tensor, up: float, low: float, out: Optional[torch.Tensor] = None,
+                 const_w: bool = False) -> torch.Tensor:
     """xIELU of ``x @ w^T``: ``up z^2 + z / 2`` for ``z > 0`` and ``low (exp(z) - 1 - z) + z / 2`` otherwise; in the epilogue of
     the product for bf16 (on ``z`` rounded to bf16), a kernel behind it for fp32."""
     M, Kd = x.shape
@@ -727,8 +733,8 @@ def xielu_linear(x: torch.Tensor, w: torch.Tensor, up: float, low: float, out: O
         out = torch.empty(M, F, dtype=torch.bfloat16, device=x.device)
     for n, t in (("x", x), ("w", w), ("out", out)):
         _check_bf16_2d(t, n)
-    if _few_ok(x, w) and _whole_pieces(out):
-        return _gemm_few(x, w, out, act=5, act_up=up, act_low=low)
+    if _few_ok(x, w, const=const_w) and _whole_pieces(out):
+        return _gemm_few(x, w, out, act=5, act_up=up, act_low=low, early=const_w)
     pair, bn, splits = _plan_tiles(M, F, Kd, 0, False, False, False)
     _rc(lib().tahb_gemm_xielu(_p(w), _p(x), _p(out), c_int(M), c_int(F), c_int(Kd), c_ll(w.stride(0)), c_ll(x.stride(0)), c_ll(out.stride(0)),
                               c_float(up), c_float(low), c_int(int(pair)), c_int(splits), c_int(bn), _p(status_word(x.device)), _stream()),
@@ -940,15 +946,15 @@ def window_attn_tiles(q, out, pool, page_table, pos, row, tile_q0, tile_qn, n_pa
     in pairs)."""
     a = window_attn_args(q, out, pool, page_table, pos, row, **kw)
     pooled = kw.get("pooled")
+    if heads is None:
+        heads = 2 if (two_heads_per_cta(tile_q0.numel(), kw["nq"], kw["nkv"], longest) and not kw.get("softcap") and pooled is None and
+                      64 < kw["dk"] <= 128 and 64 < kw["dv"] <= 128) else 1
     _rc(lib().tahb_window_attn_tiles(ctypes.byref(a), _p(tile_q0), _p(tile_qn), c_int(tile_q0.numel()), c_int(n_pages),
                                      c_ll(kv_ld), _p(pool_base), c_int(0 if pooled is None else pooled.shape[0] // 16), c_int(heads), _stream()),
         "tahb_window_attn_tiles")
     return out
 
 
-    if heads is None:
-        heads = 2 if (two_heads_per_cta(tile_q0.numel(), kw["nq"], kw["nkv"], longest) and not kw.get("softcap") and pooled is None and
-                      64 < kw["dk"] <= 128 and 64 < kw["dv"] <= 128) else 1
 class _TiedKeys(ctypes.Structure):
     _fields_ = [(n, c_void_p) for n in ("k", "cache", "pooled", "slot", "pos", "row", "page_table")] + \
                [(n, c_int) for n in ("M", "nkv", "dk", "page_size", "max_pages", "pool", "pool_rows")] + [("ld", c_ll)]
@@ -1506,7 +1512,7 @@ def packed_pass(weights, final_norm, h, xn, pools, k_own, v_own, seg_k, seg_v, b
 
     def plan(rows, K, R=0, glu=False):
         stacked, il = glu and not gu_interleaved, glu and gu_interleaved
-        if few_shape(n, rows, K, R, glu):
+        if few_shape(n, rows, K, R, True):
             return _ProductPlan(1, 4 if il else 1 if stacked else 0, 1, 0)
         pair, bn, splits = _plan_tiles(n, rows, K, R, stacked, False, il)
         return _ProductPlan(0, 1 if stacked else (6 if pair else 4) if il else 2 if pair else 0, splits, bn)
@@ -1547,15 +1553,22 @@ def attn_kv_items(seq_kv_counts: torch.Tensor, seq_kv_base: torch.Tensor, seq_q_
 
 
 def attn_bwd_dq(q, dout, ks, vs, bases, counts, tile_q0, tile_qn, nq, nkv, hd, scale, lse, dsum, out=None,
-                bounds=None):
-    """dQ of :func:`prefill_attn` (``csrc/attn_prefill_bwd.cu``); ``dsum = rowsum(dO * O)`` per (query, head)."""
+                bounds=None, longest: int = 0, heads: Optional[int] = None):
+    """dQ of :func:`prefill_attn` (``csrc/attn_prefill_bwd.cu``); ``dsum = rowsum(dO * O)`` per (query, head).  ``longest``: tokens of the
+    longest sequence, if known; ``heads``: query heads per CTA (default: by :func:`two_heads_per_cta`, for a single sequence from one and
+    a half waves on).  us, 16 heads of 128 on 8 KV heads, one / two: four sequences of 700 tokens 38.9 / 33.3, two of 2048 100 / 85, four 181 / 173;
+    one of 1500 54.5 / 62.7, of 3000 109 / 117, 16 of 512 74.8 / 76.9, 64 of 64 23.7 / 29.0."""
+    n_tiles = tile_q0.numel()
+    if heads is None:
+        several = n_tiles * 128 >= longest + 128
+        heads = 2 if two_heads_per_cta(n_tiles, nq, nkv, longest) and (several or n_tiles * nq >= 3 * SM_COUNT) else 1
     if out is None:
         out = torch.empty_like(q)
     n = len(ks)
     n_kv = (c_ll * n)(*[k.shape[0] for k in ks])
     _rc(lib().tahb_attn_bwd_dq(_p(q), _p(dout), _p(out), _ptr_array(ks), _ptr_array(vs), n_kv, _ptr_array(bases),
-                               _ptr_array(counts), _ptr_array(bounds if bounds is not None else counts), c_int(n), _p(tile_q0), _p(tile_qn), c_int(tile_q0.numel()),
-                               c_ll(q.shape[0]), c_int(nq), c_int(nkv), c_int(hd), c_float(scale), _p(lse), _p(dsum),
+                               _ptr_array(counts), _ptr_array(bounds if bounds is not None else counts), c_int(n), _p(tile_q0), _p(tile_qn), c_int(n_tiles),
+                               c_ll(q.shape[0]), c_int(nq), c_int(nkv), c_int(hd), c_float(scale), _p(lse), _p(dsum), c_int(heads),
                                _p(status_word(q.device)), _stream()), "tahb_attn_bwd_dq")
     return out
 

@@ -200,7 +200,7 @@ def bench_attn_bwd(a):
     dsum = (do.float() * out.float()).view(ntok, nq, hd).sum(-1).contiguous()
     dq = torch.empty_like(q)
     dk, dv = torch.zeros_like(k), torch.zeros_like(v)
-    f_dq = lambda i: K.attn_bwd_dq(q, do, [k], [v], [base], [cnt], tq0, tqn, nq, nkv, hd, hd ** -0.5, lse, dsum, out=dq)
+    f_dq = lambda i: K.attn_bwd_dq(q, do, [k], [v], [base], [cnt], tq0, tqn, nq, nkv, hd, hd ** -0.5, lse, dsum, out=dq, longest=L)
     f_kv = lambda i: K.attn_bwd_dkv(q, do, k, v, cnt, items, nq, nkv, hd, hd ** -0.5, lse, dsum, dk=dk, dv=dv)
     t_dq = _time(f_dq, a.iters, a.warmup)
     t_kv = _time(f_kv, a.iters, a.warmup)
