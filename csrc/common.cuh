@@ -363,6 +363,13 @@ struct alignas(EPL * 2) QkvPiece {
   }
 };
 
+// How many CTAs the heads of a token are dealt out to: one head per warp while tokens x CTAs stay below `most`, else half as many, ...
+inline int qk_head_groups(int tokens, int heads, int warps, int most) {
+  int g = (heads + warps - 1) / warps;
+  while (g > 1 && (long long)tokens * g > most) g = (g + 1) / 2;
+  return g;
+}
+
 struct __align__(16) bf16x8 {
   __nv_bfloat162 v[4];
 };

@@ -248,11 +248,12 @@ struct QkvRopeParams {
   float eps, log2_theta;
 };
 
-// One CTA per token; a warp takes QKV_U heads at a time, whose loads are all in flight before the first is used, and the
-// token's sines and cosines are computed once for all of them.  Bound: HBM (at 16384 tokens of 16 + 16 heads: 134 MB in, 134 MB out, of
+// One CTA per token, several for few tokens; a warp takes QKV_U heads at a time, whose loads are all in flight before the first is used, and
+// the token's sines and cosines are computed once for all of them.  Bound: HBM (at 16384 tokens of 16 + 16 heads: 134 MB in, 134 MB out, of
 // which 67 MB go to the cache as well); with a warp per head, one 8-byte load in flight and sincosf and exp2f in every warp, the
 // instruction issue was: the two passes over seven prompts of up to 3500 tokens 281 us, now 121 us (139 with the sines in every warp);
-// 3072 tokens 19.2 us; one row 3.5 and 3.2 us.
+// 3072 tokens 19.2 us.  Few tokens leave SMs idle and a warp with four heads in turn: a CTA per token / four of them / a warp per head, 16 + 16
+// heads, back to back: 1 token 2.95 / 2.02 / 2.26 us, 64 3.09 / 2.36 / 3.20, 200 3.43 / 3.70 / 5.33 (two of them: 2.93).
 // WIDE: every pointer and row lies on a boundary of a lane's piece (8 bytes of a head of 128); else element by element.
 constexpr int QKV_U = 4, QKV_WARPS = 8;
 template <int HD, bool WIDE>
@@ -261,14 +262,14 @@ __global__ void __launch_bounds__(QKV_WARPS * 32) qk_norm_rope_kv_kernel(const Q
   constexpr int EPL = HD / 32;  // elements per lane
   using Piece = QkvPiece<EPL, WIDE>;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int heads = p.nq + 2 * p.nkv;
+  const int all = p.nq + 2 * p.nkv, per = (all + gridDim.y - 1) / gridDim.y, first = blockIdx.y * per, heads = min(all, first + per);
   const int t = blockIdx.x;
   const bool upper = lane >= 16;
   const __nv_bfloat16* src = p.qkv + (size_t)t * p.ld_qkv + lane * EPL;
   Piece in[QKV_U];
 #pragma unroll
   for (int u = 0; u < QKV_U; ++u) {
-    const int h = warp + u * QKV_WARPS;
+    const int h = first + warp + u * QKV_WARPS;
     if (h < heads) in[u].load(src + (size_t)h * HD);
   }
   __shared__ float2 s_cs[HD / 2];               // cosine and sine of the token's angles, each computed once
@@ -284,7 +285,7 @@ __global__ void __launch_bounds__(QKV_WARPS * 32) qk_norm_rope_kv_kernel(const Q
   float2 cs[EPL];
 #pragma unroll
   for (int i = 0; i < EPL; ++i) cs[i] = s_cs[(lane & 15) * EPL + i];      // frequency of dim d: d mod HD / 2
-  for (int h0 = warp; h0 < heads; h0 += QKV_U * QKV_WARPS) {
+  for (int h0 = first + warp; h0 < heads; h0 += QKV_U * QKV_WARPS) {
 #pragma unroll
     for (int u = 0; u < QKV_U; ++u) {
       const int h = h0 + u * QKV_WARPS;
@@ -786,8 +787,9 @@ extern "C" int tahb_qk_norm_rope_kv(const void* qkv, const void* q_w, const void
                  (uintptr_t)(ld_qkv * 2);
   for (int i = 0; i < n_caches; ++i) at |= reinterpret_cast<uintptr_t>(caches[i]);
   const bool wide = at % (hd / 16) == 0;
-#define TAHB_QKV(HD_) (wide ? launch_chain(qk_norm_rope_kv_kernel<HD_, true>, dim3(M), dim3(QKV_WARPS * 32), 0, stream, p) \
-                            : launch_chain(qk_norm_rope_kv_kernel<HD_, false>, dim3(M), dim3(QKV_WARPS * 32), 0, stream, p))
+  const int groups = qk_head_groups(M, nq + 2 * nkv, QKV_WARPS, 4 * 148);
+#define TAHB_QKV(HD_) (wide ? launch_chain(qk_norm_rope_kv_kernel<HD_, true>, dim3(M, groups), dim3(QKV_WARPS * 32), 0, stream, p) \
+                            : launch_chain(qk_norm_rope_kv_kernel<HD_, false>, dim3(M, groups), dim3(QKV_WARPS * 32), 0, stream, p))
   if (hd == 128) e = TAHB_QKV(128);
   else if (hd == 64) e = TAHB_QKV(64);
   else return -2;

@@ -169,8 +169,8 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __
 //   n = w * (x * rstd),  y = n * cos + rot(n) * sin      (q and k heads; v heads pass through)
 //   gn = gy * cos +/- partner(gy) * sin ;  gx = rstd * (gn*w - xn * mean(gn*w*xn)) ;  gw += gn * xn
 // The weight gradients are summed per CTA in shared memory and added to the fp32 buffers once.
-// A CTA takes a token at a time, a warp four of its heads with all their loads in flight and the sines and cosines once for them (once
-// per CTA, by way of shared memory, 38 us: a barrier per token).  Bound: HBM (3072 tokens of 16 + 16 heads: 75 MB, 11 us); a warp per
+// A CTA takes a token at a time (several CTAs up to 64 tokens), a warp four of its heads with all their loads in flight and the sines and
+// cosines once for them (once per CTA, by way of shared memory, 38 us: a barrier per token).  Bound: HBM (3072 tokens of 16 + 16 heads: 75 MB, 11 us); a warp per
 // head with one in flight and its own sincosf: 50 us, now 34.4 us.
 // ---------------------------------------------------------------------------------------------
 struct QkRopeBwdParams {
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(QKB_WARPS * 32) qk_norm_rope_bwd_kernel(const 
   for (int i = threadIdx.x; i < 2 * HD; i += blockDim.x) (&s_gw[0][0])[i] = 0.f;
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int heads = p.nq + 2 * p.nkv;
+  const int heads = p.nq + 2 * p.nkv, per = (heads + gridDim.y - 1) / gridDim.y, first = blockIdx.y * per, last = min(heads, first + per);
   const bool upper = lane >= 16;
   float gw_q[EPL], gw_k[EPL];
   float inv[EPL];
@@ -210,26 +210,29 @@ __global__ void __launch_bounds__(QKB_WARPS * 32) qk_norm_rope_bwd_kernel(const 
   for (int i = 0; i < EPL; ++i) gw_q[i] = gw_k[i] = 0.f;
   for (int t = blockIdx.x; t < p.M; t += gridDim.x) {
     float2 cs[EPL];
-#pragma unroll
-    for (int i = 0; i < EPL; ++i) {
-      const float ang = (float)p.pos[t] * inv[i];
-      cs[i] = make_float2(bf16_round(cosf(ang)), bf16_round(sinf(ang)));
-    }
-    for (int h0 = warp; h0 < heads; h0 += QKB_U * QKB_WARPS) {
+    const float posf = (float)p.pos[t];
+    for (int h0 = first + warp; h0 < last; h0 += QKB_U * QKB_WARPS) {
       Piece xin[QKB_U], gin[QKB_U];
 #pragma unroll
       for (int u = 0; u < QKB_U; ++u) {
         const int h = h0 + u * QKB_WARPS;
-        if (h >= heads) continue;
+        if (h >= last) continue;
         if (h < p.nq + p.nkv) xin[u].load(p.qkv + ((size_t)t * heads + h) * HD + lane * EPL);
         gin[u].load((h < p.nq ? p.gq + ((size_t)t * p.nq + h) * HD
                               : h < p.nq + p.nkv ? p.gk + ((size_t)t * p.nkv + h - p.nq) * HD
                                                  : p.gv + ((size_t)t * p.nkv + h - p.nq - p.nkv) * HD) + lane * EPL);
       }
+      if (h0 == first + warp) {                      // once per token, with the first loads on their way
+#pragma unroll
+        for (int i = 0; i < EPL; ++i) {
+          const float ang = posf * inv[i];
+          cs[i] = make_float2(bf16_round(cosf(ang)), bf16_round(sinf(ang)));
+        }
+      }
 #pragma unroll
       for (int u = 0; u < QKB_U; ++u) {
         const int h = h0 + u * QKB_WARPS;
-        if (h >= heads) continue;
+        if (h >= last) continue;
         Piece out = gin[u];
         if (h < p.nq + p.nkv) {
           const bool is_q = h < p.nq;
@@ -348,10 +351,11 @@ extern "C" int tahb_qk_norm_rope_bwd(const void* qkv, const void* q_w, const voi
   uintptr_t at = 0;
   for (const void* q : {qkv, q_w, k_w, gq, gk, gv, (const void*)gqkv}) at |= reinterpret_cast<uintptr_t>(q);
   const bool wide = at % (hd / 16) == 0;
-  const int blocks = M < 296 ? M : 296;            // two CTAs per SM, whose sums meet in the weight gradients' few lines
+  // two CTAs per SM, whose sums meet in the weight gradients' few lines
+  const dim3 grid(M < 296 ? M : 296, qk_head_groups(M, nq + 2 * nkv, QKB_WARPS, 128));
 #define TAHB_QKB(HD_)                                                                          \
-  (wide ? (void)(qk_norm_rope_bwd_kernel<HD_, true><<<blocks, QKB_WARPS * 32, 0, stream>>>(p)) \
-        : (void)(qk_norm_rope_bwd_kernel<HD_, false><<<blocks, QKB_WARPS * 32, 0, stream>>>(p)))
+  (wide ? (void)(qk_norm_rope_bwd_kernel<HD_, true><<<grid, QKB_WARPS * 32, 0, stream>>>(p)) \
+        : (void)(qk_norm_rope_bwd_kernel<HD_, false><<<grid, QKB_WARPS * 32, 0, stream>>>(p)))
   if (hd == 128) TAHB_QKB(128);
   else if (hd == 64) TAHB_QKB(64);
   else return -2;

@@ -1199,3 +1199,54 @@ def test_gemm_few_tokens_wide_swiglu(M, rows):
         out = Kc.gemm(x, w, swiglu_interleaved=True, const_w=const)
         assert bool(((out.double() - ref).abs() <= 1.01 * tol + 2e-5).all())
     Kc.check_status()
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("nq,nkv", [(4, 2), (4, 1)])
+def test_attention_backward_two_heads_per_cta(hd, nq, nkv):
+    """dQ of two query heads per CTA: the same products in the same order as of one, so the same bits; sequences around the sizes of key
+    blocks and query tiles."""
+    Kc = _cuda()
+    lens = [1, 63, 64, 65, 129, 300, 700]
+    n = sum(lens)
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    b = i32([starts[i] for i, L in enumerate(lens) for _ in range(L)])
+    c = i32([j + 1 for L in lens for j in range(L)])
+    q, k, v, dout = (_rand(n, h * hd, seed=j) for j, h in enumerate((nq, nkv, nkv, nq)))
+    tq0, tqn = Kc.attn_tiles(torch.tensor(lens, device="cuda"))
+    lse = torch.empty(n, nq, dtype=torch.float32, device="cuda")
+    out = Kc.prefill_attn(q, [k], [v], [b], [c], tq0, tqn, nq, nkv, hd, hd ** -0.5, lse=lse)
+    dsum = Kc.rows_dot(dout, out, hd)
+    one, two = (Kc.attn_bwd_dq(q, dout, [k], [v], [b], [c], tq0, tqn, nq, nkv, hd, hd ** -0.5, lse, dsum, heads=h) for h in (1, 2))
+    Kc.check_status()
+    assert torch.equal(one, two)
+    with pytest.raises(RuntimeError):
+        Kc.attn_bwd_dq(q, dout, [k], [v], [b], [c], tq0, tqn, nq, nq, hd, hd ** -0.5, lse, dsum, heads=2)
+
+
+@pytest.mark.parametrize("hd,nq,nkv", [(128, 16, 8), (128, 40, 8), (64, 8, 1)])
+def test_qk_norm_rope_of_few_tokens(hd, nq, nkv):
+    """However many CTAs the heads of a token are dealt out to, a token's rows have the same bits, forward and backward; the weight gradients
+    are 32-bit sums in any order."""
+    Kc = _cuda()
+    F = (nq + 2 * nkv) * hd
+    x, qw, kw = _rand(700, F, seed=1), _rand(hd, seed=2), _rand(hd, seed=3)
+    pos = torch.arange(700, device="cuda", dtype=torch.int32) * 57
+    grads = [_rand(700, h * hd, seed=4 + h) for h in (nq, nkv, nkv)]
+
+    def run(m):
+        k, v = (torch.empty(m, nkv * hd, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        q = Kc.qk_norm_rope_kv(x[:m], qw, kw, pos[:m], nq, nkv, hd, 1e-6, 1e6, k_dense=k, v_dense=v)
+        gx, gq, gk = Kc.qk_norm_rope_bwd(x[:m], qw, kw, *(g[:m] for g in grads), pos[:m], nq, nkv, hd, 1e-6, 1e6)
+        return (q, k, v, gx), (gq, gk)
+    full = run(700)[0]
+    for m in (1, 18, 19, 32, 64, 65, 85, 128, 129, 148, 149, 296, 297, 592, 593):
+        rows, (gq, gk) = run(m)
+        assert all(torch.equal(a, b[:m]) for a, b in zip(rows, full)), m
+        one = [torch.zeros(hd, device="cuda", dtype=torch.float64) for _ in range(2)]
+        for a in range(0, m, 7):
+            part = Kc.qk_norm_rope_bwd(x[a:min(m, a + 7)], qw, kw, *(g[a:min(m, a + 7)] for g in grads), pos[a:min(m, a + 7)], nq, nkv, hd, 1e-6, 1e6)
+            one = [s + p.double() for s, p in zip(one, part[1:])]
+        for a, b, heads in zip((gq, gk), one, (nq, nkv)):
+            _close(a, b, atol=2e-5 * (m * heads) ** 0.5 + 1e-4, rtol=1e-5)
