@@ -11,10 +11,10 @@ namespace tahb {
 // registers over those rows and adds it to the fp32 gw buffer once at the end.  Bound: HBM (2048 columns, 3072 rows: 38 MB, 6 us); a
 // row is a chain of load, block reduction and store, so the next row is on its way while one is reduced, and two CTAs per SM share
 // the rows evenly.  32 rows in turn per CTA without that: 39 us at 3072 rows (96 CTAs), now 12.3 us.
-// FEW: up to 64 rows (of a second pass, say) go to one cluster of eight CTAs, whose sums meet in a fixed order through distributed shared
+// FEW: 3 to 64 rows (of a second pass, say) go to one cluster of eight CTAs, whose sums meet in a fixed order through distributed shared
 // memory: the gradients of a few rows repeat themselves bit by bit.  64 rows 8.4 us, with atomics 3.9, in two CTAs 19.
 // ---------------------------------------------------------------------------------------------
-constexpr int RMSB_GRID = 296, RMSB_FEW_ROWS = 64, RMSB_FEW_CTAS = 8;
+constexpr int RMSB_GRID = 296, RMSB_FEW_ROWS = 64, RMSB_FEW_CTAS = 8;      // two additions to a zeroed sum have no order
 
 template <int VPT, bool FEW>
 __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x,
@@ -374,7 +374,7 @@ extern "C" int tahb_rmsnorm_bwd(const void* x, const void* w, const void* gy, vo
   auto GX = reinterpret_cast<__nv_bfloat16*>(gx);
 #define TAHB_RMSB(VPT_)                                                                                                   \
   {                                                                                                                       \
-    if (M > RMSB_FEW_ROWS) {                                                                                              \
+    if (M > RMSB_FEW_ROWS || M <= 2) {                                                                                              \
       rmsnorm_bwd_kernel<VPT_, false><<<M < RMSB_GRID ? M : RMSB_GRID, 256, 0, stream>>>(X, W, GY, GX, gw, M, H, eps);     \
     } else {                                                                                                              \
       cudaLaunchAttribute attr = {};                                                                                      \
