@@ -411,7 +411,8 @@ def test_decode_attention_two_caches(hd, nq, nkv, n_split):
 @pytest.mark.parametrize("n_split", [1, 2])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_decode_attention_more_items_than_ctas(hd, nq, nkv, n_split, shift):
-    """Every CTA walks several rows: empty ones, one entry, whole pages, more pages than a stage ring and than 32 page numbers."""
+    """Several items for every CTA that fits at once, rows of every kind: empty ones, one entry, whole pages, more than the 32 page numbers of a
+    turn, more than a warp has in flight; queries off the 16-byte boundary."""
     Kc = _cuda()
     page, rows = 16, 5 * 148 * 4 // (nkv * n_split) // 2
     some0, some1 = [0, 1, 16, 33, 96, 7, 560, 32], [0, 5, 16, 0, 40]
@@ -472,6 +473,28 @@ def test_decode_attention_warps_per_item(hd, nq, nkv, warps):
         ref = torch.einsum("hn,nhd->hd", torch.softmax(torch.einsum("hd,nhd->hn", q[r].view(nq, hd).float(), k) * scale, -1), v)
         # fp32 inside, one rounding to bf16 (2^-8 of the value) at the end; fp32 sums of 200 terms of order one stay below 1e-4
         _close(out[r].view(nq, hd), ref, atol=1e-4, rtol=2 ** -8)
+
+
+@pytest.mark.parametrize("hd,nq,nkv,n_split", [(128, 4, 2, 1), (64, 8, 2, 2), (128, 2, 2, 3)])
+def test_decode_attention_infinite_and_undefined_values(hd, nq, nkv, n_split):
+    """An infinite or undefined value shows in its own dimension of the heads that read it, also where parts of a weight are zero or
+    negative, and nowhere else."""
+    Kc = _cuda()
+    page, lens = 16, [70, 1, 33]
+    c, pt, ln = _paged_setup(3, lens, nkv, hd, page, 1)
+    q = _rand(3, nq * hd, seed=3)
+    run = lambda: Kc.decode_attn(q, [c], [pt], [ln], None, nq, nkv, hd, page, hd ** -0.5, n_split=n_split).view(3, nkv, nq // nkv, hd).clone()
+    clean = run()
+    inf, nan = float("inf"), float("nan")
+    want = clean.clone()
+    for row, entry, head, dim, value in ((0, 69, 0, 5, inf), (0, 3, 1, 6, -inf), (1, 0, 1, 0, inf), (2, 20, 0, 9, nan), (2, 32, 1, 1, -inf)):
+        c[int(pt[row, entry // page]), 1, head, entry % page, dim] = value
+        want[row, head, :, dim] = value
+    c[int(pt[2, 0]), 1, 0, 1, 9], c[int(pt[0, 0]), 1, 0, 7, 5] = inf, inf       # beside the undefined one, beside one of its sign
+    got = run()
+    Kc.check_status()
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got.nan_to_num(7.0), want.nan_to_num(7.0))
 
 
 def test_varlen_attention_duo_segments():
