@@ -184,10 +184,7 @@ template <int NT, int MT, int NW>
 static int launch_few(const FewParams& p, cudaStream_t stream) {
   constexpr int bytes = FewCfg<NT, MT>::red_bytes(NW);
   auto kern = gemm_few_kernel<NT, MT, NW>;
-  if constexpr (bytes > 48 * 1024) {
-    static const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
-    if (!ok) return -10;
-  }
+  static_assert(bytes <= 48 * 1024, "no opt-in for more shared memory");
   return launch_chain(kern, dim3((p.F + 16 * MT - 1) / (16 * MT), (p.M + 8 * NT - 1) / (8 * NT)), dim3(NW * 32), bytes, stream, p) == cudaSuccess ? 0 : -12;
 }
 

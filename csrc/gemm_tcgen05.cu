@@ -265,7 +265,7 @@ __device__ __noinline__ void qkv_epilogue(const GemmParams& p, const __nv_bfloat
   const __nv_bfloat16* nw = is_q ? p.q_norm_w : p.k_norm_w;
   // Packed bf16x2 arithmetic: a bf16 x bf16 product is exact in fp32, so __hmul2 rounds once exactly like the
   // scalar statement bf16(float(a) * float(b)); this more than halves the instruction count of the loop, which
-  // only four warps execute.
+  // only the epilogue warps execute.
   __nv_bfloat162 w01 = __floats2bfloat162_rn(0.f, 0.f), w23 = w01;
   float inv[4] = {0.f, 0.f, 0.f, 0.f};
   const bool upper = lane >= 16;

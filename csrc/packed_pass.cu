@@ -42,7 +42,7 @@ struct TahbPass {
   const int* count[3];
   const int *pos, *slots, *tile_q0, *tile_qn;
   int* status;
-  int n_layers, n, hidden, inter, nq, nkv, hd, page_size, n_seg, n_tiles, gu_dual;
+  int n_layers, n, hidden, inter, nq, nkv, hd, page_size, n_seg, n_tiles;
   int r_qkv, r_o, r_gu, r_down;                     // 0 without the adapter
   float eps, theta, scale;
   TahbProductPlan p_qkv, p_o, p_gu, p_down, p_a_qkv, p_a_o, p_a_gu, p_a_down;

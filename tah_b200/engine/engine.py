@@ -239,8 +239,8 @@ class TaHEngine(DecodeEngine):
         t_down = bf(n, w.r_down) if lora else None
         tap_layers = self._tap_layers()
         tensor_core_attn = hd in (64, 128) and os.environ.get("TAH_B200_NAIVE_PREFILL", "0") != "1"
-        # off by default here as well: at thousands of tokens per tile column the epilogue's QK-norm / RoPE arithmetic
-        # on four warps costs as much as the tile's main loop (prefill 272 ms fused, 254 ms with the separate kernel)
+        # off by default here as well: the epilogue's QK-norm / RoPE arithmetic stands behind the main loop of every tile (seven prompts of up
+        # to 3500 tokens 68.8 ms fused, on eight epilogue warps and launch by launch, 65.2 ms with the separate kernel; one of 700 12.4 and 10.2)
         fuse_qkv = hd == 128 and "qkv" in _fusions("")
         if tensor_core_attn:
             tile_q0, tile_qn = K.attn_tiles(seq_counts, by_work=True)
@@ -547,7 +547,8 @@ class TaHEngine(DecodeEngine):
         nL = len(w.layers)
         # Optional fusions of the decode chain.  RMSNorm and LoRA-A in one launch pays while launches are what a tick is made of (1 row:
         # 1.49 -> 1.35 ms, 6 rows 1.75 -> 1.67 ms); from 20 rows on the gated rows' products hold up the norm (2.98 -> 3.12 ms), and at
-        # 256 rows the chain of separate launches is faster, also than the QKV epilogue on the GEMM's epilogue warps.
+        # 256 rows the chain of separate launches is faster, also than the QKV epilogue on the GEMM's eight epilogue warps (a generation of 32
+        # tokens 205.7 ms, fused 212.2; 20 rows of up to 1900 172.9 and 182.3).
         fuse = _fusions("lora" if B <= 8 else "")
         fuse_norm_lora = "lora" in fuse and lora and tp is None  # RMSNorm + LoRA-A of the gated rows in one launch
         fuse_qkv = "qkv" in fuse and hd == 128                   # QK-norm + RoPE + KV write in the QKV GEMM epilogue

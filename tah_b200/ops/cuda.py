@@ -1455,7 +1455,7 @@ class _Pass(ctypes.Structure):
         [(f, _VP) for f in ("taps", "k_own", "v_own", "pool")] + \
         [("k_seg", _VP * 3), ("v_seg", _VP * 3), ("n_kv", c_ll * 3), ("base", c_void_p * 3), ("count", c_void_p * 3)] + \
         [(f, c_void_p) for f in ("pos", "slots", "tile_q0", "tile_qn", "status")] + \
-        [(f, c_int) for f in ("n_layers", "n", "hidden", "inter", "nq", "nkv", "hd", "page_size", "n_seg", "n_tiles", "gu_dual", "r_qkv",
+        [(f, c_int) for f in ("n_layers", "n", "hidden", "inter", "nq", "nkv", "hd", "page_size", "n_seg", "n_tiles", "r_qkv",
                               "r_o", "r_gu", "r_down")] + \
         [(f, c_float) for f in ("eps", "theta", "scale")] + \
         [(f, _ProductPlan) for f in ("p_qkv", "p_o", "p_gu", "p_down", "p_a_qkv", "p_a_o", "p_a_gu", "p_a_down")]
@@ -1506,7 +1506,7 @@ def packed_pass(weights, final_norm, h, xn, pools, k_own, v_own, seg_k, seg_v, b
     a.pos, a.slots, a.tile_q0, a.tile_qn = pos.data_ptr(), slots.data_ptr(), tile_q0.data_ptr(), tile_qn.data_ptr()
     a.status = status_word(h.device).data_ptr()
     a.n_layers, a.n, a.hidden, a.inter, a.nq, a.nkv, a.hd, a.page_size = L, n, H, inter, nq, nkv, hd, page_size
-    a.n_seg, a.n_tiles, a.gu_dual = len(bases), tile_q0.numel(), 0 if gu_interleaved else 1
+    a.n_seg, a.n_tiles = len(bases), tile_q0.numel()
     a.r_qkv, a.r_o, a.r_gu, a.r_down = ranks
     a.eps, a.theta, a.scale = eps, theta, scale
 
