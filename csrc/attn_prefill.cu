@@ -1,8 +1,7 @@
 // Duo-causal attention forward for packed (varlen) passes on the 5th-generation tensor cores.
 //
-// One CTA handles a tile of up to 128 consecutive query tokens of ONE sequence and one query head; two CTAs share an SM (112 KB of shared
-// memory and 256 tensor-memory columns each).  For each of up to three KV segments (depth-0 K/V, depth-1 K/V, ...) the tile walks the keys of
-// its sequence in blocks of 64:
+// One CTA handles a tile of up to 128 consecutive query tokens of ONE sequence and one query head, or two of one KV head.  For each of up to
+// three KV segments (depth-0 K/V, depth-1 K/V, ...) the tile walks the keys of its sequence in blocks of 64; two heads use the same blocks:
 //
 //     S = Q K^T          tcgen05.mma, Q and K K-major (head_dim contiguous), S in tensor memory
 //     P = exp2(S - m)    128 threads, one per query row, straight out of tensor memory; the duo-causal
@@ -12,17 +11,19 @@
 //
 // The running maximum is only refreshed when it grows by more than 8 (in log2 units), so the
 // accumulator in tensor memory is rescaled rarely; the final division uses the matching row sums.
-// No mask tensor exists.  K/V blocks arrive by TMA into a two-stage ring.  All waits are bounded.
+// No mask tensor exists.  K/V blocks arrive by TMA into a ring.  All waits are bounded.
 //
 // What bounds it: per head and block the tensor pipe needs 256 cycles, the softmax of a warp's 32 rows about 350 (one exponential, one
 // multiply-add and half a conversion per score, four warps).  S has two buffers: the product for block i + 1 is issued ahead of P V of block
 // i.  A thread owns a whole row; with two threads per row their maxima met through tensor memory and a barrier in every block.  The long
-// tiles of all heads go first (a tail of long tiles stood behind the rest).  Two heads per CTA, with four stages for both, give the same
-// from 1500 tokens on and hold up short sequences, which have fewer CTAs then.  us, 16 heads of 128 on 8 KV heads, with two threads per row / two
-// heads per CTA / this form: 100 tokens 8.4 / 9.2 / 7.5, 700 22.3 / 21.1 / 18.4, 64 sequences of 128 42.6 / 43.1 / 36.7, 3000 tokens 122 / 74.4 /
-// 69.6, four sequences of 2048 162 / 112 / 112, two of 4000 298 / 183 / 186.
+// tiles of all heads go first (a tail of long tiles stood behind the rest: four sequences of 2048 head by head 117 us, now 111).
+// One head per CTA, two CTAs per SM, have room for two stages each; two heads in one CTA read each block once and have four, which pays where
+// there is more than a wave of long sequences, and holds up short ones, which have half the CTAs then (the rule: prefill_heads in
+// tah_b200/ops/cuda.py).  us, 16 heads of 128 on 8 KV heads, two threads per row / one head / two heads: 100 tokens 8.4 / 7.5 / 9.2, 700 22.3 / 18.4 /
+// 21.1, 64 sequences of 128 42.6 / 36.7 / 43.1, 3000 tokens 122 / 69.9 / 74.0, four of 2048 162 / 112 / 112, of 4000 - / 382 / 360, their second pass
+// of 0.3 of the tokens - / 184 / 166.  One sequence of 8192: 345 us (798 TFLOP/s).
 //
-// Warp roles: warp 0 = TMA producer, warp 1 = tensor-memory owner + MMA issuer, the others = softmax / epilogue
+// Warp roles: warp 0 = TMA producer, warp 1 = tensor-memory owner + MMA issuer, four warps per head = softmax / epilogue
 // (warp w reads tensor-memory lanes 32*(w%4)..+31 = query rows).
 #include <cuda.h>
 
@@ -44,50 +45,53 @@ struct PrefillParams {
   int* status;
 };
 
-template <int HD>
+// NH: query heads of a CTA
+template <int HD, int NH>
 struct PfCfg {
   static constexpr int BK = 64;                               // keys per block
   static constexpr int HALVES = HD / 64;                      // 64-element (128-byte) column groups
   static constexpr int QTILE = 128 * 64 * 2;                  // [128 rows][64] bf16 = 16 KiB
   static constexpr int KTILE = BK * 64 * 2;                   // [64 keys][64] bf16 = 8 KiB
-  static constexpr int Q_BYTES = HALVES * QTILE;
+  static constexpr int Q_BYTES = HALVES * QTILE;              // of a head
   static constexpr int K_BYTES = HALVES * KTILE;
   static constexpr int V_BYTES = HALVES * KTILE;
-  static constexpr int P_BYTES = 128 * BK * 2;                // 128 rows x 64 keys = 16 KiB
+  static constexpr int P_BYTES = 128 * BK * 2;                // 128 rows x 64 keys = 16 KiB, of a head
   static constexpr int STAGE_BYTES = K_BYTES + V_BYTES;
-  static constexpr int NSTAGE = 2;
-  static constexpr int SMEM_BYTES = Q_BYTES + P_BYTES + NSTAGE * STAGE_BYTES + 128;      // 1 KiB per CTA is reserved: two fit 228
-  static constexpr int TMEM_COLS = 256;                       // S: 2 x 64 columns, behind them O
-  static constexpr int O_COL = 128;
-  static constexpr int THREADS = 192;
+  static constexpr int NSTAGE = NH == 2 ? 4 : 2;
+  // 224 KiB of tiles + barriers with two heads; 112 KiB with one, two CTAs in an SM's 228 KiB (1 KiB is reserved per CTA)
+  static constexpr int SMEM_BYTES = NH * (Q_BYTES + P_BYTES) + NSTAGE * STAGE_BYTES + 192;
+  // of every head: S, 2 x 64 columns; behind all of them O, 128 columns each
+  static constexpr int O_COL = NH * 128;
+  static constexpr int TMEM_COLS = NH * 256;
+  static constexpr int THREADS = 64 + NH * 128;
 };
 
-template <int HD>
-__global__ void __launch_bounds__(PfCfg<HD>::THREADS, 2)
+template <int HD, int NH>
+__global__ void __launch_bounds__(PfCfg<HD, NH>::THREADS, NH == 2 ? 1 : 2)
 prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k0,
                     const __grid_constant__ CUtensorMap tm_v0, const __grid_constant__ CUtensorMap tm_k1,
                     const __grid_constant__ CUtensorMap tm_v1, const __grid_constant__ CUtensorMap tm_k2,
                     const __grid_constant__ CUtensorMap tm_v2, const PrefillParams p) {
-  using C = PfCfg<HD>;
+  using C = PfCfg<HD, NH>;
   constexpr int BK = C::BK;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* q_s = smem;
-  uint8_t* p_s = q_s + C::Q_BYTES;
-  uint8_t* kv_s = p_s + C::P_BYTES;
+  uint8_t* p_s = q_s + NH * C::Q_BYTES;
+  uint8_t* kv_s = p_s + NH * C::P_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(kv_s + C::NSTAGE * C::STAGE_BYTES);
   uint64_t* q_full = bars;
   uint64_t* kv_full = bars + 1;                 // [NSTAGE]
   uint64_t* kv_empty = kv_full + C::NSTAGE;     // [NSTAGE]
-  uint64_t* s_full = kv_empty + C::NSTAGE;      // [2] S = QK^T complete
-  uint64_t* p_ready = s_full + 2;               // P written, O rescaled (128 arrivals)
-  uint64_t* pv_done = p_ready + 1;              // O += PV complete
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 1);
+  uint64_t* s_full = kv_empty + C::NSTAGE;      // [NH][2] S = QK^T complete
+  uint64_t* p_ready = s_full + 2 * NH;          // [NH] P written, O rescaled (128 arrivals)
+  uint64_t* pv_done = p_ready + NH;             // [NH] O += PV complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + NH);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // the last tiles of a sequence walk the most keys: all heads of them first, so that the short ones fill the last wave
-  const int tile = gridDim.x / p.nq - 1 - blockIdx.x / p.nq, head = blockIdx.x % p.nq;
-  const int kvh = head / (p.nq / p.nkv);
+  const int n_hg = p.nq / NH, tile = gridDim.x / n_hg - 1 - blockIdx.x / n_hg, head0 = blockIdx.x % n_hg * NH;
+  const int kvh = head0 / (p.nq / p.nkv);
   const int q0 = p.tile_q0[tile], qn = p.tile_qn[tile];
   if ((smem_u32(smem) & 1023u) != 0) {          // the swizzled tiles need a 1024-byte aligned base
     if (threadIdx.x == 0) atomicCAS(p.status, 0, STATUS_BAD_INDEX);
@@ -110,10 +114,12 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int s = 0; s < C::NSTAGE; ++s) { mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 1); }
-    mbar_init(&s_full[0], 1);
-    mbar_init(&s_full[1], 1);
-    mbar_init(p_ready, 128);
-    mbar_init(pv_done, 1);
+    for (int h = 0; h < NH; ++h) {
+      mbar_init(&s_full[2 * h], 1);
+      mbar_init(&s_full[2 * h + 1], 1);
+      mbar_init(&p_ready[h], 128);
+      mbar_init(&pv_done[h], 1);
+    }
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -130,9 +136,9 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
-      mbar_expect_tx(q_full, C::Q_BYTES);
+      mbar_expect_tx(q_full, NH * C::Q_BYTES);
 #pragma unroll
-      for (int h = 0; h < C::HALVES; ++h) tma_load_2d(q_s + h * C::QTILE, &tm_q, head * HD + h * 64, q0, q_full);
+      for (int h = 0; h < NH * C::HALVES; ++h) tma_load_2d(q_s + h * C::QTILE, &tm_q, head0 * HD + h * 64, q0, q_full);
       int i = 0;
       for (int s = 0; s < p.n_seg; ++s) {
         const CUtensorMap* mk = s == 0 ? &tm_k0 : s == 1 ? &tm_k1 : &tm_k2;
@@ -167,12 +173,15 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tc_fence_after();
         const uint32_t k_addr = smem_u32(kv_s + st * C::STAGE_BYTES);
 #pragma unroll
-        for (int ks = 0; ks < HD / 16; ++ks) {
-          const uint32_t qo = (ks / 4) * C::QTILE + (ks % 4) * 32;
-          const uint32_t ko = (ks / 4) * C::KTILE + (ks % 4) * 32;
-          umma_bf16(tmem_s + (i & 1) * BK, umma_desc_sw128(q_addr + qo), umma_desc_sw128(k_addr + ko), idesc_s, ks > 0 ? 1u : 0u);
+        for (int h = 0; h < NH; ++h) {
+#pragma unroll
+          for (int ks = 0; ks < HD / 16; ++ks) {
+            const uint32_t qo = h * C::Q_BYTES + (ks / 4) * C::QTILE + (ks % 4) * 32;
+            const uint32_t ko = (ks / 4) * C::KTILE + (ks % 4) * 32;
+            umma_bf16(tmem_s + h * 128 + (i & 1) * BK, umma_desc_sw128(q_addr + qo), umma_desc_sw128(k_addr + ko), idesc_s, ks > 0 ? 1u : 0u);
+          }
+          umma_commit(&s_full[2 * h + (i & 1)]);
         }
-        umma_commit(&s_full[i & 1]);
       };
       if (total_blocks > 0) scores(0);
       for (int i = 0; i < total_blocks; ++i) {
@@ -180,24 +189,30 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         if (i + 1 < total_blocks) scores(i + 1);
         const int st = i % C::NSTAGE;
         const uint32_t v_addr = smem_u32(kv_s + st * C::STAGE_BYTES) + C::K_BYTES;
-        // wait for P (and the rescaled O) of this block
-        mbar_wait(p_ready, i & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
-        tc_fence_after();
-        // O += P V : BK / 16 k-steps over the keys; V is MN-major (head_dim contiguous)
 #pragma unroll
-        for (int ks = 0; ks < BK / 16; ++ks) {
-          const uint64_t db = umma_desc_mn_sw128(v_addr + ks * 2048, C::KTILE);
-          umma_bf16(tmem_o, umma_desc_sw128(p_addr + ks * 32), db, idesc_o, (i > 0 || ks > 0) ? 1u : 0u);
+        for (int h = 0; h < NH; ++h) {
+          // wait for P (and the rescaled O) of this block
+          mbar_wait(&p_ready[h], i & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+          tc_fence_after();
+          // O += P V : BK / 16 k-steps over the keys; V is MN-major (head_dim contiguous)
+#pragma unroll
+          for (int ks = 0; ks < BK / 16; ++ks) {
+            const uint64_t db = umma_desc_mn_sw128(v_addr + ks * 2048, C::KTILE);
+            umma_bf16(tmem_o + h * 128, umma_desc_sw128(p_addr + h * C::P_BYTES + ks * 32), db, idesc_o, (i > 0 || ks > 0) ? 1u : 0u);
+          }
+          if (h == NH - 1) umma_commit(&kv_empty[st]);     // K/V stage may be refilled
+          umma_commit(&pv_done[h]);                        // P buffer and O are free for the next block
         }
-        umma_commit(&kv_empty[st]);     // K/V stage may be refilled
-        umma_commit(pv_done);           // P buffer and O are free for the next block
       }
     }
     __syncwarp();
   } else {
     // ---------------- softmax / epilogue: one thread per query row ----------------
     const int qd = warp & 3;                    // tensor-memory lane quadrant this warp may access
+    const int hd = (warp - 2) >> 2, head = head0 + hd;
     const int row = qd * 32 + lane;
+    const uint32_t my_s = tmem_s + hd * 128, my_o = tmem_o + hd * 128;
+    uint8_t* my_p = p_s + hd * C::P_BYTES;
     const bool row_ok = row < qn;
     const uint32_t lane_off = static_cast<uint32_t>(qd * 32) << 16;
     const float sc = p.scale_log2;
@@ -206,12 +221,12 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     for (int s = 0; s < p.n_seg; ++s) {
       const int cnt = row_ok ? p.seg_count[s][q0 + row] : 0;
       for (int b = 0; b < seg_blocks[s]; ++b, ++i) {
-        mbar_wait(&s_full[i & 1], (i >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+        mbar_wait(&s_full[2 * hd + (i & 1)], (i >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
         tc_fence_after();
         const int valid = cnt - b * BK;         // columns [0, valid) of this block are visible
         float sv[BK];
-        tmem_ld32(tmem_s + lane_off + (i & 1) * BK, sv);
-        tmem_ld32(tmem_s + lane_off + (i & 1) * BK + 32, sv + 32);
+        tmem_ld32(my_s + lane_off + (i & 1) * BK, sv);
+        tmem_ld32(my_s + lane_off + (i & 1) * BK + 32, sv + 32);
         tmem_ld_wait();
         float mx = -INFINITY, mx2 = -INFINITY;
         if (__all_sync(0xffffffffu, valid >= BK)) {
@@ -249,30 +264,30 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         }
         l += psum0 + psum1;
         // the previous block's PV must be complete before P is overwritten or O rescaled
-        if (i > 0) mbar_wait(pv_done, (i - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+        if (i > 0) mbar_wait(&pv_done[hd], (i - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
         tc_fence_after();
         if (i > 0 && __any_sync(0xffffffffu, f != 1.0f)) {
 #pragma unroll 1
           for (int c = 0; c < HD; c += 32) {
             float o[32];
-            tmem_ld32(tmem_o + lane_off + c, o);
+            tmem_ld32(my_o + lane_off + c, o);
             tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 32; ++j) o[j] *= f;
-            tmem_st32(tmem_o + lane_off + c, o);
+            tmem_st32(my_o + lane_off + c, o);
           }
           tmem_st_wait();
         }
         // written K-major with the 128-byte swizzle
 #pragma unroll
-        for (int c = 0; c < BK / 8; ++c) *reinterpret_cast<uint4*>(p_s + row * 128 + ((c ^ (row & 7)) << 4)) = pk[c];
+        for (int c = 0; c < BK / 8; ++c) *reinterpret_cast<uint4*>(my_p + row * 128 + ((c ^ (row & 7)) << 4)) = pk[c];
         fence_proxy_async_smem();
         tc_fence_before();
-        mbar_arrive(p_ready);
+        mbar_arrive(&p_ready[hd]);
       }
     }
     // epilogue: O / l
-    if (total_blocks > 0) mbar_wait(pv_done, (total_blocks - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+    if (total_blocks > 0) mbar_wait(&pv_done[hd], (total_blocks - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
     tc_fence_after();
     const float inv = l > 0.f ? 1.0f / l : 0.f;
     if (p.lse != nullptr && row_ok) p.lse[(size_t)(q0 + row) * p.nq + head] = l > 0.f ? m_ref + log2f(l) : -INFINITY;
@@ -281,7 +296,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     for (int c = 0; c < HD; c += 32) {
       float o[32];
       if (total_blocks > 0) {
-        tmem_ld32(tmem_o + lane_off + c, o);
+        tmem_ld32(my_o + lane_off + c, o);
         tmem_ld_wait();
       } else {
 #pragma unroll
@@ -312,14 +327,16 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 using namespace tahb;
 
 // q [n_q, nq*hd], out same; ks/vs[s] [n_kv[s], nkv*hd] (contiguous, bf16); tiles: tile_q0/tile_qn [n_tiles];
-// bases/counts[s]: per query token.  Counts must be non-decreasing inside a tile.
+// bases/counts[s]: per query token.  Counts must be non-decreasing inside a tile.  heads: query heads per CTA, 1 or (an even number per KV
+// head, heads of 128) 2.
 extern "C" int tahb_prefill_attn(const void* q, void* out, void* const* ks, void* const* vs, const long long* n_kv,
                                  const int* const* bases, const int* const* counts, const int* const* bounds,
                                  int n_seg, const int* tile_q0,
                                  const int* tile_qn, int n_tiles, long long n_q, int nq, int nkv, int hd, float scale,
-                                 float* lse, int* status, cudaStream_t stream) {
+                                 float* lse, int heads, int* status, cudaStream_t stream) {
   if (n_tiles <= 0 || n_q <= 0) return 0;
   if (n_seg < 1 || n_seg > PF_MAX_SEG || (nq % nkv)) return -1;
+  if (heads != 1 && (heads != 2 || (nq / nkv) % 2 || hd != 128)) return -1;
   CUtensorMap mq, mk[PF_MAX_SEG], mv[PF_MAX_SEG];
   int rc;
   if ((rc = pf_make_map(&mq, q, n_q, (long long)nq * hd, 128u))) return rc;
@@ -342,21 +359,23 @@ extern "C" int tahb_prefill_attn(const void* q, void* out, void* const* ks, void
   p.scale_log2 = scale * 1.4426950408889634f;
   p.lse = lse;
   p.status = status;
-#define TAHB_PF(HD_)                                                                                               \
+  const bool two = heads == 2;
+#define TAHB_PF(HD_, NH_)                                                                                          \
   {                                                                                                                \
-    using C = PfCfg<HD_>;                                                                                          \
+    using C = PfCfg<HD_, NH_>;                                                                                     \
     static bool configured = false;                                                                                \
     if (!configured) {                                                                                             \
-      if (cudaFuncSetAttribute(prefill_attn_kernel<HD_>, cudaFuncAttributeMaxDynamicSharedMemorySize,              \
+      if (cudaFuncSetAttribute(prefill_attn_kernel<HD_, NH_>, cudaFuncAttributeMaxDynamicSharedMemorySize,         \
                                C::SMEM_BYTES) != cudaSuccess)                                                      \
         return -10;                                                                                                \
       configured = true;                                                                                           \
     }                                                                                                              \
-    prefill_attn_kernel<HD_><<<dim3(n_tiles * nq), C::THREADS, C::SMEM_BYTES, stream>>>(                              \
+    prefill_attn_kernel<HD_, NH_><<<dim3(n_tiles * (nq / NH_)), C::THREADS, C::SMEM_BYTES, stream>>>(                 \
         mq, mk[0], mv[0], mk[1], mv[1], mk[2], mv[2], p);                                                          \
   }
-  if (hd == 128) TAHB_PF(128)
-  else if (hd == 64) TAHB_PF(64)
+  if (hd == 128 && two) TAHB_PF(128, 2)
+  else if (hd == 128) TAHB_PF(128, 1)
+  else if (hd == 64) TAHB_PF(64, 1)
   else return -2;
 #undef TAHB_PF
   return cudaGetLastError() == cudaSuccess ? 0 : -3;

@@ -14,7 +14,7 @@ int tahb_rmsnorm(const void*, const void*, void*, int, int, long long, long long
 int tahb_qk_norm_rope_kv(const void*, const void*, const void*, void*, void*, void*, void* const*, int, const int*, const int*, const int*,
                          int, int, int, int, int, long long, float, float, cudaStream_t);
 int tahb_prefill_attn(const void*, void*, void* const*, void* const*, const long long*, const int* const*, const int* const*,
-                      const int* const*, int, const int*, const int*, int, long long, int, int, int, float, float*, int*, cudaStream_t);
+                      const int* const*, int, const int*, const int*, int, long long, int, int, int, float, float*, int, int*, cudaStream_t);
 }
 
 // Kernel-ready weights of a layer (tah_b200/engine/weights.py); a_* / b_* are null without an adapter.
@@ -42,7 +42,7 @@ struct TahbPass {
   const int* count[3];
   const int *pos, *slots, *tile_q0, *tile_qn;
   int* status;
-  int n_layers, n, hidden, inter, nq, nkv, hd, page_size, n_seg, n_tiles;
+  int n_layers, n, hidden, inter, nq, nkv, hd, page_size, n_seg, n_tiles, attn_heads;
   int r_qkv, r_o, r_gu, r_down;                     // 0 without the adapter
   float eps, theta, scale;
   TahbProductPlan p_qkv, p_o, p_gu, p_down, p_a_qkv, p_a_o, p_a_gu, p_a_down;
@@ -93,7 +93,7 @@ extern "C" int tahb_packed_pass(const TahbPass* a, int* launches, cudaStream_t s
     ks[a->n_seg - 1] = a->k_own[li];
     vs[a->n_seg - 1] = a->v_own[li];
     rc = tahb_prefill_attn(a->q, a->o, ks, vs, a->n_kv, a->base, a->count, a->count, a->n_seg, a->tile_q0, a->tile_qn, a->n_tiles, n, a->nq,
-                           a->nkv, a->hd, a->scale, nullptr, a->status, stream);
+                           a->nkv, a->hd, a->scale, nullptr, a->attn_heads, a->status, stream);
     count += 2;
     adapter(a->p_a_o, L.a_o, a->o, a->t_o, D, a->r_o);
     product(a->p_o, L.w_o, a->o, a->h, a->h, L.b_o, a->t_o, H, D, a->r_o, H);

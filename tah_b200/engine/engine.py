@@ -257,7 +257,7 @@ class TaHEngine(DecodeEngine):
                           [v for _, v in own], seg_k, seg_v, seg_base, seg_count, pos, slots, tile_q0, tile_qn, nq=nq, nkv=nkv, hd=hd,
                           inter=w.inter, ranks=(w.r_qkv, w.r_o, w.r_gu, w.r_down) if lora else (0, 0, 0, 0),
                           gu_interleaved=w.gu_interleaved, page_size=self.page_size, eps=cfg.rms_norm_eps, theta=cfg.rope_theta, scale=scale,
-                          taps=taps)
+                          seqs=seq_counts.numel(), taps=taps)
             if taps_out is not None:
                 taps_out.update(taps)
                 if nL in tap_layers:
@@ -287,7 +287,7 @@ class TaHEngine(DecodeEngine):
             ks = [sk[li] for sk in seg_k] + [kd]
             vs = [sv[li] for sv in seg_v] + [vd]
             if tensor_core_attn:
-                o = K.prefill_attn(q, ks, vs, seg_base, seg_count, tile_q0, tile_qn, nq, nkv, hd, scale)
+                o = K.prefill_attn(q, ks, vs, seg_base, seg_count, tile_q0, tile_qn, nq, nkv, hd, scale, seqs=seq_counts.numel())
             else:
                 o = K.varlen_attn_naive(q, ks, vs, seg_base, seg_count, nq, nkv, hd, scale)
             xn = self._row_parallel(o, L.w_o, L.a_o if lora else None, L.b_o, t_o, None, h, L.ln2, xn_buf, n, push=push)

@@ -373,7 +373,7 @@ class _SegmentAttention(torch.autograd.Function):
         vs = [kv[2 * s + 1].reshape(-1, nkv * hd).contiguous() for s in range(n_seg)]
         lse = torch.empty(B * Tq, nq, dtype=torch.float32, device=q.device)
         out = K.prefill_attn(q2, ks, vs, meta.bases, meta.counts, meta.tile_q0, meta.tile_qn, nq, nkv, hd, hd ** -0.5,
-                             lse=lse, bounds=meta.bounds)
+                             lse=lse, bounds=meta.bounds, seqs=B)
         ctx.meta, ctx.dims = meta, (B, Tq, nq, nkv, hd, n_seg)
         ctx.save_for_backward(q2, out, lse, *ks, *vs)
         return out.view(B, Tq, nq, hd)

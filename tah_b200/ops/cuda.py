@@ -1399,7 +1399,7 @@ def attn_tiles(seq_counts: torch.Tensor, tile: int = 128, by_work: bool = False)
     """Query tiles for :func:`prefill_attn`: every sequence's packed tokens (``seq_counts[b]`` of
     them, sequences laid out back to back) are cut into runs of at most ``tile`` tokens.  Returns
     int32 ``(tile_q0, tile_qn)``; ``by_work``: every sequence's first tiles first instead of sequence by sequence (the kernels
-    start at the end, where the work is: four sequences of 2048 forward 134 and 110 us)."""
+    start at the end, where the work is: four sequences of 2048 forward 117 and 111 us)."""
     cnt = seq_counts.to(torch.int64)
     per = (cnt + tile - 1) // tile
     n_tiles = int(per.sum())
@@ -1414,7 +1414,24 @@ def attn_tiles(seq_counts: torch.Tensor, tile: int = 128, by_work: bool = False)
     return q0.to(torch.int32).contiguous(), qn.to(torch.int32).contiguous()
 
 
-def prefill_attn(q, ks, vs, bases, counts, tile_q0, tile_qn, nq, nkv, hd, scale, out=None, lse=None, bounds=None):
+def prefill_heads(n_tiles: int, nq: int, nkv: int, hd: int, n_seg: int, keys: int, seqs: int) -> int:
+    """Query heads of a CTA of :func:`prefill_attn`, for ``keys`` keys of all segments over ``seqs`` sequences.  Two read a key block once and
+    have four in flight, but halve the CTAs: for long sequences that make three waves (of two one-head CTAs per SM), in deeper passes,
+    whose tiles are fewer and walk more keys, one and a quarter, a single sequence one and a half.  The rule is 0.2 % behind the better
+    form on average over 250 first and second passes of 1 to 12 sequences of 700 to 12000 tokens (9 % at most: second passes of 12 of 1000); one
+    head always 1.3 and 12 %.
+    us, 16 heads of 128 on 8 KV heads, one / two: seven sequences of up to 3500 tokens 304 / 289, three of 2000 86.1 / 86.3, two of 3000 117 / 119, four of
+    4000 382 / 360, 12 of 700 66 / 68; second passes of 0.3 of the tokens: four of 2500 88 / 82, two of 4000 123 / 123, two of 3000 85 / 91.  Heads
+    of 64 lose by two everywhere (four of 2000 85 / 90)."""
+    if (nq // nkv) % 2 or hd != 128 or not seqs:
+        return 1
+    if n_seg == 1:
+        return 2 if n_tiles * nq >= 6 * SM_COUNT and keys >= 2000 * seqs else 1
+    return 2 if 2 * n_tiles * nq >= (5 if seqs > 1 else 6) * SM_COUNT and keys >= 1800 * seqs else 1
+
+
+def prefill_attn(q, ks, vs, bases, counts, tile_q0, tile_qn, nq, nkv, hd, scale, out=None, lse=None, bounds=None, seqs: int = 0,
+                 heads: Optional[int] = None):
     """Packed duo-causal attention on the tensor cores (``csrc/attn_prefill.cu``).  The reference builds a
     dense additive mask ``(kv_pos <= q_pos) & (kv_iter <= q_iter) & kv_valid`` per pass (reference
     ``tah/model/tah_model.py:744-791``) and hands it to SDPA; here the same rule is the per-query prefix
@@ -1422,7 +1439,8 @@ def prefill_attn(q, ks, vs, bases, counts, tile_q0, tile_qn, nq, nkv, hd, scale,
     :func:`varlen_attn_naive` plus the query tiling of :func:`attn_tiles`: the tokens of a tile belong
     to one sequence and share ``bases[s]``.  ``counts[s]`` must be non-decreasing along a sequence's rows, or
     ``bounds[s]`` must give such a non-decreasing upper bound (rows whose count was zeroed, e.g. padding).  ``lse`` (optional fp32
-    ``[n_q, nq]``) receives the base-2 log-sum-exp of the scaled scores, which the backward kernels take."""
+    ``[n_q, nq]``) receives the base-2 log-sum-exp of the scaled scores, which the backward kernels take.  ``seqs``: how many sequences the tokens
+    are of, if known; ``heads``: query heads per CTA (default: by :func:`prefill_heads`)."""
     if out is None:
         out = torch.empty_like(q)
     n = len(ks)
@@ -1430,9 +1448,11 @@ def prefill_attn(q, ks, vs, bases, counts, tile_q0, tile_qn, nq, nkv, hd, scale,
         if t.dtype != torch.bfloat16 or not t.is_contiguous():
             raise ValueError("prefill_attn wants contiguous bf16 tensors")
     n_kv = (c_ll * n)(*[k.shape[0] for k in ks])
+    if heads is None:
+        heads = prefill_heads(tile_q0.numel(), nq, nkv, hd, n, sum(n_kv), seqs)
     _rc(lib().tahb_prefill_attn(_p(q), _p(out), _ptr_array(ks), _ptr_array(vs), n_kv, _ptr_array(bases),
                                 _ptr_array(counts), _ptr_array(bounds if bounds is not None else counts), c_int(n), _p(tile_q0), _p(tile_qn), c_int(tile_q0.numel()),
-                                c_ll(q.shape[0]), c_int(nq), c_int(nkv), c_int(hd), c_float(scale), _p(lse),
+                                c_ll(q.shape[0]), c_int(nq), c_int(nkv), c_int(hd), c_float(scale), _p(lse), c_int(heads),
                                 _p(status_word(q.device)), _stream()), "tahb_prefill_attn")
     return out
 
@@ -1455,7 +1475,7 @@ class _Pass(ctypes.Structure):
         [(f, _VP) for f in ("taps", "k_own", "v_own", "pool")] + \
         [("k_seg", _VP * 3), ("v_seg", _VP * 3), ("n_kv", c_ll * 3), ("base", c_void_p * 3), ("count", c_void_p * 3)] + \
         [(f, c_void_p) for f in ("pos", "slots", "tile_q0", "tile_qn", "status")] + \
-        [(f, c_int) for f in ("n_layers", "n", "hidden", "inter", "nq", "nkv", "hd", "page_size", "n_seg", "n_tiles", "r_qkv",
+        [(f, c_int) for f in ("n_layers", "n", "hidden", "inter", "nq", "nkv", "hd", "page_size", "n_seg", "n_tiles", "attn_heads", "r_qkv",
                               "r_o", "r_gu", "r_down")] + \
         [(f, c_float) for f in ("eps", "theta", "scale")] + \
         [(f, _ProductPlan) for f in ("p_qkv", "p_o", "p_gu", "p_down", "p_a_qkv", "p_a_o", "p_a_gu", "p_a_down")]
@@ -1479,10 +1499,10 @@ def pass_weights(layers):
 
 def packed_pass(weights, final_norm, h, xn, pools, k_own, v_own, seg_k, seg_v, bases, counts, pos, slots, tile_q0, tile_qn, *, nq: int, nkv: int,
                 hd: int, inter: int, ranks: Sequence[int], gu_interleaved: bool, page_size: int, eps: float, theta: float, scale: float,
-                taps=None):
+                seqs: int, taps=None):
     """All layers of a pass over the packed tokens ``h [n, H]`` (updated in place) in one call (``csrc/packed_pass.cu``); the final norm's
     output goes to ``xn``.  ``k_own`` / ``v_own``: per layer, this pass's keys and values; ``seg_k`` / ``seg_v``: those of the shallower
-    passes; ``ranks``: adapter widths of qkv, o, gate / up and down, zeros without it; ``taps``: layer -> buffer for its input."""
+    passes; ``seqs``: sequences that the tokens are of; ``ranks``: adapter widths of qkv, o, gate / up and down, zeros without it; ``taps``: layer -> buffer for its input."""
     global launch_count
     if len(bases) > 3:
         raise RuntimeError("tahb_packed_pass failed on the host side (more than three passes deep)")
@@ -1506,7 +1526,7 @@ def packed_pass(weights, final_norm, h, xn, pools, k_own, v_own, seg_k, seg_v, b
     a.pos, a.slots, a.tile_q0, a.tile_qn = pos.data_ptr(), slots.data_ptr(), tile_q0.data_ptr(), tile_qn.data_ptr()
     a.status = status_word(h.device).data_ptr()
     a.n_layers, a.n, a.hidden, a.inter, a.nq, a.nkv, a.hd, a.page_size = L, n, H, inter, nq, nkv, hd, page_size
-    a.n_seg, a.n_tiles = len(bases), tile_q0.numel()
+    a.n_seg, a.n_tiles, a.attn_heads = len(bases), tile_q0.numel(), prefill_heads(tile_q0.numel(), nq, nkv, hd, len(bases), sum(a.n_kv), seqs)
     a.r_qkv, a.r_o, a.r_gu, a.r_down = ranks
     a.eps, a.theta, a.scale = eps, theta, scale
 

@@ -1123,7 +1123,7 @@ def test_gemm_tile_forms_give_the_same_bits(M, F, K, residual):
 @pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("nq,nkv", [(3, 1), (4, 4), (4, 1), (6, 3)])
 def test_attention_heads_of_a_kv_head(hd, nq, nkv):
-    """Forward and backward with odd and even numbers of query heads per KV head (even ones go two to a CTA), sequences around the sizes
+    """Forward and backward with odd and even numbers of query heads per KV head (even ones go one or two to a CTA), sequences around the sizes
     of key blocks and query tiles; bounds as in the tests above."""
     Kc = _cuda()
     lens = [1, 63, 64, 65, 129, 300]
@@ -1273,3 +1273,30 @@ def test_qk_norm_rope_of_few_tokens(hd, nq, nkv):
             one = [s + p.double() for s, p in zip(one, part[1:])]
         for a, b, heads in zip((gq, gk), one, (nq, nkv)):
             _close(a, b, atol=2e-5 * (m * heads) ** 0.5 + 1e-4, rtol=1e-5)
+
+
+@pytest.mark.parametrize("nq,nkv", [(4, 2), (4, 1)])
+def test_prefill_attention_two_heads_per_cta(nq, nkv):
+    """Two query heads per CTA: the same products in the same order as with one, so the same bits; two passes, sequences around the sizes of
+    key blocks and query tiles."""
+    Kc, hd = _cuda(), 128
+    lens = [1, 63, 64, 65, 129, 300, 700]
+    deep = [[j for j in range(L) if j % 3 == L % 3] for L in lens]
+    starts = lambda sizes: [sum(sizes[:i]) for i in range(len(sizes))]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    n, m = sum(lens), sum(map(len, deep))
+    k0, v0 = (_rand(n, nkv * hd, seed=j) for j in (1, 2))
+    k1, v1 = (_rand(m, nkv * hd, seed=j) for j in (3, 4))
+    first = ([k0], [v0], [i32([s for s, L in zip(starts(lens), lens) for _ in range(L)])], [i32([j + 1 for L in lens for j in range(L)])], lens)
+    second = ([k0, k1], [v0, v1],
+              [i32([s for s, d in zip(at, deep) for _ in d]) for at in (starts(lens), starts([len(d) for d in deep]))],
+              [i32([j + 1 for d in deep for j in d]), i32([j + 1 for d in deep for j in range(len(d))])], [len(d) for d in deep])
+    for ks, vs, bases, counts, own in (first, second):
+        q = _rand(sum(own), nq * hd, seed=5)
+        tiles = Kc.attn_tiles(torch.tensor(own, device="cuda"), by_work=True)
+        one, two = (Kc.prefill_attn(q, ks, vs, bases, counts, *tiles, nq, nkv, hd, hd ** -0.5, heads=h) for h in (1, 2))
+        Kc.check_status()
+        assert one.isfinite().all() and torch.equal(one, two)
+        for heads, kv, width in ((nkv, nkv, hd), (2 * nq, 2 * nkv, hd // 2)):            # an odd number per KV head, heads of 64
+            with pytest.raises(RuntimeError):
+                Kc.prefill_attn(q[:, :heads * width].contiguous(), ks, vs, bases, counts, *tiles, heads, kv, width, hd ** -0.5, heads=2)
