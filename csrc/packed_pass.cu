@@ -10,6 +10,9 @@ int tahb_gemm(const void*, const void*, void*, const void*, const void*, const v
               long long, long long, long long, int, int, int, int, int*, cudaStream_t);
 int tahb_gemm_few(const void*, const void*, void*, const void*, const void*, const void*, int, int, int, int, long long, long long, long long,
                   long long, long long, long long, int, float, float, int, cudaStream_t);
+int tahb_gemm_persist(const void*, const void*, void*, const void*, const void*, const void*, int, int, int, int, long long, long long,
+                      long long, long long, long long, long long, int, float, float, int, int, int, int*, cudaStream_t, const void*, const void*,
+                      int);
 int tahb_rmsnorm(const void*, const void*, void*, int, int, long long, long long, float, cudaStream_t);
 int tahb_qk_norm_rope_kv(const void*, const void*, const void*, void*, void*, void*, void* const*, int, const int*, const int*, const int*,
                          int, int, int, int, int, long long, float, float, cudaStream_t);
@@ -22,9 +25,9 @@ struct TahbPassWeights {
   const void *ln1, *ln2, *q_norm, *k_norm, *w_qkv, *w_o, *w_gu, *w_down;
   const void *a_qkv, *b_qkv, *a_o, *b_o, *a_gu, *b_gu, *a_down, *b_down;
 };
-// How a product runs: few != 0: the few-token kernel, else tcgen05 with its form, tile width and split.
+// How a product runs: kind 1 the few-token kernel, 2 the persistent one with its tile width, 0 one tile per CTA with form, tile width and split.
 struct TahbProductPlan {
-  int few, dual, splits, bn;
+  int kind, dual, splits, bn;
 };
 struct TahbPass {
   const TahbPassWeights* layers;
@@ -58,7 +61,10 @@ extern "C" int tahb_packed_pass(const TahbPass* a, int* launches, cudaStream_t s
     if (rc) return;
     ++count;
     const bool stacked = p.dual == 1;
-    if (p.few)
+    if (p.kind == 2)
+      rc = tahb_gemm_persist(w, x, out, res, b, t, n, rows, K, R, K, K, ldo, res ? ldo : 0, R, R, p.dual ? 2 : 0, 0.f, 0.f, 0, 0, p.bn, a->status,
+                             stream, nullptr, nullptr, 0);
+    else if (p.kind == 1)
       rc = tahb_gemm_few(w, x, out, res, b, t, n, rows, K, R, K, K, ldo, ldo, R, R, p.dual, 0.f, 0.f, 1, stream);
     else
       rc = tahb_gemm(w, x, out, res, b, t, n, stacked ? rows / 2 : rows, K, R, K, K, ldo, res ? ldo : 0, R, R, p.dual, stacked ? rows / 2 : 0,

@@ -174,6 +174,11 @@ def plan_tiles(M: int, rows: int, K: int, can_pair: bool, can_split: bool, x_t: 
     the plan for up to 256 tokens (256-token pairs from 1024 on) / by this one: 1536 x 2048 at 450 tokens 11.2 / 11.0, 2048 x 2048 at 1000
     13.8 / 13.5, 4096 x 2048 at 400 14.3 / 13.8, 2048 x 6144 at 520 25.7 / 23.3, at 5200 136 / 117, its weight gradient over 940 tokens
     46.4 / 35.5."""
+    return _tiles_cost(M, rows, K, can_pair, can_split, x_t)[1:]
+
+
+@functools.lru_cache(maxsize=4096)
+def _tiles_cost(M: int, rows: int, K: int, can_pair: bool, can_split: bool, x_t: bool):
     best = None
     for nf in (1, 2) if can_pair else (1,):
         for bn in (64, 128, 192, 256) if nf == 1 else (128, 192, 256):
@@ -190,7 +195,34 @@ def plan_tiles(M: int, rows: int, K: int, can_pair: bool, can_split: bool, x_t: 
                 t = waves * (kb * t_kb + out + {1: 0.0, 2: 1.1 + 0.003 * bn, 4: 0.65 + 0.0133 * bn}[s])
                 if best is None or t < best[0] - 1e-9:
                     best = (t, nf == 2, bn, s)
-    return best[1:]
+    return best
+
+
+# pairs of SMs that the persistent form runs on
+SM_PAIRS = SM_COUNT // 2
+
+
+@functools.lru_cache(maxsize=4096)
+def plan_persist(M: int, rows: int, K: int, R: int = 0, glu: bool = False, x_t: bool = False, can_pair: bool = True) -> int:
+    """Tile width of the persistent form (``csrc/gemm_persist.cu``) for more than 256 tokens, or 0 where one tile per CTA is faster: few tiles
+    with a long reduction, which that form splits (us, persistent / one tile per CTA at 264 tokens: 2048 x 6144 20.3 / 17.6, 12288 x 2048 SwiGLU
+    23.7 / 22.3, 2048 x 12288 35.7 / 24.3; at 2048 x 6144 level at 504 tokens, 31.4 / 38.0 at 1504).
+
+    Both are estimated.  Microseconds, fitted to tiles of 64 to 256 features at weights of 2048 to 12288 rows, reductions of 264 to 15696 and 264 to
+    15696 tokens, K-major and transposed operands: 128 of the reduction take what the table says, or the epilogue bounds a wave (short reductions).
+    The estimate of the other form lies a ninth below what it takes beside other launches.  Of 60 measured products the choice is the faster
+    form but for 3, which lose 5 %."""
+    best = None
+    steps = -(-K // 128) + -(-R // 128)
+    for bn, kb in ((64, 0.35), (128, 0.41), (192, 0.58), (256, 0.72)):
+        if glu and bn % 128:
+            continue
+        waves = -(-(-(-M // 256) * -(-rows // bn)) // SM_PAIRS)
+        t = 3.2 + 0.004 * bn + waves * max(steps * kb, 1.25 + 0.006 * bn)
+        if best is None or t < best[0] - 1e-9:
+            best = (t, bn)
+    other = _tiles_cost(M, rows, K + R, can_pair and PAIR_AUTO and rows % 256 == 0, not glu, x_t)[0]
+    return best[1] if best[0] <= 1.12 * other else 0
 
 
 def interleave_gate_up(w: torch.Tensor) -> torch.Tensor:
@@ -315,6 +347,11 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
             not ((swiglu or gelu) and (residual is not None or swiglu and gelu)) and _few_ok(x, w, x2, w2, const_w) and
             (not (gelu or swiglu_interleaved) or _whole_pieces(out))):
         return _gemm_few(x, w, out, residual, x2, w2, 1 if swiglu else 3 if gelu else 4 if swiglu_interleaved else 0, early=const_w)
+    if (pair is None and bn == 0 and splits is None and tp_push is None and not swiglu and not (gelu and residual is not None) and
+            _persist_ok(x, w, out, residual, x2, w2)):
+        bn = plan_persist(M, F, K, R, swiglu_interleaved)
+        if bn:
+            return _gemm_persist(x, w, out, residual, x2, w2, 1 if gelu else 2 if swiglu_interleaved else 0, bn, tp_wait=tp_wait)
     pair, bn, splits = _plan_tiles(M, w.shape[0], K, R, swiglu, gelu, swiglu_interleaved, pair, bn, splits,
                                    () if tp_push is not None else (out, residual))
     args = (_p(w), _p(x), _p(out), _p(residual), _p(w2), _p(x2), c_int(M), c_int(F), c_int(K), c_int(R),
@@ -382,6 +419,30 @@ def _gemm_few(x, w, out, residual=None, x2=None, w2=None, act: int = 0, act_up: 
     return out
 
 
+def _persist_ok(x, w, out, residual=None, x2=None, w2=None, x_t: bool = False, w_t: bool = False) -> bool:
+    """Whether the persistent form takes these operands: more than 256 tokens, whole pieces of 16 bytes everywhere, whole blocks of the
+    reduction (unless both operands are transposed)."""
+    M, K = (x.shape[1], x.shape[0]) if x_t else x.shape
+    F = w.shape[1] if w_t else w.shape[0]
+    return (M > 256 and F > 0 and K > 0 and (K % 64 == 0 or x_t and w_t) and (x2 is None or x2.shape[1] % 64 == 0) and
+            (not w_t or F % 128 == 0) and (residual is None or F % 8 == 0) and
+            all(t is None or _whole_pieces(t) for t in (x, w, out, residual, x2, w2)))
+
+
+def _gemm_persist(x, w, out, residual=None, x2=None, w2=None, act: int = 0, bn: int = 256, act_up: float = 0.0, act_low: float = 0.0,
+                  x_t: bool = False, w_t: bool = False, tp_wait=None):
+    """``act``: 0 none, 1 GELU, 2 SwiGLU of interleaved rows, 3 xIELU."""
+    ld = lambda t: c_ll(0 if t is None else t.stride(0))
+    M, K = (x.shape[1], x.shape[0]) if x_t else x.shape
+    F = w.shape[1] if w_t else w.shape[0]
+    wait = (None, None, c_int(0)) if tp_wait is None else (_p(tp_wait[0]), _p(tp_wait[1]), c_int(tp_wait[0].numel()))
+    _rc(lib().tahb_gemm_persist(_p(w), _p(x), _p(out), _p(residual), _p(w2), _p(x2), c_int(M), c_int(F), c_int(K),
+                                c_int(0 if x2 is None else x2.shape[1]), ld(w), ld(x), ld(out), ld(residual), ld(w2), ld(x2), c_int(act),
+                                c_float(act_up), c_float(act_low), c_int(1 if x_t else 0), c_int(1 if w_t else 0), c_int(bn),
+                                _p(status_word(x.device)), _stream(), *wait), "tahb_gemm_persist")
+    return out
+
+
 def gemm_t(x: torch.Tensor, w: torch.Tensor, *, x_t: bool = False, w_t: bool = False, out: Optional[torch.Tensor] = None,
            residual: Optional[torch.Tensor] = None, splits: Optional[int] = None, bn: int = 0,
            pair: Optional[bool] = None) -> torch.Tensor:
@@ -411,6 +472,10 @@ def gemm_t(x: torch.Tensor, w: torch.Tensor, *, x_t: bool = False, w_t: bool = F
     if residual is not None:
         _check_bf16_2d(residual, "residual")
     can_pair = F % 256 == 0 and (not x_t or M % 64 == 0)
+    if pair is None and bn == 0 and splits is None and _persist_ok(x, w, out, residual, x_t=x_t, w_t=w_t):
+        bn = plan_persist(M, F, Kx, 0, False, x_t, can_pair)
+        if bn:
+            return _gemm_persist(x, w, out, residual, bn=bn, x_t=x_t, w_t=w_t)
     if pair is None and bn == 0 and splits is None and M > 256:
         staged = _whole_pieces(out) and (residual is None or _whole_pieces(residual))
         pair, bn, splits = plan_tiles(M, F, Kx, can_pair and PAIR_AUTO and staged, True, x_t)
@@ -735,6 +800,10 @@ def xielu_linear(x: torch.Tensor, w: torch.Tensor, up: float, low: float, out: O
         _check_bf16_2d(t, n)
     if _few_ok(x, w, const=const_w) and _whole_pieces(out):
         return _gemm_few(x, w, out, act=5, act_up=up, act_low=low, early=const_w)
+    if _persist_ok(x, w, out):
+        bn = plan_persist(M, F, Kd)
+        if bn:
+            return _gemm_persist(x, w, out, act=3, bn=bn, act_up=up, act_low=low)
     pair, bn, splits = _plan_tiles(M, F, Kd, 0, False, False, False)
     _rc(lib().tahb_gemm_xielu(_p(w), _p(x), _p(out), c_int(M), c_int(F), c_int(Kd), c_ll(w.stride(0)), c_ll(x.stride(0)), c_ll(out.stride(0)),
                               c_float(up), c_float(low), c_int(int(pair)), c_int(splits), c_int(bn), _p(status_word(x.device)), _stream()),
@@ -1458,7 +1527,7 @@ def prefill_attn(q, ks, vs, bases, counts, tile_q0, tile_qn, nq, nkv, hd, scale,
 
 
 class _ProductPlan(ctypes.Structure):
-    _fields_ = [(f, c_int) for f in ("few", "dual", "splits", "bn")]
+    _fields_ = [(f, c_int) for f in ("kind", "dual", "splits", "bn")]
 
 
 class _PassWeights(ctypes.Structure):
@@ -1534,6 +1603,9 @@ def packed_pass(weights, final_norm, h, xn, pools, k_own, v_own, seg_k, seg_v, b
         stacked, il = glu and not gu_interleaved, glu and gu_interleaved
         if few_shape(n, rows, K, R, True):
             return _ProductPlan(1, 4 if il else 1 if stacked else 0, 1, 0)
+        bn = plan_persist(n, rows, K, R, il) if n > 256 and not stacked and K % 64 == 0 and R % 64 == 0 and rows % 8 == 0 else 0
+        if bn:
+            return _ProductPlan(2, 4 if il else 0, 1, bn)
         pair, bn, splits = _plan_tiles(n, rows, K, R, stacked, False, il)
         return _ProductPlan(0, 1 if stacked else (6 if pair else 4) if il else 2 if pair else 0, splits, bn)
 

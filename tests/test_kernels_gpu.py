@@ -1300,3 +1300,65 @@ def test_prefill_attention_two_heads_per_cta(nq, nkv):
         for heads, kv, width in ((nkv, nkv, hd), (2 * nq, 2 * nkv, hd // 2)):            # an odd number per KV head, heads of 64
             with pytest.raises(RuntimeError):
                 Kc.prefill_attn(q[:, :heads * width].contiguous(), ks, vs, bases, counts, *tiles, heads, kv, width, hd ** -0.5, heads=2)
+
+
+@pytest.mark.parametrize("bn", [64, 128, 192, 256])
+@pytest.mark.parametrize("M,F,Kd,R,form", [(257, 200, 64, 0, ""), (300, 8, 192, 64, "residual"), (513, 2056, 2048, 64, "residual"), (700, 640, 320, 0, "w_t"),
+                                           (704, 640, 333, 0, "x_t"), (264, 1152, 4001, 0, "x_t residual"), (513, 448, 128, 192, "glu"),
+                                           (9000, 2048, 128, 0, "residual"), (640, 456, 512, 64, "gelu"), (640, 456, 512, 0, "xielu")])
+def test_gemm_persist(bn, M, F, Kd, R, form):
+    """The persistent product over edges of its tiles (256 tokens, bn features, chunks of 64, blocks of 128 of the reduction), one and several
+    tiles per pair of SMs, against 64 bits.  Bound: a bf16 rounding (2^-9 relative, 2^-8 for both of its neighbours) of the sum and one of
+    what is made of it; an activation carries the first with a slope of at most 1.2 (1 + |z| for up z^2), SwiGLU with its factors."""
+    Kc = _cuda()
+    if "glu" == form and bn % 128:
+        pytest.skip("tiles of whole gate / up chunks")
+    x, w = _rand(M, Kd, seed=1), _rand(F, Kd, scale=Kd ** -0.5, seed=2)
+    x2, w2 = (_rand(M, R, seed=3), _rand(F, R, scale=0.1, seed=4)) if R else (None, None)
+    z = x.double() @ w.double().t() + (x2.double() @ w2.double().t() if R else 0)
+    F_out, kw = F, {}
+    eps = 2.0 ** -8
+    if form == "glu":
+        F_out, kw = F // 2, dict(act=2)
+        g, u = z[:, 0::2], z[:, 1::2]
+        ref = torch.nn.functional.silu(g) * u
+        bound = eps * (1.2 * g.abs() * u.abs() + 3 * ref.abs())
+    elif form == "gelu":
+        ref, kw = torch.nn.functional.gelu(z), dict(act=1)
+        bound = eps * (1.2 * z.abs() + ref.abs())
+    elif form == "xielu":
+        kw = dict(act=3, act_up=0.7, act_low=0.3)
+        ref = torch.where(z > 0, 0.7 * z * z, 0.3 * (torch.exp(z) - 1 - z)) + 0.5 * z
+        bound = eps * ((1 + 1.4 * z.abs()) * z.abs() + ref.abs())
+    else:
+        ref, bound = z, eps * 2 * z.abs()
+    res = None
+    if "residual" in form:
+        res = _rand(M, F, seed=5)
+        ref = z + res.double()
+        bound = eps * (z.abs() + ref.abs())
+    pitch = (F_out + 15) // 8 * 8
+    store = torch.full((M + 2, pitch), 7.0, dtype=torch.bfloat16, device="cuda")
+    out = store[1:M + 1, :F_out]
+    if res is not None:
+        out.copy_(res)
+    x_t = form.startswith("x_t")
+    w_t = x_t or form == "w_t"
+    Kc._gemm_persist(x.t().contiguous() if x_t else x, w.t().contiguous() if w_t else w, out, out if res is not None else None, x2, w2, bn=bn, x_t=x_t,
+                     w_t=w_t, **kw)
+    Kc.check_status()
+    assert bool(((out.double() - ref).abs() <= 1.01 * bound + 2e-5).all())
+    assert bool((store[0] == 7).all()) and bool((store[-1] == 7).all()) and bool((store[:, F_out:] == 7).all())   # nothing beyond the output
+
+
+def test_gemm_persist_is_what_wide_products_take():
+    """Above 256 tokens the wrappers take the persistent form where its estimate is lower, and give what one tile per CTA gives to a rounding."""
+    Kc = _cuda()
+    x, w, res = _rand(1500, 2048, seed=1), _rand(2048, 2048, scale=2048 ** -0.5, seed=2), _rand(1500, 2048, seed=3)
+    assert Kc.plan_persist(1500, 2048, 2048) and not Kc.plan_persist(264, 2048, 12288)
+    for kw in ({}, dict(residual=res)):
+        a, b = Kc.gemm(x, w, **kw), Kc.gemm(x, w, pair=False, bn=256, **kw)
+        assert bool(((a.double() - b.double()).abs() <= 2.0 ** -7 * b.double().abs() + 1e-3).all())
+    a, b = Kc.gemm_t(x, w, w_t=True), Kc.gemm_t(x, w, w_t=True, pair=False, bn=256)
+    assert bool(((a.double() - b.double()).abs() <= 2.0 ** -7 * b.double().abs() + 1e-3).all())
+    Kc.check_status()

@@ -471,3 +471,16 @@ def test_tile_plan_counts_the_clusters_that_fit():
                 assert splits < 4 or not 132 < ctas <= 148, (M, rows, K)
     assert cuda.plan_tiles(1536, 64, 2048, False, True) == (False, 64, 4)
     assert cuda.plan_tiles(450, 1536, 2048, True, True) == (False, 128, 2)
+
+
+def test_persistent_tile_plan():
+    """Tiles of the persistent product: whole gate / up chunks for SwiGLU, narrow tiles where wide ones leave SMs idle, and none where few tiles with
+    a long reduction want a split."""
+    from tah_b200.ops import cuda
+    for rows in (64, 512, 2048, 12288, 151936):
+        for K in (64, 300, 2048, 12288):
+            for M in (257, 700, 3072, 16000):
+                assert cuda.plan_persist(M, rows, K) in (0, 64, 128, 192, 256)
+                assert cuda.plan_persist(M, rows, K, 64, True) in (0, 128, 256)
+    assert cuda.plan_persist(504, 2048, 2048) == 64 and cuda.plan_persist(16000, 2048, 2048) == 256
+    assert cuda.plan_persist(264, 2048, 12288) == 0
