@@ -56,6 +56,20 @@ static inline int make_map_mn(CUtensorMap* m, const void* base, long long red_ro
   return r == CUDA_SUCCESS ? 0 : -3;
 }
 
+// Boxes of 32 columns (64 bytes) with the 64-byte swizzle.
+static inline int make_map_half(CUtensorMap* m, const void* base, long long rows, long long cols, long long ld, int box_rows) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (!fn) return -1;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || ((ld * 2) & 15)) return -2;
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+  cuuint32_t box[2] = {32u, (cuuint32_t)box_rows};
+  cuuint32_t estr[2] = {1u, 1u};
+  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -3;
+}
+
 // Two blocks of 64 of the reduction per copy: a K-major operand [rows, cols] seen as [cols / 64][rows][64], so that a copy leaves two K-major
 // tiles of box_rows rows behind one another in shared memory.  cols is a multiple of 64; a block past it reads as zeros.
 static inline int make_map_two(CUtensorMap* m, const void* base, long long rows, long long cols, long long ld, int box_rows) {

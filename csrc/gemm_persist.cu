@@ -24,7 +24,7 @@
 //
 // Warp roles in each CTA: warp 0 = TMA producer (both CTAs signal the first CTA's barrier), warp 1 = tensor-memory owner and, in the first CTA of
 // the pair, MMA issuer, warps 2..9 = epilogue (warp w reads tensor-memory lanes 32 * (w % 4) .. + 31).  An epilogue warp stages its own 32 tokens
-// x 64 features and stores them with its own TMA store, so the epilogue warps never wait for one another.
+// x 64 weight rows and stores them with its own TMA store, so the epilogue warps never wait for one another.
 #include <cuda.h>
 
 #include "attn_common.cuh"
@@ -74,10 +74,9 @@ __device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a,
       : "memory");
 }
 // arrives at this barrier of both CTAs once the products issued so far have completed
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
-               "h"(static_cast<uint16_t>(3))
-               : "memory");
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint32_t bar_peer) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_peer) : "memory");
 }
 // a copy into this CTA's shared memory that reports to a barrier of either CTA of the pair (no multicast)
 __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tmap, int x, int y, uint32_t bar) {
@@ -94,15 +93,6 @@ __device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const void* tma
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// As mbar_wait, for the loops whose every step a wait stands in: the flag and the clock are looked at only once the barrier has been
-// asked many times.  False once this CTA has given up.
-__device__ __forceinline__ bool mbar_wait_tight(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-#pragma unroll 1
-  for (int i = 0; i < 256; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  mbar_wait(bar, parity, abort_flag, status, code);
-  return *abort_flag == 0;
 }
 // groups of p.group token tiles by all feature tiles: the tiles that run at once share few rows of X and W, which stay in L2
 __device__ __forceinline__ void persist_tile(const PersistParams& p, int tile, int& tm, int& tn) {
@@ -121,58 +111,59 @@ __device__ __forceinline__ void persist_residual(const PersistParams& p, int t, 
 
 template <int MODE>
 __device__ __forceinline__ float persist_act(const PersistParams& p, float a) {
-  if constexpr (MODE == 3) {
-    const float z = bf16_round(a);
-    return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f));
-  } else if constexpr (MODE == 4) {
-    const float z = bf16_round(a);
-    const float neg = p.act_low * (ex2_approx(z * 1.4426950408889634f) - 1.0f - z);
-    return fmaf(0.5f, z, z > 0.f ? p.act_up * z * z : neg);
-  } else {
-    return a;
-  }
+  const float z = bf16_round(a);
+  if constexpr (MODE == 3) return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f));
+  const float neg = p.act_low * (ex2_approx(z * 1.4426950408889634f) - 1.0f - z);
+  return fmaf(0.5f, z, z > 0.f ? p.act_up * z * z : neg);
 }
 
-// 64 output features of this lane's token into the warp's staging buffer (row of 128 bytes, 128-byte swizzle); `acc`: the first
-// tensor-memory column
+// 64 weight rows' worth of this lane's token into the warp's staging buffer: 64 output features (row of 128 bytes, 128-byte swizzle) or 32 of a
+// SwiGLU (64 bytes, 64-byte swizzle); `acc`: the first tensor-memory column
 template <int MODE>
 __device__ __forceinline__ void persist_chunk(const PersistParams& p, uint32_t acc, uint8_t* stg, int lane, const uint4 (&res)[8]) {
-  uint8_t* row = stg + lane * 128;
+  if constexpr (MODE >= 2) {
+    // activations piece by piece: unrolled over the chunk their code is fetched for longer than it runs (256 tokens, 12288 x 2048 SwiGLU)
+    constexpr int PIECES = MODE == 2 ? 4 : 8;
+#pragma unroll 1
+    for (int c = 0; c < PIECES; ++c) {
+      float a[16];
+      if constexpr (MODE == 2) tmem_ld16(acc + c * 16, a);
+      else tmem_ld8(acc + c * 8, a);
+      tmem_ld_wait();
+      uint4 pk;
+      __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll
-  for (int h = 0; h < (MODE == 2 ? 2 : 1); ++h) {
-    float a[64];
-    tmem_ld32(acc + h * 64, a);
-    tmem_ld32(acc + h * 64 + 32, a + 32);
-    tmem_ld_wait();
-    if constexpr (MODE == 2) {
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint4 pk;
-        __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&pk);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float* v = a + c * 16 + j * 4;
+      for (int j = 0; j < 4; ++j) {
+        if constexpr (MODE == 2) {
+          const float* v = a + j * 4;
           o[j] = __floats2bfloat162_rn(bf16_round(silu(bf16_round(v[0]))) * bf16_round(v[1]), bf16_round(silu(bf16_round(v[2]))) * bf16_round(v[3]));
+        } else {
+          o[j] = __floats2bfloat162_rn(persist_act<MODE>(p, a[2 * j]), persist_act<MODE>(p, a[2 * j + 1]));
         }
-        *reinterpret_cast<uint4*>(row + (((h * 4 + c) ^ (lane & 7)) << 4)) = pk;
       }
-    } else {
+      if constexpr (MODE == 2) *reinterpret_cast<uint4*>(stg + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) = pk;
+      else *reinterpret_cast<uint4*>(stg + lane * 128 + ((c ^ (lane & 7)) << 4)) = pk;
+    }
+  } else {
+    float a[64];
+    tmem_ld32(acc, a);
+    tmem_ld32(acc + 32, a + 32);
+    tmem_ld_wait();
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        uint4 pk;
-        __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&pk);
-        const __nv_bfloat162* r = reinterpret_cast<const __nv_bfloat162*>(&res[c]);
+    for (int c = 0; c < 8; ++c) {
+      uint4 pk;
+      __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&pk);
+      const __nv_bfloat162* r = reinterpret_cast<const __nv_bfloat162*>(&res[c]);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          if constexpr (MODE == 1) {
-            const float2 f = __bfloat1622float2(r[j]);
-            o[j] = __floats2bfloat162_rn(bf16_round(a[c * 8 + 2 * j]) + f.x, bf16_round(a[c * 8 + 2 * j + 1]) + f.y);
-          } else {
-            o[j] = __floats2bfloat162_rn(persist_act<MODE>(p, a[c * 8 + 2 * j]), persist_act<MODE>(p, a[c * 8 + 2 * j + 1]));
-          }
+      for (int j = 0; j < 4; ++j) {
+        if constexpr (MODE == 1) {
+          const float2 f = __bfloat1622float2(r[j]);
+          o[j] = __floats2bfloat162_rn(bf16_round(a[c * 8 + 2 * j]) + f.x, bf16_round(a[c * 8 + 2 * j + 1]) + f.y);
+        } else {
+          o[j] = __floats2bfloat162_rn(a[c * 8 + 2 * j], a[c * 8 + 2 * j + 1]);
         }
-        *reinterpret_cast<uint4*>(row + ((c ^ (lane & 7)) << 4)) = pk;
       }
+      *reinterpret_cast<uint4*>(stg + lane * 128 + ((c ^ (lane & 7)) << 4)) = pk;
     }
   }
 }
@@ -279,6 +270,7 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
       const uint32_t a_addr = smem_u32(smem), b_addr = a_addr + PERSIST_A, stage16 = p.stage_bytes >> 4;
       const uint64_t da0 = p.a_mn ? umma_desc_mn_sw128(a_addr, 16384) : umma_desc_sw128(a_addr);
       const uint64_t db0 = p.b_mn ? umma_desc_mn_sw128(b_addr, 16384) : umma_desc_sw128(b_addr);
+      const uint32_t empty_peer = dsmem_addr(smem_u32(empty), 1), acc_full_peer = dsmem_addr(smem_u32(acc_full), 1);
       int s = 0;
       uint32_t ph = 0;
       int n = 0;
@@ -302,7 +294,7 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
 #pragma unroll
                 for (int k = 0; k < 4; ++k) umma_bf16_pair(d, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), idesc, 1u);
               }
-              umma_commit_pair(&empty[s]);
+              umma_commit_pair(&empty[s], empty_peer + s * 8);
             }
             acc = 1u;
             if (++s == p.stages) { s = 0; ph ^= 1; }
@@ -310,16 +302,17 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
         };
         blocks(p.kb_main);
         if (p.kb_ext > 0) blocks(p.kb_ext);
-        if (elect_one()) umma_commit_pair(&acc_full[buf]);
+        if (elect_one()) umma_commit_pair(&acc_full[buf], acc_full_peer + buf * 8);
       }
     }
     __syncwarp();
   } else {
-    // ---------------- epilogue: two warps per lane quarter with alternate chunks of 64 output features ----------------
+    // ---------------- epilogue: two warps per lane quarter with alternate chunks ----------------
     const int q = warp & 3, half = (warp - 2) >> 2;
     uint8_t* stg = staging + (warp - 2) * PERSIST_STG;
     const uint32_t lanes = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     const uint32_t acc_empty0 = dsmem_addr(smem_u32(acc_empty), 0);
+    constexpr int CH = MODE == 2 ? 32 : 64;          // output features of a chunk
     const int out_bn = MODE == 2 ? p.bn / 2 : p.bn;
     int n = 0;
     uint4 res[8];
@@ -327,7 +320,7 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
       int tm, tn;
       persist_tile(p, tile, tm, tn);
       const int t0 = tm * 256 + rank * 128 + q * 32, o0 = tn * out_bn;
-      const int chunks = t0 < p.M ? (min(out_bn, p.F_out - o0) + 63) / 64 : 0;
+      const int chunks = t0 < p.M ? (min(out_bn, p.F_out - o0) + CH - 1) / CH : 0;
       if constexpr (MODE == 1) {
         if (half < chunks) persist_residual(p, t0 + lane, o0 + half * 64, res);       // under the main loop
       }
@@ -338,11 +331,11 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
       for (int c = half; c < chunks; c += 2) {
         if (lane == 0) tma_store_wait_read();          // the buffer's last store has read it
         __syncwarp();
-        persist_chunk<MODE>(p, lanes + buf * 256 + c * (MODE == 2 ? 128 : 64), stg, lane, res);
+        persist_chunk<MODE>(p, lanes + buf * 256 + c * 64, stg, lane, res);
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
-          tma_store_2d(&tm_out, stg, o0 + c * 64, t0);
+          tma_store_2d(&tm_out, stg, o0 + c * CH, t0);
           tma_store_commit();
         }
         if constexpr (MODE == 1) {
@@ -384,7 +377,7 @@ using namespace tahb;
 
 // out[M, F'] = op(X) op(W)^T (+ X2 W2^T) (+ residual), F' = F or, with act 2, F / 2.  F counts weight rows.  x_t: X is stored [K, M]; w_t: W is
 // stored [K, F]; K (the reduction) is a multiple of 64 unless both are transposed (then its tail reads as zeros).  act: 0 none, 1 GELU, 2 SwiGLU of
-// interleaved rows, 3 xIELU, without a residual but for 0.  bn: weight rows of a tile, a multiple of 64 up to 256 (of 128 with act 2).  Every
+// interleaved rows, 3 xIELU, without a residual but for 0.  bn: weight rows of a tile, a multiple of 64 up to 256.  Every
 // operand, out and residual lie on 16-byte boundaries with row pitches that are multiples of 8 elements.  wait_*: see tahb_gemm_tp.
 extern "C" int tahb_gemm_persist(const void* W, const void* X, void* out, const void* residual, const void* W2, const void* X2, int M, int F,
                                  int K, int R, long long ldw, long long ldx, long long ldo, long long ldr, long long ldw2, long long ldx2,
@@ -395,7 +388,7 @@ extern "C" int tahb_gemm_persist(const void* W, const void* X, void* out, const 
   if (K <= 0 || R % 64 || (Kp != K && !(x_t && w_t))) return -20;
   if (act < 0 || act > 3 || (act && (residual != nullptr || x_t || w_t))) return -29;
   if (R > 0 && (x_t || w_t)) return -27;
-  if (bn < 64 || bn > 256 || bn % (act == 2 ? 128 : 64)) return -22;
+  if (bn < 64 || bn > 256 || bn % 64) return -22;
   if (act == 2 && F % 2) return -29;
   PersistParams p;
   p.b_mn = w_t != 0;
@@ -412,8 +405,8 @@ extern "C" int tahb_gemm_persist(const void* W, const void* X, void* out, const 
     if ((rc = make_map_two(&mw2, W2, F, R, ldw2, bn / 2))) return rc;
   }
   p.F_out = act == 2 ? F / 2 : F;
-  // output tiles: 32 tokens x 64 features with the operands' swizzle
-  if ((rc = make_map(&mo, out, M, p.F_out, ldo, 32, true))) return rc;
+  // output pieces: 32 tokens x 64 features, or 32 features
+  if ((rc = act == 2 ? make_map_half(&mo, out, M, p.F_out, ldo, 32) : make_map(&mo, out, M, p.F_out, ldo, 32, true))) return rc;
   if (residual != nullptr && ((reinterpret_cast<uintptr_t>(residual) & 15) || (ldr & 7) || (F & 7))) return -2;
   p.M = M;
   p.kb_main = Kp / 64;

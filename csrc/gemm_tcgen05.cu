@@ -31,7 +31,11 @@
 // and its arithmetic and tensor-memory loads are bound by the warps that issue them: from 64 tokens on eight warps share it, two per
 // lane quarter with alternate columns (or, in the pair form, a tile each).  Four against eight warps:
 // 12288 x 2048 with SwiGLU at 13600 tokens 604 and 553 us, at 256 tokens 21.3 and 20.4; 2048 x 6144 with a residual at 3072
-// tokens 76.7 and 69.8 (there also because the producer loads the pair form's residual tiles behind the last k block)
+// tokens 76.7 and 69.8 (there also because the producer loads the pair form's residual tiles behind the last k block).
+// A step of the producer's and of the issuer's loop costs about 500 cycles whatever it carries, which bound every tile of up to 128 tokens (0.31 us
+// per 64 of the reduction): a stage of those carries 128, and elected lanes of converged warps issue (before / after, weights out of HBM:
+// 50 tokens 4096 x 2048 8.3 / 7.6 us, 2048 x 2048 7.9 / 6.6, 12288 x 2048 SwiGLU 14.8 / 12.1, 2048 x 6144 13.6 / 10.4; 256 tokens 11.2 / 9.8,
+// 9.9 / 8.4, -, 15.5 / 13.7)
 #include <cuda.h>
 #include <stdio.h>
 
@@ -102,12 +106,13 @@ struct GemmParams {
 
 template <int BN, bool DUAL>
 struct GemmCfg {
-  static constexpr int W_TILE = 128 * 64 * 2;                 // 16 KiB
+  static constexpr int KB = !DUAL && BN <= 128 ? 2 : 1;       // blocks of 64 of the reduction in a stage
+  static constexpr int W_TILE = 128 * 64 * 2 * KB;            // 16 or 32 KiB
   static constexpr int W_BYTES = W_TILE * (DUAL ? 2 : 1);
-  static constexpr int X_BYTES = BN * 64 * 2;
+  static constexpr int X_BYTES = BN * 64 * 2 * KB;
   static constexpr int STAGE_BYTES = W_BYTES + X_BYTES;
   static constexpr int NS_RAW = (196 * 1024) / STAGE_BYTES;
-  static constexpr int NS = NS_RAW > 8 ? 8 : NS_RAW;
+  static constexpr int NS = NS_RAW > 8 / KB ? 8 / KB : NS_RAW;
   static constexpr int NACC = DUAL ? 2 : 1;
   static constexpr int COLS = BN * NACC;
   static constexpr int TMEM_COLS = COLS <= 32 ? 32 : COLS <= 64 ? 64 : COLS <= 128 ? 128 : COLS <= 256 ? 256 : 512;
@@ -407,10 +412,9 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   const int t0 = blockIdx.y * BN;
   const int S = p.splits;
   const int rank = blockIdx.z;                       // == cluster rank: cluster dims are (1, 1, S)
-  const int kb_total = p.kb_main + p.kb_ext;
-  const int kb_begin = (int)(((long long)kb_total * rank) / S);
-  const int kb_end = (int)(((long long)kb_total * (rank + 1)) / S);
-  const int n_kb = kb_end - kb_begin;
+  const int st_main = (p.kb_main + C::KB - 1) / C::KB, st_total = st_main + (p.kb_ext + C::KB - 1) / C::KB;     // stages' worth of the reduction
+  const int st_begin = (int)(((long long)st_total * rank) / S);
+  const int n_st = (int)(((long long)st_total * (rank + 1)) / S) - st_begin;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::NS; ++s) {
@@ -436,26 +440,31 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
-      if (p.wait_world > 0) {
-        if (!wait_peer_rows(p.wait_flag, p.wait_target, p.wait_world, p.status, p.wait_limit_ns)) *abort_flag = 1;
-        asm volatile("fence.proxy.async.global;" ::: "memory");   // the TMA loads below see the landed rows
-      }
-      for (int i = 0; i < n_kb; ++i) {
-        const int s = i % C::NS;
-        const uint32_t ph = (i / C::NS) & 1;
-        mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, p.status, STATUS_TIMEOUT_STAGE_EMPTY);
-        if (*abort_flag) break;           // a wait gave up: issue no further copies, let the kernel run out
+    // Producer and issuer walk their loops as whole warps and elect the lane that issues: what one lane of a diverged warp issues is wrapped in a
+    // loop over the active lanes.  A step takes some 500 cycles whatever it carries, so a stage has two blocks of 64 of the reduction where
+    // three such stages fit, each operand's brought by one copy.
+    if (p.wait_world > 0) {
+      if (lane == 0 && !wait_peer_rows(p.wait_flag, p.wait_target, p.wait_world, p.status, p.wait_limit_ns)) *abort_flag = 1;
+      __syncwarp();
+      asm volatile("fence.proxy.async.global;" ::: "memory");   // the TMA loads below see the landed rows
+    }
+    for (int i = 0; i < n_st; ++i) {
+      const int s = i % C::NS;
+      // a wait gave up: issue no further copies, let the kernel run out
+      if (!mbar_wait_tight(&empty_bar[s], ((i / C::NS) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_STAGE_EMPTY)) break;
+      if (elect_one()) {
         mbar_expect_tx(&full_bar[s], C::STAGE_BYTES);
-        const int g = kb_begin + i;
-        const bool ext = g >= p.kb_main;
-        const int x = (ext ? g - p.kb_main : g) * 64;
+        const int g = st_begin + i;
+        const bool ext = g >= st_main;
+        const int kb = (ext ? g - st_main : g) * C::KB, x = kb * 64;
         const CUtensorMap* mw = ext ? &tm_w2 : &tm_w;
         const CUtensorMap* mx = ext ? &tm_x2 : &tm_x;
         uint8_t* st = smem + s * C::STAGE_BYTES;
-        if (p.a_mn) {                       // [64 reduction rows][64 features] boxes, 8 KiB each
+        if (p.a_mn) {                       // boxes of KB * 64 reduction rows x 64 features
           tma_load_2d(st, mw, f0, x, &full_bar[s]);
-          tma_load_2d(st + 8192, mw, f0 + 64, x, &full_bar[s]);
+          tma_load_2d(st + C::KB * 8192, mw, f0 + 64, x, &full_bar[s]);
+        } else if constexpr (C::KB == 2) {
+          tma_load_3d(st, mw, 0, f0, kb, &full_bar[s]);
         } else {
           tma_load_2d(st, mw, x, f0, &full_bar[s]);
         }
@@ -470,54 +479,63 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         if (p.b_mn) {
 #pragma unroll
           for (int j = 0; j < (BN >= 64 ? BN / 64 : 1); ++j)
-            tma_load_2d(st + C::W_BYTES + j * 8192, mx, t0 + j * 64, x, &full_bar[s]);
+            tma_load_2d(st + C::W_BYTES + j * C::KB * 8192, mx, t0 + j * 64, x, &full_bar[s]);
+        } else if constexpr (C::KB == 2) {
+          tma_load_3d(st + C::W_BYTES, mx, 0, t0, kb, &full_bar[s]);
         } else {
           tma_load_2d(st + C::W_BYTES, mx, x, t0, &full_bar[s]);
         }
       }
-      if constexpr (PAIR) {
-        // the residual tiles take the first two stages as the main loop frees them
-        if (p.tma_out && p.residual != nullptr && !*abort_flag) {
-          mbar_expect_tx(res_bar, BN * 256 * 2);
-#pragma unroll
-          for (int s = 0; s < 2; ++s) {
-            if (n_kb > s) mbar_wait(&empty_bar[s], ((n_kb - 1 - s) / C::NS) & 1, abort_flag, p.status, STATUS_TIMEOUT_STAGE_EMPTY);
-            if (!*abort_flag) tma_load_2d(smem + s * C::STAGE_BYTES, &tm_res, s ? p.up_off + f0 : f0, t0, res_bar);
-          }
-        }
-      }
     }
     __syncwarp();
+    if constexpr (PAIR) {
+      // the residual tiles take the first two stages as the main loop frees them
+      if (lane == 0 && p.tma_out && p.residual != nullptr && !*abort_flag) {
+        mbar_expect_tx(res_bar, BN * 256 * 2);
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          if (n_st > s) mbar_wait(&empty_bar[s], ((n_st - 1 - s) / C::NS) & 1, abort_flag, p.status, STATUS_TIMEOUT_STAGE_EMPTY);
+          if (!*abort_flag) tma_load_2d(smem + s * C::STAGE_BYTES, &tm_res, s ? p.up_off + f0 : f0, t0, res_bar);
+        }
+      }
+      __syncwarp();
+    }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_bf16(128, BN) | (p.a_mn ? (1u << 15) : 0u) | (p.b_mn ? (1u << 16) : 0u);
-      const uint32_t a_step = (p.a_mn ? 2048u : 32u) >> 4, b_step = (p.b_mn ? 2048u : 32u) >> 4;
-      for (int i = 0; i < n_kb; ++i) {
-        const int s = i % C::NS;
-        const uint32_t ph = (i / C::NS) & 1;
-        mbar_wait(&full_bar[s], ph, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
-        tc_fence_after();
-        const uint32_t a_addr = smem_u32(smem + s * C::STAGE_BYTES);
-        const uint32_t b_addr = a_addr + C::W_BYTES;
-        // K-major: 16 reduction elements = 32 bytes along the swizzled row; MN-major: 16 reduction rows of
-        // 128 bytes = 2048 bytes, the next 64 features / columns 8192 bytes further.  The start address sits in
-        // the low bits of the descriptor in 16-byte units, so a k step is an addition.
-        const uint64_t da0 = p.a_mn ? umma_desc_mn_sw128(a_addr, 8192) : umma_desc_sw128(a_addr);
-        const uint64_t db0 = p.b_mn ? umma_desc_mn_sw128(b_addr, 8192) : umma_desc_sw128(b_addr);
-        const uint64_t da1 = p.a_mn ? umma_desc_mn_sw128(a_addr + C::W_TILE, 8192) : umma_desc_sw128(a_addr + C::W_TILE);
+    const uint32_t idesc = umma_idesc_bf16(128, BN) | (p.a_mn ? (1u << 15) : 0u) | (p.b_mn ? (1u << 16) : 0u);
+    // K-major: 16 reduction elements = 32 bytes along the swizzled row, the next 64 one tile further; MN-major: 16 reduction rows of 128 bytes
+    // = 2048 bytes, the next 64 features / columns KB * 8192 bytes further.  The start address sits in the low bits of the
+    // descriptor in 16-byte units, so a k step is an addition.
+    const uint32_t a_step = (p.a_mn ? 2048u : 32u) >> 4, b_step = (p.b_mn ? 2048u : 32u) >> 4;
+    const uint32_t a_next = (p.a_mn ? 8192u : 128 * 128u) >> 4, b_next = (p.b_mn ? 8192u : BN * 128u) >> 4;
+    const uint32_t a_addr = smem_u32(smem), b_addr = a_addr + C::W_BYTES;
+    const uint64_t da0 = p.a_mn ? umma_desc_mn_sw128(a_addr, C::KB * 8192) : umma_desc_sw128(a_addr);
+    const uint64_t db0 = p.b_mn ? umma_desc_mn_sw128(b_addr, C::KB * 8192) : umma_desc_sw128(b_addr);
+    for (int i = 0; i < n_st; ++i) {
+      const int s = i % C::NS;
+      mbar_wait_tight(&full_bar[s], (i / C::NS) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
+      tc_fence_after();
+      if (elect_one()) {
+        uint64_t da = da0 + (uint64_t)(s * (C::STAGE_BYTES >> 4)), db = db0 + (uint64_t)(s * (C::STAGE_BYTES >> 4));
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const uint64_t da = da0 + (uint64_t)(k * a_step);
-          const uint64_t db = db0 + (uint64_t)(k * b_step);
           const uint32_t acc = (i > 0 || k > 0) ? 1u : 0u;
-          umma_bf16(tmem_base, da, db, idesc, acc);
-          if constexpr (DUAL) umma_bf16(tmem_base + BN, da1 + (uint64_t)(k * a_step), db, idesc, acc);
+          umma_bf16(tmem_base, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), idesc, acc);
+          if constexpr (DUAL) umma_bf16(tmem_base + BN, da + (C::W_TILE >> 4) + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), idesc, acc);
+        }
+        if constexpr (C::KB == 2) {
+          const int g = st_begin + i;
+          if ((g < st_main ? p.kb_main - 2 * g : p.kb_ext - 2 * (g - st_main)) > 1) {
+            da += a_next;
+            db += b_next;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) umma_bf16(tmem_base, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), idesc, 1u);
+          }
         }
         umma_commit(&empty_bar[s]);   // frees the stage once these MMAs have read it
       }
-      umma_commit(accum_bar);
     }
+    if (elect_one()) umma_commit(accum_bar);
     __syncwarp();
   } else {
     // ---------------- epilogue ----------------
@@ -863,18 +881,25 @@ static int gemm_impl(const void* W, const void* X, void* out, const void* residu
   if (bn == 0) bn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
   if (b_mn && bn < 64) bn = 64;               // MN-major column tiles come in 64-wide boxes
   if (splits < 1) splits = 1;
-  const int kb = K / 64 + R / 64;
+  const bool two = !dual && bn <= 128;        // GemmCfg::KB: stages of two blocks of the reduction
+  const int kb = two ? (K + 127) / 128 + (R + 127) / 128 : K / 64 + R / 64;      // no rank of a split without a stage
   while (splits > 1 && (splits > kb || bn % splits || (bn / splits) % 16)) splits >>= 1;
   const long long w_rows = dual ? (long long)up_off + F : F;
   CUtensorMap mw, mx, mw2, mx2;
   int rc;
+  auto k_map = [&](CUtensorMap* m, const void* base, long long rows, long long cols, long long ld, int box_rows) {
+    return two ? make_map_two(m, base, rows, cols, ld, box_rows) : make_map(m, base, rows, cols, ld, box_rows, true);
+  };
+  auto mn_map = [&](CUtensorMap* m, const void* base, long long red, long long cols, long long ld) {
+    return two ? make_map_mn_two(m, base, red, cols, ld) : make_map_mn(m, base, red, cols, ld);
+  };
   // k_rows: true reduction length of MN-major operands (K is rounded up to whole k-blocks; TMA zero-fills the rest)
   const long long kr = k_rows > 0 ? k_rows : K;
-  if ((rc = a_mn ? make_map_mn(&mw, W, kr, w_rows, ldw) : make_map(&mw, W, w_rows, K, ldw, 128, true))) return rc;
-  if ((rc = b_mn ? make_map_mn(&mx, X, kr, M, ldx) : make_map(&mx, X, M, K, ldx, bn, true))) return rc;
+  if ((rc = a_mn ? mn_map(&mw, W, kr, w_rows, ldw) : k_map(&mw, W, w_rows, K, ldw, 128))) return rc;
+  if ((rc = b_mn ? mn_map(&mx, X, kr, M, ldx) : k_map(&mx, X, M, K, ldx, bn))) return rc;
   if (R > 0) {
-    if ((rc = make_map(&mw2, W2, w_rows, R, ldw2, 128, true))) return rc;
-    if ((rc = make_map(&mx2, X2, M, R, ldx2, bn, true))) return rc;
+    if ((rc = k_map(&mw2, W2, w_rows, R, ldw2, 128))) return rc;
+    if ((rc = k_map(&mx2, X2, M, R, ldx2, bn))) return rc;
   } else {
     mw2 = mw;
     mx2 = mx;

@@ -123,14 +123,25 @@ def _fits(bn: int, s: int, nacc: int) -> bool:
     return red + per * 256 <= ns * stage
 
 
-@functools.lru_cache(maxsize=4096)
-def plan_gemm(M: int, F: int, K: int, R: int = 0, dual: bool = False):
-    """Pick the token-tile width and the split-K cluster size with a small cost model.
+# CTAs of a launch with clusters of four that run at once: a cluster lies in one group of SMs, and what is left of a group holds none (of 148
+# SMs 132 did run in one wave, 144 in two)
+CLUSTER4_CTAS = 132
 
-    Measured on B200: a k-block (64 of K) costs about 0.3 us of load latency per CTA unless the
-    tensor-core time of the tile is larger, the epilogue about 0.5 us + 8 ns per token column,
-    and clusters larger than 4 CTAs (one ~200 KB CTA per SM) no longer fit in one wave.
-    """
+
+def plan_gemm(M: int, F: int, K: int, R: int = 0, dual: bool = False):
+    """Token-tile width and split-K cluster size of the one-tile form, for products that do not take :func:`plan_tiles`: see
+    :func:`_gemm_cost`."""
+    return _gemm_cost(M, F, K, R, dual)[1:]
+
+
+@functools.lru_cache(maxsize=4096)
+def _gemm_cost(M: int, F: int, K: int, R: int = 0, dual: bool = False):
+    """``(microseconds, bn, splits)`` by a small cost model.
+
+    One accumulator, measured at 40 to 256 tokens, weights of 2048 to 151936 rows and reductions of 2048 and 6144 out of HBM: a block of 64 of the
+    reduction takes 0.195, 0.25 or 0.33 us for tiles of up to 64, 128 or 256 tokens, start and epilogue 2.4 us and 8 ns a token, the exchange of two
+    partial sums 1 us and 6.5 ns, of four 1.2 us and 20 ns.  Products whose split changed with it (us, before / now): 4096 x 2048 at 128 tokens
+    9.4 / 8.5, 2048 x 2048 at 256 9.5 / 8.4.  Two accumulators: 0.3 us a block, unless the tile's tensor time is longer."""
     nacc = 2 if dual else 1
     kb = K // 64 + R // 64
     base = 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128 if M <= 128 else 256
@@ -141,26 +152,24 @@ def plan_gemm(M: int, F: int, K: int, R: int = 0, dual: bool = False):
             if s > 1 and (kb // s < 2 or not _fits(bn, s, nacc)):
                 continue
             ctas = ((F + 127) // 128) * ((M + bn - 1) // bn) * s
-            waves = (ctas + SM_COUNT - 1) // SM_COUNT
-            t_kb = max(0.30, 128 * bn * 64 * 2 * nacc / 8192 / 1900.0)
             per = bn // s
-            t_cta = (kb / s) * t_kb + 0.5 + 0.009 * per
-            if s > 1:
-                pushed_kb = (s - 1) * per * nacc * 0.5            # KiB sent to the peers through DSMEM
-                t_cta += 1.0 + pushed_kb / 19.0 + (0.07 * per if dual else 0.0)
+            if nacc == 1:
+                waves = -(-ctas // (CLUSTER4_CTAS if s == 4 else SM_COUNT))
+                t_cta = kb / s * (0.195 if bn <= 64 else 0.25 if bn == 128 else 0.33) + 2.4 + 0.008 * bn
+                t_cta += {1: 0.0, 2: 1.0 + 0.0065 * bn, 4: 1.2 + 0.02 * bn}[s]
+            else:
+                waves = -(-ctas // SM_COUNT)
+                t_cta = kb / s * max(0.30, 128 * bn * 64 * 2 * nacc / 8192 / 1900.0) + 0.5 + 0.009 * per
+                if s > 1:
+                    t_cta += 1.0 + (s - 1) * per * nacc * 0.5 / 19.0 + 0.07 * per          # KiB sent to the peers through DSMEM
             t = waves * t_cta
             if best is None or t < best[0] - 1e-9:
                 best = (t, bn, s)
-    return best[1], best[2]
+    return best
 
 
 # the two-tile ("pair") GEMM is a candidate above 256 tokens; TAH_B200_GEMM_PAIR=0 turns it off
 PAIR_AUTO = os.environ.get("TAH_B200_GEMM_PAIR", "1") != "0"
-
-
-# CTAs of a launch with clusters of four that run at once: a cluster lies in one group of SMs, and what is left of a group holds none (of 148
-# SMs 132 did run in one wave, 144 in two)
-CLUSTER4_CTAS = 132
 
 
 @functools.lru_cache(maxsize=4096)
@@ -169,11 +178,10 @@ def plan_tiles(M: int, rows: int, K: int, can_pair: bool, can_split: bool, x_t: 
     whichever fills the SMs' waves best by a cost model.  ``x_t``: activations are read transposed (weight gradients).
 
     The constants are fitted to every form at weights of 64 to 12288 rows, reductions of 300 to 12288 and 257 to 13600 tokens (weight and
-    data gradients to 4000): a wave takes a third of a microsecond per block of 64 of the reduction whatever the width of a one-tile form,
-    so wide tiles pay only where they save a wave.  The choice lies within 5 % of the best form everywhere, 0.1 % on average.  Microseconds, by
-    the plan for up to 256 tokens (256-token pairs from 1024 on) / by this one: 1536 x 2048 at 450 tokens 11.2 / 11.0, 2048 x 2048 at 1000
-    13.8 / 13.5, 4096 x 2048 at 400 14.3 / 13.8, 2048 x 6144 at 520 25.7 / 23.3, at 5200 136 / 117, its weight gradient over 940 tokens
-    46.4 / 35.5."""
+    data gradients to 4000), those of up to 128 tokens again since their stages hold two blocks of 64 of the reduction (0.21 and 0.26 us a block where
+    the others take a third of a microsecond).  Microseconds, by the plan for up to 256 tokens (256-token pairs from 1024 on) / by this one, before
+    that: 1536 x 2048 at 450 tokens 11.2 / 11.0, 2048 x 2048 at 1000 13.8 / 13.5, 2048 x 6144 at 520 25.7 / 23.3, its weight gradient over 940
+    tokens 46.4 / 35.5; since then 6144 x 2048 at 264 14.7 / 11.9, 2048 x 2048 at 264 11.6 / 10.1."""
     return _tiles_cost(M, rows, K, can_pair, can_split, x_t)[1:]
 
 
@@ -192,6 +200,8 @@ def _tiles_cost(M: int, rows: int, K: int, can_pair: bool, can_split: bool, x_t:
                     t_kb, out = (0.29 + 0.164 * bn / 256, 2.6 + 0.0195 * bn) if nf == 1 else (0.31 + 0.297 * bn / 256, 3.0 + 0.038 * bn)
                 else:
                     t_kb, out = (0.31 + 0.03 * bn / 256, 2.0 + 0.0143 * bn) if nf == 1 else (0.345 + 0.235 * bn / 256, 2.0 + 0.022 * bn)
+                if nf == 1 and bn <= 128:          # stages of two blocks
+                    t_kb = (0.21 if bn == 64 else 0.26) + (0.02 if x_t else 0.0)
                 t = waves * (kb * t_kb + out + {1: 0.0, 2: 1.1 + 0.003 * bn, 4: 0.65 + 0.0133 * bn}[s])
                 if best is None or t < best[0] - 1e-9:
                     best = (t, nf == 2, bn, s)
@@ -204,25 +214,30 @@ SM_PAIRS = SM_COUNT // 2
 
 @functools.lru_cache(maxsize=4096)
 def plan_persist(M: int, rows: int, K: int, R: int = 0, glu: bool = False, x_t: bool = False, can_pair: bool = True) -> int:
-    """Tile width of the persistent form (``csrc/gemm_persist.cu``) for more than 256 tokens, or 0 where one tile per CTA is faster: few tiles
-    with a long reduction, which that form splits (us, persistent / one tile per CTA at 264 tokens: 2048 x 6144 20.3 / 17.6, 12288 x 2048 SwiGLU
-    23.7 / 22.3, 2048 x 12288 35.7 / 24.3; at 2048 x 6144 level at 504 tokens, 31.4 / 38.0 at 1504).
+    """Tile width of the persistent form (``csrc/gemm_persist.cu``) for more than 128 tokens, or 0 where one tile per CTA is faster: few tiles
+    with a long reduction, which that form splits (us, persistent / one tile per CTA at 264 tokens: 2048 x 6144 20.2 / 17.2, 12288 x 2048 SwiGLU
+    24.0 / 21.1, 2048 x 12288 36.6 / 23.2, 6144 x 2048 14.4 / 11.9; at 2048 x 6144 level at 504 tokens, 32.1 / 35.2 at 1504), and most products of up to
+    256 tokens (4096 x 2048 at 256 9.4 / 9.6, 2048 x 2048 9.2 / 8.4; but 12288 x 2048 SwiGLU 17.1 / 18.7, 151936 x 2048 142 / 171).
 
     Both are estimated.  Microseconds, fitted to tiles of 64 to 256 features at weights of 2048 to 12288 rows, reductions of 264 to 15696 and 264 to
-    15696 tokens, K-major and transposed operands: 128 of the reduction take what the table says, or the epilogue bounds a wave (short reductions).
-    The estimate of the other form lies a ninth below what it takes beside other launches.  Of 60 measured products the choice is the faster
-    form but for 3, which lose 5 %."""
+    15696 tokens, K-major and transposed operands: 128 of the reduction take what the table says, or the epilogue bounds a wave (short reductions);
+    with one token tile the weights come from HBM, not from L2, which costs up to 2.5 us.  The estimate of the other form lies a twelfth
+    below what it takes beside other launches."""
     best = None
     steps = -(-K // 128) + -(-R // 128)
     for bn, kb in ((64, 0.35), (128, 0.41), (192, 0.58), (256, 0.72)):
-        if glu and bn % 128:
-            continue
         waves = -(-(-(-M // 256) * -(-rows // bn)) // SM_PAIRS)
-        t = 3.2 + 0.004 * bn + waves * max(steps * kb, 1.25 + 0.006 * bn)
+        t = 3.2 + 0.004 * bn + waves * max(steps * kb, 1.25 + 0.006 * bn) + (2.5 if M <= 256 else 0.0)
         if best is None or t < best[0] - 1e-9:
             best = (t, bn)
+    if M <= 256:
+        # the one-tile form of up to 256 tokens; its SwiGLU is not split and has one tile width
+        bn = 64 if M <= 64 else 128 if M <= 128 else 256
+        other = (-(-(-(-rows // 128)) // SM_COUNT) * ((K + R) / 64 * (0.195, 0.25, 0.33)[(bn > 64) + (bn > 128)] + 4.8 + 0.015 * bn) if glu else
+                 _gemm_cost(M, rows, K, R, False)[0])
+        return best[1] if best[0] < other else 0
     other = _tiles_cost(M, rows, K + R, can_pair and PAIR_AUTO and rows % 256 == 0, not glu, x_t)[0]
-    return best[1] if best[0] <= 1.12 * other else 0
+    return best[1] if best[0] <= 1.08 * other else 0
 
 
 def interleave_gate_up(w: torch.Tensor) -> torch.Tensor:
@@ -420,11 +435,11 @@ def _gemm_few(x, w, out, residual=None, x2=None, w2=None, act: int = 0, act_up: 
 
 
 def _persist_ok(x, w, out, residual=None, x2=None, w2=None, x_t: bool = False, w_t: bool = False) -> bool:
-    """Whether the persistent form takes these operands: more than 256 tokens, whole pieces of 16 bytes everywhere, whole blocks of the
+    """Whether the persistent form takes these operands: more than 128 tokens (256 of transposed ones), whole pieces of 16 bytes everywhere, whole blocks of the
     reduction (unless both operands are transposed)."""
     M, K = (x.shape[1], x.shape[0]) if x_t else x.shape
     F = w.shape[1] if w_t else w.shape[0]
-    return (M > 256 and F > 0 and K > 0 and (K % 64 == 0 or x_t and w_t) and (x2 is None or x2.shape[1] % 64 == 0) and
+    return (M > (256 if x_t or w_t else 128) and F > 0 and K > 0 and (K % 64 == 0 or x_t and w_t) and (x2 is None or x2.shape[1] % 64 == 0) and
             (not w_t or F % 128 == 0) and (residual is None or F % 8 == 0) and
             all(t is None or _whole_pieces(t) for t in (x, w, out, residual, x2, w2)))
 
@@ -1603,7 +1618,7 @@ def packed_pass(weights, final_norm, h, xn, pools, k_own, v_own, seg_k, seg_v, b
         stacked, il = glu and not gu_interleaved, glu and gu_interleaved
         if few_shape(n, rows, K, R, True):
             return _ProductPlan(1, 4 if il else 1 if stacked else 0, 1, 0)
-        bn = plan_persist(n, rows, K, R, il) if n > 256 and not stacked and K % 64 == 0 and R % 64 == 0 and rows % 8 == 0 else 0
+        bn = plan_persist(n, rows, K, R, il) if n > 128 and not stacked and K % 64 == 0 and R % 64 == 0 and rows % 8 == 0 else 0
         if bn:
             return _ProductPlan(2, 4 if il else 0, 1, bn)
         pair, bn, splits = _plan_tiles(n, rows, K, R, stacked, False, il)

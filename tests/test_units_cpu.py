@@ -474,13 +474,16 @@ def test_tile_plan_counts_the_clusters_that_fit():
 
 
 def test_persistent_tile_plan():
-    """Tiles of the persistent product: whole gate / up chunks for SwiGLU, narrow tiles where wide ones leave SMs idle, and none where few tiles with
+    """Tiles of the persistent product: narrow tiles where wide ones leave SMs idle, and none where few tiles with
     a long reduction want a split."""
     from tah_b200.ops import cuda
     for rows in (64, 512, 2048, 12288, 151936):
         for K in (64, 300, 2048, 12288):
             for M in (257, 700, 3072, 16000):
                 assert cuda.plan_persist(M, rows, K) in (0, 64, 128, 192, 256)
-                assert cuda.plan_persist(M, rows, K, 64, True) in (0, 128, 256)
+                assert cuda.plan_persist(M, rows, K, 64, True) in (0, 64, 128, 192, 256)
     assert cuda.plan_persist(504, 2048, 2048) == 64 and cuda.plan_persist(16000, 2048, 2048) == 256
     assert cuda.plan_persist(264, 2048, 12288) == 0
+    # one token tile: the wide SwiGLU and the head, which one tile per CTA does in an uneven wave or several
+    assert cuda.plan_persist(256, 12288, 2048, 64, True) == 192 and cuda.plan_persist(256, 151936, 2048) in (192, 256)
+    assert not any(cuda.plan_persist(M, rows, 2048) for M in (129, 192, 256) for rows in (1024, 2048, 4096))
