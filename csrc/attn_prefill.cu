@@ -21,7 +21,8 @@
 // there is more than a wave of long sequences, and holds up short ones, which have half the CTAs then (the rule: prefill_heads in
 // tah_b200/ops/cuda.py).  us, 16 heads of 128 on 8 KV heads, two threads per row / one head / two heads: 100 tokens 8.4 / 7.5 / 9.2, 700 22.3 / 18.4 /
 // 21.1, 64 sequences of 128 42.6 / 36.7 / 43.1, 3000 tokens 122 / 69.9 / 74.0, four of 2048 162 / 112 / 112, of 4000 - / 382 / 360, their second pass
-// of 0.3 of the tokens - / 184 / 166.  One sequence of 8192: 345 us (798 TFLOP/s).
+// of 0.3 of the tokens - / 184 / 166.  Since an elected lane issues (the rule again): 700 tokens 18.5 / 16.4, 3072 70.8 / 61.6, four of 2000
+// 110 / 104, one of 8192 339 / 289 (950 TFLOP/s).
 //
 // Warp roles: warp 0 = TMA producer, warp 1 = tensor-memory owner + MMA issuer, four warps per head = softmax / epilogue
 // (warp w reads tensor-memory lanes 32*(w%4)..+31 = query rows).
@@ -135,7 +136,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, NH * C::Q_BYTES);
 #pragma unroll
       for (int h = 0; h < NH * C::HALVES; ++h) tma_load_2d(q_s + h * C::QTILE, &tm_q, head0 * HD + h * 64, q0, q_full);
@@ -162,7 +163,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BK);
       constexpr uint32_t idesc_o = umma_idesc_bf16_bmn(128, HD);
       mbar_wait(q_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);

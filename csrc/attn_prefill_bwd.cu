@@ -132,7 +132,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, 2 * NH * C::Q_BYTES);
 #pragma unroll
       for (int h = 0; h < NH * C::HALVES; ++h) {
@@ -159,7 +159,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BK);
       constexpr uint32_t idesc_q = umma_idesc_bf16_bmn(128, HD);
       mbar_wait(q_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
@@ -375,7 +375,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
   const uint32_t tmem_dk = tmem_base + 128, tmem_dv = tmem_base + 256;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(kv_full, 2 * C::K_BYTES);
 #pragma unroll
       for (int h = 0; h < C::HALVES; ++h) {
@@ -400,7 +400,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BQ);            // S^T, dP^T: 128 keys x 64 queries
       constexpr uint32_t idesc_a = umma_idesc_bf16_bmn(128, HD);        // dK, dV: 128 keys x head_dim
       mbar_wait(kv_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);

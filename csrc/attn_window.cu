@@ -804,7 +804,7 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, NH * C::Q_BYTES);
 #pragma unroll
       for (int h = 0; h < NH * HK; ++h) tma_load_2d(q_s + h * C::QTILE, &tm_q, (head0 + h / HK) * p.dk + h % HK * 64, q0, q_full);
@@ -847,7 +847,7 @@ window_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BK);
       constexpr uint32_t idesc_o = umma_idesc_bf16_bmn(128, HV * 64);
       mbar_wait(q_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);

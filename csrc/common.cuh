@@ -77,6 +77,9 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
   return t;
 }
 
+// One lane of a converged warp.  Loops that issue copies and tensor instructions belong to a lane elected so: behind a test of the lane's number the
+// compiler wraps every such instruction in a loop over the active lanes (a tensor instruction 57 against about 15 cycles; attention with two
+// heads per CTA over 8192 tokens: forward 339 / 289 us, dQ 577 / 398, dK / dV 848 / 768).
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(

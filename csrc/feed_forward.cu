@@ -403,7 +403,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
   const int n_tiles = *p.n_blocks * p.f_tiles;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int g = 0;
       for (int tile = blockIdx.x; tile < n_tiles && !*abort_flag; tile += gridDim.x) {
         const int b = tile / p.f_tiles, w_row = p.blk_expert[b] * p.f_rows + (tile % p.f_tiles) * 128;
@@ -420,7 +420,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16(128, BN);
       int g = 0, it = 0;
       for (int tile = blockIdx.x; tile < n_tiles && !*abort_flag; tile += gridDim.x, ++it) {

@@ -473,7 +473,7 @@ gla_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_cons
   const int slices = (nv + 1) / 2;
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       for (int i = 0; i < 4 * slices; ++i) {
         const int st = i % GcOutSmem::NRING;
         mbar_wait(&empty[st], ((i / GcOutSmem::NRING) & 1) ^ 1, abort_flag, c.status, STATUS_TIMEOUT_STAGE_EMPTY);
@@ -498,7 +498,7 @@ gla_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_v, const __grid_cons
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t qhi = smem_u32(mc_smem + GcOutSmem::QHI), qlo = smem_u32(mc_smem + GcOutSmem::QLO);
       const uint32_t khi = smem_u32(mc_smem + GcOutSmem::KHI), klo = smem_u32(mc_smem + GcOutSmem::KLO);
       mbar_wait(qk_full, 0, abort_flag, c.status, STATUS_TIMEOUT_TMA_FULL);

@@ -482,7 +482,7 @@ mlstm_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   const int slices = (nv + 1) / 2;
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(qk_full, 2 * nk * MC_KCH);
       for (int k = 0; k < nk; ++k) {
         tma_load_3d(mc_smem + McOutSmem::Q + k * MC_KCH, &tm_q, k * 64, h, start, qk_full);
@@ -512,7 +512,7 @@ mlstm_chunk_out_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t q_addr = smem_u32(mc_smem + McOutSmem::Q), k_addr = smem_u32(mc_smem + McOutSmem::K);
       const uint32_t plo_addr = smem_u32(mc_smem + McOutSmem::PLO);
       mbar_wait(qk_full, 0, abort_flag, c.status, STATUS_TIMEOUT_TMA_FULL);
