@@ -19,7 +19,10 @@
 //                        P^T and dS^T to shared memory, dV += P^T dO and dK += dS^T Q with the same
 //                        Q / dO tiles consumed MN-major.  dK and dV accumulate in tensor memory over the
 //                        whole loop (4 x 128 columns with the two score tiles).  The blocks that the most queries
-//                        see go first, of all heads: 209 us there, now 172.
+//                        see go first, of all heads: 209 us there, now 172.  P^T and dS^T have two buffers and Q / dO three
+//                        stages: with one and two, the threads waited for the products of the iteration before and a load
+//                        stood in every iteration (tensor pipe 42 % busy; 3072 tokens 156 us, now 133, four of 2000 231 and
+//                        189, one of 8192 768 and 612).
 //
 // The duo-causal rule is the per-query bound key_index < count[segment][query]; no mask tensor.
 // All waits are bounded (common.cuh).
@@ -299,10 +302,10 @@ struct BwdKVCfg {
   static constexpr int K_BYTES = HALVES * KTILE;               // K and V blocks (resident)
   static constexpr int Q_BYTES = HALVES * QTILE;               // Q and dO sub-tiles
   static constexpr int STAGE_BYTES = 2 * Q_BYTES;
-  static constexpr int NSTAGE = 2;
+  static constexpr int NSTAGE = HD == 128 ? 3 : 4;
   static constexpr int PT_BYTES = 128 * BQ * 2;                // P^T and dS^T tiles
   static constexpr int META_BYTES = 2 * 3 * BQ * 4;            // [2 buffers][lse | dsum | count][64 queries]
-  static constexpr int SMEM_BYTES = 2 * K_BYTES + NSTAGE * STAGE_BYTES + 2 * PT_BYTES + META_BYTES + 128;
+  static constexpr int SMEM_BYTES = 2 * K_BYTES + NSTAGE * STAGE_BYTES + 4 * PT_BYTES + META_BYTES + 128;
   static constexpr int TMEM_COLS = 512;                        // scores at 0 / 384 (S^T, dP^T), dK at 128, dV at 256
 };
 
@@ -317,17 +320,16 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
   uint8_t* k_s = smem;
   uint8_t* v_s = k_s + C::K_BYTES;
   uint8_t* qd_s = v_s + C::K_BYTES;                             // stages: [Q | dO]
-  uint8_t* pt_s = qd_s + C::NSTAGE * C::STAGE_BYTES;
-  uint8_t* dst_s = pt_s + C::PT_BYTES;
-  float* meta_s = reinterpret_cast<float*>(dst_s + C::PT_BYTES);  // per-query lse, dsum, count of the sub-tile
-  uint64_t* bars = reinterpret_cast<uint64_t*>(dst_s + C::PT_BYTES + C::META_BYTES);
+  uint8_t* pt_s = qd_s + C::NSTAGE * C::STAGE_BYTES;           // [2 buffers][P^T | dS^T]
+  float* meta_s = reinterpret_cast<float*>(pt_s + 4 * C::PT_BYTES);  // per-query lse, dsum, count of the sub-tile
+  uint64_t* bars = reinterpret_cast<uint64_t*>(pt_s + 4 * C::PT_BYTES + C::META_BYTES);
   uint64_t* kv_full = bars;
   uint64_t* qd_full = bars + 1;                                 // [NSTAGE]
   uint64_t* qd_empty = qd_full + C::NSTAGE;                     // [NSTAGE]
   uint64_t* s_full = qd_empty + C::NSTAGE;                      // [2]: one per score buffer
   uint64_t* p_ready = s_full + 2;
-  uint64_t* acc_done = p_ready + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
+  uint64_t* acc_done = p_ready + 1;                             // [2]: one per buffer of P^T and dS^T
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -357,7 +359,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     mbar_init(&s_full[0], 1);
     mbar_init(&s_full[1], 1);
     mbar_init(p_ready, 256);
-    mbar_init(acc_done, 1);
+    mbar_init(&acc_done[0], 1);
+    mbar_init(&acc_done[1], 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -405,7 +408,6 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
       constexpr uint32_t idesc_a = umma_idesc_bf16_bmn(128, HD);        // dK, dV: 128 keys x head_dim
       mbar_wait(kv_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
       const uint32_t k_addr = smem_u32(k_s), v_addr = smem_u32(v_s);
-      const uint32_t pt_addr = smem_u32(pt_s), dst_addr = smem_u32(dst_s);
       // scores of iteration `j`: S^T = K Q^T, dP^T = V dO^T over head_dim, into score buffer j & 1
       auto issue_scores = [&](int j) {
         const int st = j % C::NSTAGE;
@@ -432,6 +434,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         if (it + 1 < n_iter) issue_scores(it + 1);
         mbar_wait(p_ready, it & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
         tc_fence_after();
+        const uint32_t pt_addr = smem_u32(pt_s) + (it & 1) * 2 * C::PT_BYTES, dst_addr = pt_addr + C::PT_BYTES;
 #pragma unroll
         for (int ks = 0; ks < BQ / 16; ++ks) {      // dV += P^T dO, dK += dS^T Q over the 64 queries
           const uint64_t b_do = umma_desc_mn_sw128(do_addr + ks * 2048, C::QTILE);
@@ -441,7 +444,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
           umma_bf16(tmem_dk, umma_desc_sw128(dst_addr + ks * 32), b_q, idesc_a, acc);
         }
         umma_commit(&qd_empty[st]);
-        umma_commit(acc_done);
+        umma_commit(&acc_done[it & 1]);
       }
     }
     __syncwarp();
@@ -492,7 +495,9 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
       tmem_ld32(tmem_sc[it & 1] + lane_off + half * 32, sv);
       tmem_ld32(tmem_sc[it & 1] + 64 + lane_off + half * 32, dp);
       tmem_ld_wait();
-      if (it > 0) mbar_wait(acc_done, (it - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+      // this buffer of P^T and dS^T was last read for iteration it - 2
+      if (it > 1) mbar_wait(&acc_done[it & 1], ((it >> 1) - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+      uint8_t* pt = pt_s + (it & 1) * 2 * C::PT_BYTES;
       // every key of the block visible to every query of this thread's 32 columns: no masking needed.  The
       // columns' counts are the same for all lanes of the warp, so the test is warp-uniform.
       int cmin = 0x7fffffff;
@@ -531,8 +536,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         }
         const int cc = half * 4 + c;
         const int off = row * 128 + ((cc ^ (row & 7)) << 4);
-        *reinterpret_cast<uint4*>(pt_s + off) = pk;
-        *reinterpret_cast<uint4*>(dst_s + off) = dk;
+        *reinterpret_cast<uint4*>(pt + off) = pk;
+        *reinterpret_cast<uint4*>(pt + C::PT_BYTES + off) = dk;
       }
       fence_proxy_async_smem();
       tc_fence_before();
@@ -540,7 +545,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
       store_meta(it + 1);
       named_bar_sync(2, 256);                      // next iteration's values visible; this buffer free again
     }
-    if (n_iter > 0) mbar_wait(acc_done, (n_iter - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+    if (n_iter > 0) mbar_wait(&acc_done[(n_iter - 1) & 1], ((n_iter - 1) >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
     tc_fence_after();
     const size_t orow = ((size_t)(row0 + row) * p.nkv + kvh) * HD + half * (HD / 2);
 #pragma unroll 1
