@@ -14,6 +14,13 @@
 // rows g and g + 8.  The order of the reduction is free as long as both operands agree, so a lane reads 16 consecutive
 // bytes (8 indices) of a row at 8 t and feeds two instructions with them: 64 contiguous bytes per row and step, no
 // shared memory, no shuffles.
+//
+// Ticks of few rows (FUSE): a layer of a decode tick was ten launches, of which the RMSNorms with the gated rows' adapter inputs (2.5 us of a
+// one-row layer's 43, 3.6 us each with six rows) and the adapter inputs of the output and down projections (1.2 and 2.1 us) do next to
+// nothing.  Here the product does it itself: a CTA normalises the rows into shared memory while its first weights are on their way (a row is
+// 4 KB, from L2), and the first CTAs of the grid form T = gate * x A^T, which the others wait for behind their main loop (bounded; a
+// CTA only waits for ones with a lower index, which run before it) and only where a row is gated; without one the adapter's weights are not
+// read at all.  Six launches a layer.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -29,6 +36,15 @@ struct FewParams {
   int stacked;           // SwiGLU of a weight with all gate rows in front of the up rows: how many gate rows; 0: interleaved
   float act_up, act_low;
   int early;             // the weights are constants of the launch chain: read them ahead of the dependency wait
+  // FUSE
+  const __nv_bfloat16* norm_w;   // RMSNorm in front of the product, or null
+  float eps;
+  const __nv_bfloat16* A;        // adapter: T [M, R] = gate * x A^T is what X2 points at
+  __nv_bfloat16* T;
+  const int* gate;               // [M]
+  int t_ctas;                    // CTAs that form T
+  int* sync;                     // [2] CTAs of T done, CTAs that have seen it; zero between launches
+  int* status;
 };
 
 __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -42,6 +58,13 @@ __device__ __forceinline__ uint4 ld_stream(const void* p) {
   return v;
 }
 
+__device__ __forceinline__ int ld_acquire(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+constexpr int FEW_ROWS_MOST = 96 * 1024;       // of shared memory for normalised rows: two CTAs per SM
+
 template <int NT, int MT>
 struct FewCfg {
   static constexpr int ST = 4 / MT;                        // steps of 32 reduction indices per buffer, two buffers: 64 registers
@@ -49,26 +72,29 @@ struct FewCfg {
   static constexpr int red_bytes(int warps) { return warps * 8 * NT * PITCH * 4; }
 };
 
-template <int NT, int MT, int NW>
+// FUSE: 1 with the adapter input of the gated rows, 2 with the RMSNorm in front as well
+template <int NT, int MT, int NW, int FUSE>
 __global__ void __launch_bounds__(NW * 32)
 gemm_few_kernel(const FewParams p) {
   using C = FewCfg<NT, MT>;
   constexpr int ST = C::ST, FT = 16 * MT;
-  extern __shared__ float red[];
+  extern __shared__ __align__(16) float red[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int f0 = blockIdx.x * FT;
+  const bool forms_t = FUSE && (int)blockIdx.x < p.t_ctas;
+  const int F = forms_t ? p.R : p.F;
+  const int f0 = (FUSE && !forms_t ? (int)blockIdx.x - p.t_ctas : (int)blockIdx.x) * FT;
   const int tok0 = blockIdx.y * 8 * NT, M = min(p.M - tok0, 8 * NT);          // this CTA's tokens
   const int steps = p.K >> 5, s0 = steps * warp / NW, s1 = steps * (warp + 1) / NW;
 
   auto row_of = [&](int m, int h) {            // weight row of this lane's feature
-    const int v = min(f0 + 16 * m + 8 * h + g, p.F - 1);
-    return (size_t)(p.stacked ? (v >> 1) + (v & 1) * p.stacked : v);
+    const int v = min(f0 + 16 * m + 8 * h + g, F - 1);
+    return (size_t)(p.stacked && !forms_t ? (v >> 1) + (v & 1) * p.stacked : v);
   };
   const __nv_bfloat16* wr[MT][2];
 #pragma unroll
   for (int m = 0; m < MT; ++m)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) wr[m][h] = p.W + row_of(m, h) * p.ldw + t * 8;
+    for (int h = 0; h < 2; ++h) wr[m][h] = (forms_t ? p.A + row_of(m, h) * p.K : p.W + row_of(m, h) * p.ldw) + t * 8;
 
   uint4 w[2][ST][MT][2];
   auto fetch = [&](uint4 (&b)[ST][MT][2], int s) {
@@ -80,10 +106,67 @@ gemm_few_kernel(const FewParams p) {
         for (int h = 0; h < 2; ++h)
           b[i][m][h] = s + i < s1 ? ld_stream(wr[m][h] + (size_t)(s + i) * 32) : make_uint4(0u, 0u, 0u, 0u);
   };
-  if (!p.early) pdl_wait();
-  fetch(w[0], s0);
-  fetch(w[1], s0 + ST);
-  if (p.early) pdl_wait();
+  bool gated = false;
+  if constexpr (FUSE) {
+    if (!forms_t) {
+      fetch(w[0], s0);
+      fetch(w[1], s0 + ST);
+    }
+    uint4* nw = reinterpret_cast<uint4*>(red);                     // [K / 8] norm weights, then the rows
+    if constexpr (FUSE == 2)
+      for (int i = threadIdx.x; i < p.K / 8; i += NW * 32) nw[i] = reinterpret_cast<const uint4*>(p.norm_w)[i];
+    pdl_wait();
+    gated = p.t_ctas > 0 && __any_sync(0xffffffffu, lane < M && p.gate[lane] != 0);
+    if (forms_t) {
+      if (!gated) return;                                          // nobody reads T
+      fetch(w[0], s0);
+      fetch(w[1], s0 + ST);
+    }
+    if constexpr (FUSE == 2) {
+      __syncthreads();                                             // the norm weights
+      const int nvec = p.K / 8, pitch = nvec + 4;                  // 64 bytes between rows: no bank conflicts between fragments
+      for (int r = warp; r < M; r += NW) {
+        const uint4* src = reinterpret_cast<const uint4*>(p.X + (size_t)r * p.ldx);
+        uint4* dst = nw + nvec + r * pitch;
+        float ss = 0.f;
+        for (int i0 = lane; i0 < nvec; i0 += 256) {
+          uint4 v[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) v[u] = i0 + u * 32 < nvec ? src[i0 + u * 32] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            if (i0 + u * 32 < nvec) dst[i0 + u * 32] = v[u];
+            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v[u]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float2 f = __bfloat1622float2(h[j]);
+              ss += f.x * f.x + f.y * f.y;
+            }
+          }
+        }
+        const float rstd = rsqrtf(warp_sum(ss) / (float)p.K + p.eps);
+#pragma unroll 4
+        for (int i = lane; i < nvec; i += 32) {                    // what this lane wrote
+          uint4 v = dst[i];
+          const uint4 wv = nw[i];
+          __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
+          const __nv_bfloat162* wh = reinterpret_cast<const __nv_bfloat162*>(&wv);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 f = __bfloat1622float2(h[j]), q = __bfloat1622float2(wh[j]);
+            h[j] = __floats2bfloat162_rn(q.x * bf16_round(f.x * rstd), q.y * bf16_round(f.y * rstd));
+          }
+          dst[i] = v;
+        }
+      }
+      __syncthreads();
+    }
+  } else {
+    if (!p.early) pdl_wait();
+    fetch(w[0], s0);
+    fetch(w[1], s0 + ST);
+    if (p.early) pdl_wait();
+  }
 
   float acc[MT][NT][4];
 #pragma unroll
@@ -95,7 +178,11 @@ gemm_few_kernel(const FewParams p) {
 
   const __nv_bfloat16* xr[NT];
 #pragma unroll
-  for (int j = 0; j < NT; ++j) xr[j] = p.X + (size_t)(tok0 + min(8 * j + g, M - 1)) * p.ldx + t * 8;
+  for (int j = 0; j < NT; ++j) {
+    const int r = min(8 * j + g, M - 1);
+    if constexpr (FUSE == 2) xr[j] = reinterpret_cast<const __nv_bfloat16*>(red) + p.K + r * (p.K + 32) + t * 8;
+    else xr[j] = p.X + (size_t)(tok0 + r) * p.ldx + t * 8;
+  }
 
   auto multiply = [&](const uint4 (&b)[MT][2], const uint4 (&x)[NT]) {
 #pragma unroll
@@ -125,7 +212,33 @@ gemm_few_kernel(const FewParams p) {
     }
   }
   // the K-extension: R / 32 more steps, one warp each in turn
-  for (int s = warp; s < (p.R >> 5); s += NW) {
+  int ext = p.R >> 5;
+  if constexpr (FUSE) {
+    if (forms_t || !gated) {
+      ext = 0;
+    } else {
+      if (threadIdx.x == 0) {
+        unsigned long long t0 = 0;
+        for (uint32_t spins = 0; ld_acquire(p.sync) < p.t_ctas;) {
+          if ((++spins & 0xff) == 0) {
+            const unsigned long long now = globaltimer_ns();
+            if (t0 == 0) t0 = now;
+            else if (now - t0 > WAIT_TIMEOUT_NS) {
+              atomicCAS(p.status, 0, STATUS_TIMEOUT_ACCUM);
+              break;
+            }
+          }
+        }
+      }
+      __syncthreads();
+      // the last CTA that has seen T leaves the counters as it found them
+      if (threadIdx.x == 0 && atomicAdd(p.sync + 1, 1) == (int)gridDim.x - p.t_ctas - 1) {
+        p.sync[0] = 0;
+        p.sync[1] = 0;
+      }
+    }
+  }
+  for (int s = warp; s < ext; s += NW) {
     uint4 b[MT][2], x[NT];
 #pragma unroll
     for (int m = 0; m < MT; ++m)
@@ -134,12 +247,13 @@ gemm_few_kernel(const FewParams p) {
         b[m][h] = ld_stream(p.W2 + row_of(m, h) * p.ldw2 + t * 8 + s * 32);
 #pragma unroll
     for (int j = 0; j < NT; ++j)
-      x[j] = *reinterpret_cast<const uint4*>(p.X2 + (size_t)(tok0 + min(8 * j + g, M - 1)) * p.ldx2 + t * 8 + s * 32);
+      x[j] = __ldcg(reinterpret_cast<const uint4*>(p.X2 + (size_t)(tok0 + min(8 * j + g, M - 1)) * p.ldx2 + t * 8 + s * 32));
     multiply(b, x);
   }
 
   pdl_launch_dependents();
 
+  if constexpr (FUSE == 2) __syncthreads();          // the sums take the place of the rows
   // the warps' sums meet: [warp][token][feature]
 #pragma unroll
   for (int m = 0; m < MT; ++m)
@@ -155,10 +269,22 @@ gemm_few_kernel(const FewParams p) {
     for (int k = 0; k < NW; ++k) v += red[(k * 8 * NT + tok) * C::PITCH + f];
     return v;
   };
+  if constexpr (FUSE) {
+    if (forms_t) {
+      for (int o = threadIdx.x; o < M * FT; o += NW * 32) {
+        const int tok = o / FT, f = f0 + o % FT;
+        if (f < p.R) p.T[(size_t)tok * p.R + f] = __float2bfloat16_rn(p.gate[tok] != 0 ? total(tok, o % FT) : 0.f);
+      }
+      __threadfence();
+      __syncthreads();
+      if (threadIdx.x == 0) atomicAdd(p.sync, 1);
+      return;
+    }
+  }
   if (p.act == 2) {
     for (int o = threadIdx.x; o < M * (FT / 2); o += NW * 32) {
       const int tok = o / (FT / 2), f = o % (FT / 2);
-      if (f0 + 2 * f >= p.F) continue;
+      if (f0 + 2 * f >= F) continue;
       const float gate = bf16_round(total(tok, 2 * f)), up = bf16_round(total(tok, 2 * f + 1));
       p.out[(size_t)(tok0 + tok) * p.ldo + f0 / 2 + f] = __float2bfloat16_rn(bf16_round(silu(gate)) * up);
     }
@@ -166,7 +292,7 @@ gemm_few_kernel(const FewParams p) {
   }
   for (int o = threadIdx.x; o < M * FT; o += NW * 32) {
     const int tok = o / FT, f = f0 + o % FT;
-    if (f >= p.F) continue;
+    if (f >= F) continue;
     float v = total(tok, o % FT);
     if (p.residual != nullptr) v = bf16_round(v) + __bfloat162float(p.residual[(size_t)(tok0 + tok) * p.ldr + f]);
     if (p.act == 1) {
@@ -180,12 +306,46 @@ gemm_few_kernel(const FewParams p) {
   }
 }
 
-template <int NT, int MT, int NW>
-static int launch_few(const FewParams& p, cudaStream_t stream) {
-  constexpr int bytes = FewCfg<NT, MT>::red_bytes(NW);
-  auto kern = gemm_few_kernel<NT, MT, NW>;
-  static_assert(bytes <= 48 * 1024, "no opt-in for more shared memory");
-  return launch_chain(kern, dim3((p.F + 16 * MT - 1) / (16 * MT), (p.M + 8 * NT - 1) / (8 * NT)), dim3(NW * 32), bytes, stream, p) == cudaSuccess ? 0 : -12;
+// norm weights and normalised rows
+static int few_rows_bytes(int M, int K) { return K * 2 + M * (K * 2 + 64); }
+
+template <int NT, int MT, int NW, int FUSE>
+static int launch_few(FewParams& p, cudaStream_t stream) {
+  int bytes = FewCfg<NT, MT>::red_bytes(NW);
+  static_assert(FewCfg<NT, MT>::red_bytes(NW) <= 48 * 1024, "no opt-in for more shared memory");
+  auto kern = gemm_few_kernel<NT, MT, NW, FUSE>;
+  if constexpr (FUSE) {
+    p.t_ctas = (p.R + 16 * MT - 1) / (16 * MT);
+    if constexpr (FUSE == 2) {
+      static bool configured = false;
+      if (!configured) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_ROWS_MOST) != cudaSuccess) return -10;
+        configured = true;
+      }
+      const int rows = few_rows_bytes(p.M, p.K);
+      bytes = bytes > rows ? bytes : rows;
+    }
+  }
+  return launch_chain(kern, dim3((FUSE ? p.t_ctas : 0) + (p.F + 16 * MT - 1) / (16 * MT), (p.M + 8 * NT - 1) / (8 * NT)), dim3(NW * 32), bytes, stream,
+                      p) == cudaSuccess ? 0 : -12;
+}
+
+// The split by sizes, see tahb_gemm_few.
+template <int FUSE>
+static int dispatch_few(FewParams& p, cudaStream_t stream) {
+  const int tiles = (p.F + 15) / 16, M = p.M, K = p.K;
+#define TAHB_FEW(NT_)                                                                         \
+  {                                                                                           \
+    if (tiles >= 4 * 148) return launch_few<NT_, 2, 4, FUSE>(p, stream);                      \
+    if (NT_ == 1 && K <= 2048) return launch_few<1, 2, 16, FUSE>(p, stream);                  \
+    if (tiles <= 148 || K >= 4096) return launch_few<NT_, 1, 16, FUSE>(p, stream);            \
+    return launch_few<NT_, 1, 8, FUSE>(p, stream);                                            \
+  }
+  if (M <= 8) TAHB_FEW(1)
+  if (M <= 16) TAHB_FEW(2)
+  if constexpr (FUSE) return -22;
+  else TAHB_FEW(4)
+#undef TAHB_FEW
 }
 
 }  // namespace tahb
@@ -226,16 +386,40 @@ extern "C" int tahb_gemm_few(const void* W, const void* X, void* out, const void
   p.stacked = act == 1 ? F / 2 : 0;
   p.act_up = act_up; p.act_low = act_low;
   p.early = early;
-  const int tiles = (F + 15) / 16;
-#define TAHB_FEW(NT_)                                                                         \
-  {                                                                                           \
-    if (tiles >= 4 * 148) return launch_few<NT_, 2, 4>(p, stream);                             \
-    if (NT_ == 1 && K <= 2048) return launch_few<1, 2, 16>(p, stream);                         \
-    if (tiles <= 148 || K >= 4096) return launch_few<NT_, 1, 16>(p, stream);                   \
-    return launch_few<NT_, 1, 8>(p, stream);                                                  \
-  }
-  if (M <= 8) TAHB_FEW(1)
-  if (M <= 16) TAHB_FEW(2)
-  TAHB_FEW(4)
-#undef TAHB_FEW
+  p.t_ctas = 0;
+  return dispatch_few<0>(p, stream);
+}
+
+// The same for up to 16 tokens with what stands around it in a decode tick: norm_w != null: X goes through RMSNorm (norm_w, eps) first;
+// R > 0: out += T B^T with T = gate * x A^T (A [R, K], B [F, R], T [M, R], all contiguous; T is written where a row is gated).
+// act as above.  sync: two ints, zero, for this stream's launches alone.
+extern "C" int tahb_gemm_few_fused(const void* W, const void* X, void* out, const void* residual, const void* norm_w, float eps, const void* A,
+                                   const void* B, void* T, const int* gate, int* sync, int M, int F, int K, int R, long long ldw,
+                                   long long ldx, long long ldo, long long ldr, int act, int* status, cudaStream_t stream) {
+  if (M <= 0 || F <= 0) return 0;
+  if (M > 16 || K <= 0 || K % 64 || R % 64 || ((act == 1 || act == 4) && (F % 2 || residual != nullptr))) return -20;
+  if (act != 0 && act != 1 && act != 4) return -29;
+  if (R > 0 && (A == nullptr || B == nullptr || T == nullptr || gate == nullptr || sync == nullptr)) return -27;
+  if (norm_w != nullptr && few_rows_bytes(M, K) > FEW_ROWS_MOST) return -22;
+  auto odd = [](const void* p, long long ld) { return (reinterpret_cast<uintptr_t>(p) & 15) || (ld & 7); };
+  if (odd(W, ldw) || odd(X, ldx) || odd(norm_w, 0) || odd(A, 0) || odd(B, 0) || odd(T, 0)) return -2;
+  FewParams p = {};
+  p.W = reinterpret_cast<const __nv_bfloat16*>(W);
+  p.X = reinterpret_cast<const __nv_bfloat16*>(X);
+  p.W2 = reinterpret_cast<const __nv_bfloat16*>(B);
+  p.X2 = reinterpret_cast<const __nv_bfloat16*>(T);
+  p.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
+  p.out = reinterpret_cast<__nv_bfloat16*>(out);
+  p.M = M; p.F = F; p.K = K; p.R = R;
+  p.ldw = ldw; p.ldx = ldx; p.ldw2 = R; p.ldx2 = R; p.ldo = ldo; p.ldr = ldr;
+  p.act = act ? 2 : 0;
+  p.stacked = act == 1 ? F / 2 : 0;
+  p.norm_w = reinterpret_cast<const __nv_bfloat16*>(norm_w);
+  p.eps = eps;
+  p.A = reinterpret_cast<const __nv_bfloat16*>(A);
+  p.T = reinterpret_cast<__nv_bfloat16*>(T);
+  p.gate = gate;
+  p.sync = sync;
+  p.status = status;
+  return norm_w != nullptr ? dispatch_few<2>(p, stream) : dispatch_few<1>(p, stream);
 }

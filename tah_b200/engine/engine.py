@@ -39,12 +39,13 @@ KV_BLOCK_BYTES = 1 << 29
 
 def _fusions(default: str):
     """Kernel fusions selected by ``TAH_B200_FUSE``: "1" = all, "0" = none, or a comma list of "qkv" (QK-norm, RoPE
-    and the K/V write in the QKV GEMM's epilogue) and "lora" (LoRA-A of the gated rows inside the RMSNorm launch);
-    unset = ``default`` ("lora" in ticks of up to eight rows, else nothing)."""
+    and the K/V write in the QKV GEMM's epilogue), "lora" (LoRA-A of the gated rows inside the RMSNorm launch) and "few"
+    (RMSNorm and LoRA-A inside the products of up to 16 rows, in place of the others); unset = ``default`` ("few" in ticks of up to 16 rows, else
+    nothing).  "1" is "qkv" and "lora"."""
     v = os.environ.get("TAH_B200_FUSE", default)
     if v == "1":
         return {"qkv", "lora"}
-    return {t for t in v.split(",") if t in ("qkv", "lora")}
+    return {t for t in v.split(",") if t in ("qkv", "lora", "few")}
 
 
 class TaHEngine(DecodeEngine):
@@ -486,6 +487,7 @@ class TaHEngine(DecodeEngine):
         s.logits, s.cum = bf(B, w.vocab_shard[2]), bf(B, w.vocab_shard[2])
         s.topv = torch.zeros(B, self.topk, dtype=torch.float32, device=dev)
         s.topi = i32(B, self.topk)
+        s.few_sync = i32(2)
         tl = self._tap_layers()
         # the learned decider's Linear(topk -> H) output is written behind the tapped hidden states
         tap_w = (max(1, len(tl)) + (1 if self._needs_topk_for_decider() else 0)) * H
@@ -535,6 +537,28 @@ class TaHEngine(DecodeEngine):
         K.gemm(x, w_, out=tp.partial[:M], **kw)
         return tp.fused_reduce_norm(M, h, ln_w, cfg.rms_norm_eps, add_residual=True)
 
+    def _few_fits(self, B: int) -> bool:
+        """Whether a tick of ``B`` rows takes the products that normalise their input themselves."""
+        w, cfg = self.w, self.cfg
+        aligned = all(t.data_ptr() % 16 == 0 for L in w.layers for t in (L.ln1, L.ln2, L.w_qkv, L.w_o, L.w_gu, L.w_down))
+        return aligned and K.few_fused_fits(B, cfg.hidden_size) and w.nq * cfg.head_dim % 64 == 0 and w.inter % 64 == 0
+
+    def _few_layer(self, s, L, pools, lora: bool) -> None:
+        """A layer of a tick of few rows in six or seven launches: the products take the RMSNorm in front of them and the gated rows' LoRA-A
+        along (``csrc/gemm_few.cu``)."""
+        cfg, w, kv = self.cfg, self.w, self.kv
+        nq, nkv, hd = w.nq, w.nkv, cfg.head_dim
+        fused = lambda x, wt, out, A, t, Bx, **kw: K.gemm_few_fused(x, wt, out, s.gate, s.few_sync, lora=(A, t, Bx) if lora else None,
+                                                                    eps=cfg.rms_norm_eps, **kw)
+        fused(s.h, L.w_qkv, s.qkv, L.a_qkv, s.t_qkv, L.b_qkv, norm=L.ln1)
+        K.qk_norm_rope_kv(s.qkv, L.q_norm, L.k_norm, s.pos, nq, nkv, hd, cfg.rms_norm_eps, cfg.rope_theta, q_out=s.q, caches=pools,
+                          cache_sel=s.depth, slot=s.slot, page_size=self.page_size)
+        K.decode_attn(s.q, pools, kv.page_table, kv.len, s.depth, nq, nkv, hd, self.page_size, hd ** -0.5, out=s.o, n_split=s.attn_split,
+                      ws=s.attn_ws)
+        fused(s.o, L.w_o, s.h, L.a_o, s.t_o, L.b_o, residual=s.h)
+        fused(s.h, L.w_gu, s.act, L.a_gu, s.t_gu, L.b_gu, norm=L.ln2, act=4 if w.gu_interleaved else 1)
+        fused(s.act, L.w_down, s.h, L.a_down, s.t_down, L.b_down, residual=s.h)
+
     def _tick(self, s, sampling):
         """Enqueue one decode tick on the current stream (graph-capturable)."""
         cfg, w, kv, tp = self.cfg, self.w, self.kv, self.tp
@@ -545,13 +569,14 @@ class TaHEngine(DecodeEngine):
         tl = self._tap_layers()
         H = cfg.hidden_size
         nL = len(w.layers)
-        # Optional fusions of the decode chain.  RMSNorm and LoRA-A in one launch pays while launches are what a tick is made of (1 row:
-        # 1.49 -> 1.35 ms, 6 rows 1.75 -> 1.67 ms); from 20 rows on the gated rows' products hold up the norm (2.98 -> 3.12 ms), and at
-        # 256 rows the chain of separate launches is faster, also than the QKV epilogue on the GEMM's eight epilogue warps (a generation of 32
+        # Optional fusions of the decode chain.  While launches are what a tick is made of, the products of up to 16 rows take the RMSNorm in front of
+        # them and the gated rows' LoRA-A along.  RMSNorm and LoRA-A in one launch hold up the norm from 20 rows on (2.98 -> 3.12 ms), and at 256
+        # rows the chain of separate launches is faster, also than the QKV epilogue on the GEMM's eight epilogue warps (a generation of 32
         # tokens 205.7 ms, fused 212.2; 20 rows of up to 1900 172.9 and 182.3).
-        fuse = _fusions("lora" if B <= 8 else "")
-        fuse_norm_lora = "lora" in fuse and lora and tp is None  # RMSNorm + LoRA-A of the gated rows in one launch
+        fuse = _fusions("few" if B <= K.FUSED_TOKENS else "")
         fuse_qkv = "qkv" in fuse and hd == 128                   # QK-norm + RoPE + KV write in the QKV GEMM epilogue
+        few = "few" in fuse and tp is None and not fuse_qkv and self._few_fits(B)
+        fuse_norm_lora = "lora" in fuse and lora and tp is None and not few  # RMSNorm + LoRA-A of the gated rows in one launch
         rope = dict(rope_cs=s.rope_cs, hd=hd, theta=cfg.rope_theta) if fuse_qkv else {}
         if tp is None:
             s.binding.tick_begin(w.embed, s.soft, s.h, **rope)   # the input embedding is the residual stream
@@ -559,7 +584,9 @@ class TaHEngine(DecodeEngine):
             s.binding.tick_begin(w.embed, s.soft, s.x_in, **rope)
             s.h.copy_(s.x_in)
         pools = [[kv.layer_pool(d, li) for d in range(kv.n_depths)] for li in range(nL)]
-        if fuse_norm_lora:
+        if few:
+            xn = None              # every product normalises its own input
+        elif fuse_norm_lora:
             xn = K.rms_norm_lora(s.h, w.layers[0].ln1, cfg.rms_norm_eps, s.gate, w.layers[0].a_qkv, out=s.xn,
                                  t_out=s.t_qkv)[0]
         else:
@@ -577,6 +604,9 @@ class TaHEngine(DecodeEngine):
                     s.taps[:, j * H:(j + 1) * H].copy_(s.x_in)      # the embeddings: every rank has all rows
                 else:
                     s.taps[:, j * H:(j + 1) * H].copy_(tp.gather_rows(s.h, B))
+            if few:
+                self._few_layer(s, L, pools[li], lora)
+                continue
             if lora and not fuse_norm_lora:
                 K.lora_a_rows(xn, L.a_qkv, s.gate, out=s.t_qkv, tp_wait=self._xn_wait)
             kw = dict(x2=s.t_qkv, w2=L.b_qkv) if lora else {}
@@ -605,6 +635,8 @@ class TaHEngine(DecodeEngine):
             tap = (s.tap_buf, tl.index(li + 1) * H) if kernel_taps and li + 1 < nL and (li + 1) in tl else None
             xn = self._row_parallel(s.act, L.w_down, L.a_down if lora else None, L.b_down, s.t_down, s.gate, s.h,
                                     next_ln, s.xn, B, push=push, final=li + 1 == nL, next_lora=nxt_lora, tap=tap)
+        if few:
+            xn = K.rms_norm(s.h, w.final_norm, cfg.rms_norm_eps, out=s.xn)
         # xn is now the final-norm output of every row
         if cfg.num_hidden_layers in tl:
             j = tl.index(cfg.num_hidden_layers)

@@ -434,6 +434,38 @@ def _gemm_few(x, w, out, residual=None, x2=None, w2=None, act: int = 0, act_up: 
     return out
 
 
+FUSED_TOKENS = 16
+
+
+def few_fused_fits(M: int, K: int) -> bool:
+    """Whether :func:`gemm_few_fused` takes ``M`` tokens of ``K`` numbers (its rows lie in shared memory, two CTAs per SM)."""
+    return 0 < M <= FUSED_TOKENS and K > 0 and K % 64 == 0 and 2 * K + M * (2 * K + 64) <= 96 * 1024
+
+
+def gemm_few_fused(x, w, out, gate, sync, *, norm=None, eps: float = 0.0, lora=None, residual=None, act: int = 0):
+    """A few-token product of a decode tick with what stands around it, in one launch: ``out = norm(x) w^T (+ (gate * norm(x) A^T) B^T)
+    (+ residual)``.
+
+    ``norm``: RMSNorm weight (with ``eps``), None: ``x`` as it is; ``lora``: ``(A [R, K], t [M, R], B [F, R])``, contiguous, or None; ``act``: 0
+    none, 1 SwiGLU of stacked rows, 4 of interleaved rows; ``sync``: two int32 zeros that no other stream uses meanwhile."""
+    for t, n in ((x, "x"), (w, "w"), (out, "out")) + (() if residual is None else ((residual, "residual"),)):
+        _check_bf16_2d(t, n)
+    M, Kd = x.shape
+    F = w.shape[0]
+    if w.shape[1] != Kd or out.shape != (M, F // 2 if act else F) or (norm is not None and (norm.numel() != Kd or not norm.is_contiguous())):
+        raise ValueError(f"gemm_few_fused: x {tuple(x.shape)} w {tuple(w.shape)} out {tuple(out.shape)}")
+    A, t, B = lora or (None, None, None)
+    R = 0 if A is None else A.shape[0]
+    if R and (A.shape != (R, Kd) or t.shape != (M, R) or B.shape != (F, R) or not (A.is_contiguous() and t.is_contiguous() and B.is_contiguous()) or
+              gate.dtype != torch.int32 or gate.numel() < M or sync.dtype != torch.int32 or sync.numel() < 2):
+        raise ValueError("gemm_few_fused: adapter operands do not match")
+    _rc(lib().tahb_gemm_few_fused(_p(w), _p(x), _p(out), _p(residual), _p(norm), c_float(eps), _p(A), _p(B), _p(t), _p(gate if R else None),
+                                  _p(sync if R else None), c_int(M), c_int(F), c_int(Kd), c_int(R), c_ll(w.stride(0)), c_ll(x.stride(0)),
+                                  c_ll(out.stride(0)), c_ll(0 if residual is None else residual.stride(0)), c_int(act),
+                                  _p(status_word(x.device)), _stream()), "tahb_gemm_few_fused")
+    return out
+
+
 def _persist_ok(x, w, out, residual=None, x2=None, w2=None, x_t: bool = False, w_t: bool = False) -> bool:
     """Whether the persistent form takes these operands: more than 128 tokens (256 of transposed ones), whole pieces of 16 bytes everywhere, whole blocks of the
     reduction (unless both operands are transposed)."""

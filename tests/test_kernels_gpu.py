@@ -1360,3 +1360,44 @@ def test_gemm_persist_is_what_wide_products_take():
     a, b = Kc.gemm_t(x, w, w_t=True), Kc.gemm_t(x, w, w_t=True, pair=False, bn=256)
     assert bool(((a.double() - b.double()).abs() <= 2.0 ** -7 * b.double().abs() + 1e-3).all())
     Kc.check_status()
+
+
+@pytest.mark.parametrize("M", [1, 6, 8, 9, 16])
+@pytest.mark.parametrize("F,Kd,R,norm,act", [(4096, 2048, 192, True, 0), (2048, 2048, 64, False, 0), (12288, 2048, 128, True, 4), (2048, 6144, 64, False, 0),
+                                             (96, 64, 0, True, 0), (200, 192, 64, True, 1), (1000, 2304, 64, True, 0)])
+def test_gemm_few_fused(M, F, Kd, R, norm, act):
+    """The few-token product with RMSNorm and gated adapter inside, against 64 bits with its roundings (normed rows, adapter inputs and activation
+    parts in bf16), with no, some and all rows gated, the counters at zero behind it.  Bound: a bf16 rounding of the sum and of the result;
+    a normed row or an adapter input that rounds the other way moves its column by 2^-8 of its share."""
+    Kc = _cuda()
+    x, w, nw = _rand(M, Kd, seed=1), _rand(F, Kd, scale=Kd ** -0.5, seed=2), 1 + 0.1 * _rand(Kd, seed=3)
+    A, B = (_rand(R, Kd, scale=Kd ** -0.5, seed=4), _rand(F, R, scale=R ** -0.5, seed=5)) if R else (None, None)
+    res = None if act else _rand(M, F, seed=6)
+    sync = torch.zeros(2, dtype=torch.int32, device="cuda")
+    r16 = lambda t: t.to(torch.bfloat16).double()
+    xd = x.double()
+    if norm:
+        xd = r16(nw.double() * r16(xd * torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-6)))
+    for gate in ([0] * M, [i % 3 == 1 for i in range(M)], [1] * M):
+        g = torch.tensor(gate, device="cuda").int()
+        t = torch.full((M, R), float("nan"), dtype=torch.bfloat16, device="cuda") if R else None
+        out = torch.empty(M, F // 2 if act else F, dtype=torch.bfloat16, device="cuda") if act else res.clone()
+        for _ in range(2):                              # again with the counters that the first launch left
+            if res is not None:
+                out.copy_(res)
+            Kc.gemm_few_fused(x, w, out, g, sync, norm=nw if norm else None, eps=1e-6, lora=(A, t, B) if R else None, act=act,
+                              residual=None if act else out)
+        z, part = xd @ w.double().t(), (xd.abs() @ w.double().abs().t()) * 2.0 ** -8 / 8
+        if R:
+            z = z + r16(xd @ A.double().t() * g.double().view(-1, 1)) @ B.double().t()
+        if act:
+            gate_, up = (z[:, 0::2], z[:, 1::2]) if act == 4 else (z[:, :F // 2], z[:, F // 2:])
+            pg, pu = (part[:, 0::2], part[:, 1::2]) if act == 4 else (part[:, :F // 2], part[:, F // 2:])
+            ref = torch.nn.functional.silu(gate_) * up
+            bound = 2.0 ** -8 * (1.2 * gate_.abs() * up.abs() + 3 * ref.abs()) + 1.2 * pg * up.abs() + pu * gate_.abs()
+        else:
+            ref = z + res.double()
+            bound = 2.0 ** -8 * (z.abs() + ref.abs()) + part
+        assert bool(((out.double() - ref).abs() <= 1.01 * bound + 1e-4).all())
+        assert sync.tolist() == [0, 0]
+    Kc.check_status()
