@@ -65,6 +65,107 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
 }
 constexpr int FEW_ROWS_MOST = 96 * 1024;       // of shared memory for normalised rows: two CTAs per SM
 
+// T[r] = gate[r] ? x[r] A^T : 0 for a decode tick of many rows, of which a few are gated.  What bounds it: latency; a row's product is R dot
+// products of K, and as dot products of one row at a time (lora_a_rows_kernel in elementwise.cu) 14 gated rows of 256 read A 14 times: 3.5 to 6.6 us
+// a launch, four launches a layer.  Here the gated rows are gathered, 16 at a time, into the token side of warp-level tensor
+// instructions; 16 outputs per cluster of eight CTAs that split the reduction, so that a warp holds all it needs of A in registers, read
+// ahead of the dependency wait; the partial sums meet in the first CTA's shared memory, in a fixed order.  256 rows, 192 outputs of 2048, us, rows
+// of dot products / this: 1 gated row 4.1 / 2.9, 14 5.3 / 3.0; 64 outputs of 6144: 4.2 / 3.2, 5.1 / 3.3.  27 KB of shared memory and 256 threads
+// fit an SM beside a CTA of the one-tile GEMM, so that the start-up stands under its tail.
+constexpr int LG_WARPS = 8, LG_CL = 8, LG_STEPS = 4, LG_NT = 2, LG_TOK = 8 * LG_NT, LG_PITCH = 17;
+struct LoraGatedParams {
+  const __nv_bfloat16 *x, *A;
+  __nv_bfloat16* T;
+  const int* gate;
+  int M, K, R;
+  long long ldx, ldt;
+};
+__global__ void __launch_bounds__(LG_WARPS * 32) lora_gated_kernel(const LoraGatedParams p) {
+  __shared__ float red[LG_WARPS * LG_TOK * LG_PITCH];
+  __shared__ float part[2][LG_CL][LG_TOK * 16];               // [buffer][CTA of the cluster], used in the first CTA
+  __shared__ short rows[1024];
+  __shared__ int counts[32];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int rank = (int)cluster_ctarank(), f0 = (int)(blockIdx.x / LG_CL) * 16;
+  const int steps = p.K >> 5, c0 = steps * rank / LG_CL, cn = steps * (rank + 1) / LG_CL - c0;
+  const int s0 = c0 + cn * warp / LG_WARPS, s1 = c0 + cn * (warp + 1) / LG_WARPS;
+  uint4 a[LG_STEPS][2];
+#pragma unroll
+  for (int i = 0; i < LG_STEPS; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      a[i][h] = s0 + i < s1 ? ld_stream(p.A + (size_t)min(f0 + 8 * h + g, p.R - 1) * p.K + t * 8 + (s0 + i) * 32) : make_uint4(0u, 0u, 0u, 0u);
+  cluster_sync_all();                                         // the first CTA's shared memory exists before anyone writes to it
+  pdl_wait();
+  // the gated rows, in order
+  unsigned m[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const int r = (warp + c * LG_WARPS) * 32 + lane;
+    m[c] = __ballot_sync(0xffffffffu, r < p.M && p.gate[r] != 0);
+    if (lane == 0) counts[warp + c * LG_WARPS] = __popc(m[c]);
+  }
+  __syncthreads();
+  const int n = __reduce_add_sync(0xffffffffu, counts[lane]);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const int chunk = warp + c * LG_WARPS, r = chunk * 32 + lane;
+    const int before = __reduce_add_sync(0xffffffffu, lane < chunk ? counts[lane] : 0);
+    if (m[c] >> lane & 1u) {
+      rows[before + __popc(m[c] & ((1u << lane) - 1u))] = (short)r;
+    } else if (r < p.M && r % LG_CL == rank && blockIdx.y == 0) {     // zeros for the others, rows dealt out to the CTAs of the cluster
+      uint4* dst = reinterpret_cast<uint4*>(p.T + (size_t)r * p.ldt + f0);
+      dst[0] = make_uint4(0u, 0u, 0u, 0u);
+      if (f0 + 8 < p.R) dst[1] = make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
+  __syncthreads();
+  const uint32_t part0 = dsmem_addr(smem_u32(&part[0][rank][0]), 0);
+  const int stride = LG_TOK * gridDim.y;
+  for (int base = LG_TOK * blockIdx.y, pass = 0; base < n; base += stride, ++pass) {
+    float acc[LG_NT][4];
+#pragma unroll
+    for (int j = 0; j < LG_NT; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[j][c] = 0.f;
+    uint4 x[LG_STEPS][LG_NT];
+#pragma unroll
+    for (int j = 0; j < LG_NT; ++j) {
+      const __nv_bfloat16* src = p.x + (size_t)rows[min(base + 8 * j + g, n - 1)] * p.ldx + t * 8;
+#pragma unroll
+      for (int i = 0; i < LG_STEPS; ++i)
+        x[i][j] = s0 + i < s1 ? *reinterpret_cast<const uint4*>(src + (s0 + i) * 32) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int i = 0; i < LG_STEPS; ++i)
+#pragma unroll
+      for (int j = 0; j < LG_NT; ++j) {
+        mma_16816(acc[j], a[i][0].x, a[i][1].x, a[i][0].y, a[i][1].y, x[i][j].x, x[i][j].y);
+        mma_16816(acc[j], a[i][0].z, a[i][1].z, a[i][0].w, a[i][1].w, x[i][j].z, x[i][j].w);
+      }
+    if (base + stride >= n) pdl_launch_dependents();
+#pragma unroll
+    for (int j = 0; j < LG_NT; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) red[(warp * LG_TOK + 8 * j + 2 * t + (c & 1)) * LG_PITCH + g + 8 * (c >> 1)] = acc[j][c];
+    __syncthreads();
+    if (tid < LG_TOK * 16) {
+      float v = 0.f;
+#pragma unroll
+      for (int k = 0; k < LG_WARPS; ++k) v += red[(k * LG_TOK + tid / 16) * LG_PITCH + tid % 16];
+      st_dsmem_f32(part0 + ((pass & 1) * LG_CL * LG_TOK * 16 + tid) * 4, v);
+    }
+    cluster_sync_all();       // two buffers: a CTA writes the one of pass + 2 behind the barrier that follows the reading of this one
+    if (rank == 0 && tid < LG_TOK * 16) {
+      float v = 0.f;
+#pragma unroll
+      for (int k = 0; k < LG_CL; ++k) v += part[pass & 1][k][tid];
+      const int tok = base + tid / 16, f = f0 + tid % 16;
+      if (tok < n && f < p.R) p.T[(size_t)rows[tok] * p.ldt + f] = __float2bfloat16_rn(v);
+    }
+  }
+}
+
 template <int NT, int MT>
 struct FewCfg {
   static constexpr int ST = 4 / MT;                        // steps of 32 reduction indices per buffer, two buffers: 64 registers
@@ -343,7 +444,7 @@ static int dispatch_few(FewParams& p, cudaStream_t stream) {
   }
   if (M <= 8) TAHB_FEW(1)
   if (M <= 16) TAHB_FEW(2)
-  if constexpr (FUSE) return -22;
+  if constexpr (FUSE == 2) return -22;
   else TAHB_FEW(4)
 #undef TAHB_FEW
 }
@@ -390,14 +491,14 @@ extern "C" int tahb_gemm_few(const void* W, const void* X, void* out, const void
   return dispatch_few<0>(p, stream);
 }
 
-// The same for up to 16 tokens with what stands around it in a decode tick: norm_w != null: X goes through RMSNorm (norm_w, eps) first;
+// The same for up to 32 tokens (16 with norm_w) with what stands around it in a decode tick: norm_w != null: X goes through RMSNorm (norm_w, eps) first;
 // R > 0: out += T B^T with T = gate * x A^T (A [R, K], B [F, R], T [M, R], all contiguous; T is written where a row is gated).
 // act as above.  sync: two ints, zero, for this stream's launches alone.
 extern "C" int tahb_gemm_few_fused(const void* W, const void* X, void* out, const void* residual, const void* norm_w, float eps, const void* A,
                                    const void* B, void* T, const int* gate, int* sync, int M, int F, int K, int R, long long ldw,
                                    long long ldx, long long ldo, long long ldr, int act, int* status, cudaStream_t stream) {
   if (M <= 0 || F <= 0) return 0;
-  if (M > 16 || K <= 0 || K % 64 || R % 64 || ((act == 1 || act == 4) && (F % 2 || residual != nullptr))) return -20;
+  if (M > (norm_w != nullptr ? 16 : 32) || K <= 0 || K % 64 || R % 64 || ((act == 1 || act == 4) && (F % 2 || residual != nullptr))) return -20;
   if (act != 0 && act != 1 && act != 4) return -29;
   if (R > 0 && (A == nullptr || B == nullptr || T == nullptr || gate == nullptr || sync == nullptr)) return -27;
   if (norm_w != nullptr && few_rows_bytes(M, K) > FEW_ROWS_MOST) return -22;
@@ -422,4 +523,34 @@ extern "C" int tahb_gemm_few_fused(const void* W, const void* X, void* out, cons
   p.sync = sync;
   p.status = status;
   return norm_w != nullptr ? dispatch_few<2>(p, stream) : dispatch_few<1>(p, stream);
+}
+
+// T [M, R] = gate[r] ? x[r] A^T : 0 (see lora_gated_kernel).  M <= 1024, K a multiple of 64 up to 8192, R of 8; everything on 16-byte boundaries;
+// A is a constant of the launch chain.
+extern "C" int tahb_lora_gated(const void* x, const void* A, void* T, const int* gate, int M, int K, int R, long long ldx, long long ldt,
+                               cudaStream_t stream) {
+  if (M <= 0 || R <= 0) return 0;
+  if (M > 1024 || K <= 0 || K % 64 || K > 32 * LG_CL * LG_WARPS * LG_STEPS || R % 8 || gate == nullptr) return -20;
+  auto odd = [](const void* p, long long ld) { return (reinterpret_cast<uintptr_t>(p) & 15) || (ld & 7); };
+  if (odd(x, ldx) || odd(A, K) || odd(T, ldt)) return -2;
+  LoraGatedParams p;
+  p.x = reinterpret_cast<const __nv_bfloat16*>(x);
+  p.A = reinterpret_cast<const __nv_bfloat16*>(A);
+  p.T = reinterpret_cast<__nv_bfloat16*>(T);
+  p.gate = gate;
+  p.M = M; p.K = K; p.R = R;
+  p.ldx = ldx; p.ldt = ldt;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((R + 15) / 16 * LG_CL, M <= 64 ? 1 : 2);       // gated rows come 16 at a time, rarely more than 32
+  cfg.blockDim = dim3(LG_WARPS * 32);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = LG_CL;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, lora_gated_kernel, p) == cudaSuccess ? 0 : -12;
 }

@@ -487,7 +487,7 @@ class TaHEngine(DecodeEngine):
         s.logits, s.cum = bf(B, w.vocab_shard[2]), bf(B, w.vocab_shard[2])
         s.topv = torch.zeros(B, self.topk, dtype=torch.float32, device=dev)
         s.topi = i32(B, self.topk)
-        s.few_sync = i32(2)
+        s.few_sync = self._few_sync = i32(2)
         tl = self._tap_layers()
         # the learned decider's Linear(topk -> H) output is written behind the tapped hidden states
         tap_w = (max(1, len(tl)) + (1 if self._needs_topk_for_decider() else 0)) * H
@@ -514,9 +514,13 @@ class TaHEngine(DecodeEngine):
         residual rows into that column of every rank's tap buffer."""
         cfg, tp = self.cfg, self.tp
         lora = a_ is not None and t_buf is not None
+        if lora and tp is None and gate is not None and next_lora is None and K.few_gated_fits(x, w_, h, M):
+            # few rows: the product forms the gated rows' adapter input itself
+            K.gemm_few_fused(x, w_, h, gate, self._few_sync, lora=(a_, t_buf, b_), residual=h)
+            return K.rms_norm(h, ln_w, cfg.rms_norm_eps, out=xn_out)
         if lora:
             if gate is not None:
-                K.lora_a_rows(x, a_, gate, out=t_buf)
+                K.lora_a_rows(x, a_, gate, out=t_buf, const_w=True)
             else:
                 K.gemm(x, a_, out=t_buf)
         kw = dict(x2=t_buf, w2=b_) if lora else {}
@@ -608,7 +612,7 @@ class TaHEngine(DecodeEngine):
                 self._few_layer(s, L, pools[li], lora)
                 continue
             if lora and not fuse_norm_lora:
-                K.lora_a_rows(xn, L.a_qkv, s.gate, out=s.t_qkv, tp_wait=self._xn_wait)
+                K.lora_a_rows(xn, L.a_qkv, s.gate, out=s.t_qkv, tp_wait=self._xn_wait, const_w=True)
             kw = dict(x2=s.t_qkv, w2=L.b_qkv) if lora else {}
             if fuse_qkv:
                 K.gemm_qkv(xn, L.w_qkv, L.q_norm, L.k_norm, s.pos, nq, nkv, cfg.rms_norm_eps, cfg.rope_theta, q_out=s.q,
@@ -623,7 +627,7 @@ class TaHEngine(DecodeEngine):
             xn = self._row_parallel(s.o, L.w_o, L.a_o if lora else None, L.b_o, s.t_o, s.gate, s.h, L.ln2, s.xn, B,
                                     push=push, next_lora=(L.a_gu, s.t_gu) if fuse_norm_lora else None)
             if lora and not fuse_norm_lora:
-                K.lora_a_rows(xn, L.a_gu, s.gate, out=s.t_gu, tp_wait=self._xn_wait)
+                K.lora_a_rows(xn, L.a_gu, s.gate, out=s.t_gu, tp_wait=self._xn_wait, const_w=True)
             sw = dict(swiglu_interleaved=True, const_w=True) if w.gu_interleaved else dict(swiglu=True, const_w=True)
             if lora:
                 K.gemm(xn, L.w_gu, x2=s.t_gu, w2=L.b_gu, out=s.act, tp_wait=self._xn_wait, **sw)

@@ -442,6 +442,11 @@ def few_fused_fits(M: int, K: int) -> bool:
     return 0 < M <= FUSED_TOKENS and K > 0 and K % 64 == 0 and 2 * K + M * (2 * K + 64) <= 96 * 1024
 
 
+def few_gated_fits(x, w, out, M: int) -> bool:
+    """Whether a product of a tick of up to 32 rows takes its gated adapter input along (:func:`gemm_few_fused` without a norm)."""
+    return few_shape(M, w.shape[0], w.shape[1], 0, True) and M <= FEW_TOKENS and all(_whole_pieces(t) for t in (x, w, out))
+
+
 def gemm_few_fused(x, w, out, gate, sync, *, norm=None, eps: float = 0.0, lora=None, residual=None, act: int = 0):
     """A few-token product of a decode tick with what stands around it, in one launch: ``out = norm(x) w^T (+ (gate * norm(x) A^T) B^T)
     (+ residual)``.
@@ -754,14 +759,25 @@ def embed_gather(E, tok, out=None):
     return out
 
 
-def lora_a_rows(x, A, gate=None, out=None, tp_wait=None):
+def lora_gated_fits(M: int, K: int, R: int) -> bool:
+    """Whether the gated adapter input of ``M`` rows takes the gathered tensor-core form."""
+    return 0 < M <= 1024 and 0 < K <= 8192 and K % 64 == 0 and R > 0 and R % 8 == 0
+
+
+def lora_a_rows(x, A, gate=None, out=None, tp_wait=None, const_w: bool = False):
     """``out[r] = gate[r] ? x[r] @ A^T : 0`` for the few gated rows of a decode tick.  ``tp_wait =
-    (flags, targets)``: gated rows first wait for the tensor-parallel broadcast of ``x``."""
+    (flags, targets)``: gated rows first wait for the tensor-parallel broadcast of ``x``.  ``const_w``: ``A`` is a weight that no kernel of this
+    library writes: it is then read ahead, and the gated rows are gathered for tensor instructions (sums in another order)."""
     _check_bf16_2d(x, "x")
     M, K = x.shape
     R = A.shape[0]
     if out is None:
         out = torch.empty(M, R, dtype=torch.bfloat16, device=x.device)
+    if const_w and gate is not None and tp_wait is None and lora_gated_fits(M, K, R) and A.is_contiguous() and gate.is_contiguous() and \
+            all(_whole_pieces(t) for t in (x, A, out)):
+        _rc(lib().tahb_lora_gated(_p(x), _p(A), _p(out), _p(gate), c_int(M), c_int(K), c_int(R), c_ll(x.stride(0)), c_ll(out.stride(0)),
+                                  _stream()), "tahb_lora_gated")
+        return out
     if tp_wait is None:
         _rc(lib().tahb_lora_a_rows(_p(x), _p(A), _p(out), _p(gate), c_int(M), c_int(K), c_int(R), c_ll(x.stride(0)),
                                    c_ll(out.stride(0)), _stream()), "tahb_lora_a_rows")

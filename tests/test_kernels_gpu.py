@@ -1401,3 +1401,35 @@ def test_gemm_few_fused(M, F, Kd, R, norm, act):
         assert bool(((out.double() - ref).abs() <= 1.01 * bound + 1e-4).all())
         assert sync.tolist() == [0, 0]
     Kc.check_status()
+
+
+@pytest.mark.parametrize("M,Kd,R,n", [(1, 64, 8, 1), (20, 2048, 192, 2), (33, 2048, 64, 0), (256, 6144, 64, 15), (256, 2048, 128, 17), (300, 8192, 24, 300),
+                                      (1024, 192, 64, 1024)])
+def test_lora_gated(M, Kd, R, n):
+    """Adapter inputs of the gated rows, gathered 16 at a time: none, a few, one more than a pass, all.  Bound: the bf16 rounding and 32-bit sums."""
+    Kc = _cuda()
+    x, A = _rand(M, Kd, seed=1), _rand(R, Kd, scale=Kd ** -0.5, seed=2)
+    gate = torch.zeros(M, dtype=torch.int32, device="cuda")
+    gate[torch.randperm(M, generator=torch.Generator().manual_seed(3))[:n].to("cuda")] = 1
+    out = torch.full((M, R + 8), float("nan"), dtype=torch.bfloat16, device="cuda")[:, :R]
+    assert Kc.lora_gated_fits(M, Kd, R)
+    Kc.lora_a_rows(x, A, gate, out=out, const_w=True)
+    ref = x.double() @ A.double().t() * gate.double().view(-1, 1)
+    part = x.double().abs() @ A.double().abs().t()
+    assert bool(((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2.0 ** -20 * part).all())
+    assert bool((out[gate == 0] == 0).all())
+
+
+@pytest.mark.parametrize("M", [17, 24, 32])
+def test_gemm_few_fused_up_to_32_rows(M):
+    """Without a norm the fused product takes up to 32 rows."""
+    Kc = _cuda()
+    x, w, A, B = _rand(M, 6144, seed=1), _rand(2048, 6144, scale=6144 ** -0.5, seed=2), _rand(64, 6144, scale=6144 ** -0.5, seed=3), _rand(2048, 64, seed=4)
+    g = (torch.arange(M, device="cuda") % 5 == 2).int()
+    t, h, sync = torch.empty(M, 64, dtype=torch.bfloat16, device="cuda"), _rand(M, 2048, seed=5), torch.zeros(2, dtype=torch.int32, device="cuda")
+    plain = Kc.gemm(x, w, x2=Kc.lora_a_rows(x, A, g), w2=B, residual=h)
+    out = Kc.gemm_few_fused(x, w, h.clone(), g, sync, lora=(A, t, B), residual=h)
+    # both round the adapter inputs, the sum and the result to bf16
+    scale = (x.double().abs() @ w.double().abs().t()) * 2.0 ** -16 + 2.0 ** -7 * out.double().abs() + 64 ** 0.5 * 2.0 ** -8
+    assert bool(((out.double() - plain.double()).abs() <= scale).all()) and sync.tolist() == [0, 0]
+    Kc.check_status()
