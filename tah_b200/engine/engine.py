@@ -23,6 +23,7 @@ from __future__ import annotations
 import os
 from typing import Optional, Sequence
 
+import numpy as np
 import torch
 
 from tah_b200.engine.base import DecodeEngine, GenerationResult  # noqa: F401
@@ -46,6 +47,35 @@ def _fusions(default: str):
     if v == "1":
         return {"qkv", "lora"}
     return {t for t in v.split(",") if t in ("qkv", "lora", "few")}
+
+
+class HostArrays:
+    """Small host arrays that go to the device in one copy: ``put`` gives a function that returns the array on the device once ``send`` was
+    called."""
+
+    def __init__(self):
+        self._parts, self._bytes, self._dev, self._after = [], 0, None, []
+
+    def put(self, a, dtype):
+        a = np.ascontiguousarray(a, dtype=dtype)
+        at, self._bytes = self._bytes, self._bytes + (a.nbytes + 15) // 16 * 16
+        self._parts.append((at, a))
+        kind = {np.int32: torch.int32, np.int64: torch.int64}[dtype]
+        return lambda: self._dev[at:at + a.nbytes].view(kind)
+
+    def then(self, f) -> None:
+        """``f`` runs right behind the copy."""
+        self._after.append(f)
+
+    def send(self, device) -> None:
+        # page-locked (from torch's pool, which keeps it until the copy is done), so that the copy does not wait for the stream
+        host = torch.empty(max(16, self._bytes), dtype=torch.uint8, pin_memory=torch.device(device).type == "cuda")
+        view = host.numpy()
+        for at, a in self._parts:
+            view[at:at + a.nbytes] = a.reshape(-1).view(np.uint8)
+        self._dev = host.to(device, non_blocking=True)
+        for f in self._after:
+            f()
 
 
 class TaHEngine(DecodeEngine):
@@ -221,10 +251,10 @@ class TaHEngine(DecodeEngine):
     # ------------------------------------------------------------------------------------------
     # one backbone pass over packed tokens (prefill)
     # ------------------------------------------------------------------------------------------
-    def _packed_pass(self, x, pos, depth: int, slots, seg_k, seg_v, seg_base, seg_count, seq_counts, taps_out=None):
+    def _packed_pass(self, x, pos, depth: int, slots, seg_k, seg_v, seg_base, seg_count, seq_counts, taps_out=None, tiles=None):
         """x ``[n, H]`` packed tokens at iteration ``depth``.  seg_k/seg_v: per layer lists of the
         dense K/V of shallower passes; this pass's K/V are appended as the last segment.
-        ``seq_counts [B]``: how many of the packed tokens each sequence owns (query tiling).  Returns
+        ``seq_counts [B]``: how many of the packed tokens each sequence owns; ``tiles``: their query tiles where they are known.  Returns
         (final-norm hidden, list of this pass's dense (k, v) per layer)."""
         cfg, w, tp = self.cfg, self.w, self.tp
         n = x.shape[0]
@@ -244,7 +274,7 @@ class TaHEngine(DecodeEngine):
         # to 3500 tokens 68.8 ms fused, on eight epilogue warps and launch by launch, 65.2 ms with the separate kernel; one of 700 12.4 and 10.2)
         fuse_qkv = hd == 128 and "qkv" in _fusions("")
         if tensor_core_attn:
-            tile_q0, tile_qn = K.attn_tiles(seq_counts, by_work=True)
+            tile_q0, tile_qn = K.attn_tiles(seq_counts, by_work=True) if tiles is None else tiles
         native = w.native_pass() if tp is None and tensor_core_attn and not fuse_qkv and (lora or depth == 0 or w.r == 0) else None
         if native is not None:
             # the plain form on one GPU: every launch of the pass from one native call
@@ -317,9 +347,11 @@ class TaHEngine(DecodeEngine):
         state; without it the cache is (re)built for exactly this batch."""
         cfg, w, dev = self.cfg, self.w, self.device
         B, T = input_ids.shape
-        valid = attention_mask[:, -T:].bool() if attention_mask is not None else torch.ones(B, T, dtype=torch.bool, device=dev)
-        lens = valid.sum(1)
-        max_total = int(lens.max()) + max_new_tokens + 1
+        # Everything that depends on lengths and decisions alone is worked out on the host and goes to the device in one copy per pass: as device
+        # operations these were 60 small kernels and 25 synchronisations (one prompt of 700 tokens: 5.6 of 9.5 ms without a kernel running).
+        mask = None if attention_mask is None else attention_mask[:, -T:].bool().cpu().numpy()
+        lens_h = np.full(B, T, np.int64) if mask is None else mask.sum(1).astype(np.int64)
+        max_total = int(lens_h.max()) + max_new_tokens + 1
         if row_ids is not None:
             if self.kv is None or self.kv.max_pages[0] * self.page_size < max_total:
                 raise RuntimeError("admission needs an existing KV cache whose rows can hold prompt + new tokens")
@@ -328,71 +360,73 @@ class TaHEngine(DecodeEngine):
             self._new_cache(B, max(max_total, 1))
         if row_ids is None:
             self.kv.reset()
-        assign = (lambda d, c: self.kv.assign_prefill(d, c)) if row_ids is None else \
-                 (lambda d, c: self.kv.assign_rows(d, row_ids, c))
         self._prefill_rows = row_ids
+        n0 = int(lens_h.sum())
         if self.tp is not None:
-            self.tp.allocate(cfg.hidden_size, max(int(valid.sum()), B))
-        rows_idx, cols_idx = valid.nonzero(as_tuple=True)
-        ids = input_ids[rows_idx, cols_idx].to(torch.int32).contiguous()
-        n0 = ids.numel()
-        seq_start = (torch.cumsum(lens, 0) - lens).to(torch.int32)
-        pos = (torch.arange(n0, device=dev, dtype=torch.int32) - seq_start[rows_idx]).contiguous()
-        seq = rows_idx.to(torch.int32)
+            self.tp.allocate(cfg.hidden_size, max(n0, B))
+        flat = np.arange(B * T) if mask is None else np.flatnonzero(mask)
+        start = np.cumsum(lens_h) - lens_h
+        seq = np.repeat(np.arange(B), lens_h)
+        pos = np.arange(n0) - start[seq]
+        # decisions that are known before the first pass: the override's
+        extra = None
+        if self.max_iter <= 1:
+            extra = np.zeros(n0, np.int64)
+        elif self.hard_override is not None:
+            rows = self.hard_override[:B, :int(lens_h.max())] if row_ids is None else self.hard_override[row_ids, :int(lens_h.max())]
+            extra = rows.cpu().numpy()[seq, pos].astype(np.int64)
 
         # ---- pass 0 -------------------------------------------------------------------------
-        slots0 = assign(0, lens)
+        up = HostArrays()
+        slots0 = self._assign_pages(up, 0, lens_h, row_ids)
+        flat_t, lens = up.put(flat, np.int64), up.put(lens_h, np.int64)
+        pos_t, seq_t, base0_t, count0_t = (up.put(v, np.int32) for v in (pos, seq, start[seq], pos + 1))
+        tiles = [up.put(v, np.int32) for v in K.attn_tiles_host(lens_h)]
+        up.send(dev)
+        ids = input_ids.reshape(-1).index_select(0, flat_t()).to(torch.int32)
         x = K.embed_gather(w.embed, ids)
         taps = {}
-        base0 = seq_start[rows_idx].contiguous()
-        count0 = (pos + 1).contiguous()
         with nvtx_range("prefill/pass0"):
-            hn, kv0 = self._packed_pass(x, pos, 0, slots0, [], [], [base0], [count0], lens, taps_out=taps)
+            hn, kv0 = self._packed_pass(x, pos_t(), 0, slots0(), [], [], [base0_t()], [count0_t()], lens(), taps_out=taps,
+                                        tiles=[t() for t in tiles])
         seg_k, seg_v = [[k for k, _ in kv0]], [[v for _, v in kv0]]
 
         # ---- continue decision for every prompt token ----------------------------------------
-        last_idx = (seq_start.long() + lens - 1)
-        is_last = torch.zeros(n0, dtype=torch.bool, device=dev)
-        is_last[last_idx] = True
-        extra = self._prompt_extra_passes(hn, taps, seq, pos)                 # [n0] int: extra passes wanted
-        cur_idx = torch.arange(n0, device=dev)                                # packed indices of the current set
-        cur_cum = None                                                        # cumulative logits of current set
+        is_last = np.zeros(n0, bool)
+        is_last[start + lens_h - 1] = True
+        extra_t = self._prompt_extra_passes(hn, taps, seq_t(), pos_t())       # [n0] int: extra passes wanted
+        if extra is None:
+            extra = extra_t.cpu().numpy().astype(np.int64)
         final_last_logits = torch.empty(B, w.vocab_shard[1] - w.vocab_shard[0], dtype=torch.bfloat16, device=dev)
         # tokens needing logits after pass 0: last tokens + hard tokens
-        need0 = is_last | (extra > 0)
-        sel = need0.nonzero().flatten()
-        logits_sel = self._lm_head(hn[sel])
-        done_last = is_last[sel] & (extra[sel] == 0)
-        final_last_logits[seq[sel][done_last].long()] = logits_sel[done_last]
-        go = extra[sel] > 0
-        cur_idx = sel[go]
-        cur_cum = logits_sel[go]
-        prev_bases = [base0]
-        prev_counts = [count0]
+        sel = np.flatnonzero(is_last | (extra > 0))
+        done_last = np.flatnonzero(is_last[sel] & (extra[sel] == 0))
+        go = np.flatnonzero(extra[sel] > 0)
+        cur = sel[go]                                                         # packed indices of the current set
+        # (base, count) of every packed token in the packed arrays of each pass so far
+        bases, counts = [start[seq]], [pos + 1]
+        learned = self.hard_override is None and isinstance(self._decider()[1], (MLPIterDecider, SimpleMLPIterDecider))
         depth = 1
-        iter_extra_prompt = extra.clone()
-        while depth < self.max_iter and cur_idx.numel() > 0:
-            n1 = cur_idx.numel()
-            rows1 = seq[cur_idx].long()
-            cnt1 = torch.bincount(rows1, minlength=B)
-            slots1 = assign(depth, cnt1)
+        up = HostArrays()
+        sel_t, done_t, done_rows_t, go_t = (up.put(v, np.int64) for v in (sel, done_last, seq[sel[done_last]], go))
+        more = self.max_iter > 1 and cur.size > 0
+        plan = self._deep_pass(up, depth, cur, seq, pos, bases, counts, B, row_ids) if more else None
+        up.send(dev)
+        logits_sel = self._lm_head(hn.index_select(0, sel_t()))
+        if done_last.size:
+            final_last_logits.index_copy_(0, done_rows_t(), logits_sel.index_select(0, done_t()))
+        cur_cum = logits_sel.index_select(0, go_t()) if more else None        # cumulative logits of the current set
+        while plan is not None:
+            n1 = cur.size
             val = torch.zeros(n1, self.topk, dtype=torch.float32, device=dev)
             idx = torch.zeros(n1, self.topk, dtype=torch.int32, device=dev)
             self._topk(cur_cum, self.topk, None, val, idx)
             x1 = K.soft_embed_rows(val, idx, w.embed)
-            pos1 = pos[cur_idx].contiguous()
-            start1 = (torch.cumsum(cnt1, 0) - cnt1).to(torch.int32)
-            rank1 = (torch.arange(n1, device=dev, dtype=torch.int32) - start1[rows1])
-            bases = [b[cur_idx].contiguous() for b in prev_bases] + [start1[rows1].contiguous()]
-            counts = [c[cur_idx].contiguous() for c in prev_counts] + [(rank1 + 1).contiguous()]
-            # shallower segments (1..depth-1) index into the packed arrays of those passes: their
-            # (base, count) were computed against those arrays when the passes ran
-            learned = self.hard_override is None and isinstance(self._decider()[1], (MLPIterDecider, SimpleMLPIterDecider))
             taps1 = {} if learned and depth + 1 < self.max_iter else None
             with nvtx_range(f"prefill/pass{depth}"):
-                hn1, kv1 = self._packed_pass(x1, pos1, depth, slots1, seg_k, seg_v, bases, counts, cnt1, taps_out=taps1)
-            logits1 = self._lm_head(hn1)
-            cum1 = cur_cum + logits1
+                hn1, kv1 = self._packed_pass(x1, plan["pos"](), depth, plan["slots"](), seg_k, seg_v, [t() for t in plan["bases"]],
+                                             [t() for t in plan["counts"]], plan["seq_counts"](), taps_out=taps1, tiles=[t() for t in plan["tiles"]])
+            cum1 = cur_cum + self._lm_head(hn1)
             if taps1 is not None:
                 # a learned decider is asked again after every pass, on this pass's hidden states and the cumulative
                 # logits, as the model's forward and the decode tick do (reference tah_model.py:625-645)
@@ -403,27 +437,50 @@ class TaHEngine(DecodeEngine):
                 if isinstance(inner, MLPIterDecider):
                     tv = torch.zeros(n1, inner.topk, dtype=torch.float32, device=dev)
                     self._topk(cum1, inner.topk, None, tv, torch.zeros(n1, inner.topk, dtype=torch.int32, device=dev))
-                z1 = self._score(tcat, tv)
-                want_more = torch.sigmoid(z1) > self._thr
+                want_more = (torch.sigmoid(self._score(tcat, tv)) > self._thr).cpu().numpy()
             else:
-                want_more = (extra[cur_idx] > depth) & (depth + 1 < self.max_iter)
-            fin = ~want_more
-            lastfin = fin & is_last[cur_idx]
-            final_last_logits[rows1[lastfin]] = cum1[lastfin]
+                want_more = (extra[cur] > depth) & (depth + 1 < self.max_iter)
+            lastfin, go = np.flatnonzero(~want_more & is_last[cur]), np.flatnonzero(want_more)
             # next pass: subset of this one; its view of this pass's segment
             seg_k.append([k for k, _ in kv1])
             seg_v.append([v for _, v in kv1])
-            full_b = torch.zeros(n0, dtype=torch.int32, device=dev)
-            full_c = torch.zeros(n0, dtype=torch.int32, device=dev)
-            full_b[cur_idx] = bases[-1]
-            full_c[cur_idx] = counts[-1]
-            prev_bases.append(full_b)
-            prev_counts.append(full_c)
-            cur_idx = cur_idx[want_more]
-            cur_cum = cum1[want_more]
+            for full, here in ((bases, plan["own_base"]), (counts, plan["own_count"])):
+                f = np.zeros(n0, np.int64)
+                f[cur] = here
+                full.append(f)
+            up = HostArrays()
+            last_t, last_rows_t, go_t = (up.put(v, np.int64) for v in (lastfin, seq[cur[lastfin]], go))
+            cur = cur[go]
             depth += 1
+            plan = self._deep_pass(up, depth, cur, seq, pos, bases, counts, B, row_ids) if depth < self.max_iter and cur.size else None
+            up.send(dev)
+            if lastfin.size:
+                final_last_logits.index_copy_(0, last_rows_t(), cum1.index_select(0, last_t()))
+            if plan is not None:
+                cur_cum = cum1.index_select(0, go_t())
         del seg_k, seg_v
-        return final_last_logits, lens, iter_extra_prompt
+        return final_last_logits, lens(), extra_t.clone()
+
+    def _assign_pages(self, up: "HostArrays", depth: int, counts, row_ids):
+        """Pages of ``counts [B]`` entries per row at ``depth``; the slots of the entries as an array of ``up``."""
+        if row_ids is not None:
+            slots = self.kv.assign_rows(depth, row_ids, torch.from_numpy(counts))
+            return lambda: slots
+        table, slots = self.kv.assign_fresh(depth, counts)
+        table, held, slots = up.put(table, np.int32), up.put(counts, np.int32), up.put(slots, np.int32)
+        up.then(lambda: (self.kv.page_table[depth].copy_(table().view_as(self.kv.page_table[depth])), self.kv.len[depth].copy_(held())))
+        return slots
+
+    def _deep_pass(self, up: "HostArrays", depth: int, cur, seq, pos, bases, counts, B: int, row_ids) -> dict:
+        """What the pass at ``depth`` over the packed tokens ``cur`` needs, as arrays of ``up``."""
+        rows1 = seq[cur]
+        cnt1 = np.bincount(rows1, minlength=B).astype(np.int64)
+        start1 = np.cumsum(cnt1) - cnt1
+        rank1 = np.arange(cur.size) - start1[rows1]
+        put = lambda v: up.put(v, np.int32)
+        return dict(slots=self._assign_pages(up, depth, cnt1, row_ids), pos=put(pos[cur]), seq_counts=up.put(cnt1, np.int64), own_base=start1[rows1],
+                    own_count=rank1 + 1, bases=[put(b[cur]) for b in bases] + [put(start1[rows1])],
+                    counts=[put(c[cur]) for c in counts] + [put(rank1 + 1)], tiles=[put(v) for v in K.attn_tiles_host(cnt1)])
 
     def _prompt_extra_passes(self, hn, taps, seq, pos) -> torch.Tensor:
         """How many extra passes each prompt token takes (0 = easy)."""

@@ -26,6 +26,7 @@ from typing import List, Optional, Sequence, Tuple
 
 import os
 
+import numpy as np
 import torch
 
 
@@ -171,6 +172,25 @@ class PagedKVCache:
         j = torch.arange(int(counts.sum()), device=dev) - start[row_of_entry]
         pg = self.page_table[depth][row_of_entry, (j // ps)].long()
         return (pg * ps + j % ps).to(torch.int32)
+
+    def assign_fresh(self, depth: int, counts):
+        """:meth:`assign_prefill` right after :meth:`reset`, when the host knows the free stack: the page table ``[rows, max_pages]`` and the entries'
+        slots as numpy arrays, for the caller to copy into ``page_table`` and ``len``.  ``counts``: numpy, one per row."""
+        ps, pages = self.page_size, self.n_pages[depth]
+        counts = np.asarray(counts, np.int64)
+        need = (counts + ps - 1) // ps
+        total = int(need.sum())
+        if total > pages or int(need.max() if need.size else 0) > self.max_pages[depth]:
+            raise RuntimeError(f"KV pool of depth {depth} too small: need {total} pages, {pages} free")
+        first = np.cumsum(need) - need
+        row_of_page = np.repeat(np.arange(self.rows), need)
+        rank = np.arange(total)
+        table = np.zeros((self.rows, self.max_pages[depth]), np.int32)
+        table[row_of_page, rank - first[row_of_page]] = pages - 1 - rank          # the top of a stack that holds 0, 1, ...
+        self.free_count[depth].fill_(pages - total)
+        row_of_entry = np.repeat(np.arange(self.rows), counts)
+        j = np.arange(int(counts.sum())) - (np.cumsum(counts) - counts)[row_of_entry]
+        return table, table[row_of_entry, j // ps].astype(np.int64) * ps + j % ps
 
     def assign_rows(self, depth: int, rows: torch.Tensor, counts: torch.Tensor) -> torch.Tensor:
         """Like :meth:`assign_prefill` for a subset of rows (request admission while other rows keep decoding):

@@ -14,6 +14,7 @@ import functools
 import os
 from typing import List, Optional, Sequence
 
+import numpy as np
 import torch
 
 _LIB = None
@@ -1544,6 +1545,18 @@ def attn_tiles(seq_counts: torch.Tensor, tile: int = 128, by_work: bool = False)
     q0 = (torch.cumsum(cnt, 0) - cnt)[seq_of] + tile * rank
     qn = torch.clamp(cnt[seq_of] - tile * rank, max=tile)
     return q0.to(torch.int32).contiguous(), qn.to(torch.int32).contiguous()
+
+
+def attn_tiles_host(counts, tile: int = 128):
+    """:func:`attn_tiles` by work, of host counts (numpy) and as numpy arrays."""
+    cnt = np.asarray(counts, np.int64)
+    per = (cnt + tile - 1) // tile
+    seq_of = np.repeat(np.arange(cnt.size), per)
+    rank = np.arange(int(per.sum())) - (np.cumsum(per) - per)[seq_of]
+    if cnt.size > 1:
+        order = np.argsort(rank, kind="stable")
+        rank, seq_of = rank[order], seq_of[order]
+    return (np.cumsum(cnt) - cnt)[seq_of] + tile * rank, np.minimum(cnt[seq_of] - tile * rank, tile)
 
 
 def prefill_heads(n_tiles: int, nq: int, nkv: int, hd: int, n_seg: int, keys: int, seqs: int) -> int:

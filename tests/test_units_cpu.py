@@ -487,3 +487,35 @@ def test_persistent_tile_plan():
     # one token tile: the wide SwiGLU and the head, which one tile per CTA does in an uneven wave or several
     assert cuda.plan_persist(256, 12288, 2048, 64, True) == 192 and cuda.plan_persist(256, 151936, 2048) in (192, 256)
     assert not any(cuda.plan_persist(M, rows, 2048) for M in (129, 192, 256) for rows in (1024, 2048, 4096))
+
+
+def test_host_plan_of_a_prefill_is_the_device_one():
+    """Query tiles and page assignment of a prefill worked out on the host: what the tensor operations give, over row counts and lengths
+    (empty rows, whole pages, one past them), and the same refusal of a pool that is too small."""
+    import numpy as np
+    import torch
+    from tah_b200.engine.kv_cache import CacheGeometry, PagedKVCache
+    from tah_b200.ops import cuda
+    gen = torch.Generator().manual_seed(0)
+    for rows in (1, 2, 7, 40):
+        counts = torch.randint(0, 400, (rows,), generator=gen)
+        counts[0], counts[-1] = 128, 129
+        want = cuda.attn_tiles(counts, by_work=True)
+        got = cuda.attn_tiles_host(counts.numpy())
+        assert all(torch.equal(a, torch.from_numpy(b).int()) for a, b in zip(want, got))
+        kv = PagedKVCache(CacheGeometry(1, 1, 64, 16), rows, 400, 2, 0.5, "cpu")
+        for depth in (0, 1):
+            c = counts // (1 + 3 * depth)
+            slots = kv.assign_prefill(depth, c)
+            table, free = kv.page_table[depth].clone(), kv.free_count[depth].clone()
+            kv.reset()
+            t, s = kv.assign_fresh(depth, c.numpy())
+            assert torch.equal(table, torch.from_numpy(t)) and torch.equal(slots, torch.from_numpy(s).int()) and torch.equal(free, kv.free_count[depth])
+            kv.reset()
+        for call in (lambda: kv.assign_prefill(0, counts * 50), lambda: kv.assign_fresh(0, counts.numpy() * 50)):
+            try:
+                call()
+                raise AssertionError("accepted")
+            except RuntimeError as e:
+                assert "too small" in str(e)
+        kv.reset()
