@@ -135,9 +135,19 @@ def plan_gemm(M: int, F: int, K: int, R: int = 0, dual: bool = False):
     return _gemm_cost(M, F, K, R, dual)[1:]
 
 
+def _gemm_forms(M: int, F: int, K: int, R: int, nacc: int):
+    """``(bn, splits, CTAs)`` that the one-tile form of up to 256 tokens has."""
+    kb = K // 64 + R // 64
+    base = 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128 if M <= 128 else 256
+    for bn in [base] + ([128, 64] if base == 256 else [64] if base == 128 else []):
+        for s in (1, 2, 4):
+            if s == 1 or (kb // s >= 2 and _fits(bn, s, nacc)):
+                yield bn, s, ((F + 127) // 128) * ((M + bn - 1) // bn) * s
+
+
 @functools.lru_cache(maxsize=4096)
-def _gemm_cost(M: int, F: int, K: int, R: int = 0, dual: bool = False):
-    """``(microseconds, bn, splits)`` by a small cost model.
+def _gemm_cost(M: int, F: int, K: int, R: int = 0, dual: bool = False, splits: int = 0):
+    """``(microseconds, bn, splits)`` by a small cost model; ``splits``: only forms with so many.
 
     One accumulator, measured at 40 to 256 tokens, weights of 2048 to 151936 rows and reductions of 2048 and 6144 out of HBM: a block of 64 of the
     reduction takes 0.195, 0.25 or 0.33 us for tiles of up to 64, 128 or 256 tokens, start and epilogue 2.4 us and 8 ns a token, the exchange of two
@@ -145,28 +155,35 @@ def _gemm_cost(M: int, F: int, K: int, R: int = 0, dual: bool = False):
     9.4 / 8.5, 2048 x 2048 at 256 9.5 / 8.4.  Two accumulators: 0.3 us a block, unless the tile's tensor time is longer."""
     nacc = 2 if dual else 1
     kb = K // 64 + R // 64
-    base = 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128 if M <= 128 else 256
-    cands = [base] + ([128, 64] if base == 256 else [64] if base == 128 else [])
     best = None
-    for bn in cands:
-        for s in (1, 2, 4):
-            if s > 1 and (kb // s < 2 or not _fits(bn, s, nacc)):
-                continue
-            ctas = ((F + 127) // 128) * ((M + bn - 1) // bn) * s
-            per = bn // s
-            if nacc == 1:
-                waves = -(-ctas // (CLUSTER4_CTAS if s == 4 else SM_COUNT))
-                t_cta = kb / s * (0.195 if bn <= 64 else 0.25 if bn == 128 else 0.33) + 2.4 + 0.008 * bn
-                t_cta += {1: 0.0, 2: 1.0 + 0.0065 * bn, 4: 1.2 + 0.02 * bn}[s]
-            else:
-                waves = -(-ctas // SM_COUNT)
-                t_cta = kb / s * max(0.30, 128 * bn * 64 * 2 * nacc / 8192 / 1900.0) + 0.5 + 0.009 * per
-                if s > 1:
-                    t_cta += 1.0 + (s - 1) * per * nacc * 0.5 / 19.0 + 0.07 * per          # KiB sent to the peers through DSMEM
-            t = waves * t_cta
-            if best is None or t < best[0] - 1e-9:
-                best = (t, bn, s)
+    for bn, s, ctas in _gemm_forms(M, F, K, R, nacc):
+        if splits and s != splits:
+            continue
+        if nacc == 1:
+            waves = -(-ctas // (CLUSTER4_CTAS if s == 4 else SM_COUNT))
+            t = kb / s * (0.195 if bn <= 64 else 0.25 if bn == 128 else 0.33) + 2.4 + 0.008 * bn + {1: 0.0, 2: 1.0 + 0.0065 * bn, 4: 1.2 + 0.02 * bn}[s]
+        else:
+            waves, t = -(-ctas // SM_COUNT), _block_cost(bn, s, kb, nacc)
+        if best is None or waves * t < best[0] - 1e-9:
+            best = (waves * t, bn, s)
     return best
+
+
+def _block_cost(bn: int, s: int, kb: int, nacc: int) -> float:
+    """Microseconds of a CTA with stages of one block of 64 of the reduction: 0.3 us each unless the tensor time is longer."""
+    per = bn // s
+    t = kb / s * max(0.30, 128 * bn * 64 * 2 * nacc / 8192 / 1900.0) + 0.5 + 0.009 * per
+    return t if s == 1 else t + 1.0 + (s - 1) * per * nacc * 0.5 / 19.0 + (0.07 * per if nacc == 2 else 0.0)    # KiB sent through DSMEM
+
+
+@functools.lru_cache(maxsize=4096)
+def plan_gemm_kept(M: int, F: int, K: int, R: int = 0):
+    """:func:`plan_gemm` with the split that stages of one block of the reduction would take.  The split decides how sums are rounded, and
+    the gradients of an adapter that few tokens take are far apart in size: weights that training changes keep it, so that a step's rounding
+    does not follow the tuning of this kernel."""
+    split = min((-(-ctas // SM_COUNT) * _block_cost(bn, s, K // 64 + R // 64, 1), i, s)
+                for i, (bn, s, ctas) in enumerate(_gemm_forms(M, F, K, R, 1)))[2]
+    return _gemm_cost(M, F, K, R, False, split)[1:]
 
 
 # the two-tile ("pair") GEMM is a candidate above 256 tokens; TAH_B200_GEMM_PAIR=0 turns it off
@@ -286,7 +303,7 @@ def wait_flags(flags: torch.Tensor, targets: torch.Tensor) -> None:
 
 
 def _plan_tiles(M: int, rows: int, K: int, R: int, swiglu: bool, gelu: bool, swiglu_interleaved: bool, pair=None, bn: int = 0, splits=None,
-                stores=()):
+                stores=(), kept: bool = False):
     """``(pair, bn, splits)`` of a tcgen05 product with a weight of ``rows`` rows.  ``stores``: the output and the residual where there is
     one; the pair form can only move them as whole tiles (:func:`_whole_pieces`)."""
     can_pair = not swiglu and not gelu and rows % 256 == 0
@@ -303,7 +320,7 @@ def _plan_tiles(M: int, rows: int, K: int, R: int, swiglu: bool, gelu: bool, swi
         if bn == 0:
             bn = 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128 if M <= 128 else 256
     elif splits is None and bn == 0:
-        bn, splits = plan_gemm(M, rows // 2 if swiglu else rows, K, R, swiglu)
+        bn, splits = plan_gemm_kept(M, rows, K, R) if kept and not swiglu else plan_gemm(M, rows // 2 if swiglu else rows, K, R, swiglu)
     elif splits is None:
         splits = 1
     return pair, bn, splits
@@ -366,10 +383,10 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
     if (pair is None and bn == 0 and splits is None and tp_push is None and not swiglu and not (gelu and residual is not None) and
             _persist_ok(x, w, out, residual, x2, w2)):
         bn = plan_persist(M, F, K, R, swiglu_interleaved)
-        if bn:
+        if bn and (M > 256 or const_w or swiglu_interleaved or plan_gemm_kept(M, F, K, R)[1] == 1):
             return _gemm_persist(x, w, out, residual, x2, w2, 1 if gelu else 2 if swiglu_interleaved else 0, bn, tp_wait=tp_wait)
     pair, bn, splits = _plan_tiles(M, w.shape[0], K, R, swiglu, gelu, swiglu_interleaved, pair, bn, splits,
-                                   () if tp_push is not None else (out, residual))
+                                   () if tp_push is not None else (out, residual), kept=not const_w and tp_push is None and tp_wait is None)
     args = (_p(w), _p(x), _p(out), _p(residual), _p(w2), _p(x2), c_int(M), c_int(F), c_int(K), c_int(R),
             c_ll(w.stride(0)), c_ll(x.stride(0)), c_ll(out.stride(0)),
             c_ll(residual.stride(0) if residual is not None else 0),
@@ -536,7 +553,7 @@ def gemm_t(x: torch.Tensor, w: torch.Tensor, *, x_t: bool = False, w_t: bool = F
     if pair:
         bn, splits = bn or 256, 1
     elif splits is None and bn == 0:
-        bn, splits = plan_gemm(M, F, (Kx + 63) // 64 * 64, 0, False)
+        bn, splits = plan_gemm_kept(M, F, (Kx + 63) // 64 * 64)
         if x_t:
             bn = max(bn, 64)
     elif splits is None:
