@@ -230,13 +230,39 @@ __global__ void __launch_bounds__(RN_THREADS) embed_norm_kernel(const T* __restr
   }
 }
 
+// f(j, e) for the rows slot[j] of y_ex, j = 0 .. top - 1 in order: e: this thread's pieces of the row.  Row numbers eight at a time and the rows
+// four at a time on their way together: one after the other (a number, then a row) the loads of eight experts were two thirds of a seam of 12
+// tokens (8.3 us).
+// Without __restrict__: loads that the compiler may take for constant may move ahead of the dependency wait.
+template <typename T, int VPT, typename F>
+__device__ __forceinline__ void for_experts(const T* y_ex, const int* slot, int top, int ld, int nvec, const F& f) {
+  constexpr int G = VPT <= 4 ? 4 : 1;
+  for (int j0 = 0; j0 < top; j0 += 8) {
+    int s[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s[u] = slot[min(j0 + u, top - 1)];
+#pragma unroll
+    for (int u0 = 0; u0 < 8; u0 += G) {
+      if (j0 + u0 >= top) break;
+      float4 e[G][VPT];
+#pragma unroll
+      for (int u = 0; u < G; ++u)
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) {
+          const int c = threadIdx.x + i * RN_THREADS;
+          e[u][i] = c < nvec ? Vec4<T>::load(y_ex + (size_t)s[u0 + u] * ld + c * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+      for (int u = 0; u < G; ++u)
+        if (j0 + u0 + u < top) f(j0 + u0 + u, e[u]);
+    }
+  }
+}
+
 // y_ex / slot: expert outputs [list rows, ld] and the list rows slot[row * top ..] of this token, or null
 template <typename T, int VPT>
-__global__ void __launch_bounds__(RN_THREADS) residual_add_norm_kernel(const T* __restrict__ y, long long ldy,
-                                                                       const T* __restrict__ y_ex,
-                                                                       const int* __restrict__ slot, int top, float mult,
-                                                                       float* __restrict__ x, const float* __restrict__ w_next,
-                                                                       T* __restrict__ h, int width, int groups, int ld,
+__global__ void __launch_bounds__(RN_THREADS) residual_add_norm_kernel(const T* y, long long ldy, const T* y_ex, const int* slot,
+                                                                       int top, float mult, float* x, const float* w_next, T* h, int width, int groups, int ld,
                                                                        float eps) {
   pdl_launch_dependents();
   pdl_wait();
@@ -247,26 +273,20 @@ __global__ void __launch_bounds__(RN_THREADS) residual_add_norm_kernel(const T* 
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int c = threadIdx.x + i * RN_THREADS;
-    if (c < nvec) r[i] = Vec4<T>::load(y + row * ldy + c * 4);
-  }
-  if (y_ex != nullptr) {
-    for (int j = 0; j < top; ++j) {
-      const T* src = y_ex + (size_t)slot[row * top + j] * ld;
-#pragma unroll
-      for (int i = 0; i < VPT; ++i) {
-        const int c = threadIdx.x + i * RN_THREADS;
-        if (c < nvec) {
-          const float4 e = Vec4<T>::load(src + c * 4);
-          r[i].x += e.x; r[i].y += e.y; r[i].z += e.z; r[i].w += e.w;
-        }
-      }
+    if (c < nvec) {
+      r[i] = Vec4<T>::load(y + row * ldy + c * 4);
+      v[i] = Vec4<float>::load(x + row * ld + c * 4);
     }
   }
+  if (y_ex != nullptr)
+    for_experts<T, VPT>(y_ex, slot + row * top, top, ld, nvec, [&](int, const float4 (&e)[VPT]) {
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) { r[i].x += e[i].x; r[i].y += e[i].y; r[i].z += e[i].z; r[i].w += e[i].w; }
+    });
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int c = threadIdx.x + i * RN_THREADS;
     if (c < nvec) {
-      v[i] = Vec4<float>::load(x + row * ld + c * 4);
       v[i].x = fmaf(mult, r[i].x, v[i].x); v[i].y = fmaf(mult, r[i].y, v[i].y);
       v[i].z = fmaf(mult, r[i].z, v[i].z); v[i].w = fmaf(mult, r[i].w, v[i].w);
       Vec4<float>::store(x + row * ld + c * 4, v[i]);
@@ -322,21 +342,15 @@ __global__ void __launch_bounds__(RN_THREADS) streams_norm_kernel(const StreamsP
       r[i].x += b.x; r[i].y += b.y; r[i].z += b.z; r[i].w += b.w;
     }
   }
-  if (p.y_ex != nullptr) {
-    for (int j = 0; j < p.top; ++j) {
-      const T* src = reinterpret_cast<const T*>(p.y_ex) + (size_t)p.slot[row * p.top + j] * p.ld;
+  if (p.y_ex != nullptr)
+    for_experts<T, VPT>(reinterpret_cast<const T*>(p.y_ex), p.slot + row * p.top, p.top, p.ld, nvec, [&](int j, const float4 (&e)[VPT]) {
       const float w = p.y_weight != nullptr ? p.y_weight[row * p.top + j] : 1.0f;
 #pragma unroll
       for (int i = 0; i < VPT; ++i) {
-        const int c = threadIdx.x + i * RN_THREADS;
-        if (c < nvec) {
-          const float4 e = Vec4<T>::load(src + c * 4);
-          r[i].x = fmaf(w, e.x, r[i].x); r[i].y = fmaf(w, e.y, r[i].y);
-          r[i].z = fmaf(w, e.z, r[i].z); r[i].w = fmaf(w, e.w, r[i].w);
-        }
+        r[i].x = fmaf(w, e[i].x, r[i].x); r[i].y = fmaf(w, e[i].y, r[i].y);
+        r[i].z = fmaf(w, e[i].z, r[i].z); r[i].w = fmaf(w, e[i].w, r[i].w);
       }
-    }
-  }
+    });
   float mix[S][S], out[S], in[S];
 #pragma unroll
   for (int s = 0; s < S; ++s) {
@@ -410,13 +424,27 @@ struct ResidualNormParams {
 };
 
 // CENTER: layer norms; ENTER: add / E / before may be given
+// The norms' weights are read ahead of the dependency wait where they fit the registers: behind each reduction their latency stood in the
+// open, twice in a launch of 5.6 us (50 tokens).
 template <typename T, int VPT, bool CENTER, bool ENTER>
 __global__ void __launch_bounds__(RN_THREADS) residual_norm_kernel(const ResidualNormParams p) {
   pdl_launch_dependents();
-  pdl_wait();
   __shared__ float red[4];
   const size_t row = blockIdx.x;
   const int nvec = p.ld / 4;
+  constexpr bool AHEAD = VPT <= 4;
+  float4 wo[AHEAD ? VPT : 1], wn[AHEAD ? VPT : 1];
+  if constexpr (AHEAD) {
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int c = threadIdx.x + i * RN_THREADS;
+      if (c < nvec) {
+        wo[i] = Vec4<float>::load(p.w_out + c * 4);
+        wn[i] = Vec4<float>::load(p.w_next + c * 4);
+      }
+    }
+  }
+  pdl_wait();
   const T* y = reinterpret_cast<const T*>(p.y) + row * p.ldy;
   float* x = p.x + row * p.ld;
   float4 u[VPT], v[VPT];
@@ -433,7 +461,7 @@ __global__ void __launch_bounds__(RN_THREADS) residual_norm_kernel(const Residua
   for (int i = 0; i < VPT; ++i) {
     const int c = threadIdx.x + i * RN_THREADS;
     if (c < nvec) {
-      const float4 g = Vec4<float>::load(p.w_out + c * 4);
+      const float4 g = AHEAD ? wo[AHEAD ? i : 0] : Vec4<float>::load(p.w_out + c * 4);
       if constexpr (CENTER) { u[i].x -= ny.x; u[i].y -= ny.x; u[i].z -= ny.x; u[i].w -= ny.x; }
       v[i].x += u[i].x * ny.y * g.x; v[i].y += u[i].y * ny.y * g.y; v[i].z += u[i].z * ny.y * g.z; v[i].w += u[i].w * ny.y * g.w;
       if constexpr (ENTER) {
@@ -457,7 +485,7 @@ __global__ void __launch_bounds__(RN_THREADS) residual_norm_kernel(const Residua
   for (int i = 0; i < VPT; ++i) {
     const int c = threadIdx.x + i * RN_THREADS;
     if (c < nvec) {
-      const float4 g = Vec4<float>::load(p.w_next + c * 4);
+      const float4 g = AHEAD ? wn[AHEAD ? i : 0] : Vec4<float>::load(p.w_next + c * 4);
       if constexpr (CENTER) { v[i].x -= nx.x; v[i].y -= nx.x; v[i].z -= nx.x; v[i].w -= nx.x; }
       Vec4<T>::store(reinterpret_cast<T*>(p.h) + row * p.ld + c * 4,
                      make_float4(v[i].x * nx.y * g.x, v[i].y * nx.y * g.y, v[i].z * nx.y * g.z, v[i].w * nx.y * g.w));
@@ -510,14 +538,16 @@ __global__ void __launch_bounds__(FL_THREADS) few_linear_kernel(const T* __restr
 // bf16 operands: far too few features for a tcgen05 tile, so warp-level m16n8k16 products with fp32 sums.  A CTA owns 16
 // tokens and up to 32 features; its 8 warps split K.  A lane fetches 8 consecutive k of its rows with one 16-byte load:
 // which k sit in which register slot does not matter as long as x and w agree.
-constexpr int FLM_NT = 4;                  // feature tiles of 8 per CTA
-__global__ void __launch_bounds__(FL_THREADS) few_linear_mma_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
+// For few tokens (NT = 1): 8 features and 16 warps a CTA, each of which has all it reads on its way at once; 32 features of 12 tokens in a CTA
+// of 8 warps made the router of 64 experts two CTAs with four round trips (12 x 64 x 2048 9.6 us in a tick).
+template <int FLM_NT, int FLM_WARPS>       // feature tiles of 8 and warps of a CTA
+__global__ void __launch_bounds__(FLM_WARPS * 32) few_linear_mma_kernel(const __nv_bfloat16* x, long long ldx,
                                                                     const __nv_bfloat16* __restrict__ w,
                                                                     const float* __restrict__ b, float* __restrict__ out,
                                                                     int M, int K, int F) {
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ float part[FL_THREADS / 32][16][FLM_NT * 8 + 1];
+  __shared__ float part[FLM_WARPS][16][FLM_NT * 8 + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   const int t0 = blockIdx.x * 16, f0 = blockIdx.y * FLM_NT * 8;
   const int nt = min(FLM_NT, (F - f0 + 7) / 8);
@@ -532,7 +562,7 @@ __global__ void __launch_bounds__(FL_THREADS) few_linear_mma_kernel(const __nv_b
     for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
   }
 #pragma unroll 4
-  for (int k = warp * 32; k < K; k += FL_THREADS) {
+  for (int k = warp * 32; k < K; k += FLM_WARPS * 32) {
     const uint4 a = *reinterpret_cast<const uint4*>(x0 + k), c = *reinterpret_cast<const uint4*>(x1 + k);
 #pragma unroll
     for (int j = 0; j < FLM_NT; ++j) {
@@ -555,11 +585,11 @@ __global__ void __launch_bounds__(FL_THREADS) few_linear_mma_kernel(const __nv_b
     part[warp][g + 8][j * 8 + q * 2 + 1] = acc[j][3];
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 16 * nt * 8; i += FL_THREADS) {
+  for (int i = threadIdx.x; i < 16 * nt * 8; i += FLM_WARPS * 32) {
     const int r = i / (nt * 8), f = i % (nt * 8);
     float s = 0.f;
 #pragma unroll
-    for (int k = 0; k < FL_THREADS / 32; ++k) s += part[k][r][f];
+    for (int k = 0; k < FLM_WARPS; ++k) s += part[k][r][f];
     if (t0 + r < M && f0 + f < F) out[(size_t)(t0 + r) * F + f0 + f] = s + (b != nullptr ? b[f0 + f] : 0.f);
   }
 }
@@ -796,9 +826,13 @@ extern "C" int tahb_few_linear(const void* x, long long ldx, const void* w, cons
     return one ? few_linear_launch<float, 1>(x, ldx, w, b, out, M, K, F, stream)
                : few_linear_launch<float, 4>(x, ldx, w, b, out, M, K, F, stream);
   if (K % 32 || ldx % 8) return -1;
-  const dim3 grid((M + 15) / 16, (F + FLM_NT * 8 - 1) / (FLM_NT * 8));
-  cudaError_t rc = launch_chain(few_linear_mma_kernel, grid, dim3(FL_THREADS), 0, stream, reinterpret_cast<const __nv_bfloat16*>(x),
-                                ldx, reinterpret_cast<const __nv_bfloat16*>(w), b, out, M, K, F);
+  // eight features a CTA while that is one wave
+  const int tokens = (M + 15) / 16;
+  auto xx = reinterpret_cast<const __nv_bfloat16*>(x);
+  auto ww = reinterpret_cast<const __nv_bfloat16*>(w);
+  cudaError_t rc = (long long)tokens * ((F + 7) / 8) <= 148
+                       ? launch_chain(few_linear_mma_kernel<1, 16>, dim3(tokens, (F + 7) / 8), dim3(512), 0, stream, xx, ldx, ww, b, out, M, K, F)
+                       : launch_chain(few_linear_mma_kernel<4, 8>, dim3(tokens, (F + 31) / 32), dim3(256), 0, stream, xx, ldx, ww, b, out, M, K, F);
   return rc == cudaSuccess ? 0 : -3;
 }
 

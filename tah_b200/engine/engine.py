@@ -544,7 +544,7 @@ class TaHEngine(DecodeEngine):
         s.logits, s.cum = bf(B, w.vocab_shard[2]), bf(B, w.vocab_shard[2])
         s.topv = torch.zeros(B, self.topk, dtype=torch.float32, device=dev)
         s.topi = i32(B, self.topk)
-        s.few_sync = self._few_sync = i32(2)
+        s.few_sync = i32(2)
         tl = self._tap_layers()
         # the learned decider's Linear(topk -> H) output is written behind the tapped hidden states
         tap_w = (max(1, len(tl)) + (1 if self._needs_topk_for_decider() else 0)) * H
@@ -560,20 +560,21 @@ class TaHEngine(DecodeEngine):
         return s
 
     def _row_parallel(self, x, w_, a_, b_, t_buf, gate, h, ln_w, xn_out, M, push=False, final=False, next_lora=None,
-                      tap=None):
+                      tap=None, sync=None):
         """Row-parallel projection + residual + the RMSNorm that follows it.
 
         One GPU: the GEMM epilogue adds the residual in place and a norm kernel follows.  Tensor
         parallel: the GEMM writes this rank's partial result into symmetric memory and the fused
         NVLink kernel does all-reduce + residual + norm + broadcast; ``h`` stays row-sharded.
         ``next_lora = (A, t_buf)`` (one GPU, decode): fuse the LoRA-A product of the consumer of ``xn`` into the
-        norm launch.  ``tap = (tap buffer, column)`` (push path): the owner kernel also broadcasts the updated
+        norm launch.  ``sync`` (a tick's two counters): in ticks of few rows the product forms
+        the gated rows' LoRA-A itself.  ``tap = (tap buffer, column)`` (push path): the owner kernel also broadcasts the updated
         residual rows into that column of every rank's tap buffer."""
         cfg, tp = self.cfg, self.tp
         lora = a_ is not None and t_buf is not None
-        if lora and tp is None and gate is not None and next_lora is None and K.few_gated_fits(x, w_, h, M):
+        if lora and tp is None and sync is not None and next_lora is None and K.few_gated_fits(x, w_, h, M):
             # few rows: the product forms the gated rows' adapter input itself
-            K.gemm_few_fused(x, w_, h, gate, self._few_sync, lora=(a_, t_buf, b_), residual=h)
+            K.gemm_few_fused(x, w_, h, gate, sync, lora=(a_, t_buf, b_), residual=h)
             return K.rms_norm(h, ln_w, cfg.rms_norm_eps, out=xn_out)
         if lora:
             if gate is not None:
@@ -682,7 +683,7 @@ class TaHEngine(DecodeEngine):
             K.decode_attn(s.q, pools[li], kv.page_table, kv.len, s.depth, nq, nkv, hd, self.page_size, scale, out=s.o,
                           n_split=s.attn_split, ws=s.attn_ws)
             xn = self._row_parallel(s.o, L.w_o, L.a_o if lora else None, L.b_o, s.t_o, s.gate, s.h, L.ln2, s.xn, B,
-                                    push=push, next_lora=(L.a_gu, s.t_gu) if fuse_norm_lora else None)
+                                    push=push, next_lora=(L.a_gu, s.t_gu) if fuse_norm_lora else None, sync=s.few_sync)
             if lora and not fuse_norm_lora:
                 K.lora_a_rows(xn, L.a_gu, s.gate, out=s.t_gu, tp_wait=self._xn_wait, const_w=True)
             sw = dict(swiglu_interleaved=True, const_w=True) if w.gu_interleaved else dict(swiglu=True, const_w=True)
@@ -695,7 +696,7 @@ class TaHEngine(DecodeEngine):
             # a tap of the next layer's input is this projection's updated residual stream
             tap = (s.tap_buf, tl.index(li + 1) * H) if kernel_taps and li + 1 < nL and (li + 1) in tl else None
             xn = self._row_parallel(s.act, L.w_down, L.a_down if lora else None, L.b_down, s.t_down, s.gate, s.h,
-                                    next_ln, s.xn, B, push=push, final=li + 1 == nL, next_lora=nxt_lora, tap=tap)
+                                    next_ln, s.xn, B, push=push, final=li + 1 == nL, next_lora=nxt_lora, tap=tap, sync=s.few_sync)
         if few:
             xn = K.rms_norm(s.h, w.final_norm, cfg.rms_norm_eps, out=s.xn)
         # xn is now the final-norm output of every row

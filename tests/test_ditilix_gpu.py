@@ -539,3 +539,37 @@ def test_playground_command_line(tmp_path):
     assert r.returncode == 0, r.stderr[-2000:]
     rows = [[int(t) for t in l.split(",")] for l in r.stdout.split()]
     assert len(rows) == 2 and all(_tokens_follow(cfg, sd, p, o, 1e-4) for p, o in zip(prompts, rows))
+
+
+@pytest.mark.parametrize("top", [1, 3, 8, 9])
+@pytest.mark.parametrize("width", [192, 2048, 5056])
+def test_seam_gathers_what_the_launch_before_it_wrote(top, width):
+    """Lists, their gathered rows as expert outputs and the seam that sums them, launched in a row without a pause and with other logits each time:
+    the seam sees the lists of its own round.  Sums of bf16 rows in fp32: bound by their rounding."""
+    from tah_b200.ops import cuda as K
+    g = torch.Generator().manual_seed(top)
+    M, E, n = 12, 16, 12
+    L = K.ExpertLists(M, E, top, BF16, "cuda")
+    zs, hs = torch.randn(n, M, E, generator=g).cuda(), torch.randn(n, M, width, generator=g).to(BF16).cuda()
+    y, w = torch.randn(M, width, generator=g).to(BF16).cuda(), torch.ones(width, device="cuda")
+    lists, h = torch.zeros(L.rows, width, dtype=BF16, device="cuda"), torch.empty(M, width, dtype=BF16, device="cuda")
+    xs = torch.zeros(n, M, width, device="cuda")
+    torch.cuda.synchronize()
+    for i in range(n):
+        K.moe_route(zs[i], L)
+        K.moe_gather(hs[i], L, lists)
+        K.residual_add_norm(y, xs[i], 0.5, w, width, 1, 1e-6, h, lists, L.slot)
+    want = 0.5 * (y.double() + top * hs.double())              # every expert's row is the token's own
+    assert float((xs.double() - want).abs().max()) < 1e-6 * (top + 1) * float(want.abs().max())
+    check_ok()
+
+
+@pytest.mark.parametrize("M,F,K_", [(1, 8, 32), (12, 64, 2048), (50, 16, 2048), (300, 65, 2048), (148 * 16, 9, 544)])
+def test_few_linear_on_both_sides_of_a_wave(M, F, K_):
+    from tah_b200.ops import cuda as K
+    g = torch.Generator().manual_seed(M)
+    x, w, b = torch.randn(M, K_, generator=g).to(BF16), torch.randn(F, K_, generator=g).to(BF16), torch.randn(F, generator=g)
+    got = K.few_linear(x.cuda(), w.cuda(), b.cuda()).cpu().double()
+    part = x.double().abs() @ w.double().abs().T
+    assert bool(((got - x.double() @ w.double().T - b.double()).abs() <= 2.0 ** -20 * part + 1e-6).all())
+    check_ok()
