@@ -636,6 +636,7 @@ class TaHEngine(DecodeEngine):
         # rows the chain of separate launches is faster, also than the QKV epilogue on the GEMM's eight epilogue warps (a generation of 32
         # tokens 205.7 ms, fused 212.2; 20 rows of up to 1900 172.9 and 182.3).
         fuse = _fusions("few" if B <= K.FUSED_TOKENS else "")
+        sync = s.few_sync if "few" in _fusions("few") else None  # up to 32 rows: LoRA-A of the row-parallel projections inside them
         fuse_qkv = "qkv" in fuse and hd == 128                   # QK-norm + RoPE + KV write in the QKV GEMM epilogue
         few = "few" in fuse and tp is None and not fuse_qkv and self._few_fits(B)
         fuse_norm_lora = "lora" in fuse and lora and tp is None and not few  # RMSNorm + LoRA-A of the gated rows in one launch
@@ -683,7 +684,7 @@ class TaHEngine(DecodeEngine):
             K.decode_attn(s.q, pools[li], kv.page_table, kv.len, s.depth, nq, nkv, hd, self.page_size, scale, out=s.o,
                           n_split=s.attn_split, ws=s.attn_ws)
             xn = self._row_parallel(s.o, L.w_o, L.a_o if lora else None, L.b_o, s.t_o, s.gate, s.h, L.ln2, s.xn, B,
-                                    push=push, next_lora=(L.a_gu, s.t_gu) if fuse_norm_lora else None, sync=s.few_sync)
+                                    push=push, next_lora=(L.a_gu, s.t_gu) if fuse_norm_lora else None, sync=sync)
             if lora and not fuse_norm_lora:
                 K.lora_a_rows(xn, L.a_gu, s.gate, out=s.t_gu, tp_wait=self._xn_wait, const_w=True)
             sw = dict(swiglu_interleaved=True, const_w=True) if w.gu_interleaved else dict(swiglu=True, const_w=True)
@@ -696,7 +697,7 @@ class TaHEngine(DecodeEngine):
             # a tap of the next layer's input is this projection's updated residual stream
             tap = (s.tap_buf, tl.index(li + 1) * H) if kernel_taps and li + 1 < nL and (li + 1) in tl else None
             xn = self._row_parallel(s.act, L.w_down, L.a_down if lora else None, L.b_down, s.t_down, s.gate, s.h,
-                                    next_ln, s.xn, B, push=push, final=li + 1 == nL, next_lora=nxt_lora, tap=tap, sync=s.few_sync)
+                                    next_ln, s.xn, B, push=push, final=li + 1 == nL, next_lora=nxt_lora, tap=tap, sync=sync)
         if few:
             xn = K.rms_norm(s.h, w.final_norm, cfg.rms_norm_eps, out=s.xn)
         # xn is now the final-norm output of every row
