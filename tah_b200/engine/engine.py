@@ -74,7 +74,8 @@ class HostArrays:
         for at, a in self._parts:
             view[at:at + a.nbytes] = a.reshape(-1).view(np.uint8)
         self._dev = host.to(device, non_blocking=True)
-        for f in self._after:
+        after, self._after = self._after, []       # they hold this object and their engine: memory would wait for the cycle collector
+        for f in after:
             f()
 
 

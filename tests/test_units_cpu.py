@@ -519,3 +519,30 @@ def test_host_plan_of_a_prefill_is_the_device_one():
             except RuntimeError as e:
                 assert "too small" in str(e)
         kv.reset()
+
+
+def test_host_arrays_keep_nothing_alive():
+    """Arrays sent in one copy, with what runs behind it: the values arrive, and what the functions hold (an engine and its caches) is freed by
+    the last reference, not by the cycle collector."""
+    import gc
+    import weakref
+    import numpy as np
+    import torch
+    from tah_b200.engine.engine import HostArrays
+
+    class Holder:
+        pass
+
+    holder = Holder()
+    alive = weakref.ref(holder)
+    gc.disable()
+    try:
+        up = HostArrays()
+        a, b = up.put([1, 2, 3], np.int32), up.put(np.arange(5), np.int64)
+        up.then(lambda: setattr(holder, "got", a() + 1))
+        up.send("cpu")
+        assert holder.got.tolist() == [2, 3, 4] and b().tolist() == [0, 1, 2, 3, 4] and b().dtype == torch.int64
+        del holder, up, a, b
+        assert alive() is None
+    finally:
+        gc.enable()
