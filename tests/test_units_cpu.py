@@ -533,16 +533,16 @@ def test_host_arrays_keep_nothing_alive():
     class Holder:
         pass
 
-    holder = Holder()
-    alive = weakref.ref(holder)
-    gc.disable()
-    try:
+    def send(holder):
         up = HostArrays()
         a, b = up.put([1, 2, 3], np.int32), up.put(np.arange(5), np.int64)
         up.then(lambda: setattr(holder, "got", a() + 1))
         up.send("cpu")
         assert holder.got.tolist() == [2, 3, 4] and b().tolist() == [0, 1, 2, 3, 4] and b().dtype == torch.int64
-        del holder, up, a, b
-        assert alive() is None
+        return weakref.ref(holder)
+
+    gc.disable()
+    try:
+        assert send(Holder())() is None
     finally:
         gc.enable()
