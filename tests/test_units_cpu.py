@@ -543,6 +543,7 @@ def test_host_arrays_keep_nothing_alive():
 
     gc.disable()
     try:
-        assert send(Holder())() is None
+        alive = send(Holder())
+        assert alive() is None
     finally:
         gc.enable()
