@@ -374,7 +374,8 @@ __device__ __forceinline__ float silu(float x) { return __fdividef(x, 1.0f + __e
 template <int EPL, bool WIDE>
 struct alignas(EPL * 2) QkvPiece {
   __nv_bfloat16 v[EPL];
-  using Word = typename std::conditional<EPL == 4, uint2, uint32_t>::type;
+  using Word = typename std::conditional<EPL == 8, uint4, typename std::conditional<EPL == 4, uint2, uint32_t>::type>::type;
+  __device__ __forceinline__ __nv_bfloat162& pair(int i) { return reinterpret_cast<__nv_bfloat162*>(v)[i]; }
   __device__ __forceinline__ void load(const __nv_bfloat16* src) {
     if constexpr (WIDE) *reinterpret_cast<Word*>(v) = *reinterpret_cast<const Word*>(src);
     else

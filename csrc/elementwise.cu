@@ -248,82 +248,111 @@ struct QkvRopeParams {
   float eps, log2_theta;
 };
 
-// One CTA per token, several for few tokens; a warp takes QKV_U heads at a time, whose loads are all in flight before the first is used, and
-// the token's sines and cosines are computed once for all of them.  Bound: HBM (at 16384 tokens of 16 + 16 heads: 134 MB in, 134 MB out, of
-// which 67 MB go to the cache as well); with a warp per head, one 8-byte load in flight and sincosf and exp2f in every warp, the
-// instruction issue was: the two passes over seven prompts of up to 3500 tokens 281 us, now 121 us (139 with the sines in every warp);
-// 3072 tokens 19.2 us.  Few tokens leave SMs idle and a warp with four heads in turn: a CTA per token / four of them / a warp per head, 16 + 16
-// heads, back to back: 1 token 2.95 / 2.02 / 2.26 us, 64 3.09 / 2.36 / 3.20, 200 3.43 / 3.70 / 5.33 (two of them: 2.93).
-// WIDE: every pointer and row lies on a boundary of a lane's piece (8 bytes of a head of 128); else element by element.
-constexpr int QKV_U = 4, QKV_WARPS = 8;
+// One CTA per token, two for few tokens; a lane has 8 elements of a head (16 bytes), so that a warp takes two heads of 128 or four of 64, and QKV_U
+// such items at a time, whose loads are all in flight before the first is used; the token's sines and cosines are computed once for all of
+// them.  Bound: HBM (at 16384 tokens of 16 + 16 heads: 134 MB in, 134 MB out, of which 67 MB go to the cache as well: 51 us), in fact the
+// instruction issue: with four elements a lane and 32-bit arithmetic behind the norm 117 us; here the norm's weight, the rotation and their
+// sum are 16-bit operations on pairs (the same bits: products of two 16-bit numbers are exact in 32), the partner's dims come two to a
+// shuffle, and the squares are summed as 32 lanes would: 77 us, 4096 tokens 35 -> 27 us, 1024 14.3 -> 12.3 us.  48 registers (five CTAs an SM):
+// with 64 84 us.  A loop over tokens in four CTAs an SM, the next token's loads ahead, took longer: 131 us with four elements a lane.
+// WIDE: every pointer and row lies on a 16-byte boundary; else element by element.
+constexpr int QKV_U = 2, QKV_WARPS = 8;
 template <int HD, bool WIDE>
-__global__ void __launch_bounds__(QKV_WARPS * 32) qk_norm_rope_kv_kernel(const QkvRopeParams p) {
+__global__ void __launch_bounds__(QKV_WARPS * 32, 5) qk_norm_rope_kv_kernel(const QkvRopeParams p) {
   pdl_wait();
-  constexpr int EPL = HD / 32;  // elements per lane
-  using Piece = QkvPiece<EPL, WIDE>;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int all = p.nq + 2 * p.nkv, per = (all + gridDim.y - 1) / gridDim.y, first = blockIdx.y * per, heads = min(all, first + per);
+  constexpr int LPH = HD / 8, HPW = 32 / LPH;   // lanes of a head, heads of a warp
+  constexpr int CH = HPW;                       // 128: two sums of four squares a lane, 64: four of two
+  using Piece = QkvPiece<8, WIDE>;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, hl = lane / LPH, d0 = lane % LPH * 8;
+  const int all = p.nq + 2 * p.nkv, items = (all + HPW - 1) / HPW, per = (items + gridDim.y - 1) / gridDim.y;
+  const int first = blockIdx.y * per, end = min(items, first + per);
   const int t = blockIdx.x;
-  const bool upper = lane >= 16;
-  const __nv_bfloat16* src = p.qkv + (size_t)t * p.ld_qkv + lane * EPL;
+  const __nv_bfloat16* src = p.qkv + (size_t)t * p.ld_qkv + hl * HD + d0;
   Piece in[QKV_U];
+  auto fetch = [&](int it) {
 #pragma unroll
-  for (int u = 0; u < QKV_U; ++u) {
-    const int h = first + warp + u * QKV_WARPS;
-    if (h < heads) in[u].load(src + (size_t)h * HD);
-  }
-  __shared__ float2 s_cs[HD / 2];               // cosine and sine of the token's angles, each computed once
+    for (int u = 0; u < QKV_U; ++u) {
+      const int i = it + u * QKV_WARPS;
+      if (i < end && i * HPW + hl < all) in[u].load(src + (size_t)i * HPW * HD);
+    }
+  };
+#pragma unroll
+  for (int u = 0; u < QKV_U; ++u)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) in[u].pair(i) = __floats2bfloat162_rn(0.f, 0.f);
+  fetch(first + warp);
+  __shared__ __align__(16) __nv_bfloat16 s_cos[HD / 2], s_sin[HD / 2];      // of the token's angles, each computed once
   for (int j = threadIdx.x; j < HD / 2; j += QKV_WARPS * 32) {
     const float ang = (float)p.pos[t] * exp2f(-(2.0f * (float)j / (float)HD) * p.log2_theta);
-    s_cs[j] = make_float2(bf16_round(cosf(ang)), bf16_round(sinf(ang)));
+    s_cos[j] = __float2bfloat16_rn(cosf(ang));
+    s_sin[j] = __float2bfloat16_rn(sinf(ang));
   }
   const int sl = p.slot != nullptr ? p.slot[t] : -1;
   __nv_bfloat16* cache = nullptr;
   if (sl >= 0)
     cache = p.cache[p.cache_sel ? p.cache_sel[t] : 0] + ((size_t)(sl / p.page_size) * 2 * p.nkv * p.page_size + sl % p.page_size) * HD;
   __syncthreads();
-  float2 cs[EPL];
+  QkvPiece<8, true> co, si;                     // frequency of dim d: d mod HD / 2; the lower half takes away the partner's sine
+  co.load(s_cos + d0 % (HD / 2));
+  si.load(s_sin + d0 % (HD / 2));
+  if (d0 < HD / 2) {
 #pragma unroll
-  for (int i = 0; i < EPL; ++i) cs[i] = s_cs[(lane & 15) * EPL + i];      // frequency of dim d: d mod HD / 2
-  for (int h0 = first + warp; h0 < heads; h0 += QKV_U * QKV_WARPS) {
+    for (int i = 0; i < 4; ++i) si.pair(i) = __hneg2(si.pair(i));
+  }
+  for (int it = first + warp; it < end; it += QKV_U * QKV_WARPS) {
 #pragma unroll
     for (int u = 0; u < QKV_U; ++u) {
-      const int h = h0 + u * QKV_WARPS;
-      if (h >= heads) break;
+      const int i = it + u * QKV_WARPS, h = i * HPW + hl;
+      if (i >= end) break;
       const bool is_q = h < p.nq;
       const bool is_k = !is_q && h < p.nq + p.nkv;
       Piece out = in[u];
-      if (is_q || is_k) {
+      if (i * HPW < p.nq + p.nkv) {             // one of the warp's heads is a query or a key
         Piece w;
-        w.load((is_q ? p.q_w : p.k_w) + lane * EPL);
-        float x[EPL], ss = 0.f;
+        w.load((is_q ? p.q_w : p.k_w) + d0);
+        float2 x[4];
+        float ss[CH];
 #pragma unroll
-        for (int i = 0; i < EPL; ++i) {
-          x[i] = __bfloat162float(in[u].v[i]);
-          ss += x[i] * x[i];
+        for (int j = 0; j < 4; ++j) x[j] = __bfloat1622float2(in[u].pair(j));
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+          ss[c] = 0.f;
+#pragma unroll
+          for (int j = c * 4 / CH; j < (c + 1) * 4 / CH; ++j) {
+            ss[c] += x[j].x * x[j].x;
+            ss[c] += x[j].y * x[j].y;
+          }
         }
-        const float rstd = rsqrtf(warp_sum(ss) / (float)HD + p.eps);
+        // in the order of a sum over 32 lanes of HD / 32 elements
 #pragma unroll
-        for (int i = 0; i < EPL; ++i) {
-          const float n = bf16_round(__bfloat162float(w.v[i]) * bf16_round(x[i] * rstd));
-          const float partner = __shfl_xor_sync(0xffffffffu, n, 16);
-          out.v[i] = __float2bfloat16_rn(bf16_round(n * cs[i].x) + bf16_round((upper ? partner : -partner) * cs[i].y));
+        for (int o = LPH / 2; o > 0; o >>= 1)
+#pragma unroll
+          for (int c = 0; c < CH; ++c) ss[c] += __shfl_xor_sync(0xffffffffu, ss[c], o);
+#pragma unroll
+        for (int o = CH / 2; o > 0; o >>= 1)
+#pragma unroll
+          for (int c = 0; c < o; ++c) ss[c] += ss[c + o];
+        const float rstd = rsqrtf(ss[0] / (float)HD + p.eps);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          // products of 16-bit numbers, exact in 32 bits: rounded once either way
+          const __nv_bfloat162 n = __hmul2_rn(w.pair(j), __floats2bfloat162_rn(x[j].x * rstd, x[j].y * rstd));
+          const __nv_bfloat162 partner = __shfl_xor_sync(0xffffffffu, n, LPH / 2);
+          const __nv_bfloat162 r = __hadd2_rn(__hmul2_rn(n, co.pair(j)), __hmul2_rn(partner, si.pair(j)));
+          if (is_q || is_k) out.pair(j) = r;
         }
       }
+      if (h >= all) continue;
       if (is_q) {
-        out.store(p.q_out + ((size_t)t * p.nq + h) * HD + lane * EPL);
+        out.store(p.q_out + ((size_t)t * p.nq + h) * HD + d0);
         continue;
       }
       const int kvh = is_k ? h - p.nq : h - p.nq - p.nkv;
       __nv_bfloat16* dense = is_k ? p.k_dense : p.v_dense;
-      if (dense != nullptr) out.store(dense + ((size_t)t * p.nkv + kvh) * HD + lane * EPL);
-      if (cache != nullptr) out.store(cache + ((size_t)((is_k ? 0 : p.nkv) + kvh) * p.page_size) * HD + lane * EPL);
+      if (dense != nullptr) out.store(dense + ((size_t)t * p.nkv + kvh) * HD + d0);
+      if (cache != nullptr) out.store(cache + ((size_t)((is_k ? 0 : p.nkv) + kvh) * p.page_size) * HD + d0);
     }
-#pragma unroll
-    for (int u = 0; u < QKV_U; ++u) {
-      const int h = h0 + (QKV_U + u) * QKV_WARPS;
-      if (h < heads) in[u].load(src + (size_t)h * HD);
-    }
+    fetch(it + QKV_U * QKV_WARPS);
   }
   pdl_launch_dependents();
 }
@@ -786,8 +815,8 @@ extern "C" int tahb_qk_norm_rope_kv(const void* qkv, const void* q_w, const void
                  reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(k_dense) | reinterpret_cast<uintptr_t>(v_dense) |
                  (uintptr_t)(ld_qkv * 2);
   for (int i = 0; i < n_caches; ++i) at |= reinterpret_cast<uintptr_t>(caches[i]);
-  const bool wide = at % (hd / 16) == 0;
-  const int groups = qk_head_groups(M, nq + 2 * nkv, QKV_WARPS, 4 * 148);
+  const bool wide = at % 16 == 0;
+  const int groups = qk_head_groups(M, (nq + 2 * nkv + 256 / hd - 1) / (256 / hd), QKV_WARPS, 4 * 148);
 #define TAHB_QKV(HD_) (wide ? launch_chain(qk_norm_rope_kv_kernel<HD_, true>, dim3(M, groups), dim3(QKV_WARPS * 32), 0, stream, p) \
                             : launch_chain(qk_norm_rope_kv_kernel<HD_, false>, dim3(M, groups), dim3(QKV_WARPS * 32), 0, stream, p))
   if (hd == 128) e = TAHB_QKV(128);

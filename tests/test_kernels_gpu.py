@@ -1248,6 +1248,31 @@ def test_attention_backward_two_heads_per_cta(hd, nq, nkv):
         Kc.attn_bwd_dq(q, dout, [k], [v], [b], [c], tq0, tqn, nq, nq, hd, hd ** -0.5, lse, dsum, heads=2)
 
 
+@pytest.mark.parametrize("hd,nq,nkv", [(128, 3, 1), (128, 2, 1), (64, 3, 1), (64, 5, 3), (64, 1, 1)])
+@pytest.mark.parametrize("shift", [0, 4])
+def test_qk_norm_rope_heads_that_share_a_warp(hd, nq, nkv, shift):
+    """Queries, keys and values that meet in one warp, and warps that are not full, on and off 16-byte boundaries; 600 tokens: a CTA each."""
+    Kc = _cuda()
+    F = (nq + 2 * nkv) * hd
+    for M in (1, 600):
+        flat = _rand(M * F + 8, seed=1)
+        x, qw, kw = flat[shift:shift + M * F].view(M, F), _rand(hd, seed=2), _rand(hd, seed=3)
+        pos = torch.arange(M, device="cuda", dtype=torch.int32) % 64
+        k, v = (torch.empty(M, nkv * hd, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        q = Kc.qk_norm_rope_kv(x, qw, kw, pos, nq, nkv, hd, 1e-6, 1e6, k_dense=k, v_dense=v)
+        assert torch.equal(v, x[:, (nq + nkv) * hd:])
+        ang = pos[:, None, None].float() * torch.exp2(-torch.arange(hd // 2, device="cuda") * 2 / hd * torch.log2(torch.tensor(1e6)).item())
+        cos, sin = (f(ang).bfloat16().float().repeat(1, 1, 2) for f in (torch.cos, torch.sin))
+        for out, w, first, n in ((q, qw, 0, nq), (k, kw, nq, nkv)):
+            h = x[:, first * hd:(first + n) * hd].float().view(M, n, hd)
+            h = w.float() * h * torch.rsqrt(h.pow(2).mean(-1, keepdim=True) + 1e-6)
+            part = torch.cat([-h[..., hd // 2:], h[..., :hd // 2]], -1)
+            # normed, weighted, its products and their sum: four roundings to 8 significant bits, 2^-8 each; a rounded sine or cosine may lie one
+            # step off, 2^-7; angles up to 64 to 2^-22
+            bound = (4 + 2) * 2.0 ** -8 * ((h * cos).abs() + (part * sin).abs()) + 64 * 2.0 ** -22 * (h.abs() + part.abs())
+            assert ((out.view(M, n, hd).float() - (h * cos + part * sin)).abs() <= bound).all()
+
+
 @pytest.mark.parametrize("hd,nq,nkv", [(128, 16, 8), (128, 40, 8), (64, 8, 1)])
 def test_qk_norm_rope_of_few_tokens(hd, nq, nkv):
     """However many CTAs the heads of a token are dealt out to, a token's rows have the same bits, forward and backward; the weight gradients
