@@ -380,11 +380,13 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
             not ((swiglu or gelu) and (residual is not None or swiglu and gelu)) and _few_ok(x, w, x2, w2, const_w) and
             (not (gelu or swiglu_interleaved) or _whole_pieces(out))):
         return _gemm_few(x, w, out, residual, x2, w2, 1 if swiglu else 3 if gelu else 4 if swiglu_interleaved else 0, early=const_w)
+    # the plan, which is kept, before the look at every operand (4 us of host time)
     if (pair is None and bn == 0 and splits is None and tp_push is None and not swiglu and not (gelu and residual is not None) and
-            _persist_ok(x, w, out, residual, x2, w2)):
-        bn = plan_persist(M, F, K, R, swiglu_interleaved)
-        if bn and (M > 256 or const_w or swiglu_interleaved or plan_gemm_kept(M, F, K, R)[1] == 1):
-            return _gemm_persist(x, w, out, residual, x2, w2, 1 if gelu else 2 if swiglu_interleaved else 0, bn, tp_wait=tp_wait)
+            M > 128 and F > 0 and K > 0):
+        wide = plan_persist(M, F, K, R, swiglu_interleaved)
+        if (wide and (M > 256 or const_w or swiglu_interleaved or plan_gemm_kept(M, F, K, R)[1] == 1) and
+                _persist_ok(x, w, out, residual, x2, w2)):
+            return _gemm_persist(x, w, out, residual, x2, w2, 1 if gelu else 2 if swiglu_interleaved else 0, wide, tp_wait=tp_wait)
     pair, bn, splits = _plan_tiles(M, w.shape[0], K, R, swiglu, gelu, swiglu_interleaved, pair, bn, splits,
                                    () if tp_push is not None else (out, residual), kept=not const_w and tp_push is None and tp_wait is None)
     args = (_p(w), _p(x), _p(out), _p(residual), _p(w2), _p(x2), c_int(M), c_int(F), c_int(K), c_int(R),
@@ -542,10 +544,10 @@ def gemm_t(x: torch.Tensor, w: torch.Tensor, *, x_t: bool = False, w_t: bool = F
     if residual is not None:
         _check_bf16_2d(residual, "residual")
     can_pair = F % 256 == 0 and (not x_t or M % 64 == 0)
-    if pair is None and bn == 0 and splits is None and _persist_ok(x, w, out, residual, x_t=x_t, w_t=w_t):
-        bn = plan_persist(M, F, Kx, 0, False, x_t, can_pair)
-        if bn:
-            return _gemm_persist(x, w, out, residual, bn=bn, x_t=x_t, w_t=w_t)
+    if pair is None and bn == 0 and splits is None and M > 256 and F > 0 and Kx > 0:
+        wide = plan_persist(M, F, Kx, 0, False, x_t, can_pair)
+        if wide and _persist_ok(x, w, out, residual, x_t=x_t, w_t=w_t):
+            return _gemm_persist(x, w, out, residual, bn=wide, x_t=x_t, w_t=w_t)
     if pair is None and bn == 0 and splits is None and M > 256:
         staged = _whole_pieces(out) and (residual is None or _whole_pieces(residual))
         pair, bn, splits = plan_tiles(M, F, Kx, can_pair and PAIR_AUTO and staged, True, x_t)
