@@ -86,6 +86,19 @@ def test_left_padded_prompts_and_eos():
     assert cut.tokens[0] == full.tokens[0][:first]
 
 
+def test_prefill_with_a_mask_narrower_than_the_ids():
+    """The tokens are the columns that the mask has, in every row: what ids cut to its width give."""
+    B, T = 3, 20
+    _, _, eng, ids = _setup(2, B, T)
+    mask = torch.ones(B, 13, dtype=torch.long)
+    mask[1, :4] = 0
+    want, lens, _ = eng.prefill(ids[:, :13].cuda(), mask.cuda(), 4)
+    got, lens2, _ = eng.prefill(ids.cuda(), mask.cuda(), 4)
+    assert torch.equal(want, got) and torch.equal(lens, lens2) and lens.tolist() == [13, 9, 13]
+    with pytest.raises(ValueError, match="attention mask"):
+        eng.prefill(ids.cuda(), mask[:2].cuda(), 4)
+
+
 def test_sampling_runs_and_is_seeded():
     B, T, n_new = 3, 20, 8
     model, ref, eng, ids = _setup(2, B, T, n_new)

@@ -521,6 +521,26 @@ def test_host_plan_of_a_prefill_is_the_device_one():
         kv.reset()
 
 
+def test_packed_tokens_of_masks_narrower_than_the_ids():
+    """A mask's columns are the ids' first ones, whatever its pitch; the rows have to be the ids'."""
+    import numpy as np
+    import torch
+    from tah_b200.engine.engine import packed_tokens
+    gen = torch.Generator().manual_seed(0)
+    ids = torch.randint(0, 1000, (3, 6), generator=gen)
+    for width in (1, 4, 6):
+        mask = torch.rand(3, width, generator=gen) < 0.7
+        mask[:, 0] = True
+        want = ids[mask.nonzero(as_tuple=True)]
+        assert torch.equal(ids.reshape(-1)[torch.from_numpy(packed_tokens(mask.numpy(), 3, 6))], want)
+    for bad in (np.ones((1, 6), bool), np.ones((4, 6), bool), np.ones(6, bool)):
+        try:
+            packed_tokens(bad, 3, 6)
+            raise AssertionError("accepted")
+        except ValueError as e:
+            assert "attention mask" in str(e)
+
+
 def test_host_arrays_keep_nothing_alive():
     """Arrays sent in one copy, with what runs behind it: the values arrive, and what the functions hold (an engine and its caches) is freed by
     the last reference, not by the cycle collector."""
