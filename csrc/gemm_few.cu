@@ -43,7 +43,7 @@ struct FewParams {
   __nv_bfloat16* T;
   const int* gate;               // [M]
   int t_ctas;                    // CTAs that form T
-  int* sync;                     // [2] CTAs of T done, CTAs that have seen it; zero between launches
+  unsigned long long* sync;      // CTAs of T done and, in the high half, CTAs that look at it no more; zero between launches
   int* status;
 };
 
@@ -58,10 +58,16 @@ __device__ __forceinline__ uint4 ld_stream(const void* p) {
   return v;
 }
 
-__device__ __forceinline__ int ld_acquire(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
+}
+// Every CTA of a launch with gated rows, those that form T included, leaves once, when it will not look at the counters again; the last one
+// finds all of T counted and puts them back to zero.  So they are zero behind every launch, also one whose wait for T ran out (the
+// CTAs of T then leave behind the others).  A CTA of T counts and leaves in one step: one word, T's CTAs in the low half.
+__device__ __forceinline__ void few_leave(unsigned long long* sync, unsigned long long formed) {
+  if (atomicAdd(sync, (1ull << 32) + formed) >> 32 == gridDim.x - 1) *sync = 0;
 }
 constexpr int FEW_ROWS_MOST = 96 * 1024;       // of shared memory for normalised rows: two CTAs per SM
 
@@ -320,7 +326,7 @@ gemm_few_kernel(const FewParams p) {
     } else {
       if (threadIdx.x == 0) {
         unsigned long long t0 = 0;
-        for (uint32_t spins = 0; ld_acquire(p.sync) < p.t_ctas;) {
+        for (uint32_t spins = 0; (int)(uint32_t)ld_acquire(p.sync) < p.t_ctas;) {
           if ((++spins & 0xff) == 0) {
             const unsigned long long now = globaltimer_ns();
             if (t0 == 0) t0 = now;
@@ -332,11 +338,7 @@ gemm_few_kernel(const FewParams p) {
         }
       }
       __syncthreads();
-      // the last CTA that has seen T leaves the counters as it found them
-      if (threadIdx.x == 0 && atomicAdd(p.sync + 1, 1) == (int)gridDim.x - p.t_ctas - 1) {
-        p.sync[0] = 0;
-        p.sync[1] = 0;
-      }
+      if (threadIdx.x == 0) few_leave(p.sync, 0);
     }
   }
   for (int s = warp; s < ext; s += NW) {
@@ -378,7 +380,7 @@ gemm_few_kernel(const FewParams p) {
       }
       __threadfence();
       __syncthreads();
-      if (threadIdx.x == 0) atomicAdd(p.sync, 1);
+      if (threadIdx.x == 0) few_leave(p.sync, 1);
       return;
     }
   }
@@ -493,9 +495,9 @@ extern "C" int tahb_gemm_few(const void* W, const void* X, void* out, const void
 
 // The same for up to 32 tokens (16 with norm_w) with what stands around it in a decode tick: norm_w != null: X goes through RMSNorm (norm_w, eps) first;
 // R > 0: out += T B^T with T = gate * x A^T (A [R, K], B [F, R], T [M, R], all contiguous; T is written where a row is gated).
-// act as above.  sync: two ints, zero, for this stream's launches alone.
+// act as above.  sync: eight bytes, zero, on their own boundary, for this stream's launches alone.
 extern "C" int tahb_gemm_few_fused(const void* W, const void* X, void* out, const void* residual, const void* norm_w, float eps, const void* A,
-                                   const void* B, void* T, const int* gate, int* sync, int M, int F, int K, int R, long long ldw,
+                                   const void* B, void* T, const int* gate, void* sync, int M, int F, int K, int R, long long ldw,
                                    long long ldx, long long ldo, long long ldr, int act, int* status, cudaStream_t stream) {
   if (M <= 0 || F <= 0) return 0;
   if (M > (norm_w != nullptr ? 16 : 32) || K <= 0 || K % 64 || R % 64 || ((act == 1 || act == 4) && (F % 2 || residual != nullptr))) return -20;
@@ -503,7 +505,7 @@ extern "C" int tahb_gemm_few_fused(const void* W, const void* X, void* out, cons
   if (R > 0 && (A == nullptr || B == nullptr || T == nullptr || gate == nullptr || sync == nullptr)) return -27;
   if (norm_w != nullptr && few_rows_bytes(M, K) > FEW_ROWS_MOST) return -22;
   auto odd = [](const void* p, long long ld) { return (reinterpret_cast<uintptr_t>(p) & 15) || (ld & 7); };
-  if (odd(W, ldw) || odd(X, ldx) || odd(norm_w, 0) || odd(A, 0) || odd(B, 0) || odd(T, 0)) return -2;
+  if (odd(W, ldw) || odd(X, ldx) || odd(norm_w, 0) || odd(A, 0) || odd(B, 0) || odd(T, 0) || (reinterpret_cast<uintptr_t>(sync) & 7)) return -2;
   FewParams p = {};
   p.W = reinterpret_cast<const __nv_bfloat16*>(W);
   p.X = reinterpret_cast<const __nv_bfloat16*>(X);
@@ -520,7 +522,7 @@ extern "C" int tahb_gemm_few_fused(const void* W, const void* X, void* out, cons
   p.A = reinterpret_cast<const __nv_bfloat16*>(A);
   p.T = reinterpret_cast<__nv_bfloat16*>(T);
   p.gate = gate;
-  p.sync = sync;
+  p.sync = reinterpret_cast<unsigned long long*>(sync);
   p.status = status;
   return norm_w != nullptr ? dispatch_few<2>(p, stream) : dispatch_few<1>(p, stream);
 }

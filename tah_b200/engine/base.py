@@ -66,6 +66,7 @@ class DecodeEngine:
         s.samp_v = torch.zeros(B, 128, dtype=torch.float32, device=dev)
         s.samp_i = i32(B, 128)
         s.seed_dev = torch.zeros(1, dtype=torch.int64, device=dev)     # per-call sampling seed, read on the device
+        s.counters = []                       # what kernels of the tick count in, zero between launches
         s.graph = None
         kv = self.kv
         pad = lambda lst: list(lst) + [lst[0]] * (4 - len(lst))
@@ -159,7 +160,7 @@ class DecodeEngine:
             self._states[key] = s
         else:
             for t in (s.tok, s.depth, s.pos, s.finished, s.n_out, s.out_tokens, s.iter_sum, s.cur_iters, s.slot,
-                      s.gate, s.tokens_done, s.need_soft, s.best, s.sampled):
+                      s.gate, s.tokens_done, s.need_soft, s.best, s.sampled, *s.counters):
                 t.zero_()
         return s
 

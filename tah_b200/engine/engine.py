@@ -554,6 +554,7 @@ class TaHEngine(DecodeEngine):
         s.topv = torch.zeros(B, self.topk, dtype=torch.float32, device=dev)
         s.topi = i32(B, self.topk)
         s.few_sync = i32(2)
+        s.counters.append(s.few_sync)
         tl = self._tap_layers()
         # the learned decider's Linear(topk -> H) output is written behind the tapped hidden states
         tap_w = (max(1, len(tl)) + (1 if self._needs_topk_for_decider() else 0)) * H

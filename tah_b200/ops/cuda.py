@@ -472,7 +472,8 @@ def gemm_few_fused(x, w, out, gate, sync, *, norm=None, eps: float = 0.0, lora=N
     (+ residual)``.
 
     ``norm``: RMSNorm weight (with ``eps``), None: ``x`` as it is; ``lora``: ``(A [R, K], t [M, R], B [F, R])``, contiguous, or None; ``act``: 0
-    none, 1 SwiGLU of stacked rows, 4 of interleaved rows; ``sync``: two int32 zeros that no other stream uses meanwhile."""
+    none, 1 SwiGLU of stacked rows, 4 of interleaved rows; ``sync``: two int32 zeros (on an 8-byte boundary) that no other stream uses meanwhile; zeros again behind
+    the launch."""
     for t, n in ((x, "x"), (w, "w"), (out, "out")) + (() if residual is None else ((residual, "residual"),)):
         _check_bf16_2d(t, n)
     M, Kd = x.shape
@@ -482,7 +483,7 @@ def gemm_few_fused(x, w, out, gate, sync, *, norm=None, eps: float = 0.0, lora=N
     A, t, B = lora or (None, None, None)
     R = 0 if A is None else A.shape[0]
     if R and (A.shape != (R, Kd) or t.shape != (M, R) or B.shape != (F, R) or not (A.is_contiguous() and t.is_contiguous() and B.is_contiguous()) or
-              gate.dtype != torch.int32 or gate.numel() < M or sync.dtype != torch.int32 or sync.numel() < 2):
+              gate.dtype != torch.int32 or gate.numel() < M or sync.dtype != torch.int32 or sync.numel() < 2 or not sync.is_contiguous()):
         raise ValueError("gemm_few_fused: adapter operands do not match")
     _rc(lib().tahb_gemm_few_fused(_p(w), _p(x), _p(out), _p(residual), _p(norm), c_float(eps), _p(A), _p(B), _p(t), _p(gate if R else None),
                                   _p(sync if R else None), c_int(M), c_int(F), c_int(Kd), c_int(R), c_ll(w.stride(0)), c_ll(x.stride(0)),

@@ -150,6 +150,18 @@ def test_graph_is_reused_across_calls_and_results_repeat():
     assert c.tokens == d.tokens
 
 
+def test_tick_counters_start_from_zero_on_every_call():
+    """Counters of the fused products that a call found or left above zero do not reach the next call on the same state."""
+    B, T, n_new = 3, 20, 16
+    _, _, eng, ids = _setup(2, B, T, n_new)
+    want = eng.generate(ids.cuda(), None, max_new_tokens=n_new).tokens
+    s = next(iter(eng._states.values()))
+    assert any(t is s.few_sync for t in s.counters) and s.few_sync.tolist() == [0, 0]
+    s.few_sync.copy_(torch.tensor([5, 3]))
+    assert eng.generate(ids.cuda(), None, max_new_tokens=n_new).tokens == want
+    assert s.few_sync.tolist() == [0, 0]
+
+
 def test_default_seed_follows_torch_generator():
     """Without an explicit seed two sampled calls differ, and re-seeding torch reproduces them (the evaluation
     driver repeats a prompt ``repeat_size`` times and relies on the samples being different)."""

@@ -11,6 +11,11 @@ symmetric buffers are shared Python lists, peer stores / flag updates are ordina
 * landing-flag protocol of the push all-gather (``shard_gather_push_kernel`` + the consumer's ``wait_peer_rows``):
   the consumer's target grows by the push grid size per use; a consumer never reads a buffer before all sources
   of THAT use have landed, and a producer never overwrites it before every consumer released the previous use.
+* counters of the fused few-token product (``gemm_few_kernel`` in ``csrc/gemm_few.cu``): a CTA that forms T counts itself and
+  leaves in one step, the others wait for T (bounded) and leave, and whoever leaves last puts the counters back to zero.  Every
+  order of the CTAs' steps and every moment at which a wait may run out is walked through: the counters are zero behind each launch, so no
+  CTA of the next one reads T early.  (An earlier form, in which only the CTAs that wait left, could end above zero after a wait that
+  ran out; the model shows it.)
 """
 import random
 import threading
@@ -104,3 +109,35 @@ def test_push_gather_flags_order_producers_and_consumers():
     for t in threads:
         t.join(timeout=60)
     assert not any(t.is_alive() for t in threads) and bad == []
+
+
+def _counter_ends(formers, waiters, formers_leave):
+    """``(T formed, left)`` as every order of a launch's steps from zeroed counters can leave them, its waits running out at any moment."""
+    last = (formers + waiters if formers_leave else waiters) - 1
+    # a former counts itself (and leaves); a waiter passes its wait, then leaves
+    seen, ends, todo = set(), set(), [((1,) * formers + (0,) * waiters, 0, 0)]
+    while todo:
+        state = todo.pop()
+        if state in seen:
+            continue
+        seen.add(state)
+        at, done, left = state
+        if all(a == 2 for a in at):
+            ends.add((done, left))
+        for i, a in enumerate(at):
+            step = lambda to, done, left: todo.append((at[:i] + (to,) + at[i + 1:], done, left))
+            leave = lambda done: step(2, 0, 0) if left == last else step(2, done, left + 1)
+            if a == 0:
+                step(1, done, left)                                        # T is there, or the wait runs out
+            elif a == 1 and i < formers:
+                leave(done + 1) if formers_leave else step(2, done + 1, left)
+            elif a == 1:
+                leave(done)
+    return ends
+
+
+def test_counters_of_the_fused_product_are_zero_behind_every_launch():
+    for formers in (1, 2, 3):
+        for waiters in (1, 2, 4):
+            assert _counter_ends(formers, waiters, formers_leave=True) == {(0, 0)}
+    assert any(done > 0 for done, _ in _counter_ends(2, 2, formers_leave=False))

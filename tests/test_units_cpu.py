@@ -541,6 +541,18 @@ def test_packed_tokens_of_masks_narrower_than_the_ids():
             assert "attention mask" in str(e)
 
 
+def test_reused_tick_state_clears_the_kernels_counters():
+    """A cached tick state starts as a new one does: its scheduler tensors and the counters of its kernels are zero."""
+    import types
+    import torch
+    from tah_b200.engine.base import DecodeEngine
+    names = "tok depth pos finished n_out out_tokens iter_sum cur_iters slot gate tokens_done need_soft best sampled".split()
+    s = types.SimpleNamespace(**{n: torch.ones(2, dtype=torch.int32) for n in names}, counters=[torch.tensor([5, 3], dtype=torch.int32)])
+    eng = types.SimpleNamespace(hard_override=None, _states={(2, 8, None, None, None): s})
+    assert DecodeEngine._tick_state(eng, 2, 8, None, None) is s
+    assert all(not t.any() for t in [getattr(s, n) for n in names] + s.counters)
+
+
 def test_host_arrays_keep_nothing_alive():
     """Arrays sent in one copy, with what runs behind it: the values arrive, and what the functions hold (an engine and its caches) is freed by
     the last reference, not by the cycle collector."""
