@@ -139,14 +139,31 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
-// As mbar_wait, for the loops whose every step a wait stands in: the flag and the clock are looked at only once the barrier has been
-// asked many times.  False once this CTA has given up.
+// As mbar_wait, for the loops of a converged warp whose every step a wait stands in: nothing but the barrier is looked at while it answers at once.
+// False, in all lanes alike, once this CTA has given up and the barrier is not there yet: the caller leaves its loop.
 __device__ __forceinline__ bool mbar_wait_tight(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  unsigned long long t0 = 0;
 #pragma unroll 1
-  for (int i = 0; i < 256; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  mbar_wait(bar, parity, abort_flag, status, code);
-  return *abort_flag == 0;
+  for (uint32_t spins = 1;; ++spins) {
+    if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if ((spins & 0x3ff) == 0) {
+      const unsigned long long now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      else if (__any_sync(0xffffffffu, now - t0 > WAIT_TIMEOUT_NS)) {
+        *abort_flag = 1;
+        atomicCAS(status, 0, code);
+        return false;
+      }
+    }
+  }
+}
+
+// For copies and products that are on their way in a CTA that may have given up: they are waited for whatever the flag says (bounded).
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+  const unsigned long long t0 = globaltimer_ns();
+  while (!mbar_try_wait(bar, parity) && globaltimer_ns() - t0 < WAIT_TIMEOUT_NS) {}
 }
 
 // Bounded wait of ONE thread until flag[q] has reached target[q] (wrap-around safe) for every q <
@@ -330,6 +347,9 @@ __device__ __forceinline__ void st_dsmem_v4(uint32_t cluster_addr, float4 v) {
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};"
                ::"r"(cluster_addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
                : "memory");
+}
+__device__ __forceinline__ void st_dsmem_u32(uint32_t cluster_addr, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
 __device__ __forceinline__ void st_dsmem_f32(uint32_t cluster_addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr), "f"(v) : "memory");

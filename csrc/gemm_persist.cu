@@ -73,9 +73,12 @@ __device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a,
       ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// arrives at this barrier of both CTAs once the products issued so far have completed
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint32_t bar_peer) {
+// arrives at this CTA's barrier, or at this barrier of both CTAs, once the products issued so far have completed
+__device__ __forceinline__ void umma_commit_own(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint32_t bar_peer) {
+  umma_commit_own(bar);
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_peer) : "memory");
 }
 // a copy into this CTA's shared memory that reports to a barrier of either CTA of the pair (no multicast)
@@ -182,10 +185,12 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
   uint64_t* acc_empty = acc_full + 2;                                        // [2], used in the first CTA: 8 epilogue warps of 2 CTAs
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint64_t* last = reinterpret_cast<uint64_t*>(tmem_slot + 2);               // products in flight when the issuer gives up
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_ctarank();
-  const int n_tiles = p.tiles_m * p.tiles_n, first = blockIdx.x >> 1, step = gridDim.x >> 1;
+  int n_tiles = p.tiles_m * p.tiles_n;
+  const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) {
@@ -196,6 +201,7 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
       mbar_init(&acc_full[b], 1);
       mbar_init(&acc_empty[b], 16);
     }
+    mbar_init(last, 1);
     *abort_flag = 0;
     mbar_fence_init();
     prefetch_tensormap(&tm_x);
@@ -211,18 +217,24 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
   tc_fence_after();
   pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
+  if (p.wait_world > 0) {
+    // Both CTAs wait for the peers' rows in front of everything, and skip all tiles if one of them does not see them come.
+    if (threadIdx.x == 0 && !wait_peer_rows(p.wait_flag, p.wait_target, p.wait_world, p.status, p.wait_limit_ns)) {
+      *abort_flag = 1;
+      st_dsmem_u32(dsmem_addr(smem_u32(const_cast<int*>(abort_flag)), rank ^ 1), 1);
+    }
+    cluster_sync_all();
+    asm volatile("fence.proxy.async.global;" ::: "memory");   // the TMA loads below see the landed rows
+    if (*abort_flag) n_tiles = 0;
+  }
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (p.wait_world > 0) {
-      if (lane == 0 && !wait_peer_rows(p.wait_flag, p.wait_target, p.wait_world, p.status, p.wait_limit_ns)) *abort_flag = 1;
-      __syncwarp();
-      asm volatile("fence.proxy.async.global;" ::: "memory");
-    }
     const uint32_t full0 = dsmem_addr(smem_u32(full), 0);
     int s = 0;
     uint32_t ph = 1;
     bool going = true;
+    int issued = 0;
     for (int tile = first; tile < n_tiles && going; tile += step) {
       int tm, tn;
       persist_tile(p, tile, tm, tn);
@@ -250,6 +262,7 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
               tma_load_3d_pair(st + PERSIST_A, mb, 0, f0, g, bar);
             }
           }
+          ++issued;
           if (++s == p.stages) { s = 0; ph ^= 1; }
         }
       };
@@ -257,6 +270,9 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
       if (p.kb_ext > 0 && going) blocks(&tm_x2, &tm_w2, p.kb_ext);
     }
     __syncwarp();
+    // Given up: the first CTA, whose barriers both CTAs' copies report to, stays until they have landed (bounded); the other one leaves with it.
+    if (*abort_flag && rank == 0)
+      for (int j = issued > p.stages ? issued - p.stages : 0; j < issued; ++j) mbar_drain(&full[j % p.stages], (j / p.stages) & 1);
     pdl_launch_dependents();
   } else if (warp == 1) {
     // ---------------- MMA issuer (first CTA of the pair) ----------------
@@ -274,15 +290,22 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
       int s = 0;
       uint32_t ph = 0;
       int n = 0;
+      bool going = true;
       for (int tile = first; tile < n_tiles; tile += step, ++n) {
         const int buf = n & 1;
-        mbar_wait(&acc_empty[buf], ((n >> 1) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+        if (!mbar_wait_tight(&acc_empty[buf], ((n >> 1) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM)) {
+          going = false;
+          break;
+        }
         tc_fence_after();
         const uint32_t d = tmem_base + buf * 256;
         uint32_t acc = 0u;
         auto blocks = [&](int n_blocks) {
           for (int g = 0; g < n_blocks; g += 2) {
-            mbar_wait_tight(&full[s], ph, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
+            if (!mbar_wait_tight(&full[s], ph, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL)) {
+              going = false;
+              break;
+            }
             tc_fence_after();
             if (elect_one()) {
               uint64_t da = da0 + (uint64_t)(s * stage16), db = db0 + (uint64_t)(s * stage16);
@@ -301,8 +324,13 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
           }
         };
         blocks(p.kb_main);
-        if (p.kb_ext > 0) blocks(p.kb_ext);
+        if (p.kb_ext > 0 && going) blocks(p.kb_ext);
+        if (!going) break;
         if (elect_one()) umma_commit_pair(&acc_full[buf], acc_full_peer + buf * 8);
+      }
+      if (!going) {
+        if (elect_one()) umma_commit_own(last);
+        mbar_drain(last, 0);
       }
     }
     __syncwarp();
@@ -325,7 +353,7 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
         if (half < chunks) persist_residual(p, t0 + lane, o0 + half * 64, res);       // under the main loop
       }
       const int buf = n & 1;
-      mbar_wait(&acc_full[buf], (n >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+      if (!mbar_wait_tight(&acc_full[buf], (n >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM)) break;
       tc_fence_after();
 #pragma unroll 1
       for (int c = half; c < chunks; c += 2) {

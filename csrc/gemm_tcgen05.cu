@@ -414,7 +414,7 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   const int rank = blockIdx.z;                       // == cluster rank: cluster dims are (1, 1, S)
   const int st_main = (p.kb_main + C::KB - 1) / C::KB, st_total = st_main + (p.kb_ext + C::KB - 1) / C::KB;     // stages' worth of the reduction
   const int st_begin = (int)(((long long)st_total * rank) / S);
-  const int n_st = (int)(((long long)st_total * (rank + 1)) / S) - st_begin;
+  int n_st = (int)(((long long)st_total * (rank + 1)) / S) - st_begin;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::NS; ++s) {
@@ -437,18 +437,22 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   tc_fence_after();
   pdl_wait();                   // set-up above touched no global memory; operands may be read from here on
   const uint32_t tmem_base = *tmem_slot;
+  if (p.wait_world > 0) {
+    // All warps wait for the peers' rows, so that no wait inside starts its clock before they are there.  If they do not come, nothing is copied
+    // or multiplied; the rest of the kernel runs out (the others of the cluster and the peers count on it).
+    if (threadIdx.x == 0 && !wait_peer_rows(p.wait_flag, p.wait_target, p.wait_world, p.status, p.wait_limit_ns)) *abort_flag = 1;
+    __syncthreads();
+    asm volatile("fence.proxy.async.global;" ::: "memory");   // the TMA loads below see the landed rows
+    if (*abort_flag) n_st = 0;
+  }
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     // Producer and issuer walk their loops as whole warps and elect the lane that issues: what one lane of a diverged warp issues is wrapped in a
     // loop over the active lanes.  A step takes some 500 cycles whatever it carries, so a stage has two blocks of 64 of the reduction where
     // three such stages fit, each operand's brought by one copy.
-    if (p.wait_world > 0) {
-      if (lane == 0 && !wait_peer_rows(p.wait_flag, p.wait_target, p.wait_world, p.status, p.wait_limit_ns)) *abort_flag = 1;
-      __syncwarp();
-      asm volatile("fence.proxy.async.global;" ::: "memory");   // the TMA loads below see the landed rows
-    }
-    for (int i = 0; i < n_st; ++i) {
+    int i = 0;
+    for (; i < n_st; ++i) {
       const int s = i % C::NS;
       // a wait gave up: issue no further copies, let the kernel run out
       if (!mbar_wait_tight(&empty_bar[s], ((i / C::NS) & 1) ^ 1, abort_flag, p.status, STATUS_TIMEOUT_STAGE_EMPTY)) break;
@@ -488,6 +492,8 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       }
     }
     __syncwarp();
+    if (*abort_flag)
+      for (int j = i > C::NS ? i - C::NS : 0; j < i; ++j) mbar_drain(&full_bar[j % C::NS], (j / C::NS) & 1);
     if constexpr (PAIR) {
       // the residual tiles take the first two stages as the main loop frees them
       if (lane == 0 && p.tma_out && p.residual != nullptr && !*abort_flag) {
@@ -495,7 +501,7 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
           if (n_st > s) mbar_wait(&empty_bar[s], ((n_st - 1 - s) / C::NS) & 1, abort_flag, p.status, STATUS_TIMEOUT_STAGE_EMPTY);
-          if (!*abort_flag) tma_load_2d(smem + s * C::STAGE_BYTES, &tm_res, s ? p.up_off + f0 : f0, t0, res_bar);
+          tma_load_2d(smem + s * C::STAGE_BYTES, &tm_res, s ? p.up_off + f0 : f0, t0, res_bar);
         }
       }
       __syncwarp();
@@ -513,7 +519,7 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     const uint64_t db0 = p.b_mn ? umma_desc_mn_sw128(b_addr, C::KB * 8192) : umma_desc_sw128(b_addr);
     for (int i = 0; i < n_st; ++i) {
       const int s = i % C::NS;
-      mbar_wait_tight(&full_bar[s], (i / C::NS) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
+      if (!mbar_wait_tight(&full_bar[s], (i / C::NS) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL)) break;
       tc_fence_after();
       if (elect_one()) {
         uint64_t da = da0 + (uint64_t)(s * (C::STAGE_BYTES >> 4)), db = db0 + (uint64_t)(s * (C::STAGE_BYTES >> 4));
@@ -557,7 +563,10 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         __nv_bfloat16* stg1 = reinterpret_cast<__nv_bfloat16*>(smem + C::STAGE_BYTES);
         const bool il = p.act == 2;
         static_assert(!PAIR || (C::STAGE_BYTES >= BN * 256 && C::NS >= 2), "a staged tile fits a stage");
-        if (res_tma) mbar_wait(res_bar, 0, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
+        if (res_tma) {
+          mbar_wait(res_bar, 0, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
+          if (*abort_flag && n_st > 0) mbar_drain(res_bar, 0);
+        }
         if (il) {
           swiglu_interleaved_tile<BN, C::CHUNK>(trow + half * BN, half ? stg1 : stg, row, 0, C::CHUNK);
         } else {
@@ -597,6 +606,7 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           tma_load_2d(stg, &tm_res, f0, t0, res_bar);
         }
         mbar_wait(res_bar, 0, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
+        if (*abort_flag) mbar_drain(res_bar, 0);
       }
       const bool swiglu_il = !DUAL && p.act == 2;
       if (swiglu_il) {
@@ -705,6 +715,7 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           tma_load_2d(stg, &tm_res, f0, t0 + rank * per, res_bar);
         }
         mbar_wait(res_bar, 0, abort_flag, p.status, STATUS_TIMEOUT_TMA_FULL);
+        if (*abort_flag) mbar_drain(res_bar, 0);
       }
       const int c_first = C::EPI_WARPS == 8 ? ((warp - 2) >> 2) * 16 : 0, c_step = C::EPI_WARPS * 4;
 #pragma unroll 1
@@ -763,6 +774,7 @@ gemm_fl_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
 
   __syncthreads();
   if (warp == 1) {
+    if (*abort_flag) mbar_drain(accum_bar, 0);        // products that nobody waited for
     tc_fence_after();
     tmem_dealloc(tmem_base, C::TMEM_COLS);
   }

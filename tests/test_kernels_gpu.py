@@ -941,20 +941,25 @@ def test_training_step_kernel_path_matches_torch_path_multi_tile(monkeypatch):
         assert float(cos) > 0.97, (name, float(cos))
 
 
-def test_peer_flag_wait_runs_out_and_reports_a_timeout():
+@pytest.mark.parametrize("M,F,Kd,res,how", [(64, 256, 256, False, {}), (64, 256, 256, True, dict(splits=2, bn=64)), (64, 256, 256, True, dict(splits=1, bn=64)),
+                                            (300, 512, 256, True, dict(pair=True)), (1500, 2048, 2048, False, {}), (1500, 2048, 2048, True, {})])
+def test_peer_flag_wait_runs_out_and_reports_a_timeout(M, F, Kd, res, how):
     """A consumer GEMM that waits for rows a peer would broadcast: nothing advances the landing flags, the wait
     limit is 5 ms, so the kernel gives up, records the timeout code and returns; the host reads the status word
-    and raises.  Nothing traps or hangs, and the context stays usable."""
+    and raises.  Nothing traps or hangs, and the context stays usable.  The persistent form writes nothing then."""
     import time
     Kc = _cuda()
-    x, w = _rand(64, 256, seed=1), _rand(256, 256, scale=256 ** -0.5, seed=2)
+    x, w, r = _rand(M, Kd, seed=1), _rand(F, Kd, scale=Kd ** -0.5, seed=2), _rand(M, F, seed=3) if res else None
+    out, persist = torch.full((M, F), 7.0, dtype=torch.bfloat16, device="cuda"), M > 1000 and Kc.plan_persist(M, F, Kd) > 0
+    assert persist == (M == 1500)
+    Kc.gemm(x, w, residual=r, tp_wait=(torch.ones(2, dtype=torch.int32, device="cuda"),) * 2, **how)       # first launch of this form
     flags = torch.zeros(2, dtype=torch.int32, device="cuda")
     targets = torch.ones(2, dtype=torch.int32, device="cuda")
     prev = Kc.set_peer_wait_limit_ns(5_000_000)
     try:
         torch.cuda.synchronize()
         t0 = time.time()
-        Kc.gemm(x, w, tp_wait=(flags, targets))
+        Kc.gemm(x, w, residual=r, out=out, tp_wait=(flags, targets), **how)
         Kc.wait_flags(flags, targets)
         torch.cuda.synchronize()
         assert time.time() - t0 < 1.0                                   # two 5 ms limits, not the 2 s default
@@ -963,10 +968,12 @@ def test_peer_flag_wait_runs_out_and_reports_a_timeout():
     finally:
         Kc.set_peer_wait_limit_ns(prev)
     Kc.check_status()                                                   # the status word was cleared
+    assert not persist or bool((out == 7.0).all())
     flags.fill_(1)                                                      # the flags arrive: same launch succeeds
-    y = Kc.gemm(x, w, tp_wait=(flags, targets))
+    y = Kc.gemm(x, w, residual=r, tp_wait=(flags, targets), **how)
     Kc.check_status()
-    _close(y, x.float() @ w.float().t(), atol=2e-2, rtol=2e-2)
+    ref = x.float() @ w.float().t()
+    _close(y, ref if r is None else ref + r.float(), atol=2e-2, rtol=2e-2)
 
 
 @pytest.mark.parametrize("rows,V", [(37, 151936), (300, 1024), (5, 1000)])
