@@ -306,6 +306,7 @@ struct BwdKVCfg {
   static constexpr int PT_BYTES = 128 * BQ * 2;                // P^T and dS^T tiles
   static constexpr int META_BYTES = 2 * 3 * BQ * 4;            // [2 buffers][lse | dsum | count][64 queries]
   static constexpr int SMEM_BYTES = 2 * K_BYTES + NSTAGE * STAGE_BYTES + 4 * PT_BYTES + META_BYTES + 128;
+  static_assert((1 + 2 * NSTAGE + 6) * 8 + 8 <= 128, "barriers, tensor-memory address and flag");
   static constexpr int TMEM_COLS = 512;                        // scores at 0 / 384 (S^T, dP^T), dK at 128, dV at 256
 };
 
@@ -327,8 +328,10 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
   uint64_t* qd_full = bars + 1;                                 // [NSTAGE]
   uint64_t* qd_empty = qd_full + C::NSTAGE;                     // [NSTAGE]
   uint64_t* s_full = qd_empty + C::NSTAGE;                      // [2]: one per score buffer
+  // [2] each: one per buffer of P^T and dS^T.  The threads may be an iteration ahead of the issuer (the buffer that they fill next is free once the
+  // products of the iteration before last are done), so both phases of one p_ready barrier could pass while the issuer is on its way to it.
   uint64_t* p_ready = s_full + 2;
-  uint64_t* acc_done = p_ready + 1;                             // [2]: one per buffer of P^T and dS^T
+  uint64_t* acc_done = p_ready + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -358,7 +361,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     for (int s = 0; s < C::NSTAGE; ++s) { mbar_init(&qd_full[s], 1); mbar_init(&qd_empty[s], 1); }
     mbar_init(&s_full[0], 1);
     mbar_init(&s_full[1], 1);
-    mbar_init(p_ready, 256);
+    mbar_init(&p_ready[0], 256);
+    mbar_init(&p_ready[1], 256);
     mbar_init(&acc_done[0], 1);
     mbar_init(&acc_done[1], 1);
     *abort_flag = 0;
@@ -432,7 +436,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
         const uint32_t do_addr = q_addr + C::Q_BYTES;
         // the other score buffer was last read for iteration it-1, whose p_ready has been waited for
         if (it + 1 < n_iter) issue_scores(it + 1);
-        mbar_wait(p_ready, it & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
+        mbar_wait(&p_ready[it & 1], (it >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_ACCUM);
         tc_fence_after();
         const uint32_t pt_addr = smem_u32(pt_s) + (it & 1) * 2 * C::PT_BYTES, dst_addr = pt_addr + C::PT_BYTES;
 #pragma unroll
@@ -541,7 +545,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
       }
       fence_proxy_async_smem();
       tc_fence_before();
-      mbar_arrive(p_ready);
+      mbar_arrive(&p_ready[it & 1]);
       store_meta(it + 1);
       named_bar_sync(2, 256);                      // next iteration's values visible; this buffer free again
     }

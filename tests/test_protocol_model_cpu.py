@@ -16,6 +16,9 @@ symmetric buffers are shared Python lists, peer stores / flag updates are ordina
   order of the CTAs' steps and every moment at which a wait may run out is walked through: the counters are zero behind each launch, so no
   CTA of the next one reads T early.  (An earlier form, in which only the CTAs that wait left, could end above zero after a wait that
   ran out; the model shows it.)
+* phases of the dK / dV kernel (``attn_bwd_dkv_kernel`` in ``csrc/attn_prefill_bwd.cu``): the threads may fill one buffer of P and dS while the
+  issuer has not yet seen that the other one is full.  Every order of both sides' steps ends with all iterations done.  (With one barrier
+  for both buffers two of its phases can pass unseen, and a wait for a parity then never ends; the model shows it.)
 """
 import random
 import threading
@@ -141,3 +144,37 @@ def test_counters_of_the_fused_product_are_zero_behind_every_launch():
         for waiters in (1, 2, 4):
             assert _counter_ends(formers, waiters, formers_leave=True) == {(0, 0)}
     assert any(done > 0 for done, _ in _counter_ends(2, 2, formers_leave=False))
+
+
+def _backward_gets_stuck(iterations, ready):
+    """Whether some order of the steps of issuer and threads ends before the last iteration, with ``ready`` barriers of full buffers.  A barrier is
+    its number of completed phases; a wait for a parity passes while the current phase has the other one."""
+    passed = lambda phases, parity: phases & 1 != parity
+    # issuer: scores of iteration 0, then for each iteration: scores of the next, wait for its buffers, products
+    plan = [("scores", 0)] + [x for i in range(iterations) for x in ([("scores", i + 1)] if i + 1 < iterations else []) + [("products", i)]]
+    seen, todo = set(), [(0, 0, (0, 0), (0,) * ready, (0, 0))]
+    while todo:
+        state = todo.pop()
+        if state in seen:
+            continue
+        seen.add(state)
+        at, it, scores, full, done = state
+        up = lambda t, i: t[:i] + (t[i] + 1,) + t[i + 1:]
+        n = len(todo)
+        if at < len(plan):
+            what, i = plan[at]
+            if what == "scores":
+                todo.append((at + 1, it, up(scores, i & 1), full, done))
+            elif passed(full[i % ready], i & 1 if ready == 1 else i >> 1 & 1):
+                todo.append((at + 1, it, scores, full, up(done, i & 1)))
+        if it < iterations and passed(scores[it & 1], it >> 1 & 1) and (it < 2 or passed(done[it & 1], (it >> 1) - 1 & 1)):
+            todo.append((at, it + 1, scores, up(full, it % ready), done))
+        if len(todo) == n and (at < len(plan) or it < iterations):
+            return True
+    return False
+
+
+def test_backward_buffers_never_leave_issuer_and_threads_waiting():
+    for iterations in range(1, 9):
+        assert not _backward_gets_stuck(iterations, ready=2)
+    assert _backward_gets_stuck(4, ready=1)
