@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(NW * 32, AttCfg<HD, G>::WARPS / NW) decode_att
 }
 
 template <int HD>
-__global__ void decode_attn_merge_kernel(const float* __restrict__ ws, __nv_bfloat16* __restrict__ out, int n_split) {
+__global__ void decode_attn_merge_kernel(const float* ws, __nv_bfloat16* out, int n_split) {
   pdl_launch_dependents();
   pdl_wait();
   const int rh = blockIdx.x;   // row * nq + head

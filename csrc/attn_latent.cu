@@ -143,23 +143,30 @@ __global__ void __launch_bounds__(256) latent_query_kernel(const LatentQueryPara
 }
 
 // Pages of the cache one after another as rows of pitch lp (16-byte units; zero behind the cached row).
-__global__ void __launch_bounds__(128) latent_gather_kernel(const uint4* __restrict__ cache, const int* __restrict__ src, int n_pool,
-                                                            int page_size, int units, int lp_units, uint4* __restrict__ out) {
+__global__ void __launch_bounds__(128) latent_gather_kernel(const uint4* cache, const int* src, int n_pool,
+                                                            int page_size, int units, int lp_units, uint4* out) {
   pdl_launch_dependents();
   pdl_wait();
   const int page = src[blockIdx.x];
-  for (int i = threadIdx.x; i < page_size * lp_units; i += 128) {
-    const int r = i / lp_units, c = i % lp_units;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (c < units && page >= 0 && page < n_pool) v = cache[((size_t)page * page_size + r) * units + c];
-    out[((size_t)blockIdx.x * page_size + r) * lp_units + c] = v;
+  const int all = page_size * lp_units;
+  const bool held = page >= 0 && page < n_pool;
+  for (int i0 = threadIdx.x; i0 < all; i0 += 4 * 128) {       // four loads on their way together
+    uint4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + u * 128, r = i / lp_units, c = i % lp_units;
+      v[u] = held && i < all && c < units ? cache[((size_t)page * page_size + r) * units + c] : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i0 + u * 128 < all) out[(size_t)blockIdx.x * all + i0 + u * 128] = v[u];
   }
 }
 
 // out[t, h * dv + d] = list[h * npad + t, d] * sigmoid(gate[t, h * dv + d]) (gate null: no factor), 8 elements per thread
 template <typename T>
-__global__ void __launch_bounds__(256) latent_gate_kernel(const T* __restrict__ list, int npad, int ld_list, const T* __restrict__ gate,
-                                                          long long ld_gate, T* __restrict__ out, long long ld_out, int n, int heads,
+__global__ void __launch_bounds__(256) latent_gate_kernel(const T* list, int npad, int ld_list, const T* gate,
+                                                          long long ld_gate, T* out, long long ld_out, int n, int heads,
                                                           int dv) {
   pdl_launch_dependents();
   pdl_wait();

@@ -69,16 +69,23 @@ __global__ void __launch_bounds__(128) tied_keys_kernel(const TiedKeysParams p) 
 
 // Pooled rows one after another for the portion kernel: out[r][g * dk + d] = pooled row src[r] (page * pool_rows + row), zeros
 // where src[r] is negative.  16-byte units.
-__global__ void __launch_bounds__(128) pool_gather_kernel(const uint4* __restrict__ pooled, const int* __restrict__ src, int nkv, int units,
-                                                          int pool_rows, int n_pages, uint4* __restrict__ out) {
+__global__ void __launch_bounds__(128) pool_gather_kernel(const uint4* pooled, const int* src, int nkv, int units,
+                                                          int pool_rows, int n_pages, uint4* out) {
   pdl_launch_dependents();
   pdl_wait();
   const int s = src[blockIdx.x], page = s < 0 ? -1 : s / pool_rows;
-  for (int i = threadIdx.x; i < nkv * units; i += 128) {
-    const int g = i / units, c = i % units;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (page >= 0 && page < n_pages) v = pooled[(((size_t)page * nkv + g) * pool_rows + s % pool_rows) * units + c];
-    out[(size_t)blockIdx.x * nkv * units + i] = v;
+  const int all = nkv * units;
+  const bool held = page >= 0 && page < n_pages;
+  for (int i0 = threadIdx.x; i0 < all; i0 += 4 * 128) {       // four loads on their way together
+    uint4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + u * 128, g = i / units, c = i % units;
+      v[u] = held && i < all ? pooled[(((size_t)page * nkv + g) * pool_rows + s % pool_rows) * units + c] : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i0 + u * 128 < all) out[(size_t)blockIdx.x * all + i0 + u * 128] = v[u];
   }
 }
 

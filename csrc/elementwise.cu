@@ -16,9 +16,9 @@ namespace tahb {
 // registers (H <= 128 * 8 * VPT elements).
 // ---------------------------------------------------------------------------------------------
 template <int VPT>
-__global__ void __launch_bounds__(128) rmsnorm_kernel(const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(128) rmsnorm_kernel(const __nv_bfloat16* x,
                                                       const __nv_bfloat16* __restrict__ w,
-                                                      __nv_bfloat16* __restrict__ y, int H, long long ldx,
+                                                      __nv_bfloat16* y, int H, long long ldx,
                                                       long long ldy, float eps) {
   pdl_wait();
   const int row = blockIdx.x;
@@ -83,12 +83,12 @@ __global__ void __launch_bounds__(128) rmsnorm_kernel(const __nv_bfloat16* __res
 constexpr int NORM_LORA_SLICES = 8;
 constexpr int NORM_LORA_SLOTS = 32;
 
-__global__ void __launch_bounds__(256) rmsnorm_lora_kernel(const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(256) rmsnorm_lora_kernel(const __nv_bfloat16* x,
                                                            const __nv_bfloat16* __restrict__ w,
-                                                           __nv_bfloat16* __restrict__ y, int M, int H, long long ldx,
-                                                           long long ldy, float eps, const int* __restrict__ gate,
+                                                           __nv_bfloat16* y, int M, int H, long long ldx,
+                                                           long long ldy, float eps, const int* gate,
                                                            const __nv_bfloat16* __restrict__ A,
-                                                           __nv_bfloat16* __restrict__ T, int R, long long ldt) {
+                                                           __nv_bfloat16* T, int R, long long ldt) {
   pdl_wait();
   extern __shared__ uint4 srow[];            // H / 8 vectors: the normalised row (LoRA CTAs only)
   __shared__ float red[8];
@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(256) rmsnorm_lora_kernel(const __nv_bfloat16* 
   int want = lid / NORM_LORA_SLICES;         // index of this CTA's gated row among the gated rows
   const int nvec = H / 8;
   const uint4* wr = reinterpret_cast<const uint4*>(w);
+  const bool clear = norm_cta && (gate == nullptr || gate[blockIdx.x] == 0);
   for (;;) {
     int row;
     if (norm_cta) {
@@ -183,7 +184,7 @@ __global__ void __launch_bounds__(256) rmsnorm_lora_kernel(const __nv_bfloat16* 
     }
     __nv_bfloat16* out = T + (size_t)row * ldt;
     if (norm_cta) {
-      if (gate == nullptr || gate[row] == 0)
+      if (clear)
         for (int j = tid; j < R; j += 256) out[j] = __float2bfloat16_rn(0.f);
       return;
     }
@@ -379,11 +380,11 @@ __global__ void rope_table_kernel(const int* __restrict__ pos, __nv_bfloat16* __
 // One warp per row (D <= 4096, D % 8 == 0); with `dot_w` the normalised row is not stored but reduced
 // against dot_w (+ dot_b) into z[r] (fp32): the output layer LayerNorm -> Linear(D, 1) of the decider.
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) layernorm_kernel(const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(128) layernorm_kernel(const __nv_bfloat16* x,
                                                         const __nv_bfloat16* __restrict__ w,
-                                                        const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y,
+                                                        const __nv_bfloat16* __restrict__ b, __nv_bfloat16* y,
                                                         const __nv_bfloat16* __restrict__ dot_w,
-                                                        const __nv_bfloat16* __restrict__ dot_b, float* __restrict__ z,
+                                                        const __nv_bfloat16* __restrict__ dot_b, float* z,
                                                         int M, int D, long long ldx, long long ldy, float eps) {
   pdl_launch_dependents();
   pdl_wait();
@@ -473,9 +474,9 @@ __global__ void embed_gather_kernel(const __nv_bfloat16* __restrict__ E, const i
 // Rows whose gate is 0 only clear their output.  Meant for decode ticks where a handful of rows
 // are at depth >= 1; dense passes use the tensor-core GEMM instead.
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) lora_a_rows_dense_kernel(const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(256) lora_a_rows_dense_kernel(const __nv_bfloat16* x,
                                                           const __nv_bfloat16* __restrict__ A,
-                                                          __nv_bfloat16* __restrict__ T, const int* __restrict__ gate,
+                                                          __nv_bfloat16* T, const int* gate,
                                                           int K, int R, long long ldx, long long ldt,
                                                           const uint32_t* wait_flag, const uint32_t* wait_target,
                                                           int wait_world, int* status, unsigned long long wait_limit) {
@@ -519,9 +520,9 @@ __global__ void __launch_bounds__(256) lora_a_rows_dense_kernel(const __nv_bfloa
 // ... for its 8 outputs (one per warp); the x == 0 CTAs also clear their 8 columns of the rows that
 // are gated off.
 constexpr int LORA_SLOTS = 32;
-__global__ void __launch_bounds__(256) lora_a_rows_kernel(const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(256) lora_a_rows_kernel(const __nv_bfloat16* x,
                                                           const __nv_bfloat16* __restrict__ A,
-                                                          __nv_bfloat16* __restrict__ T, const int* __restrict__ gate,
+                                                          __nv_bfloat16* T, const int* gate,
                                                           int M, int K, int R, long long ldx, long long ldt,
                                                           const uint32_t* wait_flag, const uint32_t* wait_target,
                                                           int wait_world, int* status, unsigned long long wait_limit) {

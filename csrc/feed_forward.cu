@@ -69,8 +69,8 @@ template <> struct Vec8<__nv_bfloat16> {
 constexpr int PN_THREADS = 256;
 
 template <typename T, int VPT>
-__global__ void __launch_bounds__(PN_THREADS) poly_norm_kernel(const T* __restrict__ z, long long ldz,
-                                                               const float* __restrict__ act, T* __restrict__ out,
+__global__ void __launch_bounds__(PN_THREADS) poly_norm_kernel(const T* z, long long ldz,
+                                                               const float* __restrict__ act, T* out,
                                                                long long ldo, int n, int np, float eps) {
   pdl_launch_dependents();
   pdl_wait();
@@ -304,11 +304,11 @@ __global__ void __launch_bounds__(ROUTE_THREADS) moe_route_kernel(const RoutePar
 }
 
 // One CTA per token: its row (16-byte units) goes to a list row of each of its experts; list_weight and slot on the way.
-__global__ void __launch_bounds__(128) moe_gather_kernel(const uint4* __restrict__ h, int units, long long ld_units, int top,
-                                                         const int* __restrict__ expert, const int* __restrict__ rank,
-                                                         const float* __restrict__ weight, const int* __restrict__ seg,
-                                                         uint4* __restrict__ list, float* __restrict__ list_weight,
-                                                         int* __restrict__ slot, int list_rows, int* status) {
+__global__ void __launch_bounds__(128) moe_gather_kernel(const uint4* h, int units, long long ld_units, int top,
+                                                         const int* expert, const int* rank,
+                                                         const float* weight, const int* seg,
+                                                         uint4* list, float* list_weight,
+                                                         int* slot, int list_rows, int* status) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ int s_slot[64];
@@ -325,9 +325,15 @@ __global__ void __launch_bounds__(128) moe_gather_kernel(const uint4* __restrict
     list_weight[s] = weight[a];
   }
   __syncthreads();
-  for (int c = threadIdx.x; c < units; c += 128) {
-    const uint4 v = h[t * ld_units + c];
-    for (int j = 0; j < top; ++j) list[(size_t)s_slot[j] * units + c] = v;
+  for (int c0 = threadIdx.x; c0 < units; c0 += 2 * 128) {     // two loads on their way together: rows of 2048
+    uint4 v[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (c0 + u * 128 < units) v[u] = h[t * ld_units + c0 + u * 128];
+    for (int j = 0; j < top; ++j)
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (c0 + u * 128 < units) list[(size_t)s_slot[j] * units + c0 + u * 128] = v[u];
   }
 }
 

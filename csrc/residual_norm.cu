@@ -163,11 +163,11 @@ __device__ __forceinline__ float2 sin_cos_pair(float p, float hi, float lo) {
 // sees (null: one stream as it is).  add [ld]: vector added to the scaled embedding (zero in the padding), or null.  CENTER: layer
 // norm (groups is 1).
 template <typename T, int VPT, bool CENTER>
-__global__ void __launch_bounds__(RN_THREADS) embed_norm_kernel(const T* __restrict__ E, const int* __restrict__ tok,
-                                                                float scale, const int* __restrict__ pos,
+__global__ void __launch_bounds__(RN_THREADS) embed_norm_kernel(const T* __restrict__ E, const int* tok,
+                                                                float scale, const int* pos,
                                                                 const float* __restrict__ freq, int streams, const float* __restrict__ w_in,
-                                                                const float* __restrict__ add, float* __restrict__ x, const float* __restrict__ w,
-                                                                T* __restrict__ h, int vocab, int width, int groups, int ld,
+                                                                const float* add, float* x, const float* __restrict__ w,
+                                                                T* h, int vocab, int width, int groups, int ld,
                                                                 float eps) {
   pdl_launch_dependents();
   pdl_wait();
@@ -395,8 +395,8 @@ __global__ void __launch_bounds__(RN_THREADS) streams_norm_kernel(const StreamsP
 }
 
 // out[t][i] = mscale * (cos, sin) of pos[t] * f_i; freq: [2, half] high parts, then low parts
-__global__ void rotary_table_kernel(const int* __restrict__ pos, const float* __restrict__ freq, float mscale,
-                                    float2* __restrict__ out, int M, int half) {
+__global__ void rotary_table_kernel(const int* pos, const float* __restrict__ freq, float mscale,
+                                    float2* out, int M, int half) {
   pdl_launch_dependents();
   pdl_wait();
   const int n = M * half;
@@ -500,9 +500,9 @@ __global__ void __launch_bounds__(RN_THREADS) residual_norm_kernel(const Residua
 constexpr int FL_THREADS = 256;
 
 template <typename T, int TOK>
-__global__ void __launch_bounds__(FL_THREADS) few_linear_kernel(const T* __restrict__ x, long long ldx,
+__global__ void __launch_bounds__(FL_THREADS) few_linear_kernel(const T* x, long long ldx,
                                                                 const T* __restrict__ w, const float* __restrict__ b,
-                                                                float* __restrict__ out, int M, int K, int F) {
+                                                                float* out, int M, int K, int F) {
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ float xs[];              // [TOK][K]
@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(FL_THREADS) few_linear_kernel(const T* __restr
 template <int FLM_NT, int FLM_WARPS>       // feature tiles of 8 and warps of a CTA
 __global__ void __launch_bounds__(FLM_WARPS * 32) few_linear_mma_kernel(const __nv_bfloat16* x, long long ldx,
                                                                     const __nv_bfloat16* __restrict__ w,
-                                                                    const float* __restrict__ b, float* __restrict__ out,
+                                                                    const float* __restrict__ b, float* out,
                                                                     int M, int K, int F) {
   pdl_launch_dependents();
   pdl_wait();

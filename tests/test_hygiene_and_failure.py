@@ -49,13 +49,42 @@ def test_no_cluster_multicast_no_triton_no_disassembly():
 
 def test_every_device_wait_is_bounded():
     """Every spin in the kernels goes through a helper with a time limit."""
-    for name in ("gemm_tcgen05.cu", "attn_decode.cu", "attn_prefill.cu", "attn_window.cu", "mlstm.cu"):
+    for name in ("gemm_tcgen05.cu", "gemm_persist.cu", "attn_decode.cu", "attn_prefill.cu", "attn_prefill_bwd.cu", "attn_window.cu", "mlstm.cu"):
         text = open(os.path.join(ROOT, "csrc", name)).read()
         assert "mbar_try_wait(" not in text            # only the bounded mbar_wait() may be called from kernels
         assert "while (true)" not in text and "while(1)" not in text
     for name in ("comm.cu", "optim.cu"):
         text = open(os.path.join(ROOT, "csrc", name)).read()
         assert "WAIT_TIMEOUT_NS" in text and "STATUS_TIMEOUT_PEER_FLAG" in text
+    text = open(os.path.join(ROOT, "csrc", "gemm_few.cu")).read()
+    assert text.count("ld_acquire(p.sync)") == text.count("now - t0 > WAIT_TIMEOUT_NS") == 1
+
+
+# operands that are constants of a chain of launches: weights and tables
+_CONSTANTS = {"w", "A", "E", "b", "freq", "w_in", "act", "dot_w", "dot_b"}
+
+
+def _balanced(text, i, opening, closing):
+    depth = 1
+    while depth:
+        depth += (text[i] == opening) - (text[i] == closing)
+        i += 1
+    return i
+
+
+def test_kernels_that_start_early_read_what_was_written_before_through_plain_pointers():
+    """A kernel that waits for the launch before it (pdl_wait) has ``__restrict__`` on weights and tables alone: what is read or written through
+    such a pointer may move ahead of the wait."""
+    seen, bad = 0, []
+    for path in _sources((".cu", ".cuh")):
+        text = open(path, encoding="utf-8").read()
+        for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\([^()]*(?:\([^()]*\)[^()]*)*\)\s*)?(\w+)\s*\(", text):
+            end = _balanced(text, m.end(), "(", ")")
+            body = re.compile(r"[{;]").search(text, end).start()
+            if text[body] == "{" and "pdl_wait()" in text[body:_balanced(text, body + 1, "{", "}")]:
+                seen += 1
+                bad += [(m.group(1), n) for n in re.findall(r"__restrict__\s+(\w+)", text[m.end():end]) if n not in _CONSTANTS]
+    assert seen > 20 and not bad, bad
 
 
 class _DictStore(dict):
