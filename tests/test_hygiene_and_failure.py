@@ -49,13 +49,20 @@ def test_no_cluster_multicast_no_triton_no_disassembly():
 
 def test_every_device_wait_is_bounded():
     """Every spin in the kernels goes through a helper with a time limit."""
-    for name in ("gemm_tcgen05.cu", "gemm_persist.cu", "attn_decode.cu", "attn_prefill.cu", "attn_prefill_bwd.cu", "attn_window.cu", "mlstm.cu"):
+    for name in ("gemm_tcgen05.cu", "attn_decode.cu", "attn_prefill.cu", "attn_window.cu", "mlstm.cu"):
         text = open(os.path.join(ROOT, "csrc", name)).read()
         assert "mbar_try_wait(" not in text            # only the bounded mbar_wait() may be called from kernels
         assert "while (true)" not in text and "while(1)" not in text
     for name in ("comm.cu", "optim.cu"):
         text = open(os.path.join(ROOT, "csrc", name)).read()
         assert "WAIT_TIMEOUT_NS" in text and "STATUS_TIMEOUT_PEER_FLAG" in text
+
+
+def test_waits_of_the_persistent_backward_and_few_token_kernels_are_bounded():
+    """The same for the persistent product, the attention backward and the one wait of the fused few-token product."""
+    for name in ("gemm_persist.cu", "attn_prefill_bwd.cu"):
+        text = open(os.path.join(ROOT, "csrc", name)).read()
+        assert "mbar_try_wait(" not in text and "while (true)" not in text and "while(1)" not in text
     text = open(os.path.join(ROOT, "csrc", "gemm_few.cu")).read()
     assert text.count("ld_acquire(p.sync)") == text.count("now - t0 > WAIT_TIMEOUT_NS") == 1
 

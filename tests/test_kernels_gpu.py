@@ -941,12 +941,39 @@ def test_training_step_kernel_path_matches_torch_path_multi_tile(monkeypatch):
         assert float(cos) > 0.97, (name, float(cos))
 
 
-@pytest.mark.parametrize("M,F,Kd,res,how", [(64, 256, 256, False, {}), (64, 256, 256, True, dict(splits=2, bn=64)), (64, 256, 256, True, dict(splits=1, bn=64)),
-                                            (300, 512, 256, True, dict(pair=True)), (1500, 2048, 2048, False, {}), (1500, 2048, 2048, True, {})])
-def test_peer_flag_wait_runs_out_and_reports_a_timeout(M, F, Kd, res, how):
+def test_peer_flag_wait_runs_out_and_reports_a_timeout():
     """A consumer GEMM that waits for rows a peer would broadcast: nothing advances the landing flags, the wait
     limit is 5 ms, so the kernel gives up, records the timeout code and returns; the host reads the status word
-    and raises.  Nothing traps or hangs, and the context stays usable.  The persistent form writes nothing then."""
+    and raises.  Nothing traps or hangs, and the context stays usable."""
+    import time
+    Kc = _cuda()
+    x, w = _rand(64, 256, seed=1), _rand(256, 256, scale=256 ** -0.5, seed=2)
+    flags = torch.zeros(2, dtype=torch.int32, device="cuda")
+    targets = torch.ones(2, dtype=torch.int32, device="cuda")
+    prev = Kc.set_peer_wait_limit_ns(5_000_000)
+    try:
+        torch.cuda.synchronize()
+        t0 = time.time()
+        Kc.gemm(x, w, tp_wait=(flags, targets))
+        Kc.wait_flags(flags, targets)
+        torch.cuda.synchronize()
+        assert time.time() - t0 < 1.0                                   # two 5 ms limits, not the 2 s default
+        with pytest.raises(Kc.KernelTimeout, match="peer flag"):
+            Kc.check_status()
+    finally:
+        Kc.set_peer_wait_limit_ns(prev)
+    Kc.check_status()                                                   # the status word was cleared
+    flags.fill_(1)                                                      # the flags arrive: same launch succeeds
+    y = Kc.gemm(x, w, tp_wait=(flags, targets))
+    Kc.check_status()
+    _close(y, x.float() @ w.float().t(), atol=2e-2, rtol=2e-2)
+
+
+@pytest.mark.parametrize("M,F,Kd,res,how", [(64, 256, 256, True, dict(splits=2, bn=64)), (64, 256, 256, True, dict(splits=1, bn=64)),
+                                            (300, 512, 256, True, dict(pair=True)), (1500, 2048, 2048, False, {}), (1500, 2048, 2048, True, {})])
+def test_peer_flag_wait_runs_out_in_every_form(M, F, Kd, res, how):
+    """The wait for peers' rows runs out in split, paired and persistent products, with and without a residual: the status is reported, the
+    persistent form writes nothing, and the same launch succeeds once the flags are there."""
     import time
     Kc = _cuda()
     x, w, r = _rand(M, Kd, seed=1), _rand(F, Kd, scale=Kd ** -0.5, seed=2), _rand(M, F, seed=3) if res else None
