@@ -186,7 +186,7 @@ def plan_gemm_kept(M: int, F: int, K: int, R: int = 0):
     return _gemm_cost(M, F, K, R, False, split)[1:]
 
 
-# the two-tile ("pair") GEMM is a candidate above 256 tokens; TAH_B200_GEMM_PAIR=0 turns it off
+# the persistent GEMM on pairs of SMs and the two-tile ("pair") GEMM are candidates above 128 and 256 tokens; TAH_B200_GEMM_PAIR=0 turns both off
 PAIR_AUTO = os.environ.get("TAH_B200_GEMM_PAIR", "1") != "0"
 
 
@@ -230,9 +230,15 @@ def _tiles_cost(M: int, rows: int, K: int, can_pair: bool, can_split: bool, x_t:
 SM_PAIRS = SM_COUNT // 2
 
 
-@functools.lru_cache(maxsize=4096)
 def plan_persist(M: int, rows: int, K: int, R: int = 0, glu: bool = False, x_t: bool = False, can_pair: bool = True) -> int:
-    """Tile width of the persistent form (``csrc/gemm_persist.cu``) for more than 128 tokens, or 0 where one tile per CTA is faster: few tiles
+    """Tile width of the persistent form (``csrc/gemm_persist.cu``) for more than 128 tokens, or 0 where it is turned off or one tile per CTA is
+    faster."""
+    return _persist_cost(M, rows, K, R, glu, x_t, can_pair) if PAIR_AUTO else 0
+
+
+@functools.lru_cache(maxsize=4096)
+def _persist_cost(M: int, rows: int, K: int, R: int, glu: bool, x_t: bool, can_pair: bool) -> int:
+    """:func:`plan_persist` by estimates of both forms.  One tile per CTA is faster for few tiles
     with a long reduction, which that form splits (us, persistent / one tile per CTA at 264 tokens: 2048 x 6144 20.2 / 17.2, 12288 x 2048 SwiGLU
     24.0 / 21.1, 2048 x 12288 36.6 / 23.2, 6144 x 2048 14.4 / 11.9; at 2048 x 6144 level at 504 tokens, 32.1 / 35.2 at 1504), and most products of up to
     256 tokens (4096 x 2048 at 256 9.4 / 9.6, 2048 x 2048 9.2 / 8.4; but 12288 x 2048 SwiGLU 17.1 / 18.7, 151936 x 2048 142 / 171).
@@ -254,7 +260,7 @@ def plan_persist(M: int, rows: int, K: int, R: int = 0, glu: bool = False, x_t: 
         other = (-(-(-(-rows // 128)) // SM_COUNT) * ((K + R) / 64 * (0.195, 0.25, 0.33)[(bn > 64) + (bn > 128)] + 4.8 + 0.015 * bn) if glu else
                  _gemm_cost(M, rows, K, R, False)[0])
         return best[1] if best[0] < other else 0
-    other = _tiles_cost(M, rows, K + R, can_pair and PAIR_AUTO and rows % 256 == 0, not glu, x_t)[0]
+    other = _tiles_cost(M, rows, K + R, can_pair and rows % 256 == 0, not glu, x_t)[0]
     return best[1] if best[0] <= 1.08 * other else 0
 
 

@@ -489,6 +489,43 @@ def test_persistent_tile_plan():
     assert not any(cuda.plan_persist(M, rows, 2048) for M in (129, 192, 256) for rows in (1024, 2048, 4096))
 
 
+def _launches(monkeypatch):
+    """The products' entry points as fakes: what is called, in a list."""
+    from tah_b200.ops import cuda
+    called = []
+
+    class Lib:
+        def __getattr__(self, name):
+            return lambda *a: called.append(name) or 0
+
+    monkeypatch.setattr(cuda, "lib", Lib)
+    monkeypatch.setattr(cuda, "_check_bf16_2d", lambda t, name: None)
+    monkeypatch.setattr(cuda, "status_word", lambda device: None)
+    monkeypatch.setattr(cuda, "_stream", lambda: None)
+    monkeypatch.setattr(cuda, "_p", lambda t: None)
+    return cuda, called
+
+
+def test_one_tile_switch_turns_off_the_persistent_form(monkeypatch):
+    """``TAH_B200_GEMM_PAIR=0``: one-tile forms only, whatever was planned before."""
+    cuda, called = _launches(monkeypatch)
+    t = lambda *s: torch.zeros(*s, dtype=torch.bfloat16)
+    x, w = t(1500, 2048), t(2048, 2048)
+
+    def forms():
+        called.clear()
+        cuda.gemm(x, w)
+        cuda.gemm_t(x, w, w_t=True)
+        cuda.xielu_linear(x, w, 0.8, 0.5)
+        return called[:]
+
+    assert forms() == ["tahb_gemm_persist"] * 3
+    monkeypatch.setattr(cuda, "PAIR_AUTO", False)
+    assert forms() == ["tahb_gemm", "tahb_gemm_t", "tahb_gemm_xielu"]
+    for M in (200, 600, 1504, 16000):
+        assert cuda.plan_persist(M, 4096, 2048) == 0
+
+
 def test_host_plan_of_a_prefill_is_the_device_one():
     """Query tiles and page assignment of a prefill worked out on the host: what the tensor operations give, over row counts and lengths
     (empty rows, whole pages, one past them), and the same refusal of a pool that is too small."""
