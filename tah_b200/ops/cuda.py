@@ -308,6 +308,40 @@ def wait_flags(flags: torch.Tensor, targets: torch.Tensor) -> None:
         "tahb_wait_flags")
 
 
+def _persist_width(M: int, rows: int, K: int, R: int, swiglu_interleaved: bool, const_w: bool) -> int:
+    """:func:`plan_persist` for :func:`gemm`: up to 256 tokens with weights that training changes only where their split (:func:`plan_gemm_kept`)
+    is none."""
+    wide = plan_persist(M, rows, K, R, swiglu_interleaved)
+    return wide if wide and (M > 256 or const_w or swiglu_interleaved or plan_gemm_kept(M, rows, K, R)[1] == 1) else 0
+
+
+def gemm_form(M: int, rows: int, K: int, R: int = 0, *, swiglu: bool = False, gelu: bool = False, swiglu_interleaved: bool = False,
+              const_w: bool = False):
+    """``(form, tile width, split)`` that :func:`gemm` takes by sizes, for operands on whole pieces of 16 bytes: "few", "persist", "pair" or
+    "tile"."""
+    if few_shape(M, rows, K, R, const_w):
+        return "few", 0, 1
+    wide = _persist_width(M, rows, K, R, swiglu_interleaved, const_w) if M > 128 and not swiglu else 0
+    if wide:
+        return "persist", wide, 1
+    pair, bn, splits = _plan_tiles(M, rows, K, R, swiglu, gelu, swiglu_interleaved, kept=not const_w)
+    return "pair" if pair else "tile", bn, splits
+
+
+def gemm_t_form(M: int, F: int, K: int, x_t: bool, w_t: bool):
+    """The same of :func:`gemm_t`."""
+    can_pair = F % 256 == 0 and (not x_t or M % 64 == 0)
+    if M > 256:
+        whole = (K % 64 == 0 or x_t and w_t) and (not w_t or F % 128 == 0)
+        wide = plan_persist(M, F, K, 0, False, x_t, can_pair) if whole else 0
+        if wide:
+            return "persist", wide, 1
+        pair, bn, splits = plan_tiles(M, F, K, can_pair and PAIR_AUTO, True, x_t)
+        return "pair" if pair else "tile", bn or 256, 1 if pair else splits
+    bn, splits = plan_gemm_kept(M, F, (K + 63) // 64 * 64)
+    return "tile", max(bn, 64) if x_t else bn, splits
+
+
 def _plan_tiles(M: int, rows: int, K: int, R: int, swiglu: bool, gelu: bool, swiglu_interleaved: bool, pair=None, bn: int = 0, splits=None,
                 stores=(), kept: bool = False):
     """``(pair, bn, splits)`` of a tcgen05 product with a weight of ``rows`` rows.  ``stores``: the output and the residual where there is
@@ -344,8 +378,9 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
 
     ``pair``: every CTA computes two 128-feature output tiles (features ``f`` and ``F/2 + f``) from one activation tile
     of 256 tokens (or ``bn`` 128, 192), unsplit.  It halves the activation bytes a CTA pulls per unit of work, which is what
-    bounds the kernel at large token counts (1350-1400 vs 915-1100 TFLOP/s at 8192+ tokens); default: by
-    :func:`plan_tiles` above 256 tokens (also with ``swiglu_interleaved``).
+    bounds that kernel at large token counts.  Default: the few-token form, above 128 tokens the persistent one where :func:`plan_persist` gives
+    it a width, else one tile or a pair by :func:`plan_tiles` above 256 tokens (:func:`gemm_form`).  A tile width, a split or ``pair`` that the
+    caller gives excludes the persistent form.
 
     ``swiglu_interleaved``: the rows of ``w`` (and ``w2``) alternate ``gate_i, up_i`` (see :func:`interleave_gate_up`)
     and ``out[M, F/2] = silu(gate) * up``: one accumulator and one wide MMA per k step, the faster SwiGLU form.
@@ -389,9 +424,8 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
     # the plan, which is kept, before the look at every operand (4 us of host time)
     if (pair is None and bn == 0 and splits is None and tp_push is None and not swiglu and not (gelu and residual is not None) and
             M > 128 and F > 0 and K > 0):
-        wide = plan_persist(M, F, K, R, swiglu_interleaved)
-        if (wide and (M > 256 or const_w or swiglu_interleaved or plan_gemm_kept(M, F, K, R)[1] == 1) and
-                _persist_ok(x, w, out, residual, x2, w2)):
+        wide = _persist_width(M, F, K, R, swiglu_interleaved, const_w)
+        if wide and _persist_ok(x, w, out, residual, x2, w2):
             return _gemm_persist(x, w, out, residual, x2, w2, 1 if gelu else 2 if swiglu_interleaved else 0, wide, tp_wait=tp_wait)
     pair, bn, splits = _plan_tiles(M, w.shape[0], K, R, swiglu, gelu, swiglu_interleaved, pair, bn, splits,
                                    () if tp_push is not None else (out, residual), kept=not const_w and tp_push is None and tp_wait is None)

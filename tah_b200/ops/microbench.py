@@ -92,10 +92,14 @@ def bench_gemm(a):
     t = _time(fn, a.iters, a.warmup)
     flops = 2.0 * M * wrows * (Kd + R)
     byts = (wrows * (Kd + R) + M * (Kd + R) + M * F) * 2
-    auto_pair = M > 256 and not a.bn and not a.swiglu and K.plan_tiles(M, wrows, Kd + R, K.PAIR_AUTO and wrows % 256 == 0, not il)[0]
+    if a.bn or a.pair is not None:
+        form = ["pair" if a.pair else "tile", a.bn, a.splits]
+    elif a.transposed:
+        form = K.gemm_t_form(M, F, Kd, a.transposed == "wgrad", True)
+    else:
+        form = K.gemm_form(M, wrows, Kd, R, swiglu=a.swiglu, swiglu_interleaved=il)
     res = {"op": "gemm", "M": M, "F": F, "K": Kd, "R": R, "swiglu": a.swiglu, "swiglu_interleaved": il,
-           "transposed": a.transposed, "pair": bool(a.pair) if a.pair is not None else auto_pair,
-           "plan_bn_splits": [a.bn, a.splits] if a.bn else K.plan_gemm(M, F, Kd, R, a.swiglu)}
+           "transposed": a.transposed, "form_bn_splits": list(form)}
     if a.cublas:
         ref = lambda i: torch.matmul(xs[i % n], ws[i % n].t())
         res["cublas_us"] = round(_time(ref, a.iters, a.warmup) * 1e6, 2)

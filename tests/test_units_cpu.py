@@ -523,7 +523,25 @@ def test_one_tile_switch_turns_off_the_persistent_form(monkeypatch):
     monkeypatch.setattr(cuda, "PAIR_AUTO", False)
     assert forms() == ["tahb_gemm", "tahb_gemm_t", "tahb_gemm_xielu"]
     for M in (200, 600, 1504, 16000):
-        assert cuda.plan_persist(M, 4096, 2048) == 0
+        assert cuda.plan_persist(M, 4096, 2048) == 0 and cuda.gemm_form(M, 4096, 2048)[0] == cuda.gemm_t_form(M, 4096, 2048, True, True)[0] == "tile"
+
+
+def test_form_of_a_product_is_the_one_launched(monkeypatch):
+    """What :func:`gemm_form` and :func:`gemm_t_form` name is what :func:`gemm` and :func:`gemm_t` launch."""
+    cuda, called = _launches(monkeypatch)
+    entry = {"few": "tahb_gemm_few", "persist": "tahb_gemm_persist", "pair": "tahb_gemm", "tile": "tahb_gemm"}
+    t = lambda *s: torch.empty(*s, dtype=torch.bfloat16)
+    for M in (1, 16, 40, 100, 130, 256, 257, 504, 1500, 5000):
+        for rows, K in ((64, 256), (320, 448), (2048, 2048), (4096, 1024), (2048, 6144), (12288, 2048)):
+            for how in ({}, dict(const_w=True), dict(swiglu=True), dict(swiglu_interleaved=True), dict(gelu=True)):
+                called.clear()
+                cuda.gemm(t(M, K), t(rows, K), **how)
+                assert called == [entry[cuda.gemm_form(M, rows, K, **how)[0]]], (M, rows, K, how)
+            for x_t, w_t in ((False, True), (True, True)):
+                called.clear()
+                cuda.gemm_t(t(K, M + -M % 8) if x_t else t(M, K), t(K, rows), x_t=x_t, w_t=w_t)
+                form = cuda.gemm_t_form(M + -M % 8 if x_t else M, rows, K, x_t, w_t)[0]
+                assert called == ["tahb_gemm_persist" if form == "persist" else "tahb_gemm_t"], (M, rows, K, x_t, w_t)
 
 
 def test_host_plan_of_a_prefill_is_the_device_one():
