@@ -123,6 +123,8 @@ def bench_tied_keys(a):
     """``--m`` tokens of rows of ``--ctx``."""
     from tah_b200.engine.kv_cache import LayerKV
     M, T = a.m, min(a.ctx, a.m)
+    if T % 16 or M % T:
+        raise ValueError("--m takes whole rows of --ctx (or one row) and whole pages of 16")
     pages, S = M // 16, LayerKV(block=a.block or 16).pool_rows(16)
     k, pool, means = _bf(M, a.nkv * a.hd + 2048), _bf(pages, a.nkv * 16 * a.hd), _bf(pages, a.nkv * S * a.hd)
     slot = torch.arange(M, device="cuda", dtype=torch.int32)
@@ -303,7 +305,7 @@ def bench_latent_query(a):
 
 
 def bench_latent_gather(a):
-    pages, row = a.m // 16, a.rank + a.rot
+    pages, row = (a.m + 15) // 16, a.rank + a.rot
     pool, src = _bf(pages, 16 * row), torch.randperm(pages, device="cuda").to(torch.int32)
     out = _bf(pages * 16, (row + 63) // 64 * 64)
     return {"op": "latent_gather", "tokens": a.m}, lambda i: K.latent_gather(pool, src, 16, row, out), 0.0, a.m * (row + out.shape[1]) * 2
