@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(QKVP_WARPS * 32) qkv_post_128_kernel(const Qkv
   if (sl >= 0)
     page = reinterpret_cast<__nv_bfloat16*>(p.cache) + ((size_t)(sl / p.page_size) * 2 * p.nkv * p.page_size + sl % p.page_size) * HD + c;
   for (int h0 = warp; h0 < heads; h0 += QKVP_U * QKVP_WARPS) {
-    QkvPiece<4, true> in[QKVP_U];
+    QkvPiece<4> in[QKVP_U];
     float4 b[QKVP_U];
 #pragma unroll
     for (int u = 0; u < QKVP_U; ++u) {
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(QKVP_WARPS * 32) qkv_post_128_kernel(const Qkv
         const float4 g = *reinterpret_cast<const float4*>(w + c);
         x[0] *= r * g.x; x[1] *= r * g.y; x[2] *= r * g.z; x[3] *= r * g.w;
       }
-      QkvPiece<4, true> out;
+      QkvPiece<4> out;
 #pragma unroll
       for (int i = 0; i < 4; ++i) out.v[i] = __float2bfloat16_rn(x[i]);
       if (is_q) out.store(reinterpret_cast<__nv_bfloat16*>(p.q_out) + ((size_t)t * p.nq + h) * HD + c);

@@ -390,23 +390,48 @@ __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(_
 // main loop).  Relative error ~2^-21, far below the bf16 rounding that follows every use.
 __device__ __forceinline__ float silu(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
 
-// EPL consecutive bf16 of a lane, moved in one access when they lie on a boundary of their size (WIDE), else one by one.
-template <int EPL, bool WIDE>
+// EPL consecutive bf16 of a lane, moved BYTES (a power of two from 2 on) at a time: everything they lie on has to start on such a boundary.
+// 2 also takes words of 4 bytes, off their boundary shifted out of the words around the piece (loads) or with one element at each end (stores).
+template <int EPL, int BYTES = EPL * 2>
 struct alignas(EPL * 2) QkvPiece {
+  static_assert(BYTES >= 2 && BYTES <= EPL * 2 && BYTES <= 16, "words of a piece");
   __nv_bfloat16 v[EPL];
-  using Word = typename std::conditional<EPL == 8, uint4, typename std::conditional<EPL == 4, uint2, uint32_t>::type>::type;
+  using Word = typename std::conditional<
+      BYTES == 16, uint4, typename std::conditional<BYTES == 8, uint2, typename std::conditional<BYTES == 4, uint32_t, __nv_bfloat16>::type>::type>::type;
   __device__ __forceinline__ __nv_bfloat162& pair(int i) { return reinterpret_cast<__nv_bfloat162*>(v)[i]; }
   __device__ __forceinline__ void load(const __nv_bfloat16* src) {
-    if constexpr (WIDE) *reinterpret_cast<Word*>(v) = *reinterpret_cast<const Word*>(src);
-    else
+    if constexpr (BYTES == 2) {
+      uint32_t* o = reinterpret_cast<uint32_t*>(v);
+      const uint32_t odd = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 2) / 2;
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(src - odd);
+      uint32_t a = w[0];
 #pragma unroll
-      for (int i = 0; i < EPL; ++i) v[i] = src[i];
+      for (int i = 0; i < EPL / 2; ++i) {
+        const uint32_t b = i + 1 < EPL / 2 || odd ? w[i + 1] : 0u;      // the last word of an odd piece holds its last element
+        o[i] = __funnelshift_r(a, b, odd * 16);
+        a = b;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < EPL * 2 / BYTES; ++i) reinterpret_cast<Word*>(v)[i] = reinterpret_cast<const Word*>(src)[i];
+    }
   }
   __device__ __forceinline__ void store(__nv_bfloat16* dst) const {
-    if constexpr (WIDE) *reinterpret_cast<Word*>(dst) = *reinterpret_cast<const Word*>(v);
-    else
+    if constexpr (BYTES == 2) {
+      const uint32_t* o = reinterpret_cast<const uint32_t*>(v);
+      if (reinterpret_cast<uintptr_t>(dst) & 2) {
+        dst[0] = v[0];
 #pragma unroll
-      for (int i = 0; i < EPL; ++i) dst[i] = v[i];
+        for (int i = 0; i + 1 < EPL / 2; ++i) reinterpret_cast<uint32_t*>(dst + 1)[i] = __funnelshift_r(o[i], o[i + 1], 16);
+        dst[EPL - 1] = v[EPL - 1];
+      } else {
+#pragma unroll
+        for (int i = 0; i < EPL / 2; ++i) reinterpret_cast<uint32_t*>(dst)[i] = o[i];
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < EPL * 2 / BYTES; ++i) reinterpret_cast<Word*>(dst)[i] = reinterpret_cast<const Word*>(v)[i];
+    }
   }
 };
 

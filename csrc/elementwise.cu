@@ -256,14 +256,15 @@ struct QkvRopeParams {
 // sum are 16-bit operations on pairs (the same bits: products of two 16-bit numbers are exact in 32), the partner's dims come two to a
 // shuffle, and the squares are summed as 32 lanes would: 77 us, 4096 tokens 35 -> 27 us, 1024 14.3 -> 12.3 us.  48 registers (five CTAs an SM):
 // with 64 84 us.  A loop over tokens in four CTAs an SM, the next token's loads ahead, took longer: 131 us with four elements a lane.
-// WIDE: every pointer and row lies on a 16-byte boundary; else element by element.
+// BYTES: the boundary that every pointer and row lies on, 16, 8, 4 or 2; a lane's 16 bytes are moved so many at a time.  us, 3000 tokens of
+// 16 + 16 heads: 12.9, 13.6, 16.0, 24.4 (two bytes element by element 36.0).
 constexpr int QKV_U = 2, QKV_WARPS = 8;
-template <int HD, bool WIDE>
+template <int HD, int BYTES>
 __global__ void __launch_bounds__(QKV_WARPS * 32, 5) qk_norm_rope_kv_kernel(const QkvRopeParams p) {
   pdl_wait();
   constexpr int LPH = HD / 8, HPW = 32 / LPH;   // lanes of a head, heads of a warp
   constexpr int CH = HPW;                       // 128: two sums of four squares a lane, 64: four of two
-  using Piece = QkvPiece<8, WIDE>;
+  using Piece = QkvPiece<8, BYTES>;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, hl = lane / LPH, d0 = lane % LPH * 8;
   const int all = p.nq + 2 * p.nkv, items = (all + HPW - 1) / HPW, per = (items + gridDim.y - 1) / gridDim.y;
   const int first = blockIdx.y * per, end = min(items, first + per);
@@ -293,7 +294,7 @@ __global__ void __launch_bounds__(QKV_WARPS * 32, 5) qk_norm_rope_kv_kernel(cons
   if (sl >= 0)
     cache = p.cache[p.cache_sel ? p.cache_sel[t] : 0] + ((size_t)(sl / p.page_size) * 2 * p.nkv * p.page_size + sl % p.page_size) * HD;
   __syncthreads();
-  QkvPiece<8, true> co, si;                     // frequency of dim d: d mod HD / 2; the lower half takes away the partner's sine
+  QkvPiece<8> co, si;                     // frequency of dim d: d mod HD / 2; the lower half takes away the partner's sine
   co.load(s_cos + d0 % (HD / 2));
   si.load(s_sin + d0 % (HD / 2));
   if (d0 < HD / 2) {
@@ -816,14 +817,14 @@ extern "C" int tahb_qk_norm_rope_kv(const void* qkv, const void* q_w, const void
                  reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(k_dense) | reinterpret_cast<uintptr_t>(v_dense) |
                  (uintptr_t)(ld_qkv * 2);
   for (int i = 0; i < n_caches; ++i) at |= reinterpret_cast<uintptr_t>(caches[i]);
-  const bool wide = at % 16 == 0;
   const int groups = qk_head_groups(M, (nq + 2 * nkv + 256 / hd - 1) / (256 / hd), QKV_WARPS, 4 * 148);
-#define TAHB_QKV(HD_) (wide ? launch_chain(qk_norm_rope_kv_kernel<HD_, true>, dim3(M, groups), dim3(QKV_WARPS * 32), 0, stream, p) \
-                            : launch_chain(qk_norm_rope_kv_kernel<HD_, false>, dim3(M, groups), dim3(QKV_WARPS * 32), 0, stream, p))
+#define TAHB_QKV_AT(HD_, BYTES_) launch_chain(qk_norm_rope_kv_kernel<HD_, BYTES_>, dim3(M, groups), dim3(QKV_WARPS * 32), 0, stream, p)
+#define TAHB_QKV(HD_) (at % 16 == 0 ? TAHB_QKV_AT(HD_, 16) : at % 8 == 0 ? TAHB_QKV_AT(HD_, 8) : at % 4 == 0 ? TAHB_QKV_AT(HD_, 4) : TAHB_QKV_AT(HD_, 2))
   if (hd == 128) e = TAHB_QKV(128);
   else if (hd == 64) e = TAHB_QKV(64);
   else return -2;
 #undef TAHB_QKV
+#undef TAHB_QKV_AT
   return e == cudaSuccess ? 0 : -3;
 }
 

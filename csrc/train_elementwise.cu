@@ -192,7 +192,7 @@ constexpr int QKB_U = 4, QKB_WARPS = 8;
 template <int HD, bool WIDE>
 __global__ void __launch_bounds__(QKB_WARPS * 32) qk_norm_rope_bwd_kernel(const QkRopeBwdParams p) {
   constexpr int EPL = HD / 32;
-  using Piece = QkvPiece<EPL, WIDE>;
+  using Piece = QkvPiece<EPL, WIDE ? EPL * 2 : 2>;
   __shared__ float s_gw[2][HD];
   for (int i = threadIdx.x; i < 2 * HD; i += blockDim.x) (&s_gw[0][0])[i] = 0.f;
   __syncthreads();

@@ -1282,6 +1282,29 @@ def test_attention_backward_two_heads_per_cta(hd, nq, nkv):
         Kc.attn_bwd_dq(q, dout, [k], [v], [b], [c], tq0, tqn, nq, nq, hd, hd ** -0.5, lse, dsum, heads=2)
 
 
+@pytest.mark.parametrize("hd,nq,nkv", [(128, 5, 2), (64, 7, 3)])
+def test_qk_norm_rope_on_every_boundary(hd, nq, nkv):
+    """Rows, outputs and caches on boundaries of 8, 4 and 2 bytes give the bits that they give on 16: only the width of an access changes."""
+    Kc = _cuda()
+    M, W, ps = 37, (nq + 2 * nkv) * hd, 16
+    pages = M // ps + 1
+    x, qw, kw = _rand(M, W, seed=1), _rand(hd, seed=2), _rand(hd, seed=3)
+    pos = torch.arange(M, device="cuda", dtype=torch.int32) * 7
+    slot = torch.randperm(pages * ps, generator=torch.Generator().manual_seed(4))[:M].to(torch.int32).cuda()
+
+    def at(shift, *shape):
+        n = torch.Size(shape).numel()
+        return torch.zeros(n + 8, dtype=torch.bfloat16, device="cuda")[shift:shift + n].view(shape)
+
+    outs = []
+    for shift in (0, 4, 2, 1):
+        xs, q, k, v, cache = at(shift, M, W).copy_(x), at(shift, M, nq * hd), at(shift, M, nkv * hd), at(shift, M, nkv * hd), at(shift, pages, 2, nkv, ps, hd)
+        Kc.qk_norm_rope_kv(xs, qw, kw, pos, nq, nkv, hd, 1e-6, 1e6, q_out=q, k_dense=k, v_dense=v, caches=[cache], slot=slot, page_size=ps)
+        outs.append((q, k, v, cache))
+    for got in outs[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(outs[0], got))
+
+
 @pytest.mark.parametrize("hd,nq,nkv", [(128, 3, 1), (128, 2, 1), (64, 3, 1), (64, 5, 3), (64, 1, 1)])
 @pytest.mark.parametrize("shift", [0, 4])
 def test_qk_norm_rope_heads_that_share_a_warp(hd, nq, nkv, shift):
