@@ -190,6 +190,13 @@ def plan_gemm_kept(M: int, F: int, K: int, R: int = 0):
 PAIR_AUTO = os.environ.get("TAH_B200_GEMM_PAIR", "1") != "0"
 
 
+# A weight gradient over so many tokens takes constants of its own.  Those of long reductions, fitted from 264 on, left short ones to the persistent form
+# where one tile or pair per CTA is faster.  Over 18 weights of 320 to 12288 rows and 1 to 800 tokens the choice lies 0.5 % above the best form on average, 6 % at
+# most, in place of 4 and 24 %.  us, before that / by it: 1000 x 2048 over 50 tokens 5.1 / 4.8, 200 5.7 / 5.1, 576 x 1536 over 320 5.1 / 4.2,
+# 2560 x 2560 over 8 7.7 / 7.0.
+SHORT_REDUCTION = 1024
+
+
 @functools.lru_cache(maxsize=4096)
 def plan_tiles(M: int, rows: int, K: int, can_pair: bool, can_split: bool, x_t: bool = False):
     """``(pair, bn, splits)`` for more than 256 tokens: tiles of 128 features by 64 to 256 tokens or (pair) 256 features by 128 to 256,
@@ -214,12 +221,14 @@ def _tiles_cost(M: int, rows: int, K: int, can_pair: bool, can_split: bool, x_t:
                     continue
                 waves = -(-(-(-rows // (128 * nf)) * -(-M // bn) * s) // (CLUSTER4_CTAS if s == 4 else SM_COUNT))
                 # microseconds: the main loop, the epilogue, the exchange of split sums
-                if x_t:
+                if x_t and K <= SHORT_REDUCTION:
+                    t_kb, out = (0.07 + 0.281 * bn / 256, 2.3 + 0.0105 * bn) if nf == 1 else (0.16 + 0.451 * bn / 256, 2.3 + 0.019 * bn)
+                elif x_t:
                     t_kb, out = (0.29 + 0.164 * bn / 256, 2.6 + 0.0195 * bn) if nf == 1 else (0.31 + 0.297 * bn / 256, 3.0 + 0.038 * bn)
                 else:
                     t_kb, out = (0.31 + 0.03 * bn / 256, 2.0 + 0.0143 * bn) if nf == 1 else (0.345 + 0.235 * bn / 256, 2.0 + 0.022 * bn)
                 if nf == 1 and bn <= 128:          # stages of two blocks
-                    t_kb = (0.21 if bn == 64 else 0.26) + (0.02 if x_t else 0.0)
+                    t_kb = (0.18 if bn == 64 else 0.23) if x_t and K <= SHORT_REDUCTION else (0.21 if bn == 64 else 0.26) + (0.02 if x_t else 0.0)
                 t = waves * (kb * t_kb + out + {1: 0.0, 2: 1.1 + 0.003 * bn, 4: 0.65 + 0.0133 * bn}[s])
                 if best is None or t < best[0] - 1e-9:
                     best = (t, nf == 2, bn, s)
@@ -249,9 +258,11 @@ def _persist_cost(M: int, rows: int, K: int, R: int, glu: bool, x_t: bool, can_p
     below what it takes beside other launches."""
     best = None
     steps = -(-K // 128) + -(-R // 128)
-    for bn, kb in ((64, 0.35), (128, 0.41), (192, 0.58), (256, 0.72)):
+    short = x_t and K <= SHORT_REDUCTION
+    for bn, kb in ((64, 0.395), (128, 0.435), (192, 0.635), (256, 0.725)) if short else ((64, 0.35), (128, 0.41), (192, 0.58), (256, 0.72)):
         waves = -(-(-(-M // 256) * -(-rows // bn)) // SM_PAIRS)
-        t = 3.2 + 0.004 * bn + waves * max(steps * kb, 1.25 + 0.006 * bn) + (2.5 if M <= 256 else 0.0)
+        start, out = (2.8 + 0.003 * bn, 1.45 + 0.004 * bn) if short else (3.2 + 0.004 * bn, 1.25 + 0.006 * bn)
+        t = start + waves * max(steps * kb, out) + (2.5 if M <= 256 else 0.0)
         if best is None or t < best[0] - 1e-9:
             best = (t, bn)
     if M <= 256:
@@ -261,7 +272,7 @@ def _persist_cost(M: int, rows: int, K: int, R: int, glu: bool, x_t: bool, can_p
                  _gemm_cost(M, rows, K, R, False)[0])
         return best[1] if best[0] < other else 0
     other = _tiles_cost(M, rows, K + R, can_pair and rows % 256 == 0, not glu, x_t)[0]
-    return best[1] if best[0] <= 1.08 * other else 0
+    return best[1] if best[0] <= (1.04 if short else 1.08) * other else 0
 
 
 def interleave_gate_up(w: torch.Tensor) -> torch.Tensor:
