@@ -20,7 +20,8 @@
 // nothing.  Here the product does it itself: a CTA normalises the rows into shared memory while its first weights are on their way (a row is
 // 4 KB, from L2), and the first CTAs of the grid form T = gate * x A^T, which the others wait for behind their main loop (bounded; a
 // CTA only waits for ones with a lower index, which run before it) and only where a row is gated; without one the adapter's weights are not
-// read at all.  Six launches a layer.
+// read at all.  Six launches a layer, in ticks of up to eight rows (few_fused_pays in tah_b200/ops/cuda.py: above that all CTAs' norms of all rows cost more
+// than the launches).
 #include <cuda.h>
 
 #include "common.cuh"

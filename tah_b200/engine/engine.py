@@ -41,7 +41,7 @@ KV_BLOCK_BYTES = 1 << 29
 def _fusions(default: str):
     """Kernel fusions selected by ``TAH_B200_FUSE``: "1" = all, "0" = none, or a comma list of "qkv" (QK-norm, RoPE
     and the K/V write in the QKV GEMM's epilogue), "lora" (LoRA-A of the gated rows inside the RMSNorm launch) and "few"
-    (RMSNorm and LoRA-A inside the products of up to 16 rows, in place of the others); unset = ``default`` ("few" in ticks of up to 16 rows, else
+    (RMSNorm and LoRA-A inside the products of up to 16 rows, in place of the others); unset = ``default`` ("few" in ticks of up to eight rows, else
     nothing).  "1" is "qkv" and "lora"."""
     v = os.environ.get("TAH_B200_FUSE", default)
     if v == "1":
@@ -641,11 +641,11 @@ class TaHEngine(DecodeEngine):
         tl = self._tap_layers()
         H = cfg.hidden_size
         nL = len(w.layers)
-        # Optional fusions of the decode chain.  While launches are what a tick is made of, the products of up to 16 rows take the RMSNorm in front of
-        # them and the gated rows' LoRA-A along.  RMSNorm and LoRA-A in one launch hold up the norm from 20 rows on (2.98 -> 3.12 ms), and at 256
+        # Optional fusions of the decode chain.  While launches are what a tick is made of, the products of up to eight rows take the RMSNorm in front of
+        # them and the gated rows' LoRA-A along (K.few_fused_pays).  RMSNorm and LoRA-A in one launch hold up the norm from 20 rows on (2.98 -> 3.12 ms), and at 256
         # rows the chain of separate launches is faster, also than the QKV epilogue on the GEMM's eight epilogue warps (a generation of 32
         # tokens 205.7 ms, fused 212.2; 20 rows of up to 1900 172.9 and 182.3).
-        fuse = _fusions("few" if B <= K.FUSED_TOKENS else "")
+        fuse = _fusions("few" if K.few_fused_pays(B, H) else "")
         sync = s.few_sync if "few" in _fusions("few") else None  # up to 32 rows: LoRA-A of the row-parallel projections inside them
         fuse_qkv = "qkv" in fuse and hd == 128                   # QK-norm + RoPE + KV write in the QKV GEMM epilogue
         few = "few" in fuse and tp is None and not fuse_qkv and self._few_fits(B)

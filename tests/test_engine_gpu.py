@@ -249,6 +249,52 @@ def test_engine_with_head_dim_128_fused_kernels_match_unfused(monkeypatch):
     assert same >= 0.9 * B * n_new, same
 
 
+@pytest.mark.parametrize("B", [1, 8, 12, 16, 17, 24, 32])
+def test_default_ticks_of_few_rows_match_separate_launches(monkeypatch, B):
+    """Up to 16 rows a tick's products take norm and adapter inputs along, up to 32 the row-parallel ones the adapter inputs; their logits are those of
+    the chain of separate launches, whose second passes the adapters change by far more than the two may differ."""
+    from tah_b200.engine import TaHEngine
+    T, n_new = 16, 6
+    model = tiny_tah(max_iter=2, dtype=torch.bfloat16, head_dim=128, num_attention_heads=2, num_key_value_heads=1).cuda().eval()
+    ids = torch.randint(0, 1024, (B, T), generator=torch.Generator().manual_seed(2)).cuda()
+    hard = torch.zeros(B, T + n_new + 2, dtype=torch.int8)
+    hard[:, T:] = (torch.arange(n_new + 2)[None] + torch.arange(B)[:, None]) % 2 == 0         # about half of the rows in every tick
+
+    def ticks(fuse, adapters=True):
+        monkeypatch.delenv("TAH_B200_FUSE", raising=False)
+        if fuse is not None:
+            monkeypatch.setenv("TAH_B200_FUSE", fuse)
+        eng = TaHEngine(model, max_rows=B, max_seq_len=T + n_new + 2, use_cuda_graph=True, deep_fraction=1.0)
+        eng.hard_override = hard.cuda()
+        if not adapters:
+            for L in eng.w.layers:
+                for b in (L.b_qkv, L.b_o, L.b_gu, L.b_down):
+                    b.zero_()
+        kept = []
+        eng.generate(ids, None, max_new_tokens=n_new, do_sample=False, on_tick=lambda t, s: kept.append((s.cum[:B].float().clone(), s.tok[:B].clone(),
+                                                                                                       s.gate[:B].clone())))
+        return kept, eng.kernel_launches_per_tick
+
+    got, few = ticks(None)
+    want, all_ = ticks("0")
+    bare, _ = ticks("0", adapters=False)
+    assert few < all_
+    # A layer rounds the residual stream, norms, products and attention about ten times on its way, 2^-9 of a number at most each and adding up as
+    # squares do over four layers and two passes: sqrt(80) * 2^-9 = 0.0175; a little over twice that.
+    bound, alive, seen = 0.04, torch.ones(B, dtype=torch.bool, device="cuda"), 0
+    for (a, ta, ga), (b, tb, gb), (c, _, _) in zip(got[:n_new - 2], want, bare):       # before a row is done
+        if not alive.any():
+            break
+        assert torch.equal(ga[alive], gb[alive])
+        off = (a - b).norm(dim=1) / b.norm(dim=1)
+        assert bool((off[alive] <= bound).all()), off
+        alive &= ta == tb
+        seen += 1
+    assert seen >= 2
+    far = max(float(((c - b).norm(dim=1) / b.norm(dim=1)).max()) for (b, _, _), (c, _, _) in zip(want[:3], bare[:3]))
+    assert far > 2 * bound, far
+
+
 @pytest.mark.parametrize("head_dim,T", [(64, 5), (64, 20), (128, 150)])
 def test_native_pass_gives_the_bits_of_the_loop(head_dim, T):
     """The passes of a prompt (three deep, some tokens each) from one native call and launch by launch: the same kernels on the same plans."""

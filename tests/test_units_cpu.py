@@ -544,17 +544,6 @@ def test_form_of_a_product_is_the_one_launched(monkeypatch):
                 assert called == ["tahb_gemm_persist" if form == "persist" else "tahb_gemm_t"], (M, rows, K, x_t, w_t)
 
 
-            for how in ({}, dict(const_w=True), dict(swiglu=True), dict(swiglu_interleaved=True), dict(gelu=True)):
-                called.clear()
-                cuda.gemm(t(M, K), t(rows, K), **how)
-                assert called == [entry[cuda.gemm_form(M, rows, K, **how)[0]]], (M, rows, K, how)
-            for x_t, w_t in ((False, True), (True, True)):
-                called.clear()
-                cuda.gemm_t(t(K, M + -M % 8) if x_t else t(M, K), t(K, rows), x_t=x_t, w_t=w_t)
-                form = cuda.gemm_t_form(M + -M % 8 if x_t else M, rows, K, x_t, w_t)[0]
-                assert called == ["tahb_gemm_persist" if form == "persist" else "tahb_gemm_t"], (M, rows, K, x_t, w_t)
-
-
 def test_weight_gradients_over_few_tokens_take_one_tile_or_pair_per_cta():
     """Reductions below those that the long ones' constants were fitted to: few output tiles stay off the persistent form, many take it."""
     from tah_b200.ops import cuda
@@ -563,6 +552,13 @@ def test_weight_gradients_over_few_tokens_take_one_tile_or_pair_per_cta():
     assert [form(576, 1536, T) for T in (100, 200, 320)] == [("tile", 64, 1)] * 3
     assert form(2560, 2560, 8)[0] == form(2560, 2560, 64)[0] == "pair"
     assert form(12288, 2048, 50)[0] == form(2048, 6144, 200)[0] == form(12288, 2048, 3072)[0] == "persist"
+
+
+def test_rules_of_ticks_of_few_rows():
+    """Norms move into the products of ticks of few and narrow rows only."""
+    from tah_b200.ops import cuda
+    for K, most in ((256, 8), (1024, 8), (2048, 8), (2560, 5), (4096, 2), (8192, 0)):
+        assert [M for M in range(1, 17) if cuda.few_fused_pays(M, K)] == list(range(1, most + 1))
 
 
 def test_host_plan_of_a_prefill_is_the_device_one():
