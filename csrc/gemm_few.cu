@@ -78,7 +78,8 @@ constexpr int FEW_ROWS_MOST = 96 * 1024;       // of shared memory for normalise
 // instructions; 16 outputs per cluster of eight CTAs that split the reduction, so that a warp holds all it needs of A in registers, read
 // ahead of the dependency wait; the partial sums meet in the first CTA's shared memory, in a fixed order.  256 rows, 192 outputs of 2048, us, rows
 // of dot products / this: 1 gated row 4.1 / 2.9, 14 5.3 / 3.0; 64 outputs of 6144: 4.2 / 3.2, 5.1 / 3.3.  27 KB of shared memory and 256 threads
-// fit an SM beside a CTA of the one-tile GEMM, so that the start-up stands under its tail.
+// fit an SM beside a CTA of the one-tile GEMM, so that the start-up stands under its tail.  Small adapters and ticks of up to 32 rows keep the dot products
+// (lora_gated_pays in tah_b200/ops/cuda.py).
 constexpr int LG_WARPS = 8, LG_CL = 8, LG_STEPS = 4, LG_NT = 2, LG_TOK = 8 * LG_NT, LG_PITCH = 17;
 struct LoraGatedParams {
   const __nv_bfloat16 *x, *A;

@@ -588,7 +588,7 @@ class TaHEngine(DecodeEngine):
             return K.rms_norm(h, ln_w, cfg.rms_norm_eps, out=xn_out)
         if lora:
             if gate is not None:
-                K.lora_a_rows(x, a_, gate, out=t_buf, const_w=True)
+                K.lora_a_rows(x, a_, gate, out=t_buf, const_w=K.lora_gated_pays(M, a_.shape[1], a_.shape[0]))
             else:
                 K.gemm(x, a_, out=t_buf)
         kw = dict(x2=t_buf, w2=b_) if lora else {}
@@ -681,7 +681,7 @@ class TaHEngine(DecodeEngine):
                 self._few_layer(s, L, pools[li], lora)
                 continue
             if lora and not fuse_norm_lora:
-                K.lora_a_rows(xn, L.a_qkv, s.gate, out=s.t_qkv, tp_wait=self._xn_wait, const_w=True)
+                K.lora_a_rows(xn, L.a_qkv, s.gate, out=s.t_qkv, tp_wait=self._xn_wait, const_w=K.lora_gated_pays(B, H, L.a_qkv.shape[0]))
             kw = dict(x2=s.t_qkv, w2=L.b_qkv) if lora else {}
             if fuse_qkv:
                 K.gemm_qkv(xn, L.w_qkv, L.q_norm, L.k_norm, s.pos, nq, nkv, cfg.rms_norm_eps, cfg.rope_theta, q_out=s.q,
@@ -696,7 +696,7 @@ class TaHEngine(DecodeEngine):
             xn = self._row_parallel(s.o, L.w_o, L.a_o if lora else None, L.b_o, s.t_o, s.gate, s.h, L.ln2, s.xn, B,
                                     push=push, next_lora=(L.a_gu, s.t_gu) if fuse_norm_lora else None, sync=sync)
             if lora and not fuse_norm_lora:
-                K.lora_a_rows(xn, L.a_gu, s.gate, out=s.t_gu, tp_wait=self._xn_wait, const_w=True)
+                K.lora_a_rows(xn, L.a_gu, s.gate, out=s.t_gu, tp_wait=self._xn_wait, const_w=K.lora_gated_pays(B, H, L.a_gu.shape[0]))
             sw = dict(swiglu_interleaved=True, const_w=True) if w.gu_interleaved else dict(swiglu=True, const_w=True)
             if lora:
                 K.gemm(xn, L.w_gu, x2=s.t_gu, w2=L.b_gu, out=s.act, tp_wait=self._xn_wait, **sw)

@@ -555,10 +555,12 @@ def test_weight_gradients_over_few_tokens_take_one_tile_or_pair_per_cta():
 
 
 def test_rules_of_ticks_of_few_rows():
-    """Norms move into the products of ticks of few and narrow rows only."""
+    """Norms move into the products of ticks of few and narrow rows only; adapter inputs are gathered for many rows and large adapters."""
     from tah_b200.ops import cuda
     for K, most in ((256, 8), (1024, 8), (2048, 8), (2560, 5), (4096, 2), (8192, 0)):
         assert [M for M in range(1, 17) if cuda.few_fused_pays(M, K)] == list(range(1, most + 1))
+    assert not cuda.lora_gated_pays(32, 2048, 192) and cuda.lora_gated_pays(33, 2048, 192) and cuda.lora_gated_pays(256, 6144, 64)
+    assert not any(cuda.lora_gated_pays(M, K, R) for M in (64, 256) for K, R in ((2048, 64), (1024, 192), (512, 256), (16384, 64)))
 
 
 def test_host_plan_of_a_prefill_is_the_device_one():
