@@ -230,37 +230,59 @@ __global__ void __launch_bounds__(RN_THREADS) embed_norm_kernel(const T* __restr
   }
 }
 
-// f(j, e) for the rows slot[j] of y_ex, j = 0 .. top - 1 in order: e: this thread's pieces of the row.  Row numbers eight at a time and the rows
-// four at a time on their way together: one after the other (a number, then a row) the loads of eight experts were two thirds of a seam of 12
-// tokens (8.3 us).
+// f(weight(j), i, e) for the rows slot[j] of y_ex, j = 0 .. top - 1 in order: e: this thread's piece i of the row.  AHEAD: row numbers eight at a time and the
+// rows four (longer ones one) at a time on their way together: one after the other (a number, then a row) the loads of eight experts were two thirds of a seam of 12
+// tokens (8.3 us).  That takes half as many registers again (96 to 102 a thread in place of 48 to 56 for rows of 2048), so from a wave of
+// CTAs on, and for rows above 4096, they come one after the other.  us, rows of 2048, one by one / ahead: 12 tokens 8.2 / 6.2 (two streams 10.3 / 8.3), 400
+// 8.5 / 8.2 (12.3 / 10.3), 740 10.5 / 10.4 (14.4 / 18.5), 3000 36.0 / 36.3 (45.0 / 54.1).
 // Without __restrict__: loads that the compiler may take for constant may move ahead of the dependency wait.
-template <typename T, int VPT, typename F>
-__device__ __forceinline__ void for_experts(const T* y_ex, const int* slot, int top, int ld, int nvec, const F& f) {
-  constexpr int G = VPT <= 4 ? 4 : 1;
-  for (int j0 = 0; j0 < top; j0 += 8) {
-    int s[8];
+constexpr int RN_AHEAD_TOKENS = 4 * 148;           // CTAs that run at once with 102 registers
+
+template <typename T, int VPT, bool AHEAD, typename W, typename F>
+__device__ __forceinline__ void for_experts(const T* y_ex, const int* slot, int top, int ld, int nvec, const W& weight, const F& f) {
+  if constexpr (!AHEAD) {
+    int next = VPT > 8 && top > 0 ? slot[0] : 0;
+    for (int j = 0; j < top; ++j) {
+      const T* src = y_ex + (size_t)(VPT > 8 ? next : slot[j]) * ld;
+      if constexpr (VPT > 8) next = slot[min(j + 1, top - 1)];      // few long rows on an SM: the next number ahead of this row (8192: 90 / 66 us)
+      const float w = weight(j);
 #pragma unroll
-    for (int u = 0; u < 8; ++u) s[u] = slot[min(j0 + u, top - 1)];
+      for (int i = 0; i < VPT; ++i) {
+        const int c = threadIdx.x + i * RN_THREADS;
+        if (c < nvec) f(w, i, Vec4<T>::load(src + c * 4));
+      }
+    }
+  } else {
+    constexpr int G = VPT <= 4 ? 4 : 1;
+    for (int j0 = 0; j0 < top; j0 += 8) {
+      int s[8];
 #pragma unroll
-    for (int u0 = 0; u0 < 8; u0 += G) {
-      if (j0 + u0 >= top) break;
-      float4 e[G][VPT];
+      for (int u = 0; u < 8; ++u) s[u] = slot[min(j0 + u, top - 1)];
 #pragma unroll
-      for (int u = 0; u < G; ++u)
+      for (int u0 = 0; u0 < 8; u0 += G) {
+        if (j0 + u0 >= top) break;
+        float4 e[G][VPT];
 #pragma unroll
-        for (int i = 0; i < VPT; ++i) {
-          const int c = threadIdx.x + i * RN_THREADS;
-          e[u][i] = c < nvec ? Vec4<T>::load(y_ex + (size_t)s[u0 + u] * ld + c * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+        for (int u = 0; u < G; ++u)
 #pragma unroll
-      for (int u = 0; u < G; ++u)
-        if (j0 + u0 + u < top) f(j0 + u0 + u, e[u]);
+          for (int i = 0; i < VPT; ++i) {
+            const int c = threadIdx.x + i * RN_THREADS;
+            e[u][i] = c < nvec ? Vec4<T>::load(y_ex + (size_t)s[u0 + u] * ld + c * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+#pragma unroll
+        for (int u = 0; u < G; ++u)
+          if (j0 + u0 + u < top) {
+            const float w = weight(j0 + u0 + u);
+#pragma unroll
+            for (int i = 0; i < VPT; ++i) f(w, i, e[u][i]);
+          }
+      }
     }
   }
 }
 
 // y_ex / slot: expert outputs [list rows, ld] and the list rows slot[row * top ..] of this token, or null
-template <typename T, int VPT>
+template <typename T, int VPT, bool AHEAD>
 __global__ void __launch_bounds__(RN_THREADS) residual_add_norm_kernel(const T* y, long long ldy, const T* y_ex, const int* slot,
                                                                        int top, float mult, float* x, const float* w_next, T* h, int width, int groups, int ld,
                                                                        float eps) {
@@ -275,18 +297,18 @@ __global__ void __launch_bounds__(RN_THREADS) residual_add_norm_kernel(const T* 
     const int c = threadIdx.x + i * RN_THREADS;
     if (c < nvec) {
       r[i] = Vec4<T>::load(y + row * ldy + c * 4);
-      v[i] = Vec4<float>::load(x + row * ld + c * 4);
+      if constexpr (AHEAD) v[i] = Vec4<float>::load(x + row * ld + c * 4);
     }
   }
   if (y_ex != nullptr)
-    for_experts<T, VPT>(y_ex, slot + row * top, top, ld, nvec, [&](int, const float4 (&e)[VPT]) {
-#pragma unroll
-      for (int i = 0; i < VPT; ++i) { r[i].x += e[i].x; r[i].y += e[i].y; r[i].z += e[i].z; r[i].w += e[i].w; }
+    for_experts<T, VPT, AHEAD>(y_ex, slot + row * top, top, ld, nvec, [](int) { return 1.0f; }, [&](float, int i, const float4& e) {
+      r[i].x += e.x; r[i].y += e.y; r[i].z += e.z; r[i].w += e.w;
     });
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int c = threadIdx.x + i * RN_THREADS;
     if (c < nvec) {
+      if constexpr (!AHEAD) v[i] = Vec4<float>::load(x + row * ld + c * 4);
       v[i].x = fmaf(mult, r[i].x, v[i].x); v[i].y = fmaf(mult, r[i].y, v[i].y);
       v[i].z = fmaf(mult, r[i].z, v[i].z); v[i].w = fmaf(mult, r[i].w, v[i].w);
       Vec4<float>::store(x + row * ld + c * 4, v[i]);
@@ -323,7 +345,7 @@ struct StreamsParams {
   float eps;
 };
 
-template <typename T, int VPT, int S>
+template <typename T, int VPT, int S, bool AHEAD>
 __global__ void __launch_bounds__(RN_THREADS) streams_norm_kernel(const StreamsParams p) {
   pdl_launch_dependents();
   pdl_wait();
@@ -343,13 +365,11 @@ __global__ void __launch_bounds__(RN_THREADS) streams_norm_kernel(const StreamsP
     }
   }
   if (p.y_ex != nullptr)
-    for_experts<T, VPT>(reinterpret_cast<const T*>(p.y_ex), p.slot + row * p.top, p.top, p.ld, nvec, [&](int j, const float4 (&e)[VPT]) {
-      const float w = p.y_weight != nullptr ? p.y_weight[row * p.top + j] : 1.0f;
-#pragma unroll
-      for (int i = 0; i < VPT; ++i) {
-        r[i].x = fmaf(w, e[i].x, r[i].x); r[i].y = fmaf(w, e[i].y, r[i].y);
-        r[i].z = fmaf(w, e[i].z, r[i].z); r[i].w = fmaf(w, e[i].w, r[i].w);
-      }
+    for_experts<T, VPT, AHEAD>(reinterpret_cast<const T*>(p.y_ex), p.slot + row * p.top, p.top, p.ld, nvec, [&](int j) {
+      return p.y_weight != nullptr ? p.y_weight[row * p.top + j] : 1.0f;
+    }, [&](float w, int i, const float4& e) {
+      r[i].x = fmaf(w, e.x, r[i].x); r[i].y = fmaf(w, e.y, r[i].y);
+      r[i].z = fmaf(w, e.z, r[i].z); r[i].w = fmaf(w, e.w, r[i].w);
     });
   float mix[S][S], out[S], in[S];
 #pragma unroll
@@ -683,13 +703,16 @@ static int streams_norm_launch(const StreamsParams& p, int M, cudaStream_t strea
   const int need = (p.ld / 4 + RN_THREADS - 1) / RN_THREADS;
   const size_t smem = group_rms_smem(p.width, p.groups, p.ld);
   cudaError_t rc;
-#define TAHB_SN(V_) rc = launch_chain(streams_norm_kernel<T, V_, S>, dim3(M), dim3(RN_THREADS), smem, stream, p)
+  const bool ahead = p.y_ex != nullptr && M <= RN_AHEAD_TOKENS;
+#define TAHB_SN_AT(V_, A_) launch_chain(streams_norm_kernel<T, V_, S, A_>, dim3(M), dim3(RN_THREADS), smem, stream, p)
+#define TAHB_SN(V_) rc = ahead ? TAHB_SN_AT(V_, true) : TAHB_SN_AT(V_, false)
   if (need <= 1) TAHB_SN(1);
   else if (need <= 2) TAHB_SN(2);
   else if (need <= 4) TAHB_SN(4);
   else if (need <= 8) TAHB_SN(8);
-  else if (need <= 16) TAHB_SN(16);
+  else if (need <= 16) rc = TAHB_SN_AT(16, false);
   else return -2;
+#undef TAHB_SN_AT
 #undef TAHB_SN
   return rc == cudaSuccess ? 0 : -3;
 }
@@ -719,13 +742,16 @@ static int residual_add_norm_launch(const void* y, long long ldy, const void* y_
   auto ye = reinterpret_cast<const T*>(y_ex);
   auto o = reinterpret_cast<T*>(h);
   cudaError_t rc;
-#define TAHB_RA(V_) rc = launch_chain(residual_add_norm_kernel<T, V_>, dim3(M), dim3(RN_THREADS), smem, stream, yy, ldy, ye, slot, top, mult, x, w_next, o, width, groups, ld, eps)
+  const bool ahead = M <= RN_AHEAD_TOKENS;
+#define TAHB_RA_AT(V_, A_) launch_chain(residual_add_norm_kernel<T, V_, A_>, dim3(M), dim3(RN_THREADS), smem, stream, yy, ldy, ye, slot, top, mult, x, w_next, o, width, groups, ld, eps)
+#define TAHB_RA(V_) rc = ahead ? TAHB_RA_AT(V_, true) : TAHB_RA_AT(V_, false)
   if (need <= 1) TAHB_RA(1);
   else if (need <= 2) TAHB_RA(2);
   else if (need <= 4) TAHB_RA(4);
   else if (need <= 8) TAHB_RA(8);
-  else if (need <= 16) TAHB_RA(16);
+  else if (need <= 16) rc = TAHB_RA_AT(16, false);
   else return -2;
+#undef TAHB_RA_AT
 #undef TAHB_RA
   return rc == cudaSuccess ? 0 : -3;
 }

@@ -1485,6 +1485,27 @@ def test_gemm_few_fused(M, F, Kd, R, norm, act):
     Kc.check_status()
 
 
+@pytest.mark.parametrize("W,top", [(512, 3), (1000, 8), (2048, 9), (4096, 2), (8192, 4)])
+def test_seams_of_many_tokens_give_the_bits_of_few(W, top):
+    """Rows of experts fetched ahead (up to a wave of CTAs) and one by one give the same sums: 593 tokens at once and in two parts."""
+    Kc = _cuda()
+    M, S = 4 * 148 + 1, 2
+    slot = torch.randperm(M * top, generator=torch.Generator().manual_seed(1)).to(torch.int32).cuda().view(M, top)
+    y, ex = _rand(M, W, seed=2), _rand(M * top, W, seed=3)
+    w, yw = torch.rand(W, device="cuda") + 0.5, torch.rand(M, top, device="cuda")
+    hc = torch.cat([0.5 * torch.eye(S).flatten(), torch.full((2 * S,), 0.5)]).cuda()
+    x, xs = torch.randn(M, W, device="cuda"), torch.randn(M, S, W, device="cuda")
+
+    def both(parts):
+        x1, xs1, h1, h2 = x.clone(), xs.clone(), torch.empty_like(y), torch.empty_like(y)
+        for a, b in parts:
+            Kc.residual_add_norm(y[a:b], x1[a:b], 0.5, w, W, 1, 1e-6, h1[a:b], ex, slot[a:b])
+            Kc.streams_norm(None, xs1[a:b], hc, w, W, 1, 1e-6, h2[a:b], y_ex=ex, slot=slot[a:b], y_weight=yw[a:b])
+        return x1, xs1, h1, h2
+
+    assert all(torch.equal(p, q) for p, q in zip(both([(0, M)]), both([(0, 300), (300, M)])))
+
+
 @pytest.mark.parametrize("M,Kd,R,n", [(1, 64, 8, 1), (20, 2048, 192, 2), (33, 2048, 64, 0), (256, 6144, 64, 15), (256, 2048, 128, 17), (300, 8192, 24, 300),
                                       (1024, 192, 64, 1024)])
 def test_lora_gated(M, Kd, R, n):
