@@ -319,10 +319,11 @@ def wait_flags(flags: torch.Tensor, targets: torch.Tensor) -> None:
         "tahb_wait_flags")
 
 
+@functools.lru_cache(maxsize=4096)
 def _persist_width(M: int, rows: int, K: int, R: int, swiglu_interleaved: bool, const_w: bool) -> int:
-    """:func:`plan_persist` for :func:`gemm`: up to 256 tokens with weights that training changes only where their split (:func:`plan_gemm_kept`)
-    is none."""
-    wide = plan_persist(M, rows, K, R, swiglu_interleaved)
+    """:func:`plan_persist` for :func:`gemm`, where it is not turned off: up to 256 tokens with weights that training changes only where their split
+    (:func:`plan_gemm_kept`) is none."""
+    wide = _persist_cost(M, rows, K, R, swiglu_interleaved, False, True)
     return wide if wide and (M > 256 or const_w or swiglu_interleaved or plan_gemm_kept(M, rows, K, R)[1] == 1) else 0
 
 
@@ -332,7 +333,7 @@ def gemm_form(M: int, rows: int, K: int, R: int = 0, *, swiglu: bool = False, ge
     "tile"."""
     if few_shape(M, rows, K, R, const_w):
         return "few", 0, 1
-    wide = _persist_width(M, rows, K, R, swiglu_interleaved, const_w) if M > 128 and not swiglu else 0
+    wide = _persist_width(M, rows, K, R, swiglu_interleaved, const_w) if PAIR_AUTO and M > 128 and not swiglu else 0
     if wide:
         return "persist", wide, 1
     pair, bn, splits = _plan_tiles(M, rows, K, R, swiglu, gelu, swiglu_interleaved, kept=not const_w)
@@ -434,7 +435,7 @@ def gemm(x: torch.Tensor, w: torch.Tensor, *, out: Optional[torch.Tensor] = None
         return _gemm_few(x, w, out, residual, x2, w2, 1 if swiglu else 3 if gelu else 4 if swiglu_interleaved else 0, early=const_w)
     # the plan, which is kept, before the look at every operand (4 us of host time)
     if (pair is None and bn == 0 and splits is None and tp_push is None and not swiglu and not (gelu and residual is not None) and
-            M > 128 and F > 0 and K > 0):
+            M > 128 and PAIR_AUTO and F > 0 and K > 0):
         wide = _persist_width(M, F, K, R, swiglu_interleaved, const_w)
         if wide and _persist_ok(x, w, out, residual, x2, w2):
             return _gemm_persist(x, w, out, residual, x2, w2, 1 if gelu else 2 if swiglu_interleaved else 0, wide, tp_wait=tp_wait)
@@ -606,7 +607,7 @@ def gemm_t(x: torch.Tensor, w: torch.Tensor, *, x_t: bool = False, w_t: bool = F
         _check_bf16_2d(residual, "residual")
     can_pair = F % 256 == 0 and (not x_t or M % 64 == 0)
     if pair is None and bn == 0 and splits is None and M > 256 and F > 0 and Kx > 0:
-        wide = plan_persist(M, F, Kx, 0, False, x_t, can_pair)
+        wide = _persist_cost(M, F, Kx, 0, False, x_t, can_pair) if PAIR_AUTO else 0
         if wide and _persist_ok(x, w, out, residual, x_t=x_t, w_t=w_t):
             return _gemm_persist(x, w, out, residual, bn=wide, x_t=x_t, w_t=w_t)
     if pair is None and bn == 0 and splits is None and M > 256:
