@@ -55,6 +55,9 @@ constexpr int PERSIST_STG = 4096;                     // an epilogue warp's stag
 constexpr int PERSIST_THREADS = 320;
 constexpr int PERSIST_SMEM = PERSIST_STAGE_SPACE + 8 * PERSIST_STG + 1024 /*alignment*/ + 512 /*barriers*/;
 constexpr int PERSIST_MAX_STAGES = 4;
+// Where a product waits for weights that are being gathered, its CTAs may hold all SMs before those of shard_gather_push_kernel have theirs: one of 256 threads
+// of 32 registers fits beside (320 threads of up to 159), and its 8 bytes of shared memory do; every CTA costs 1 KB more.
+static_assert(PERSIST_SMEM + 1024 + 128 + 1024 <= 228 * 1024, "the gather's CTAs fit beside");
 constexpr int PERSIST_A = 32768;                      // a CTA's 128 tokens x 128 of the reduction
 
 // ---- the cta_group::2 forms ------------------------------------------------------------------
